@@ -33,6 +33,31 @@ def test_gradient_matches_oracle(ctx):
     assert np.max(np.abs(g - og)) <= 1e-3 * scale, (np.max(np.abs(g - og)), scale)
 
 
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 127, 129, 4096, 148 * 4 * 128 + 1, 200003])
+def test_gradient_sizes(ctx, n):
+    """Sizes around a warp's 32 samples, a CTA's 128 and the grid's first round, against
+    64-bit torch.  Every sum runs over at most ~100 terms per level (32 + 8 multiply-adds
+    per sample, 32 samples per tile, few tiles, then double), so the relative error of the
+    gradient's norm stays below 100 x 2^-24 = 6e-6."""
+    import torch
+    x, y = _data(n, 11)
+    p = learn.init_params(5)
+    p[256:288] = 0.05
+    p[1312:1344] = -0.03
+    ctx.mlp_set_params(p)
+    xt, yt = torch.from_numpy(x).cuda(), torch.from_numpy(y).cuda()
+    loss, g = ctx.mlp_loss_grad(xt, yt)
+    q = torch.from_numpy(p).cuda().double().requires_grad_(True)
+    w1, b1, w2, b2, w3, b3 = torch.split(q, [256, 32, 1024, 32, 32, 1])
+    h = torch.relu(xt.double() @ w1.view(32, 8).T + b1)
+    h = torch.relu(h @ w2.view(32, 32).T + b2)
+    ref = torch.nn.functional.binary_cross_entropy_with_logits(h @ w3 + b3, yt.double())
+    ref.backward()
+    rg = q.grad.cpu().numpy()
+    assert abs(loss - ref.item()) <= 6e-6 * abs(ref.item())
+    assert np.linalg.norm(g - rg) <= 6e-6 * np.linalg.norm(rg)
+
+
 def test_inference_tensor_cores_vs_fp32(ctx):
     import torch
     x, _ = _data(10007, 2)
