@@ -33,124 +33,232 @@ struct SubInfo {
     int64_t slab_off;
 };
 
-// One BFS-growth + FM bisection trial per warp.  Trial state lives in shared
-// memory when the largest subgraph of the depth fits (else in a global slab).
+// One BFS-growth + FM bisection trial per group of G threads: a warp, or a CTA of
+// TC_THREADS on large or dense subgraphs.  Trial state lives in shared memory
+// when the largest subgraph of the depth fits (SMEM), else in a global slab.
 //
 // FM without a heap: the reference's priority queues
 // (hunyuangraph_CPU_2wayrefine.h:117-225, hunyuangraph_priorityqueue.h) only
-// ever hold the vertices v with bnd[v] && moved[v] == -1, keyed by ed[v]-id[v]
-// (every insert/update/delete keeps that invariant), so popping side `from`
-// is an argmax of (ed-id desc, v asc) over {bnd, not moved, where == from}.
-// The warp computes that argmax in n/32 steps and updates the moved vertex's
-// neighbours in parallel, which is exact and needs no heap maintenance on
-// dense coarse graphs.
+// ever hold the boundary vertices that have not moved in the pass, keyed by
+// ed[v]-id[v] (every insert/update/delete keeps that invariant), so popping side
+// `from` is an argmax of (ed-id desc, v asc) over them, which is exact and
+// needs no heap maintenance on dense coarse graphs.  A vertex is on the boundary
+// exactly when ed > 0, or when it has no neighbours, in every state the
+// reference's insert and delete rules reach.  So the state keeps per vertex
+//   ed     the external weight, gain = ed - id,
+//   pop    gain while the vertex may be popped, INT_MIN otherwise,
+//   side, moved,
+// and the pop reads one 16-byte load of pop[] and one 4-byte load of side[] per
+// four vertices, all independent, where reading a boundary flag, then the moved
+// mark, the side and the two weights chained four shared-memory latencies per
+// vertex.  A trial is one dependent chain of moves on an otherwise idle SM, so
+// its latency per move is its cost; the argmax across lanes is two redux.sync.
+// The whole initial partition, before and after: 128^3 grid, k = 64 (510 vertices)
+// 3.8 -> 1.7 ms; R-MAT scale 20, k = 256 (900 vertices of 286 entries) 8.8 -> 3.7 ms;
+// RGG 2^24, k = 1024 (1,934 vertices) 8.6 -> 3.7 ms.
 struct TrialState {
-    int8_t *where, *bnd, *vis;
-    int32_t *id, *ed, *moved, *swaps;   // swaps doubles as the BFS queue
+    int8_t *side, *mark;              // mark: visited (growth), then moved (FM)
+    int32_t *pop, *gain, *ed, *list;  // list: the growth's queue, then the pass's moves
 };
+
+__host__ __device__ inline int32_t pad4(int32_t n) { return (n + 3) & ~3; }
 
 __host__ __device__ inline int64_t state_bytes(int32_t n)
 {
-    return (((int64_t)3 * n + 15) & ~(int64_t)15) + (int64_t)16 * n + 16;
+    return (((int64_t)2 * pad4(n) + 15) & ~(int64_t)15) + (int64_t)16 * pad4(n);
 }
 
 __device__ __forceinline__ TrialState carve(char *p, int32_t n)
 {
+    const int32_t np = pad4(n);
     TrialState t;
-    t.where = (int8_t *)p;
-    t.bnd = t.where + n;
-    t.vis = t.bnd + n;
-    int32_t *ip = (int32_t *)(p + (((int64_t)3 * n + 15) & ~(int64_t)15));
-    t.id = ip;
-    t.ed = ip + n;
-    t.moved = ip + 2 * n;
-    t.swaps = ip + 3 * n;
+    t.side = (int8_t *)p;
+    t.mark = t.side + np;
+    int32_t *ip = (int32_t *)(p + (((int64_t)2 * np + 15) & ~(int64_t)15));   // (16-byte aligned)
+    t.pop = ip;
+    t.gain = ip + np;
+    t.ed = ip + 2 * np;
+    t.list = ip + 3 * np;
     return t;
 }
 
-__global__ void __launch_bounds__(128)
-trial_warp_kernel(const SubInfo *__restrict__ subs, const int32_t *__restrict__ trial_sub,
-                  int32_t ntrials, const int32_t *__restrict__ fxadj, const int32_t *__restrict__ fadj,
-                  const int32_t *__restrict__ fwgt, const int32_t *__restrict__ fvwgt, char *slab_base,
-                  int32_t starts, int32_t fm_passes, int64_t *tr_cut, int64_t *tr_viol,
-                  int use_smem, int64_t smem_per_warp)
-{
-    hp::pdl_wait();
-    extern __shared__ __align__(16) char tsm[];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int32_t t = blockIdx.x * (blockDim.x >> 5) + wib;
-    if (t >= ntrials) return;
-    const SubInfo S = subs[trial_sub[t]];
-    const int32_t lt = t - S.tbeg;
-    const int32_t n = S.n;
-    const int32_t *xadj = fxadj + S.vbeg;   // global edge offsets, local neighbour ids
-    const int32_t *vwgt = fvwgt + S.vbeg;
-    char *base = use_smem ? tsm + (int64_t)wib * smem_per_warp
-                          : slab_base + S.slab_off + (int64_t)lt * state_bytes(n);
-    TrialState T = carve(base, n);
-    const int32_t start = (n <= starts) ? lt : (int32_t)(((int64_t)lt * n) / starts);
-    const int64_t tv = S.tv, want1 = S.want1, onemin = S.onemin, onemax = S.onemax;
-    int64_t pw0 = 0, pw1 = tv;
+constexpr int TC_THREADS = 256;   // a CTA per trial
+constexpr int64_t TC_DEG = 64;    // ... also where the rows are at least this long on average
+constexpr int TW_WARPS = 4;       // a warp per trial: trials per CTA at most
 
-    // ---- BFS growth of side 0 (hunyuangraph_CPU_initialpartition.h:66-120)
-    for (int32_t v = lane; v < n; v += 32) { T.where[v] = 1; T.vis[v] = 0; }
+template <int G>
+__device__ __forceinline__ void trial_sync()
+{
+    if (G == 32) __syncwarp();
+    else __syncthreads();
+}
+
+constexpr int GROW_DEPTH = 4;
+
+// BFS growth of side 0 by one warp (hunyuangraph_CPU_initialpartition.h:66-120);
+// returns the weight of side 0.  Once every vertex is visited a row adds nothing
+// to the queue and is not read.
+__device__ __forceinline__ int64_t trial_grow(const TrialState &T, int32_t n, const int32_t *__restrict__ xadj,
+                                              const int32_t *__restrict__ fadj, const int32_t *__restrict__ vwgt,
+                                              int32_t start, int64_t tv, int64_t onemin, int64_t onemax)
+{
+    const int lane = threadIdx.x & 31;
+    int64_t pw0 = 0, pw1 = tv;
+    for (int32_t v = lane; v < n; v += 32) { T.side[v] = 1; T.mark[v] = 0; }
     __syncwarp();
     int32_t first = 0, last = 1, nleft = n - 1, next_unvis = 0;
     bool drain = false;
-    if (lane == 0) { T.swaps[0] = start; T.vis[start] = 1; }
+    if (lane == 0) { T.list[0] = start; T.mark[start] = 1; }
     __syncwarp();
     for (;;) {
         if (first == last) {
             if (nleft == 0 || drain) break;
             // lowest unvisited vertex
             for (;;) {
-                int32_t v = next_unvis + lane;
-                bool un = v < n && !T.vis[v];
-                unsigned m = __ballot_sync(HP_FULL_MASK, un);
+                const int32_t v = next_unvis + lane;
+                const bool un = v < n && !T.mark[v];
+                const unsigned m = __ballot_sync(HP_FULL_MASK, un);
                 if (m) { next_unvis += __ffs(m) - 1; break; }
                 next_unvis += 32;
             }
-            if (lane == 0) { T.swaps[0] = next_unvis; T.vis[next_unvis] = 1; }
+            if (lane == 0) { T.list[0] = next_unvis; T.mark[next_unvis] = 1; }
             __syncwarp();
             first = 0; last = 1; nleft--;
         }
-        const int32_t i = T.swaps[first++];
+        const int32_t i = T.list[first++];
         const int32_t wi = vwgt[i];
         if (pw0 > 0 && pw1 - wi < onemin) { drain = true; continue; }
-        if (lane == 0) T.where[i] = 0;
+        if (lane == 0) T.side[i] = 0;
         pw0 += wi; pw1 -= wi;
         if (pw1 <= onemax) break;
         drain = false;
-        for (int32_t base_j = xadj[i]; base_j < xadj[i + 1]; base_j += 32) {
-            int32_t j = base_j + lane;
-            int32_t k = -1;
-            bool un = false;
-            if (j < xadj[i + 1]) { k = fadj[j]; un = !T.vis[k]; }
-            unsigned m = __ballot_sync(HP_FULL_MASK, un);
-            if (un) { T.swaps[last + __popc(m & hp::lanemask_lt())] = k; T.vis[k] = 1; }
-            last += __popc(m);
-            nleft -= __popc(m);
-            __syncwarp();
+        // GROW_DEPTH chunks of 32 entries in flight, taken in row order
+        const int32_t e = xadj[i + 1];
+        for (int32_t j0 = xadj[i]; j0 < e && nleft > 0; j0 += 32 * GROW_DEPTH) {
+            int32_t k[GROW_DEPTH];
+#pragma unroll
+            for (int q = 0; q < GROW_DEPTH; q++) {
+                const int32_t j = j0 + 32 * q + lane;
+                k[q] = j < e ? fadj[j] : -1;
+            }
+#pragma unroll
+            for (int q = 0; q < GROW_DEPTH; q++) {
+                if (j0 + 32 * q >= e) break;
+                const bool un = k[q] >= 0 && !T.mark[k[q]];
+                const unsigned m = __ballot_sync(HP_FULL_MASK, un);
+                if (un) { T.list[last + __popc(m & hp::lanemask_lt())] = k[q]; T.mark[k[q]] = 1; }
+                last += __popc(m);
+                nleft -= __popc(m);
+                __syncwarp();
+            }
         }
     }
     __syncwarp();
+    return pw0;
+}
+
+// The trial's FM neighbour update after h moved to `to` (all G threads).
+template <int G>
+__device__ __forceinline__ void trial_relax(const TrialState &T, int t, int32_t b, int32_t e, int to,
+                                            const int32_t *__restrict__ fadj, const int32_t *__restrict__ fwgt)
+{
+#pragma unroll 2
+    for (int32_t j = b + t; j < e; j += G) {
+        const int32_t k = fadj[j], w = fwgt[j];
+        const int32_t kw = (to == T.side[k]) ? w : -w;
+        const int32_t ned = T.ed[k] - kw, ng = T.gain[k] - kw - kw;
+        T.ed[k] = ned;
+        T.gain[k] = ng;
+        T.pop[k] = (!T.mark[k] && ned > 0) ? ng : INT_MIN;
+    }
+}
+
+template <int G, bool SMEM>
+__global__ void __launch_bounds__(G == 32 ? 32 * TW_WARPS : G)
+trial_kernel(const SubInfo *__restrict__ subs, const int32_t *__restrict__ trial_sub, int32_t ntrials,
+             const int32_t *__restrict__ fxadj, const int32_t *__restrict__ fadj, const int32_t *__restrict__ fwgt,
+             const int32_t *__restrict__ fvwgt, char *slab_base, int32_t starts, int32_t fm_passes, int64_t *tr_cut,
+             int64_t *tr_viol, int64_t smem_per_trial)
+{
+    hp::pdl_wait();
+    extern __shared__ __align__(16) char tsm[];
+    constexpr int W = G / 32;
+    __shared__ int2 s_pop[2][W];        // (key, vertex) of each warp's best, double buffered (G > 32)
+    __shared__ long long s_cut[W];
+    __shared__ long long s_pw0;
+    const int lane = threadIdx.x & 31, t = threadIdx.x % G, grp = threadIdx.x / G, wid = t >> 5;
+    const int32_t tr = blockIdx.x * (blockDim.x / G) + grp;
+    if (tr >= ntrials) return;   // the whole group
+    const SubInfo S = subs[trial_sub[tr]];
+    const int32_t lt = tr - S.tbeg;
+    const int32_t n = S.n, np = pad4(n);
+    const int32_t *xadj = fxadj + S.vbeg;   // global edge offsets, local neighbour ids
+    const int32_t *vwgt = fvwgt + S.vbeg;
+    char *gbase = slab_base + S.slab_off + (int64_t)lt * state_bytes(n);
+    const TrialState T = carve(SMEM ? tsm + (int64_t)grp * smem_per_trial : gbase, n);
+    const int32_t start = (n <= starts) ? lt : (int32_t)(((int64_t)lt * n) / starts);
+    const int64_t tv = S.tv, want1 = S.want1, onemin = S.onemin, onemax = S.onemax;
+
+    int64_t pw0 = 0;
+    if (wid == 0) {
+        pw0 = trial_grow(T, n, xadj, fadj, vwgt, start, tv, onemin, onemax);
+        if (G > 32 && lane == 0) s_pw0 = pw0;
+    }
+    trial_sync<G>();
+    if (G > 32) pw0 = s_pw0;
+    int64_t pw1 = tv - pw0;
 
     // ---- 2-way FM (hunyuangraph_CPU_2wayrefine.h:24-245)
     long long cut2 = 0;
-    for (int32_t v = lane; v < n; v += 32) {
-        int32_t tid = 0, ted = 0;
-        const int8_t wv = T.where[v];
-        for (int32_t j = xadj[v]; j < xadj[v + 1]; j++) {
-            if (T.where[fadj[j]] == wv) tid += fwgt[j];
-            else ted += fwgt[j];
+    const int32_t m = xadj[n] - xadj[0];
+    auto init_vertex = [&](int32_t v, int32_t id, int32_t ed, bool isolated) {
+        T.ed[v] = ed;
+        T.gain[v] = ed - id;
+        T.pop[v] = (ed > 0 || isolated) ? ed - id : INT_MIN;
+        T.mark[v] = 0;
+        cut2 += ed;
+    };
+    if (m >= 16 * n) {   // long rows: a warp per vertex, the row coalesced
+        for (int32_t v = wid; v < n; v += W) {
+            int32_t id = 0, ed = 0;
+            const int8_t sv = T.side[v];
+            const int32_t b = xadj[v], e = xadj[v + 1];
+#pragma unroll 4
+            for (int32_t j = b + lane; j < e; j += 32) {
+                const int32_t w = fwgt[j];
+                if (T.side[fadj[j]] == sv) id += w;
+                else ed += w;
+            }
+            id = hp::warp_sum(id);
+            ed = hp::warp_sum(ed);
+            if (lane == 0) init_vertex(v, id, ed, b == e);
         }
-        T.id[v] = tid; T.ed[v] = ted;
-        T.bnd[v] = (ted > 0 || xadj[v] == xadj[v + 1]);
-        cut2 += ted;
-        T.moved[v] = -1;
+    } else {
+        for (int32_t v = t; v < n; v += G) {
+            int32_t id = 0, ed = 0;
+            const int8_t sv = T.side[v];
+            const int32_t b = xadj[v], e = xadj[v + 1];
+#pragma unroll 4
+            for (int32_t j = b; j < e; j++) {
+                const int32_t w = fwgt[j];
+                if (T.side[fadj[j]] == sv) id += w;
+                else ed += w;
+            }
+            init_vertex(v, id, ed, b == e);
+        }
     }
-    int64_t cut = hp::warp_sum64(cut2) / 2;
-    __syncwarp();
+    for (int32_t v = n + t; v < np; v += G) { T.pop[v] = INT_MIN; T.side[v] = 0; }
+    cut2 = hp::warp_sum64(cut2);
+    if (G > 32) {
+        if (lane == 0) s_cut[wid] = cut2;
+        __syncthreads();
+        cut2 = 0;
+#pragma unroll
+        for (int w = 0; w < W; w++) cut2 += s_cut[w];
+    } else {
+        __syncwarp();
+    }
+    int64_t cut = cut2 / 2;
     const int64_t tpw0 = tv - want1, tpw1 = want1;
     int64_t limit = n / 100;
     if (limit < 15) limit = 15;
@@ -158,19 +266,6 @@ trial_warp_kernel(const SubInfo *__restrict__ subs, const int32_t *__restrict__ 
     int64_t avgvwgt = (pw0 + pw1) / 20;
     if (n > 0 && 2 * (pw0 + pw1) / n < avgvwgt) avgvwgt = 2 * (pw0 + pw1) / n;
     const int64_t origdiff = hp::iabs64(tpw0 - pw0);
-
-    // neighbour update after h moved to `to`
-    auto relax = [&](int32_t h, int to) {
-        for (int32_t j = xadj[h] + lane; j < xadj[h + 1]; j += 32) {
-            const int32_t k = fadj[j];
-            const int32_t kw = (to == T.where[k]) ? fwgt[j] : -fwgt[j];
-            const int32_t nid = T.id[k] + kw, ned = T.ed[k] - kw;
-            T.id[k] = nid; T.ed[k] = ned;
-            if (T.bnd[k]) { if (ned == 0) T.bnd[k] = 0; }
-            else if (ned > 0) T.bnd[k] = 1;
-        }
-        __syncwarp();
-    };
 
     for (int32_t pass = 0; pass < fm_passes; pass++) {
         int64_t mincutorder = -1;
@@ -180,23 +275,33 @@ trial_warp_kernel(const SubInfo *__restrict__ subs, const int32_t *__restrict__ 
         for (nswaps = 0; nswaps < n; nswaps++) {
             const int from = (tpw0 - pw0 < tpw1 - pw1) ? 0 : 1;
             const int to = 1 - from;
-            // pop: argmax (ed-id desc, v asc) over {bnd, not moved, side from}
-            int32_t bh = -1, bk = 0;
-            for (int32_t v = lane; v < n; v += 32) {
-                if (T.bnd[v] && T.moved[v] == -1 && T.where[v] == from) {
-                    int32_t key = T.ed[v] - T.id[v];
-                    if (bh < 0 || key > bk) { bh = v; bk = key; }   // ascending v per lane
+            // pop: argmax (gain desc, v asc) over the poppable vertices of side `from`
+            int32_t bk = INT_MIN, bh = INT_MAX;
+#pragma unroll 2
+            for (int32_t v = 4 * t; v < np; v += 4 * G) {   // ascending v per thread
+                const int4 k4 = *reinterpret_cast<const int4 *>(T.pop + v);
+                const char4 s4 = *reinterpret_cast<const char4 *>(T.side + v);
+                if (s4.x == from && k4.x > bk) { bk = k4.x; bh = v; }
+                if (s4.y == from && k4.y > bk) { bk = k4.y; bh = v + 1; }
+                if (s4.z == from && k4.z > bk) { bk = k4.z; bh = v + 2; }
+                if (s4.w == from && k4.w > bk) { bk = k4.w; bh = v + 3; }
+            }
+            int32_t key = __reduce_max_sync(HP_FULL_MASK, bk);
+            int32_t h = __reduce_min_sync(HP_FULL_MASK, bk == key ? bh : INT_MAX);
+            if (G > 32) {
+                // two buffers: a warp a round ahead does not overwrite what is still read
+                int2 *sp = s_pop[nswaps & 1];
+                if (lane == 0) sp[wid] = make_int2(key, h);
+                __syncthreads();
+                key = INT_MIN; h = INT_MAX;
+#pragma unroll
+                for (int w = 0; w < W; w++) {
+                    const int2 o = sp[w];
+                    if (o.x > key || (o.x == key && o.y < h)) { key = o.x; h = o.y; }
                 }
             }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                int32_t oh = __shfl_xor_sync(HP_FULL_MASK, bh, o);
-                int32_t ok = __shfl_xor_sync(HP_FULL_MASK, bk, o);
-                if (oh >= 0 && (bh < 0 || ok > bk || (ok == bk && oh < bh))) { bh = oh; bk = ok; }
-            }
-            const int32_t h = bh;
-            if (h < 0) break;
-            const int32_t gain = bk, wh = vwgt[h];
+            if (key == INT_MIN) break;
+            const int32_t gain = key, wh = vwgt[h], b = xadj[h], e = xadj[h + 1];
             newcut -= gain;
             if (to == 0) { pw0 += wh; pw1 -= wh; } else { pw1 += wh; pw0 -= wh; }
             if ((newcut < mincut && hp::iabs64(tpw0 - pw0) <= origdiff + avgvwgt) ||
@@ -209,31 +314,49 @@ trial_warp_kernel(const SubInfo *__restrict__ subs, const int32_t *__restrict__ 
                 if (to == 0) { pw0 -= wh; pw1 += wh; } else { pw1 -= wh; pw0 += wh; }
                 break;
             }
-            if (lane == 0) {
-                T.where[h] = (int8_t)to;
-                T.moved[h] = nswaps;
-                T.swaps[nswaps] = h;
-                int32_t tt = T.id[h]; T.id[h] = T.ed[h]; T.ed[h] = tt;
-                if (T.ed[h] == 0 && xadj[h] < xadj[h + 1]) T.bnd[h] = 0;
+            // (h is not its own neighbour: its entries and its neighbours' are disjoint)
+            if (t == 0) {
+                T.side[h] = (int8_t)to;
+                T.mark[h] = 1;
+                T.list[nswaps] = h;
+                T.ed[h] -= gain;
+                T.gain[h] = -gain;
+                T.pop[h] = INT_MIN;
             }
-            __syncwarp();
-            relax(h, to);
+            trial_relax<G>(T, t, b, e, to, fadj, fwgt);
+            trial_sync<G>();
         }
-        for (int32_t i = lane; i < nswaps; i += 32) T.moved[T.swaps[i]] = -1;
-        __syncwarp();
-        for (nswaps--; nswaps > mincutorder; nswaps--) {
-            const int32_t h = T.swaps[nswaps];
-            const int to = 1 - T.where[h];
-            if (lane == 0) {
-                T.where[h] = (int8_t)to;
-                int32_t tt = T.id[h]; T.id[h] = T.ed[h]; T.ed[h] = tt;
-                if (T.ed[h] == 0 && T.bnd[h] && xadj[h] < xadj[h + 1]) T.bnd[h] = 0;
-                else if (T.ed[h] > 0 && !T.bnd[h]) T.bnd[h] = 1;
+        trial_sync<G>();
+        for (int32_t i = t; i < nswaps; i += G) {
+            const int32_t h = T.list[i];
+            T.mark[h] = 0;
+            T.pop[h] = (T.ed[h] > 0 || xadj[h] == xadj[h + 1]) ? T.gain[h] : INT_MIN;
+        }
+        trial_sync<G>();
+        // undo the moves after the best prefix, last first
+        nswaps--;
+        int32_t h = nswaps > mincutorder ? T.list[nswaps] : 0;
+        int to = nswaps > mincutorder ? 1 - T.side[h] : 0;
+        trial_sync<G>();   // every thread has read side[h]
+        while (nswaps > mincutorder) {
+            const int32_t b = xadj[h], e = xadj[h + 1];
+            if (t == 0) {
+                const int32_t g = -T.gain[h], ed = T.ed[h] + g;
+                T.side[h] = (int8_t)to;
+                T.ed[h] = ed;
+                T.gain[h] = g;
+                T.pop[h] = (ed > 0 || b == e) ? g : INT_MIN;
             }
             const int32_t wh = vwgt[h];
             if (to == 0) { pw0 += wh; pw1 -= wh; } else { pw1 += wh; pw0 -= wh; }
-            __syncwarp();
-            relax(h, to);
+            trial_relax<G>(T, t, b, e, to, fadj, fwgt);
+            // the next vertex: its side is not written before the barrier
+            nswaps--;
+            if (nswaps > mincutorder) {
+                h = T.list[nswaps];
+                to = 1 - T.side[h];
+            }
+            trial_sync<G>();
         }
         cut = mincut;
         if (mincutorder <= 0 || mincut == initcut) break;
@@ -242,226 +365,9 @@ trial_warp_kernel(const SubInfo *__restrict__ subs, const int32_t *__restrict__ 
     if (pw1 > onemax) viol += pw1 - onemax;
     if (pw1 < onemin) viol += onemin - pw1;
     // the trial's sides go to the global slab for the selection kernel
-    int8_t *wout = (int8_t *)(slab_base + S.slab_off + (int64_t)lt * state_bytes(n));
-    if (use_smem)
-        for (int32_t v = lane; v < n; v += 32) wout[v] = T.where[v];
-    if (lane == 0) { tr_cut[t] = cut; tr_viol[t] = viol; }
-}
-
-// The same trial with one CTA of TC_THREADS threads per trial, for the large
-// subgraphs of the first recursion depths: the FM pop is an argmax of n/256
-// candidates per thread reduced across the warps, the BFS appends a row chunk's
-// unvisited neighbours in row order through a block scan, and every decision
-// is taken by all threads alike from shared values, so the trial's moves, cut
-// and sides are those of trial_warp_kernel.
-constexpr int TC_THREADS = 256;
-constexpr int TC_WARPS = TC_THREADS / 32;
-
-__device__ __forceinline__ int32_t tc_block_min(int32_t v, int32_t *s_red)
-{
-    v = __reduce_min_sync(HP_FULL_MASK, v);
-    __syncthreads();   // earlier readers of s_red are done
-    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    int32_t r = INT_MAX;
-#pragma unroll
-    for (int w = 0; w < TC_WARPS; w++) r = min(r, s_red[w]);
-    return r;
-}
-
-__global__ void __launch_bounds__(TC_THREADS)
-trial_cta_kernel(const SubInfo *__restrict__ subs, const int32_t *__restrict__ trial_sub,
-                 int32_t ntrials, const int32_t *__restrict__ fxadj, const int32_t *__restrict__ fadj,
-                 const int32_t *__restrict__ fwgt, const int32_t *__restrict__ fvwgt, char *slab_base,
-                 int32_t starts, int32_t fm_passes, int64_t *tr_cut, int64_t *tr_viol, int use_smem)
-{
-    hp::pdl_wait();
-    extern __shared__ __align__(16) char tsm[];
-    __shared__ int32_t s_red[TC_WARPS], s_key[TC_WARPS];
-    __shared__ int32_t s_scan[TC_WARPS + 2];
-    __shared__ long long s_cut[TC_WARPS];
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int32_t t = blockIdx.x;
-    if (t >= ntrials) return;   // whole CTA
-    const SubInfo S = subs[trial_sub[t]];
-    const int32_t lt = t - S.tbeg;
-    const int32_t n = S.n;
-    const int32_t *xadj = fxadj + S.vbeg;
-    const int32_t *vwgt = fvwgt + S.vbeg;
-    char *base = use_smem ? tsm : slab_base + S.slab_off + (int64_t)lt * state_bytes(n);
-    TrialState T = carve(base, n);
-    const int32_t start = (n <= starts) ? lt : (int32_t)(((int64_t)lt * n) / starts);
-    const int64_t tv = S.tv, want1 = S.want1, onemin = S.onemin, onemax = S.onemax;
-    int64_t pw0 = 0, pw1 = tv;
-
-    // ---- BFS growth of side 0
-    for (int32_t v = tid; v < n; v += TC_THREADS) { T.where[v] = 1; T.vis[v] = 0; }
-    __syncthreads();
-    int32_t first = 0, last = 1, nleft = n - 1, next_unvis = 0;
-    bool drain = false;
-    if (tid == 0) { T.swaps[0] = start; T.vis[start] = 1; }
-    __syncthreads();
-    for (;;) {
-        if (first == last) {
-            if (nleft == 0 || drain) break;
-            for (;;) {   // lowest unvisited vertex
-                const int32_t v = next_unvis + tid;
-                const int32_t mv = tc_block_min(v < n && !T.vis[v] ? v : INT_MAX, s_red);
-                if (mv != INT_MAX) { next_unvis = mv; break; }
-                next_unvis += TC_THREADS;
-            }
-            __syncthreads();
-            if (tid == 0) { T.swaps[0] = next_unvis; T.vis[next_unvis] = 1; }
-            __syncthreads();
-            first = 0; last = 1; nleft--;
-        }
-        const int32_t i = T.swaps[first++];
-        const int32_t wi = vwgt[i];
-        if (pw0 > 0 && pw1 - wi < onemin) { drain = true; continue; }
-        __syncthreads();   // every thread has read swaps[first - 1]
-        if (tid == 0) T.where[i] = 0;
-        pw0 += wi; pw1 -= wi;
-        if (pw1 <= onemax) break;
-        drain = false;
-        for (int32_t base_j = xadj[i]; base_j < xadj[i + 1]; base_j += TC_THREADS) {
-            const int32_t j = base_j + tid;
-            int32_t k = -1;
-            bool un = false;
-            if (j < xadj[i + 1]) { k = fadj[j]; un = !T.vis[k]; }
-            int tot;
-            const int ex = hp::block_excl_scan<TC_THREADS>(un ? 1 : 0, &tot, s_scan);
-            if (un) { T.swaps[last + ex] = k; T.vis[k] = 1; }
-            last += tot;
-            nleft -= tot;
-            __syncthreads();
-        }
-    }
-    __syncthreads();
-
-    // ---- 2-way FM
-    long long cut2 = 0;
-    for (int32_t v = tid; v < n; v += TC_THREADS) {
-        int32_t tid_ = 0, ted = 0;
-        const int8_t wv = T.where[v];
-        for (int32_t j = xadj[v]; j < xadj[v + 1]; j++) {
-            if (T.where[fadj[j]] == wv) tid_ += fwgt[j];
-            else ted += fwgt[j];
-        }
-        T.id[v] = tid_; T.ed[v] = ted;
-        T.bnd[v] = (ted > 0 || xadj[v] == xadj[v + 1]);
-        cut2 += ted;
-        T.moved[v] = -1;
-    }
-    cut2 = hp::warp_sum64(cut2);
-    if (lane == 0) s_cut[wid] = cut2;
-    __syncthreads();
-    long long call = 0;
-#pragma unroll
-    for (int w = 0; w < TC_WARPS; w++) call += s_cut[w];
-    int64_t cut = call / 2;
-    const int64_t tpw0 = tv - want1, tpw1 = want1;
-    int64_t limit = n / 100;
-    if (limit < 15) limit = 15;
-    if (limit > 100) limit = 100;
-    int64_t avgvwgt = (pw0 + pw1) / 20;
-    if (n > 0 && 2 * (pw0 + pw1) / n < avgvwgt) avgvwgt = 2 * (pw0 + pw1) / n;
-    const int64_t origdiff = hp::iabs64(tpw0 - pw0);
-
-    auto relax = [&](int32_t h, int to) {
-        for (int32_t j = xadj[h] + tid; j < xadj[h + 1]; j += TC_THREADS) {
-            const int32_t k = fadj[j];
-            const int32_t kw = (to == T.where[k]) ? fwgt[j] : -fwgt[j];
-            const int32_t nid = T.id[k] + kw, ned = T.ed[k] - kw;
-            T.id[k] = nid; T.ed[k] = ned;
-            if (T.bnd[k]) { if (ned == 0) T.bnd[k] = 0; }
-            else if (ned > 0) T.bnd[k] = 1;
-        }
-        __syncthreads();
-    };
-
-    for (int32_t pass = 0; pass < fm_passes; pass++) {
-        int64_t mincutorder = -1;
-        int64_t newcut = cut, mincut = cut, initcut = cut;
-        int64_t mindiff = hp::iabs64(tpw0 - pw0);
-        int32_t nswaps;
-        for (nswaps = 0; nswaps < n; nswaps++) {
-            const int from = (tpw0 - pw0 < tpw1 - pw1) ? 0 : 1;
-            const int to = 1 - from;
-            int32_t bh = -1, bk = 0;
-            for (int32_t v = tid; v < n; v += TC_THREADS) {
-                if (T.bnd[v] && T.moved[v] == -1 && T.where[v] == from) {
-                    const int32_t key = T.ed[v] - T.id[v];
-                    if (bh < 0 || key > bk) { bh = v; bk = key; }   // ascending v per thread
-                }
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const int32_t oh = __shfl_xor_sync(HP_FULL_MASK, bh, o);
-                const int32_t ok = __shfl_xor_sync(HP_FULL_MASK, bk, o);
-                if (oh >= 0 && (bh < 0 || ok > bk || (ok == bk && oh < bh))) { bh = oh; bk = ok; }
-            }
-            __syncthreads();   // earlier readers of s_red / s_key are done
-            if (lane == 0) { s_red[wid] = bh; s_key[wid] = bk; }
-            __syncthreads();
-            bh = -1; bk = 0;
-#pragma unroll
-            for (int w = 0; w < TC_WARPS; w++) {
-                const int32_t oh = s_red[w], ok = s_key[w];
-                if (oh >= 0 && (bh < 0 || ok > bk || (ok == bk && oh < bh))) { bh = oh; bk = ok; }
-            }
-            const int32_t h = bh;
-            if (h < 0) break;
-            const int32_t gain = bk, wh = vwgt[h];
-            newcut -= gain;
-            if (to == 0) { pw0 += wh; pw1 -= wh; } else { pw1 += wh; pw0 -= wh; }
-            if ((newcut < mincut && hp::iabs64(tpw0 - pw0) <= origdiff + avgvwgt) ||
-                (newcut == mincut && hp::iabs64(tpw0 - pw0) < mindiff)) {
-                mincut = newcut;
-                mindiff = hp::iabs64(tpw0 - pw0);
-                mincutorder = nswaps;
-            } else if (nswaps - mincutorder > limit) {
-                newcut += gain;
-                if (to == 0) { pw0 -= wh; pw1 += wh; } else { pw1 -= wh; pw0 += wh; }
-                break;
-            }
-            if (tid == 0) {
-                T.where[h] = (int8_t)to;
-                T.moved[h] = nswaps;
-                T.swaps[nswaps] = h;
-                int32_t tt = T.id[h]; T.id[h] = T.ed[h]; T.ed[h] = tt;
-                if (T.ed[h] == 0 && xadj[h] < xadj[h + 1]) T.bnd[h] = 0;
-            }
-            __syncthreads();
-            relax(h, to);
-        }
-        __syncthreads();
-        for (int32_t i = tid; i < nswaps; i += TC_THREADS) T.moved[T.swaps[i]] = -1;
-        __syncthreads();
-        for (nswaps--; nswaps > mincutorder; nswaps--) {
-            const int32_t h = T.swaps[nswaps];
-            const int to = 1 - T.where[h];
-            __syncthreads();   // every thread has read where[h]
-            if (tid == 0) {
-                T.where[h] = (int8_t)to;
-                int32_t tt = T.id[h]; T.id[h] = T.ed[h]; T.ed[h] = tt;
-                if (T.ed[h] == 0 && T.bnd[h] && xadj[h] < xadj[h + 1]) T.bnd[h] = 0;
-                else if (T.ed[h] > 0 && !T.bnd[h]) T.bnd[h] = 1;
-            }
-            const int32_t wh = vwgt[h];
-            if (to == 0) { pw0 += wh; pw1 -= wh; } else { pw1 += wh; pw0 -= wh; }
-            __syncthreads();
-            relax(h, to);
-        }
-        cut = mincut;
-        if (mincutorder <= 0 || mincut == initcut) break;
-    }
-    int64_t viol = 0;
-    if (pw1 > onemax) viol += pw1 - onemax;
-    if (pw1 < onemin) viol += onemin - pw1;
-    int8_t *wout = (int8_t *)(slab_base + S.slab_off + (int64_t)lt * state_bytes(n));
-    if (use_smem)
-        for (int32_t v = tid; v < n; v += TC_THREADS) wout[v] = T.where[v];
-    if (tid == 0) { tr_cut[t] = cut; tr_viol[t] = viol; }
+    if (SMEM)
+        for (int32_t v = t; v < n; v += G) gbase[v] = T.side[v];
+    if (t == 0) { tr_cut[tr] = cut; tr_viol[tr] = viol; }
 }
 
 // Best trial of every subgraph: min (violation, cut, trial index); copies its
@@ -624,9 +530,9 @@ inline unsigned nblk(int64_t n, int b = 256) { return (unsigned)std::max<int64_t
 
 int hp_initpart_init()
 {
-    HP_CUDA(cudaFuncSetAttribute(trial_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    HP_CUDA(cudaFuncSetAttribute(trial_kernel<32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)HP_TRIAL_SMEM));
-    HP_CUDA(cudaFuncSetAttribute(trial_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    HP_CUDA(cudaFuncSetAttribute(trial_kernel<TC_THREADS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)HP_TRIAL_SMEM));
     return HP_OK;
 }
@@ -710,17 +616,27 @@ int hp_initial_partition(hp_context *c, HpLevel &g, int32_t nparts, const int64_
         int32_t maxn = 0;
         for (const HostSub &H : subs) maxn = std::max(maxn, H.n);
         const int64_t per = (state_bytes(maxn) + 15) & ~(int64_t)15;
-        const int wpb = (int)std::max<int64_t>(1, std::min<int64_t>(4, HP_TRIAL_SMEM / per));
-        const int use_smem = per <= HP_TRIAL_SMEM ? 1 : 0;
-        const int wpb_eff = use_smem ? wpb : 4;
+        const bool smem = per <= HP_TRIAL_SMEM;
+        const int wpb = smem ? (int)std::min<int64_t>(TW_WARPS, HP_TRIAL_SMEM / per) : TW_WARPS;
         const int tok = hp_prof_begin(c);
-        if (maxn >= c->tune.trial_cta_n)   // a CTA per trial (same trial, same result)
-            HP_LAUNCH(c, trial_cta_kernel, (unsigned)tcount, TC_THREADS, use_smem ? (size_t)per : 0, d_info, d_tsub,
-                      tcount, fxadj, fadj, fwgt, fvwgt, slab, starts, fm_passes, d_cut, d_viol, use_smem);
-        else
-            HP_LAUNCH(c, trial_warp_kernel, nblk(tcount, wpb_eff), 32 * wpb_eff,
-                      use_smem ? (size_t)(per * wpb_eff) : 0, d_info, d_tsub, tcount, fxadj, fadj, fwgt, fvwgt,
-                      slab, starts, fm_passes, d_cut, d_viol, use_smem, per);
+        // a CTA per trial (same trial, same result) on large subgraphs, and on dense
+        // ones, whose moves read long rows: rows of deg0 entries on average in the
+        // whole graph, shrinking with the subgraph as in a dense one (R-MAT, 900
+        // vertices of 286 entries, 512 as the vertex bound: 6.3 ms with warps at the
+        // depths below it, 3.7 ms with CTAs)
+        const int64_t deg0 = g.m / n, deg = deg0 * maxn / n;
+        const bool cta = maxn >= c->tune.trial_cta_n || deg >= TC_DEG;
+        const unsigned tgrid = cta ? (unsigned)tcount : nblk(tcount, wpb);
+        const unsigned tblock = cta ? TC_THREADS : 32 * wpb;
+        const size_t tsmem = !smem ? 0 : cta ? (size_t)per : (size_t)(per * wpb);
+#define HP_TRIAL_LAUNCH(K)                                                                              \
+    HP_LAUNCH(c, K, tgrid, tblock, tsmem, d_info, d_tsub, tcount, fxadj, fadj, fwgt, fvwgt, slab, starts, \
+              fm_passes, d_cut, d_viol, per)
+        if (cta && smem) HP_TRIAL_LAUNCH((trial_kernel<TC_THREADS, true>));
+        else if (cta) HP_TRIAL_LAUNCH((trial_kernel<TC_THREADS, false>));
+        else if (smem) HP_TRIAL_LAUNCH((trial_kernel<32, true>));
+        else HP_TRIAL_LAUNCH((trial_kernel<32, false>));
+#undef HP_TRIAL_LAUNCH
         hp_prof_end(c, tok, HP_PROF_INIT, 0);
         HP_LAUNCH(c, select_kernel, (unsigned)ns, 256, 0, d_info, d_cut, d_viol, slab, fvwgt, side, d_res);
         std::vector<int64_t> res(2 * ns);

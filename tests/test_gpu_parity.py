@@ -456,3 +456,32 @@ def test_hybrid_contraction(ctx, hybrid):
         compare_runs(ctx, g, 64)
     finally:
         ctx.set_tuning(None)
+
+
+def dense_graph(n, p, seed, isolated=0):
+    """Random graph of edge probability p on n vertices, the last `isolated` of them without edges."""
+    rng = np.random.default_rng(seed)
+    a = np.triu(rng.random((n, n)) < p, 1)
+    a[:, n - isolated:] = False
+    a |= a.T
+    w = rng.integers(1, 50, (n, n))
+    w = np.triu(w, 1) + np.triu(w, 1).T
+    rows = [np.nonzero(a[v])[0] for v in range(n)]
+    xadj = np.concatenate([[0], np.cumsum([r.size for r in rows])]).astype(np.int32)
+    adj = np.concatenate(rows).astype(np.int32)
+    wgt = np.concatenate([w[v][r] for v, r in enumerate(rows)]).astype(np.int32)
+    return graphs.Graph(xadj, adj, rng.integers(1, 4, n).astype(np.int32), wgt)
+
+
+# the bisection trials of the coarsest graph: no coarsening (coarsen_to = n), sizes around
+# the four vertices a lane reads at once, sparse and dense rows (a warp or a CTA per trial),
+# vertices without neighbours, state in shared memory (up to 11,000 vertices) and in the slab
+@pytest.mark.parametrize("n,p,isolated,k", [(2, 1.0, 0, 2), (5, 0.6, 2, 3), (31, 0.3, 0, 4), (126, 0.9, 3, 2),
+                                            (129, 0.9, 0, 7), (257, 0.05, 9, 5), (513, 0.3, 1, 4)])
+def test_bisection_trials(ctx, n, p, isolated, k):
+    compare_runs(ctx, dense_graph(n, p, n, isolated), k, 1.1, coarsen_to=n)
+
+
+def test_bisection_trials_large_state(ctx):
+    g = graphs.grid2d(120, 100, seed=3, wmin=1, wmax=9)
+    compare_runs(ctx, g, 2, 1.1, coarsen_to=g.nvtxs, init_starts=4, fm_passes=2)
