@@ -718,7 +718,7 @@ HP_API int hp_context_create(int device, hp_context **out)
     }
     ok = ok && cudaMallocHost((void **)&c->h_pin, sizeof(long long) * HP_NSCAL) == cudaSuccess;
     for (int i = 0; ok && i < 8; i++) ok = cudaEventCreate(&c->ev[i]) == cudaSuccess;
-    ok = ok && hp_refine_init() == HP_OK;
+    ok = ok && hp_refine_init(c) == HP_OK;
     ok = ok && hp_initpart_init() == HP_OK;
     ok = ok && hp_coarsen_init() == HP_OK;
     if (!ok) {

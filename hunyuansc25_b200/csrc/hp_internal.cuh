@@ -25,6 +25,7 @@ struct HpLevel {
 struct hp_context {
     int device = 0;
     int sm_count = 148;
+    int max_cluster = 1;             // CTAs of the largest cluster refine_cluster_kernel can run in
     cudaStream_t stream = nullptr;   // stream of the current call
     cudaStream_t own_stream = nullptr;
 
@@ -104,7 +105,7 @@ constexpr int HP_TUNE_WARP_ROW_MAX = 256;        // contract_warp_radix_kernel's
 constexpr int HP_TUNE_CTA_ROW_MAX = 4096;        // contract_cta_radix_kernel<256, 4096>
 constexpr int HP_TUNE_WARP_DENSE_K_MAX = 1024;   // gain_bigwarp_kernel's shared accumulators
 constexpr int HP_TUNE_DEG_MAX = 1 << 24;
-constexpr int HP_TUNE_SMALL_LEVEL_MAX = 32768;   // refine_small_kernel's staged prefix weights
+constexpr int HP_TUNE_SMALL_LEVEL_MAX = 32768;   // vertices per CTA of refine_cluster_kernel's levels
 constexpr int HP_TUNE_SMALL_MATCH_MAX = 8192;    // match_small_kernel's shared-memory state
 constexpr int HP_TUNE_SMEM_CN_MAX = 49152;       // shared-memory dense accumulator of the contraction
 constexpr int64_t HP_LEARNED_SKEW = 16;          // learned proposals: max degree / mean degree of the input
@@ -145,30 +146,42 @@ template <class T> inline T *ralloc_t(hp_context *c, int64_t n) { return (T *)hp
 // exactly that of a plain launch.
 template <class... P, class... A>
 inline cudaError_t hp_launch_kernel(const hp_context *c, void (*kernel)(P...), unsigned grid, unsigned block,
-                                    size_t smem, A &&...args)
+                                    size_t smem, unsigned cluster, A &&...args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = c->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    unsigned na = 0;
+    if (c->tune.pdl) {
+        attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[na++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[na].id = cudaLaunchAttributeClusterDimension;
+        attr[na].val.clusterDim.x = cluster;
+        attr[na].val.clusterDim.y = 1;
+        attr[na++].val.clusterDim.z = 1;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = c->tune.pdl ? 1 : 0;
+    cfg.numAttrs = na;
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
 // Count and check every kernel launch.  Once the arena has run out nothing more is
 // launched (a pointer allocated after that is null): the call unwinds with
 // HP_ERR_NOMEM and partition_common retries with a larger arena.
-#define HP_LAUNCH(ctx, kernel, grid, block, smem, ...)                                      \
+#define HP_LAUNCH(ctx, kernel, grid, block, smem, ...) \
+    HP_LAUNCH_CLUSTER(ctx, kernel, 1, grid, block, smem, __VA_ARGS__)
+// The same with thread-block clusters of `cluster` CTAs.
+#define HP_LAUNCH_CLUSTER(ctx, kernel, cluster, grid, block, smem, ...)                     \
     do {                                                                                    \
         if ((ctx)->oom) return HP_ERR_NOMEM;                                                \
         if ((grid) > 0) {                                                                   \
             cudaError_t e__ = hp_launch_kernel((ctx), kernel, (unsigned)(grid), (unsigned)(block), \
-                                               (size_t)(smem), __VA_ARGS__);                \
+                                               (size_t)(smem), (unsigned)(cluster), __VA_ARGS__); \
             (ctx)->launches++;                                                              \
             if (e__ == cudaSuccess) e__ = cudaGetLastError();                               \
             if (e__ != cudaSuccess) {                                                       \
@@ -240,7 +253,7 @@ int hp_uncoarsen(hp_context *c, int32_t nparts, const int64_t *h_opt, const int6
 // nworkers of them, with the context's tuning.
 int hp_ensure_workers(hp_context *ctx, int nworkers);
 
-int hp_refine_init();
+int hp_refine_init(hp_context *c);
 int hp_initpart_init();
 int hp_coarsen_init();
 int hp_mlp_ensure(hp_context *c);

@@ -2482,24 +2482,37 @@ int pass_apply(hp_context *c, HpLevel &g, RefineBufs &B, const PassCfg &P, cudaG
     return HP_OK;
 }
 
-// ---- small levels: every pass of the level in one CTA --------------------------------
-// A level with few vertices runs its whole pass loop inside one CTA of
-// SL_THREADS threads.  The phases are those of the multi-kernel pass, in the
-// same order and through the same device functions -- LP selection and
-// afterburner, weak or strong rebalance (candidates, stable radix sort, ranks,
-// selection or eviction and cookie cutter), simultaneous moves, gain-row
-// maintenance, the exact cut change, the control step and the best partition --
-// separated by __syncthreads instead of kernel boundaries.  Gain rows,
-// candidates and moves equal the multi-kernel pass's, so the level's result is
-// identical; what goes away is about fifteen launches per pass, which on small
-// levels cost more than the work.
-constexpr int SL_THREADS = 1024;
-constexpr int SL_WARPS = SL_THREADS / 32;
-constexpr int SL_SORT_INTS = hp::block_sort_ints(SL_THREADS);
+// ---- small levels: every pass of the level in one cluster of CTAs --------------------
+// A level of at most cluster_level_n() vertices runs its whole pass loop inside one
+// thread-block cluster of up to CL_MAX CTAs of CL_THREADS threads.  The phases are
+// those of the multi-kernel pass, in the same order and by the same rules -- LP
+// selection and afterburner, weak or strong rebalance (candidates, stable radix
+// sort, ranks, selection or eviction and cookie cutter), simultaneous moves,
+// gain-row maintenance, the exact cut change, the control step and the best
+// partition -- separated by the hardware's cluster barrier instead of kernel
+// boundaries.  Every warp of the cluster owns one contiguous range of vertices
+// (then of sorted candidates), so ordered results need one exchange of the CTAs'
+// totals through distributed shared memory, and rows walked by a whole warp are
+// spread over all of them.  The control block and the part weights are kept by
+// every CTA alike.  Gain rows, candidates and moves equal the multi-kernel pass's,
+// so the level's result is identical; what goes away is about fifteen dependent
+// launches per pass, which on these levels cost more than the work.
+// Per level and pass, one CTA or the launched kernels before, a cluster now: 128^3 grid
+// (k = 64) 2,817 vertices 100 -> 47 us, 8,854 93 -> 58, 25,181 85 -> 62; 256^2 grid
+// (k = 8) 10,870 vertices 62 -> 28 us, 65,536 63 -> 36.  Fewer than about 512 vertices
+// per CTA buy nothing: the passes are chains of L2 latencies and barriers; above
+// CL_LEVEL_MAX the grid-wide kernels' 148 SMs win.
+constexpr int CL_THREADS = 1024;
+constexpr int CL_WARPS = CL_THREADS / 32;
+constexpr int CL_MAX = 16;                 // CTAs of a cluster (above 8: non-portable size)
+constexpr int CL_SORT_INTS = CL_WARPS * 256;
+constexpr size_t CL_COOKIE_BYTES = 100 * 1024;   // staged prefix weights of the cookie cutter
+constexpr int CL_KMAX = HP_TUNE_WARP_DENSE_K_MAX;
 
 struct SmallLevel {
     int32_t n, k, finest, bigd, small_max, key_bits, learned_mlp;
     int32_t patience, judge;    // the control block's init (the level's setup runs in the kernel)
+    int32_t cookie_cap;         // prefix weights that fit the dynamic shared memory
     const RefineCtl *coarser;   // the coarser level's control block (its best cut), or nullptr
     float mlp_threshold;
     const int32_t *xadj, *adjncy, *adjwgt, *vwgt;
@@ -2508,7 +2521,8 @@ struct SmallLevel {
     int32_t *gpart, *gconn;
     int32_t *dest, *pregain, *moves, *oldp, *dirty, *small_l, *big_l, *best_where;
     int32_t *K, *V, *K2, *V2, *pre, *P, *sp;
-    int32_t *pstart, *pend, *und, *ev_end, *es, *ee;
+    int32_t *pbase, *es, *ee;
+    int32_t *counts;        // 2 sets of 4: moves, dirty short rows, dirty long rows
     int8_t *lock;
     int8_t *prune, *accp;   // the judge of a learned pass
     unsigned long long *pw, *best_pw;
@@ -2518,55 +2532,200 @@ struct SmallLevel {
     unsigned *status;
 };
 
-// Dynamic shared memory of the small-level kernel: the largest of the phases'
-// needs (sort tables; the staged prefix weights of the cookie cutter, at most
-// n + 1; the warps' dense gain-row accumulators).
+// Dynamic shared memory: the largest of the phases' needs (sort tables; the staged
+// prefix weights of the cookie cutter, at most n + 1; the warps' dense gain-row
+// accumulators; the part weights of the setup).
 size_t small_level_smem(int32_t n, int32_t k)
 {
-    const size_t sort = sizeof(int32_t) * SL_SORT_INTS;
-    const size_t cookie = sizeof(int32_t) * ((size_t)n + 1);
-    const size_t rows = sizeof(int32_t) * SL_WARPS * ((size_t)k + (k + 31) / 32);
+    const size_t sort = sizeof(int32_t) * CL_SORT_INTS;
+    const size_t cookie = std::min(sizeof(int32_t) * ((size_t)n + 1), CL_COOKIE_BYTES);
+    const size_t rows = sizeof(int32_t) * CL_WARPS * ((size_t)k + (k + 31) / 32);
     return std::max(sort, std::max(cookie, rows));
 }
 
-// Block-wide sum / max of a long long; every thread gets the result.
-__device__ __forceinline__ long long sl_sum64(long long v, long long *s_red)
+// CTAs of a level's cluster, a power of two: CL_PER_CTA vertices and CL_ENT_PER_CTA
+// adjacency entries each.
+constexpr int32_t CL_PER_CTA = 512;
+constexpr int64_t CL_ENT_PER_CTA = 8192;
+int cluster_ctas(const hp_context *c, int32_t n, int64_t m)
 {
-    v = hp::warp_sum64(v);
-    __syncthreads();   // the previous reduction has been read
-    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    long long t = 0;
-#pragma unroll 8
-    for (int w = 0; w < SL_WARPS; w++) t += s_red[w];
-    return t;
+    int q = 1;
+    while (q < c->max_cluster && ((int64_t)q * CL_PER_CTA < n || q * CL_ENT_PER_CTA < m)) q *= 2;
+    return q;
 }
 
-__device__ __forceinline__ long long sl_max64(long long v, long long *s_red)
+// The largest level a cluster takes: small_level_n vertices per CTA, at most
+// CL_LEVEL_MAX (above it the grid-wide kernels' memory parallelism wins), and at
+// most CL_DEG entries per vertex of that bound.
+constexpr int32_t CL_LEVEL_MAX = 65536;
+constexpr int64_t CL_DEG = 16;
+int32_t cluster_level_n(const hp_context *c)
 {
-    v = hp::warp_max64(v);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    long long t = LLONG_MIN;
-#pragma unroll 8
-    for (int w = 0; w < SL_WARPS; w++) t = s_red[w] > t ? s_red[w] : t;
-    return t;
+    return (int32_t)std::min<int64_t>((int64_t)c->tune.small_level_n * c->max_cluster, CL_LEVEL_MAX);
 }
 
-__global__ void __launch_bounds__(SL_THREADS, 1)
-refine_small_kernel(SmallLevel a)
+__device__ __forceinline__ unsigned cl_rank()
+{
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+
+__device__ __forceinline__ unsigned cl_size()
+{
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return r;
+}
+
+// All threads of the cluster; writes before it (global and shared, this CTA's and
+// remote) are visible after it.
+__device__ __forceinline__ void cl_sync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n"
+                 "barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// The address of CTA `rank`'s copy of a shared-memory object.
+__device__ __forceinline__ unsigned cl_map(const void *p, unsigned rank)
+{
+    unsigned a = (unsigned)__cvta_generic_to_shared(p), r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+
+__device__ __forceinline__ void cl_st64(unsigned addr, long long v)
+{
+    asm volatile("st.shared::cluster.s64 [%0], %1;" ::"r"(addr), "l"(v) : "memory");
+}
+
+__device__ __forceinline__ int32_t cl_ld32(unsigned addr)
+{
+    int32_t v;
+    asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
+
+// Exchange of the CTAs' sums through a cluster barrier.  Two buffers in turn: a CTA
+// writes a buffer again only two barriers later, when every CTA has read it.
+struct ClXch {
+    long long x[2][CL_MAX][3];
+    long long w[CL_WARPS][3];
+    int buf;   // (thread 0 toggles it; read after a barrier)
+};
+
+// Sums of N (at most 3) values over all threads of the cluster; every thread gets
+// them.  Everything written before the call is visible after it.
+template <int N>
+__device__ __forceinline__ void cl_sum(long long (&v)[N], ClXch &X, int buf, unsigned rank, unsigned nct)
+{
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        const long long s = hp::warp_sum64(v[i]);
+        if (lane == 0) X.w[wid][i] = s;
+    }
+    __syncthreads();
+    if (wid == 0) {
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            const long long s = hp::warp_sum64(X.w[lane][i]);
+            if (lane < (int)nct) cl_st64(cl_map(&X.x[buf][rank][i], lane), s);
+        }
+    }
+    cl_sync();
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        long long s = 0;
+        for (unsigned r = 0; r < nct; r++) s += X.x[buf][r][i];
+        v[i] = s;
+    }
+}
+
+// Exclusive prefix over the cluster's warps (rank, then warp order) of two values
+// per warp (the same in all its lanes), and their totals.
+__device__ __forceinline__ void cl_warp_scan2(int32_t a, int32_t b, int32_t *ea, int32_t *eb, int32_t *ta,
+                                              int32_t *tb, ClXch &X, int buf, unsigned rank, unsigned nct)
+{
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (lane == 0) { X.w[wid][0] = a; X.w[wid][1] = b; }
+    __syncthreads();
+    if (wid == 0) {
+        const int va = (int)X.w[lane][0], vb = (int)X.w[lane][1];
+        const int ia = hp::warp_incl_scan(va), ib = hp::warp_incl_scan(vb);
+        X.w[lane][0] = ia - va;
+        X.w[lane][1] = ib - vb;
+        const int sa = __shfl_sync(HP_FULL_MASK, ia, 31), sb = __shfl_sync(HP_FULL_MASK, ib, 31);
+        if (lane < (int)nct) {
+            cl_st64(cl_map(&X.x[buf][rank][0], lane), sa);
+            cl_st64(cl_map(&X.x[buf][rank][1], lane), sb);
+        }
+    }
+    cl_sync();
+    int32_t pa = (int32_t)X.w[wid][0], pb = (int32_t)X.w[wid][1], xa = 0, xb = 0;
+    for (unsigned r = 0; r < nct; r++) {
+        const int32_t qa = (int32_t)X.x[buf][r][0], qb = (int32_t)X.x[buf][r][1];
+        if (r < rank) { pa += qa; pb += qb; }
+        xa += qa;
+        xb += qb;
+    }
+    *ea = pa;
+    *eb = pb;
+    *ta = xa;
+    *tb = xb;
+}
+
+// The gain rows of the listed vertices (short rows by lane segments, long rows by a
+// warp's dense accumulator in shared memory).
+__device__ __forceinline__ void cl_rebuild(const SmallLevel &a, int gw, int tw, int32_t ns, int32_t nb, int32_t *dyn)
+{
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (ns > 0) {
+        if (a.small_max <= 8)
+            gain_seg_rows<8>(gw, tw, a.small_l, ns, a.xadj, a.adjncy, a.adjwgt, a.where, a.goff, a.gpart, a.gconn,
+                             a.k, a.dirty);
+        else if (a.small_max <= 16)
+            gain_seg_rows<16>(gw, tw, a.small_l, ns, a.xadj, a.adjncy, a.adjwgt, a.where, a.goff, a.gpart, a.gconn,
+                              a.k, a.dirty);
+        else
+            gain_seg_rows<32>(gw, tw, a.small_l, ns, a.xadj, a.adjncy, a.adjwgt, a.where, a.goff, a.gpart, a.gconn,
+                              a.k, a.dirty);
+    }
+    if (nb > 0) {
+        const int nw = (a.k + 31) >> 5;
+        int32_t *dw = dyn + (size_t)wid * (a.k + nw);
+        unsigned *bm = (unsigned *)(dw + a.k);
+        for (int i = lane; i < a.k; i += 32) dw[i] = 0;
+        for (int i = lane; i < nw; i += 32) bm[i] = 0u;
+        __syncwarp();
+        gain_bigwarp_rows(gw, tw, dw, bm, a.big_l, nb, a.xadj, a.adjncy, a.adjwgt, a.where, a.goff, a.gpart, a.gconn,
+                          a.k, a.dirty, a.bigd, INT_MAX);
+    }
+}
+
+__global__ void __launch_bounds__(CL_THREADS, 1)
+refine_cluster_kernel(SmallLevel a)
 {
     hp::pdl_wait();
-    extern __shared__ __align__(16) int32_t sl_dyn[];
+    extern __shared__ __align__(16) int32_t cl_dyn[];
     __shared__ hp::MlpSmem s_mlp;
-    __shared__ int32_t s_scan[SL_THREADS / 32 + 2];
-    __shared__ long long s_red[SL_WARPS];
-    __shared__ int32_t s_lists[2];   // dirty rows queued this pass: short, long
-    __shared__ int32_t s_nu;         // undersized parts of a weak pass
+    __shared__ ClXch X;
+    __shared__ RefineCtl s_ctl;
+    __shared__ long long s_pw[CL_KMAX];      // part weights (of the current partition)
+    __shared__ int32_t s_part[CL_KMAX];      // weak: the undersized parts; strong: the parts' evicted ranges
+    __shared__ int8_t s_ufl[CL_KMAX];        // weak: pw < maxp
+    __shared__ int32_t s_hist[256], s_base[256];
+    __shared__ int32_t s_scan[CL_WARPS + 2];
+    __shared__ int32_t s_nu;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const unsigned lt = hp::lanemask_lt();
+    const unsigned rank = cl_rank(), nct = cl_size();
+    const int tw = (int)nct * CL_WARPS, gw = (int)rank * CL_WARPS + wid;
+    const int gt = (int)nct * CL_THREADS, gtid = (int)rank * CL_THREADS + tid;
     const int32_t n = a.n, k = a.k;
-    RefineCtl *s = a.ctl;
+    const int32_t vpw = (n + tw - 1) / tw;   // the warp's vertices [vb, ve)
+    const int32_t vb = min(n, gw * vpw), ve = min(n, vb + vpw);
+    int buf = 0;                             // exchange buffer (uniform over the cluster)
     if (a.learned_mlp) hp::mlp_load_smem(s_mlp, a.mlp_params);
     // ---- the level's setup, as the launches of the multi-kernel levels:
     // gain-row capacities min(deg, k) and offsets, cleared locks and dirty
@@ -2574,100 +2733,93 @@ refine_small_kernel(SmallLevel a)
     // the starting cut (the coarser level's best cut, else summed from the
     // rows), the excess, the best-partition copy and the control block
     {
-        int32_t run = 0, ns = 0, nb = 0;
-        for (int32_t b0 = 0; b0 < n; b0 += SL_THREADS) {
-            const int32_t v = b0 + tid;
-            int32_t cap = 0, d = 0;
-            if (v < n) {
-                d = a.xadj[v + 1] - a.xadj[v];
-                cap = d < k ? d : k;
-                a.lock[v] = 0;
-                a.dirty[v] = 0;
-                a.best_where[v] = a.where[v];
-            }
-            int tot;
-            const int ex = hp::block_excl_scan<SL_THREADS>(cap, &tot, s_scan);
-            if (v < n) a.goff[v] = run + ex;
-            run += tot;
-            const bool sh = v < n && d <= a.bigd, lg = v < n && d > a.bigd;
-            int ts, tl;
-            const int es = hp::block_excl_scan<SL_THREADS>(sh ? 1 : 0, &ts, s_scan);
-            const int el = hp::block_excl_scan<SL_THREADS>(lg ? 1 : 0, &tl, s_scan);
-            if (sh) a.small_l[ns + es] = v;
-            if (lg) a.big_l[nb + el] = v;
-            ns += ts;
-            nb += tl;
-        }
-        if (tid == 0) a.goff[n] = run;
-        unsigned long long *spw = (unsigned long long *)sl_dyn;   // k <= 1024 part weights
-        for (int32_t q = tid; q < k; q += SL_THREADS) spw[q] = 0ull;
-        __syncthreads();
-        for (int32_t v = tid; v < n; v += SL_THREADS) atomicAdd(&spw[a.where[v]], (unsigned long long)a.vwgt[v]);
-        __syncthreads();
-        for (int32_t q = tid; q < k; q += SL_THREADS) { a.pw[q] = spw[q]; a.best_pw[q] = spw[q]; }
-        __syncthreads();   // the accumulators below reuse the shared memory
-        if (ns > 0) {
-            if (a.small_max <= 8)
-                gain_seg_rows<8>(wid, SL_WARPS, a.small_l, ns, a.xadj, a.adjncy, a.adjwgt, a.where, a.goff, a.gpart,
-                                 a.gconn, k, a.dirty);
-            else if (a.small_max <= 16)
-                gain_seg_rows<16>(wid, SL_WARPS, a.small_l, ns, a.xadj, a.adjncy, a.adjwgt, a.where, a.goff, a.gpart,
-                                  a.gconn, k, a.dirty);
-            else
-                gain_seg_rows<32>(wid, SL_WARPS, a.small_l, ns, a.xadj, a.adjncy, a.adjwgt, a.where, a.goff, a.gpart,
-                                  a.gconn, k, a.dirty);
-        }
-        if (nb > 0) {
-            const int nw = (k + 31) >> 5;
-            int32_t *dw = sl_dyn + (size_t)wid * (k + nw);
-            unsigned *bm = (unsigned *)(dw + k);
-            for (int i = lane; i < k; i += 32) dw[i] = 0;
-            for (int i = lane; i < nw; i += 32) bm[i] = 0u;
-            __syncwarp();
-            gain_bigwarp_rows(wid, SL_WARPS, dw, bm, a.big_l, nb, a.xadj, a.adjncy, a.adjwgt, a.where, a.goff,
-                              a.gpart, a.gconn, k, a.dirty, a.bigd, INT_MAX);
+        int32_t *spw = cl_dyn;   // this CTA's share of the part weights (each total below 2^31)
+        for (int32_t q = tid; q < k; q += CL_THREADS) spw[q] = 0;
+        if (rank == 0) {
+            for (int32_t q = tid; q < k; q += CL_THREADS) a.pw[q] = 0ull;
+            if (tid < 8) a.counts[tid] = 0;
         }
         __syncthreads();
-        long long cut = 0;
+        int32_t caps = 0;
+        for (int32_t v = vb + lane; v < ve; v += 32) {
+            const int32_t d = a.xadj[v + 1] - a.xadj[v], p = a.where[v];
+            caps += d < k ? d : k;
+            a.lock[v] = 0;
+            a.dirty[v] = 0;
+            a.best_where[v] = p;
+            atomicAdd(&spw[p], a.vwgt[v]);
+        }
+        caps = hp::warp_sum(caps);
+        int32_t run, e1, total, t1;
+        cl_warp_scan2(caps, 0, &run, &e1, &total, &t1, X, buf, rank, nct);
+        buf ^= 1;
+        for (int32_t v0 = vb; v0 < ve; v0 += 32) {
+            const int32_t v = v0 + lane;
+            const bool in = v < ve;
+            const int32_t d = in ? a.xadj[v + 1] - a.xadj[v] : 0;
+            const int32_t cap = d < k ? d : k, incl = hp::warp_incl_scan(cap);
+            if (in) a.goff[v] = run + incl - cap;
+            run += __shfl_sync(HP_FULL_MASK, incl, 31);
+            const bool sh = in && d <= a.bigd, lg = in && d > a.bigd;
+            const int32_t ps = hp::warp_append(&a.counts[1], sh), pl = hp::warp_append(&a.counts[2], lg);
+            if (sh) a.small_l[ps] = v;
+            if (lg) a.big_l[pl] = v;
+        }
+        if (gtid == 0) a.goff[n] = total;
+        for (int32_t q = tid; q < k; q += CL_THREADS)
+            if (spw[q]) atomicAdd(&a.pw[q], (unsigned long long)spw[q]);
+        cl_sync();
+        const int32_t ns = __ldcg(&a.counts[1]), nb = __ldcg(&a.counts[2]);
+        cl_rebuild(a, gw, tw, ns, nb, cl_dyn);
+        cl_sync();
+        if (rank == 0 && tid < 4) a.counts[tid] = 0;   // (the first pass's; barriers follow before its use)
+        long long cut[1] = {0};
         if (!a.coarser) {   // the coarsest level: the cut from the gain rows
-            long long acc = 0;
-            for (int32_t v = tid; v < n; v += SL_THREADS) {
+            for (int32_t v = vb + lane; v < ve; v += 32) {
                 const int32_t p = a.where[v], o = a.goff[v], len = a.goff[v + 1] - o;
                 for (int32_t j = o; j < o + len; j++) {
                     const int32_t q = a.gpart[j];
                     if (q < 0) break;
-                    if (q != p) acc += a.gconn[j];
+                    if (q != p) cut[0] += a.gconn[j];
                 }
             }
-            cut = sl_sum64(acc, s_red) / 2;
         }
+        cl_sum<1>(cut, X, buf, rank, nct);
+        buf ^= 1;
         long long m = LLONG_MIN;
-        for (int32_t q = tid; q < k; q += SL_THREADS) {
-            const long long e = (long long)a.pw[q] - a.maxp[q];
+        for (int32_t q = tid; q < k; q += CL_THREADS) {
+            const long long w = (long long)__ldcg(&a.pw[q]), e = w - a.maxp[q];
+            s_pw[q] = w;
+            s_ufl[q] = e < 0;
+            if (rank == 0) a.best_pw[q] = (unsigned long long)w;
             m = e > m ? e : m;
         }
-        m = sl_max64(m, s_red);
-        if (tid == 0)
-            ctl_init_state(s, a.coarser ? a.coarser->best_cut : cut, m, a.patience, a.learned_mlp, a.goff[n],
+        m = hp::warp_max64(m);
+        if (lane == 0) X.w[wid][0] = m;
+        __syncthreads();
+        if (tid == 0) {
+            for (int w = 1; w < CL_WARPS; w++) m = X.w[w][0] > m ? X.w[w][0] : m;
+            ctl_init_state(&s_ctl, a.coarser ? a.coarser->best_cut : cut[0] / 2, m, a.patience, a.learned_mlp, total,
                            a.judge);
+        }
     }
     __syncthreads();
     // the control step ends the loop; the pass cap bounds it as well
     for (int32_t guard = 0; guard <= HP_MAX_REFINE_PASSES; guard++) {
-        if (!*(volatile const int32_t *)&s->cont) break;   // written by thread 0 before a barrier
-        const int mode = *(volatile const int32_t *)&s->mode;
-        if (tid < 2) s_lists[tid] = 0;
+        if (!s_ctl.cont) break;
+        const int mode = s_ctl.mode;
+        int32_t *cn = a.counts + 4 * (guard & 1);   // this pass's counters (zero; the other set is cleared below)
         long long ncand = 0, jp2 = 0, jl2 = 0;
         bool judged = false;
-        int32_t nmoves = 0;
+        long long c1 = 0;   // conn(to) - conn(from) over the moves, before any applies
         if (mode == 0) {
             // ---- LP selection (plain or learned), as lp_select[_learned]_kernel
-            const bool lrn = a.learned_mlp && *(volatile const int32_t *)&s->learned_pass;
-            const bool jdg = lrn && *(volatile const int32_t *)&s->judge_pass;
-            int32_t my_cand = 0, my_candp = 0;
-            for (int32_t b0 = 0; b0 < n; b0 += SL_THREADS) {
-                const int32_t v = b0 + tid;
-                const bool in = v < n;
+            const bool lrn = a.learned_mlp && s_ctl.learned_pass;
+            const bool jdg = lrn && s_ctl.judge_pass;
+            long long my[2] = {0, 0};
+            for (int32_t v0 = vb; v0 < ve; v0 += 32) {
+                const int32_t v = v0 + lane;
+                const bool in = v < ve;
                 int32_t p = 0, o = 0, len = 0;
                 if (in) {
                     p = a.where[v];
@@ -2686,12 +2838,12 @@ refine_small_kernel(SmallLevel a)
                         cand = 1;
                         if (lrn)
                             hp::mlp_features(rb.pc, rb.bc, rb.wd, rb.np, a.xadj[v + 1] - a.xadj[v],
-                                             a.maxp[d] - (int64_t)a.pw[d], a.opt[d], a.maxp[p] - (int64_t)a.pw[p],
+                                             a.maxp[d] - (int64_t)s_pw[d], a.opt[d], a.maxp[p] - (int64_t)s_pw[p],
                                              a.opt[p], a.finest, f);
                     }
                 }
                 int8_t pr = 0;   // dropped by the MLP: keeps the plain gain and destination for the judge
-                my_candp += cand;
+                my[1] += cand;
                 if (lrn && __any_sync(HP_FULL_MASK, cand)) {   // a warp without candidates needs no scores
                     const float logit = hp::mlp_warp_logit(s_mlp, f);
                     if (cand && logit < a.mlp_threshold) {
@@ -2705,18 +2857,18 @@ refine_small_kernel(SmallLevel a)
                     a.dest[v] = d;
                     if (jdg) a.prune[v] = pr;
                 }
-                my_cand += cand;
+                my[0] += cand;
             }
-            ncand = sl_sum64(my_cand, s_red);   // (barrier: every selection is visible)
-            const long long ncandp = jdg ? sl_sum64(my_candp, s_red) : ncand;
+            cl_sum<2>(my, X, buf, rank, nct);   // (barrier: every selection is visible)
+            buf ^= 1;
+            ncand = my[0];
             judged = jdg;
-            if (ncand > 0 || (jdg && ncandp > 0)) {
+            if (ncand > 0 || (jdg && my[1] > 0)) {
                 // ---- afterburner: every candidate re-scored against the
-                // higher-priority neighbours; locks and moves (in vertex order)
-                int32_t run = 0;
-                for (int32_t b0 = 0; b0 < n; b0 += SL_THREADS) {
-                    const int32_t v = b0 + tid;
-                    const bool in = v < n;
+                // higher-priority neighbours; locks and moves
+                for (int32_t v0 = vb; v0 < ve; v0 += 32) {
+                    const int32_t v = v0 + lane;
+                    const bool in = v < ve;
                     const int32_t g = in ? a.pregain[v] : NEG;
                     const bool act = g != NEG;
                     const int32_t ro = act ? a.xadj[v] : 0, rl = act ? a.xadj[v + 1] - ro : 0;
@@ -2724,9 +2876,8 @@ refine_small_kernel(SmallLevel a)
                     long long chp = 0, chl = 0;
                     const bool coop = rl > 32;
                     if (act && !coop)
-                        for (int32_t j = ro; j < ro + rl; j++)
-                            ab_change2(v, g, pp, bb, a.adjncy[j], a.adjwgt[j], a.pregain, a.dest, a.where, a.prune,
-                                       jdg, chp, chl);
+                        ab_row_sum2(v, g, pp, bb, ro, ro + rl, 1, a.adjncy, a.adjwgt, a.pregain, a.dest, a.where,
+                                    a.prune, jdg, chp, chl);
                     unsigned cm = __ballot_sync(HP_FULL_MASK, coop);
                     while (cm) {
                         const int src = __ffs(cm) - 1;
@@ -2741,26 +2892,27 @@ refine_small_kernel(SmallLevel a)
                         if (jdg) cl = hp::warp_sum64(cl);
                         if (lane == src) { chp = cp; chl = cl; }
                     }
-                    const int selp = act && ((long long)g + chp >= 0);
-                    const int sel = jdg ? (act && !a.prune[v] && (long long)g + chl >= 0) : selp;
+                    const bool selp = act && ((long long)g + chp >= 0);
+                    const bool sel = jdg ? (act && !a.prune[v] && (long long)g + chl >= 0) : selp;
                     if (in) {
                         a.lock[v] = (int8_t)sel;
                         if (jdg) a.accp[v] = (int8_t)selp;
                     }
-                    int tot;
-                    const int ex = hp::block_excl_scan<SL_THREADS>(sel, &tot, s_scan);
-                    if (sel) a.moves[run + ex] = v;
-                    run += tot;
+                    const int32_t pos = hp::warp_append(&cn[0], sel);
+                    if (sel) {
+                        a.moves[pos] = v;
+                        a.oldp[pos] = pp;
+                        c1 += g;   // the gain is conn(dest) - conn(own)
+                    }
                 }
-                nmoves = run;
                 if (jdg) {
                     // ---- the judge: exact cut decrease of the plain and the
                     // learned move sets on this state, as judge_delta_kernel
-                    __syncthreads();   // every lock / accp is visible
-                    long long sp = 0, sl = 0;
-                    for (int32_t b0 = 0; b0 < n; b0 += SL_THREADS) {
-                        const int32_t v = b0 + tid;
-                        const bool in = v < n;
+                    cl_sync();   // every lock / accp is visible
+                    long long sj[2] = {0, 0};
+                    for (int32_t v0 = vb; v0 < ve; v0 += 32) {
+                        const int32_t v = v0 + lane;
+                        const bool in = v < ve;
                         const bool mp = in && a.accp[v] != 0, ml = in && a.lock[v] != 0;
                         const bool act = mp || ml;
                         const int32_t ro = act ? a.xadj[v] : 0, rl = act ? a.xadj[v + 1] - ro : 0;
@@ -2769,7 +2921,7 @@ refine_small_kernel(SmallLevel a)
                         if (act && !coop)
                             for (int32_t j = ro; j < ro + rl; j++)
                                 judge_entry(pv, dv, mp, ml, a.adjncy[j], a.adjwgt[j], a.where, a.dest, a.accp, a.lock,
-                                            sp, sl);
+                                            sj[0], sj[1]);
                         unsigned cm = __ballot_sync(HP_FULL_MASK, coop);
                         while (cm) {
                             const int src = __ffs(cm) - 1;
@@ -2780,38 +2932,48 @@ refine_small_kernel(SmallLevel a)
                             const bool sml = __shfl_sync(HP_FULL_MASK, (int)ml, src) != 0;
                             for (int32_t j = so + lane; j < so + sn; j += 32)
                                 judge_entry(spv, sdv, smp, sml, a.adjncy[j], a.adjwgt[j], a.where, a.dest, a.accp,
-                                            a.lock, sp, sl);
+                                            a.lock, sj[0], sj[1]);
                         }
                     }
-                    jp2 = sl_sum64(sp, s_red);
-                    jl2 = sl_sum64(sl, s_red);
+                    cl_sum<2>(sj, X, buf, rank, nct);
+                    buf ^= 1;
+                    jp2 = sj[0];
+                    jl2 = sj[1];
                 }
             }
         } else {
             // ---- rebalance, as rb_candidates / sort / rb_rank / rw_select or
-            // evict_end / rs_evict / cookie_cutter / rs_assign
+            // rs_evict / cookie_cutter / rs_assign
             const bool strong = mode == 2;
-            if (!strong) undersized_block(k, a.pw, a.maxp, a.und, &s_nu, s_scan);
-            for (int32_t p = tid; p < k; p += SL_THREADS) {
-                a.pstart[p] = -1;
-                a.pend[p] = -1;
+            if (!strong) {   // undersized parts (pw < max(0.99 maxp, maxp - 100)) in part order; k <= CL_THREADS
+                int f = 0;
+                if (tid < k) {
+                    const int64_t mp = a.maxp[tid];
+                    int64_t md = (mp * 99) / 100;
+                    if (md < mp - 100) md = mp - 100;
+                    f = s_pw[tid] < md;
+                }
+                int tot;
+                const int pos = hp::block_excl_scan<CL_THREADS>(f, &tot, s_scan);
+                if (f) s_part[pos] = tid;
+                if (tid == 0) s_nu = tot;
+                __syncthreads();
             }
-            __syncthreads();
-            const int32_t nu = s_nu;
-            int32_t cnt = 0;
-            for (int32_t b0 = 0; b0 < n; b0 += SL_THREADS) {
-                const int32_t v = b0 + tid;
-                const bool in = v < n;
-                int32_t p = 0;
+            // candidates, by each warp in vertex order at the front of its own range
+            int32_t cw = 0;
+            for (int32_t v0 = vb; v0 < ve; v0 += 32) {
+                const int32_t v = v0 + lane;
+                const bool in = v < ve;
+                int32_t p = 0, vw = 0;
                 bool cand = false;
                 if (in) {
                     p = a.where[v];
-                    const int64_t pwp = (int64_t)a.pw[p];
-                    cand = strong ? (pwp > a.maxp[p] && (int64_t)a.vwgt[v] < 2 * (pwp - a.opt[p]))
-                                  : (pwp > a.maxp[p] && 2 * (int64_t)a.vwgt[v] < 3 * (pwp - a.opt[p]));
+                    vw = a.vwgt[v];
+                    const int64_t pwp = s_pw[p], over = pwp - a.opt[p];
+                    cand = pwp > a.maxp[p] && (strong ? (int64_t)vw < 2 * over : 2 * (int64_t)vw < 3 * over);
                 }
                 const int32_t o = cand ? a.goff[v] : 0, len = cand ? a.goff[v + 1] - o : 0;
-                int32_t d = p, kk = -1;
+                int32_t d = p, kk = -1, gain = 0;
                 if (!strong) {
                     int64_t pc = 0, bc = 0;
                     int32_t b = -1;
@@ -2822,7 +2984,7 @@ refine_small_kernel(SmallLevel a)
                             if (q < 0) break;
                             const int32_t cq = a.gconn[j];
                             if (q == p) pc = cq;
-                            if ((int64_t)a.pw[q] < a.maxp[q] && cq > bc) { bc = cq; b = q; }
+                            if (s_ufl[q] && cq > bc) { bc = cq; b = q; }
                         }
                     unsigned cm = __ballot_sync(HP_FULL_MASK, coop);
                     while (cm) {
@@ -2836,7 +2998,7 @@ refine_small_kernel(SmallLevel a)
                             if (q < 0) break;
                             const int32_t cq = a.gconn[so + j];
                             if (q == sp_) lpc = cq;
-                            if ((int64_t)a.pw[q] < a.maxp[q] && cq > lbc) { lbc = cq; lb = q; }
+                            if (s_ufl[q] && cq > lbc) { lbc = cq; lb = q; }
                         }
                         lpc = hp::warp_sum(lpc);
 #pragma unroll
@@ -2848,191 +3010,239 @@ refine_small_kernel(SmallLevel a)
                         if (lane == src) { pc = lpc; bc = lbc; b = lb; }
                     }
                     if (cand) {
-                        int64_t g = 0;
                         bool ok = true;
-                        if (b >= 0) g = bc - pc;
-                        else if (nu == 0) ok = false;
-                        else { b = a.und[v % nu]; g = -pc; }
-                        if (ok) { d = b; kk = p * 64 + hp::gain_bucket((int32_t)g, a.vwgt[v]); }
+                        if (b >= 0) gain = (int32_t)(bc - pc);
+                        else if (s_nu == 0) ok = false;
+                        else { b = s_part[v % s_nu]; gain = (int32_t)-pc; }   // (no connectivity to an undersized part)
+                        if (ok) { d = b; kk = p * 64 + hp::gain_bucket(gain, vw); }
                     }
                 } else if (cand) {
-                    const int32_t pc = row_conn(a.gpart + o, a.gconn + o, len, p, k);
-                    kk = p * 64 + hp::gain_bucket(-pc, a.vwgt[v]);
+                    gain = -row_conn(a.gpart + o, a.gconn + o, len, p, k);
+                    kk = p * 64 + hp::gain_bucket(gain, vw);
                 }
-                if (in) a.dest[v] = d;
-                int tot;
-                const int ex = hp::block_excl_scan<SL_THREADS>(kk >= 0 ? 1 : 0, &tot, s_scan);
+                const unsigned m = __ballot_sync(HP_FULL_MASK, kk >= 0);
                 if (kk >= 0) {
-                    a.K[cnt + ex] = kk;
-                    a.V[cnt + ex] = v;
+                    const int32_t pos = vb + cw + __popc(m & lt);
+                    a.K[pos] = kk;
+                    a.V[pos] = v;
+                    a.dest[v] = d;
+                    a.pregain[v] = gain;   // weak: conn(dest) - conn(own)
                 }
-                cnt += tot;
+                cw += __popc(m);
             }
-            const bool flip = hp::block_sort_pairs<SL_THREADS>(a.K, a.V, a.K2, a.V2, cnt, a.key_bits, sl_dyn, s_scan);
-            const int32_t *Ks = flip ? a.K2 : a.K, *Vs = flip ? a.V2 : a.V;
-            // prefix weights in sorted order and the part bounds
-            int32_t run = 0;
-            for (int32_t b0 = 0; b0 < cnt; b0 += SL_THREADS) {
-                const int32_t i = b0 + tid;
-                const bool valid = i < cnt;
-                const int32_t w = valid ? a.vwgt[Vs[i]] : 0;
-                int tot;
-                const int ex = hp::block_excl_scan<SL_THREADS>(w, &tot, s_scan);
+            __syncwarp();
+            // stable radix sort by key, 8-bit digits: per-warp digit counts, their
+            // prefix over the CTA's warps, the CTAs' totals read through the cluster
+            int32_t *ks = a.K, *vs = a.V, *kd = a.K2, *vd = a.V2;
+            int32_t ib = vb, ie = vb + cw, cnt = 0;   // the warp's items
+            int32_t *wc = cl_dyn + wid * 256;
+            for (int shift = 0; shift < a.key_bits; shift += 8) {
+                for (int q = lane; q < 256; q += 32) wc[q] = 0;
+                __syncwarp();
+                for (int32_t i = ib + lane; i < ie; i += 32) atomicAdd(&wc[((unsigned)ks[i] >> shift) & 255u], 1);
+                __syncthreads();
+                if (tid < 256) {
+                    int32_t s = 0;
+#pragma unroll 8
+                    for (int w = 0; w < CL_WARPS; w++) {
+                        const int32_t t = cl_dyn[w * 256 + tid];
+                        cl_dyn[w * 256 + tid] = s;
+                        s += t;
+                    }
+                    s_hist[tid] = s;
+                }
+                cl_sync();
+                int32_t before = 0, all = 0;
+                if (tid < 256)
+                    for (unsigned r = 0; r < nct; r++) {
+                        const int32_t t = cl_ld32(cl_map(&s_hist[tid], r));
+                        if (r < rank) before += t;
+                        all += t;
+                    }
+                const int ex = hp::block_excl_scan<CL_THREADS>(all, &cnt, s_scan);
+                if (tid < 256) s_base[tid] = ex + before;
+                __syncthreads();
+                for (int32_t i0 = ib; i0 < ie; i0 += 32) {
+                    const int32_t i = i0 + lane;
+                    const bool valid = i < ie;
+                    const int32_t key = valid ? ks[i] : 0, val = valid ? vs[i] : 0;
+                    const unsigned dg = valid ? (((unsigned)key >> shift) & 255u) : 256u + lane;
+                    const unsigned peers = __match_any_sync(HP_FULL_MASK, dg);
+                    const int rk = __popc(peers & lt);
+                    if (valid) {
+                        const int32_t pos = s_base[dg] + wc[dg] + rk;
+                        kd[pos] = key;
+                        vd[pos] = val;
+                    }
+                    __syncwarp();
+                    if (valid && rk == 0) wc[dg] += __popc(peers);
+                    __syncwarp();
+                }
+                cl_sync();
+                int32_t *t = ks; ks = kd; kd = t;
+                t = vs; vs = vd; vd = t;
+                const int32_t ipw = (cnt + tw - 1) / tw;
+                ib = min(cnt, gw * ipw);
+                ie = min(cnt, ib + ipw);
+            }
+            // prefix weights in sorted order; pbase[p]: the prefix at part p's first candidate
+            int32_t wsum = 0;
+            for (int32_t i = ib + lane; i < ie; i += 32) wsum += a.vwgt[vs[i]];
+            wsum = hp::warp_sum(wsum);
+            int32_t run, e1, t0, t1;
+            cl_warp_scan2(wsum, 0, &run, &e1, &t0, &t1, X, buf, rank, nct);
+            buf ^= 1;
+            for (int32_t i0 = ib; i0 < ie; i0 += 32) {
+                const int32_t i = i0 + lane;
+                const bool valid = i < ie;
+                const int32_t w = valid ? a.vwgt[vs[i]] : 0, incl = hp::warp_incl_scan(w);
                 if (valid) {
-                    a.pre[i] = run + ex;
-                    const int32_t p = Ks[i] >> 6;
-                    if (i == 0 || (Ks[i - 1] >> 6) != p) a.pstart[p] = i;
-                    if (i == cnt - 1 || (Ks[i + 1] >> 6) != p) a.pend[p] = i + 1;
+                    const int32_t p = ks[i] >> 6, pr = run + incl - w;
+                    a.pre[i] = pr;
+                    if (i == 0 || (ks[i - 1] >> 6) != p) a.pbase[p] = pr;
                 }
-                run += tot;
+                run += __shfl_sync(HP_FULL_MASK, incl, 31);
             }
-            if (tid == 0) a.pre[cnt] = run;
-            __syncthreads();
-            if (!strong) {
-                int32_t mv = 0;
-                for (int32_t b0 = 0; b0 < cnt; b0 += SL_THREADS) {
-                    const int32_t i = b0 + tid;
-                    int sel = 0;
-                    if (i < cnt) {
-                        const int32_t p = Ks[i] >> 6;
-                        const int64_t before = (int64_t)a.pre[i] - a.pre[a.pstart[p]];
-                        sel = before < (int64_t)a.pw[p] - a.maxp[p];
+            cl_sync();
+            // a candidate leaves its part when the part's candidates before it weigh
+            // less than the part's excess (weak: the moves; strong: the evicted prefix,
+            // whose end is the first candidate where that weight reaches the excess)
+            int32_t nf = 0, fw = 0;
+            for (int32_t i0 = ib; i0 < ie; i0 += 32) {
+                const int32_t i = i0 + lane;
+                int32_t p = 0, v = 0;
+                bool sel = false;
+                if (i < ie) {
+                    p = ks[i] >> 6;
+                    v = vs[i];
+                    sel = (int64_t)a.pre[i] - a.pbase[p] < s_pw[p] - a.maxp[p];
+                }
+                if (!strong) {
+                    const int32_t pos = hp::warp_append(&cn[0], sel);
+                    if (sel) {
+                        a.moves[pos] = v;
+                        a.oldp[pos] = p;
+                        c1 += a.pregain[v];
                     }
-                    int tot;
-                    const int ex = hp::block_excl_scan<SL_THREADS>(sel, &tot, s_scan);
-                    if (sel) a.moves[mv + ex] = Vs[i];
-                    mv += tot;
+                } else {
+                    nf += sel;
+                    fw += sel ? a.vwgt[v] : 0;
                 }
-                nmoves = mv;
-            } else {
-                for (int32_t p = tid; p < k; p += SL_THREADS) {   // evict_end_kernel
-                    const int32_t st = a.pstart[p], en = a.pend[p];
-                    if (st < 0) { a.ev_end[p] = -1; continue; }
-                    const int64_t need = (int64_t)a.pw[p] - a.maxp[p];
-                    int32_t lo = st, hi = en;
-                    while (lo + 1 < hi) {
-                        const int32_t mid = (lo + hi) / 2;
-                        if ((int64_t)a.pre[mid] - a.pre[st] >= need) hi = mid; else lo = mid;
+            }
+            if (strong) {
+                nf = hp::warp_sum(nf);
+                fw = hp::warp_sum(fw);
+                int32_t pc, pr, np, wt;
+                cl_warp_scan2(nf, fw, &pc, &pr, &np, &wt, X, buf, rank, nct);
+                buf ^= 1;
+                // the evicted vertices in sorted order and their prefix weights (rs_evict_kernel)
+                for (int32_t i0 = ib; i0 < ie; i0 += 32) {
+                    const int32_t i = i0 + lane;
+                    bool sel = false;
+                    int32_t v = 0, w = 0;
+                    if (i < ie) {
+                        const int32_t p = ks[i] >> 6;
+                        v = vs[i];
+                        sel = (int64_t)a.pre[i] - a.pbase[p] < s_pw[p] - a.maxp[p];
+                        w = sel ? a.vwgt[v] : 0;
                     }
-                    a.ev_end[p] = hi;
-                }
-                __syncthreads();
-                int32_t np = 0, wrun = 0;   // rs_evict_kernel
-                for (int32_t b0 = 0; b0 < cnt; b0 += SL_THREADS) {
-                    const int32_t i = b0 + tid;
-                    const int f = i < cnt && i < a.ev_end[Ks[i] >> 6];
-                    const int32_t w = f ? a.vwgt[Vs[i]] : 0;
-                    int tc, tw;
-                    const int ec = hp::block_excl_scan<SL_THREADS>(f, &tc, s_scan);
-                    const int ew = hp::block_excl_scan<SL_THREADS>(w, &tw, s_scan);
-                    if (f) {
-                        a.P[np + ec] = i;
-                        a.sp[np + ec] = wrun + ew;
+                    const unsigned m = __ballot_sync(HP_FULL_MASK, sel);
+                    const int32_t incl = hp::warp_incl_scan(w);
+                    if (sel) {
+                        a.P[pc + __popc(m & lt)] = v;
+                        a.sp[pc + __popc(m & lt)] = pr + incl - w;
                     }
-                    np += tc;
-                    wrun += tw;
+                    pc += __popc(m);
+                    pr += __shfl_sync(HP_FULL_MASK, incl, 31);
                 }
-                // cookie cutter on the prefix weights staged in shared memory
-                for (int32_t i = tid; i < np; i += SL_THREADS) sl_dyn[i] = a.sp[i];
-                if (tid == 0) {
-                    sl_dyn[np] = wrun;
-                    a.sp[np] = wrun;
+                if (gtid == 0) a.sp[np] = wt;
+                cl_sync();
+                if (rank == 0) {   // the cookie cutter, on staged prefix weights when they fit
+                    const bool staged = np + 1 <= a.cookie_cap;
+                    if (staged)
+                        for (int32_t i = tid; i <= np; i += CL_THREADS) cl_dyn[i] = a.sp[i];
+                    __syncthreads();
+                    if (wid == 0)
+                        cookie_cut_warp(k, (const unsigned long long *)s_pw, a.maxp, staged ? cl_dyn : a.sp, np, a.es,
+                                        a.ee);
                 }
+                cl_sync();
+                for (int32_t q = tid; q < k; q += CL_THREADS) s_part[q] = a.es[q];
                 __syncthreads();
-                if (wid == 0) cookie_cut_warp(k, a.pw, a.maxp, sl_dyn, np, a.es, a.ee);
-                __syncthreads();
-                int32_t mv = 0;   // rs_assign_kernel
-                for (int32_t b0 = 0; b0 < np; b0 += SL_THREADS) {
-                    const int32_t j = b0 + tid;
-                    int sel = 0;
-                    int32_t v = 0;
+                for (int32_t j0 = gw * 32; j0 < np; j0 += tw * 32) {   // rs_assign_kernel
+                    const int32_t j = j0 + lane;
+                    bool sel = false;
+                    int32_t v = 0, lo = 0, from = 0;
                     if (j < np) {
-                        int32_t lo = 0, hi = k - 1;   // last part with es[p] <= j
+                        int32_t hi = k - 1;   // last part with es[p] <= j
                         while (lo < hi) {
                             const int32_t mid = (lo + hi + 1) / 2;
-                            if (a.es[mid] <= j) lo = mid; else hi = mid - 1;
+                            if (s_part[mid] <= j) lo = mid; else hi = mid - 1;
                         }
-                        v = Vs[a.P[j]];
-                        if (j < a.ee[lo] && lo != a.where[v]) {
-                            a.dest[v] = lo;
-                            sel = 1;
-                        }
+                        v = a.P[j];
+                        from = a.where[v];
+                        sel = j < a.ee[lo] && lo != from;
                     }
-                    int tot;
-                    const int ex = hp::block_excl_scan<SL_THREADS>(sel, &tot, s_scan);
-                    if (sel) a.moves[mv + ex] = v;
-                    mv += tot;
+                    const int32_t pos = hp::warp_append(&cn[0], sel);
+                    if (sel) {
+                        a.dest[v] = lo;
+                        a.moves[pos] = v;
+                        a.oldp[pos] = from;
+                        const int32_t o = a.goff[v], len = a.goff[v + 1] - o;
+                        c1 += (long long)row_conn(a.gpart + o, a.gconn + o, len, lo, k) + a.pregain[v];
+                    }
                 }
-                nmoves = mv;
             }
         }
-        __syncthreads();
-        // ---- apply: cut change before, moves, gain-row maintenance, cut change after
-        long long acc = 0;
-        for (int32_t i = tid; i < nmoves; i += SL_THREADS) {
-            const int32_t v = a.moves[i];
-            const int32_t o = a.goff[v], len = a.goff[v + 1] - o;
-            const int32_t from = a.where[v], to = a.dest[v];
-            a.oldp[i] = from;
-            acc += (long long)row_conn(a.gpart + o, a.gconn + o, len, to, k) -
-                   row_conn(a.gpart + o, a.gconn + o, len, from, k);
+        cl_sync();   // the moves are complete
+        // ---- apply: moves, gain-row maintenance, cut change after
+        const int32_t nmoves = __ldcg(&cn[0]);
+        if (nmoves > 0) {
+            apply_moves_rows(gw, tw, a.moves, nmoves, a.where, a.dest, a.vwgt, a.pw, a.xadj, a.adjncy, a.adjwgt,
+                             a.goff, a.gconn, a.dirty, a.small_l, a.big_l, &cn[1], k, nullptr, nullptr, a.bigd,
+                             INT_MAX);
+            cl_sync();
+            cl_rebuild(a, gw, tw, __ldcg(&cn[1]), __ldcg(&cn[2]), cl_dyn);
         }
-        const long long c1 = sl_sum64(acc, s_red);
-        apply_moves_rows(wid, SL_WARPS, a.moves, nmoves, a.where, a.dest, a.vwgt, a.pw, a.xadj, a.adjncy, a.adjwgt,
-                         a.goff, a.gconn, a.dirty, a.small_l, a.big_l, s_lists, k, nullptr, nullptr, a.bigd, INT_MAX);
-        __syncthreads();
-        const int32_t ns = s_lists[0], nb = s_lists[1];
-        if (ns > 0) {
-            if (a.small_max <= 8)
-                gain_seg_rows<8>(wid, SL_WARPS, a.small_l, ns, a.xadj, a.adjncy, a.adjwgt, a.where, a.goff, a.gpart,
-                                 a.gconn, k, a.dirty);
-            else if (a.small_max <= 16)
-                gain_seg_rows<16>(wid, SL_WARPS, a.small_l, ns, a.xadj, a.adjncy, a.adjwgt, a.where, a.goff, a.gpart,
-                                  a.gconn, k, a.dirty);
-            else
-                gain_seg_rows<32>(wid, SL_WARPS, a.small_l, ns, a.xadj, a.adjncy, a.adjwgt, a.where, a.goff, a.gpart,
-                                  a.gconn, k, a.dirty);
+        if (rank == 0 && tid < 4) a.counts[4 * ((guard & 1) ^ 1) + tid] = 0;   // the next pass's set
+        long long c[2] = {c1, 0};
+        if (nmoves > 0) {
+            cl_sync();
+            for (int32_t i = gtid; i < nmoves; i += gt) {
+                const int32_t v = a.moves[i];
+                const int32_t o = a.goff[v], len = a.goff[v + 1] - o;
+                c[1] += (long long)row_conn(a.gpart + o, a.gconn + o, len, a.where[v], k) -
+                        row_conn(a.gpart + o, a.gconn + o, len, a.oldp[i], k);
+            }
         }
-        if (nb > 0) {
-            const int nw = (k + 31) >> 5;
-            int32_t *dw = sl_dyn + (size_t)wid * (k + nw);
-            unsigned *bm = (unsigned *)(dw + k);
-            for (int i = lane; i < k; i += 32) dw[i] = 0;
-            for (int i = lane; i < nw; i += 32) bm[i] = 0u;
-            __syncwarp();
-            gain_bigwarp_rows(wid, SL_WARPS, dw, bm, a.big_l, nb, a.xadj, a.adjncy, a.adjwgt, a.where, a.goff,
-                              a.gpart, a.gconn, k, a.dirty, a.bigd, INT_MAX);
-        }
-        __syncthreads();
-        acc = 0;
-        for (int32_t i = tid; i < nmoves; i += SL_THREADS) {
-            const int32_t v = a.moves[i];
-            const int32_t o = a.goff[v], len = a.goff[v + 1] - o;
-            const int32_t from = a.oldp[i], to = a.where[v];
-            acc += (long long)row_conn(a.gpart + o, a.gconn + o, len, to, k) -
-                   row_conn(a.gpart + o, a.gconn + o, len, from, k);
-        }
-        const long long c2 = sl_sum64(acc, s_red);
         long long m = LLONG_MIN;
-        for (int32_t p = tid; p < k; p += SL_THREADS) {
-            const long long e = (long long)a.pw[p] - a.maxp[p];
+        for (int32_t q = tid; q < k; q += CL_THREADS) {
+            const long long w = (long long)__ldcg(&a.pw[q]), e = w - a.maxp[q];
+            s_pw[q] = w;
+            s_ufl[q] = e < 0;
             m = e > m ? e : m;
         }
-        m = sl_max64(m, s_red);
+        m = hp::warp_max64(m);
+        cl_sum<2>(c, X, buf, rank, nct);
+        buf ^= 1;
+        if (lane == 0) X.w[wid][2] = m;
+        __syncthreads();
         if (tid == 0) {
+            for (int w = 1; w < CL_WARPS; w++) m = X.w[w][2] > m ? X.w[w][2] : m;
             // the judge's sum over the learned moves is the applied pass's exact change
-            if (judged && jl2 != c1 + c2) atomicOr(a.status, HP_STATUS_OVERFLOW);
-            ctl_advance(s, m, c1, c2, nmoves, ncand, jp2);
+            if (rank == 0 && judged && jl2 != c[0] + c[1]) atomicOr(a.status, HP_STATUS_OVERFLOW);
+            ctl_advance(&s_ctl, m, c[0], c[1], nmoves, ncand, jp2);
         }
         __syncthreads();
-        if (*(volatile const int32_t *)&s->take) {
-            for (int32_t i = tid; i < n; i += SL_THREADS) a.best_where[i] = a.where[i];
-            for (int32_t i = tid; i < k; i += SL_THREADS) a.best_pw[i] = a.pw[i];
+        if (s_ctl.take) {
+            for (int32_t v = vb + lane; v < ve; v += 32) a.best_where[v] = a.where[v];
+            if (rank == 0)
+                for (int32_t q = tid; q < k; q += CL_THREADS) a.best_pw[q] = (unsigned long long)s_pw[q];
         }
-        __syncthreads();
     }
-    if (!*(volatile const int32_t *)&s->best_current)
-        for (int32_t i = tid; i < n; i += SL_THREADS) a.where[i] = a.best_where[i];
+    if (!s_ctl.best_current)
+        for (int32_t v = vb + lane; v < ve; v += 32) a.where[v] = a.best_where[v];
+    if (gtid == 0) *a.ctl = s_ctl;
 }
 
 // Graph-capture helper: records the launches of body() into `graph`.  The capture
@@ -3222,11 +3432,10 @@ int refine_level(hp_context *c, HpLevel &g, int32_t k, bool finest, const int64_
     const bool recording = c->opt.learned == 2 && c->log_x != nullptr;
     const int patience = c->opt.refine_patience;
     const bool dbg = getenv("HP_DEBUG_PASSES") != nullptr;
-    // small levels: the whole pass loop in one CTA (same rule, same result), in
+    // small levels: the whole pass loop in one cluster (same rule, same result), in
     // either loop mode unless the per-pass move log or pass log is on
-    const int32_t small_n = c->tune.small_level_n;
-    const bool small_level = !recording && !dbg && n <= small_n && k <= HP_TUNE_WARP_DENSE_K_MAX &&
-                             g.m <= 16 * (int64_t)small_n;
+    const int32_t cl_n = cluster_level_n(c);
+    const bool small_level = !recording && !dbg && n <= cl_n && k <= CL_KMAX && g.m <= CL_DEG * cl_n;
     if (small_level) {
         // the level's setup (gain rows, part weights, cut, control block) runs
         // inside the kernel: no launch per setup step
@@ -3269,10 +3478,8 @@ int refine_level(hp_context *c, HpLevel &g, int32_t k, bool finest, const int64_
         a.pre = B.pre;
         a.P = B.P;
         a.sp = B.sp;
-        a.pstart = B.pstart;
-        a.pend = B.pend;
-        a.und = B.und;
-        a.ev_end = B.ev_end;
+        a.pbase = B.pstart;
+        a.counts = (int32_t *)c->d_scal;
         a.es = B.es;
         a.ee = B.ee;
         a.lock = B.lock;
@@ -3285,7 +3492,10 @@ int refine_level(hp_context *c, HpLevel &g, int32_t k, bool finest, const int64_
         a.maxp = B.maxp;
         a.mlp_params = c->mlp_params;
         a.ctl = ctl;
-        HP_LAUNCH(c, refine_small_kernel, 1, SL_THREADS, small_level_smem(n, k), a);
+        const size_t smem = small_level_smem(n, k);
+        a.cookie_cap = (int32_t)(smem / sizeof(int32_t));
+        const int ctas = cluster_ctas(c, n, g.m);
+        HP_LAUNCH_CLUSTER(c, refine_cluster_kernel, ctas, ctas, CL_THREADS, smem, a);
         c->hi = mark;
         return HP_OK;
     }
@@ -3369,14 +3579,36 @@ int refine_level(hp_context *c, HpLevel &g, int32_t k, bool finest, const int64_
 
 }  // namespace
 
-int hp_refine_init()
+int hp_refine_init(hp_context *c)
 {
     HP_CUDA(cudaFuncSetAttribute(cookie_cutter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(sizeof(int32_t) * COOKIE_SMEM_INTS)));
     const int bytes = HP_MAX_PARTS * 4 + (HP_MAX_PARTS / 32) * 4;
     HP_CUDA(cudaFuncSetAttribute(gain_dense_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    HP_CUDA(cudaFuncSetAttribute(refine_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)small_level_smem(HP_TUNE_SMALL_LEVEL_MAX, HP_TUNE_WARP_DENSE_K_MAX)));
+    const size_t smem = small_level_smem(CL_LEVEL_MAX, CL_KMAX);
+    HP_CUDA(cudaFuncSetAttribute(refine_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    HP_CUDA(cudaFuncSetAttribute(refine_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    // the largest cluster the device can place
+    c->max_cluster = 1;
+    for (int q = CL_MAX; q > 1; q /= 2) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(q);
+        cfg.blockDim = dim3(CL_THREADS);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)q;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int fit = 0;
+        if (cudaOccupancyMaxActiveClusters(&fit, refine_cluster_kernel, &cfg) == cudaSuccess && fit > 0) {
+            c->max_cluster = q;
+            break;
+        }
+        cudaGetLastError();
+    }
     return HP_OK;
 }
 

@@ -175,9 +175,10 @@ typedef struct hp_tuning {
     int32_t grid_ctas_per_sm;    /* grid-stride kernels: CTAs per SM              [1, 32]       8 */
     int32_t dense_sparse_ratio;  /* dense contraction rows: the two-level bitmap when
                                     entries * ratio < bitmap words                [1, 4096]     4 */
-    int32_t small_level_n;       /* refinement: levels of at most this many vertices
-                                    (and 16x as many adjacency entries, nparts <= 1024)
-                                    run all their passes in one CTA; 0 = never    [0, 32768]    4096 */
+    int32_t small_level_n;       /* refinement: levels of at most this many vertices per CTA of
+                                    a cluster (16 CTAs where the device has them; at most 65536
+                                    vertices, 16x as many adjacency entries, nparts <= 1024)
+                                    run all their passes in one cluster; 0 = never [0, 32768]    4096 */
     int32_t chunk_deg;           /* refinement: the afterburner and move application
                                     split rows longer than this into chunks of 512
                                     entries over the whole grid                  [gain_thread_deg, 2^24] 4096 */

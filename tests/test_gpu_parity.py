@@ -10,7 +10,7 @@ import pytest
 
 import hunyuansc25_b200 as hp
 import oracle
-from hunyuansc25_b200 import graphs
+from hunyuansc25_b200 import graphs, learn
 from hunyuansc25_b200._abi import (HP_ERR_INVALID_ARG, HP_ERR_INVALID_GRAPH, HP_ERR_NOMEM, HP_ERR_TIMEOUT,
                                    HP_ERR_UNSUPPORTED, default_options)
 
@@ -485,3 +485,27 @@ def test_bisection_trials(ctx, n, p, isolated, k):
 def test_bisection_trials_large_state(ctx):
     g = graphs.grid2d(120, 100, seed=3, wmin=1, wmax=9)
     compare_runs(ctx, g, 2, 1.1, coarsen_to=g.nvtxs, init_starts=4, fm_passes=2)
+
+
+# every pass of a level in one cluster: sizes around its CTAs (512 vertices each) and its
+# bound (65536), one part to the most it takes, gain rows denser and sparser than k
+@pytest.mark.parametrize("x,y,k,wmax", [(7, 73, 3, 1), (19, 27, 1, 9), (19, 27, 1024, 9), (41, 50, 33, 100),
+                                        (128, 65, 8, 1), (256, 256, 100, 5), (257, 256, 100, 5)])
+def test_cluster_levels(ctx, x, y, k, wmax):
+    compare_runs(ctx, graphs.grid2d(x, y, seed=x, wmin=1, wmax=wmax), k, 1.05)
+
+
+def test_cluster_levels_learned(ctx):
+    """The learned selection inside a cluster equals the launched passes'."""
+    g = graphs.rmat(13, 8, seed=9, wmin=1, wmax=100)
+    params, thr, _ = learn.load_params()
+    ctx.mlp_set_params(params, thr)
+    for learned in (1, 3):
+        opt = default_options(learned=learned)
+        a = ctx.partition_graph(g, 32, 1.03, options=opt)
+        ctx.set_tuning(small_level_n=0)
+        try:
+            b = ctx.partition_graph(g, 32, 1.03, options=opt)
+        finally:
+            ctx.set_tuning()
+        assert a[1] == b[1] and np.array_equal(a[0], b[0])
