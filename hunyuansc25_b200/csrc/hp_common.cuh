@@ -139,6 +139,43 @@ __device__ __forceinline__ int32_t warp_find_row(const int32_t *__restrict__ xad
     return m ? lo + 1 + (31 - __clz(m)) : lo;
 }
 
+// 32 consecutive rows of a CSR held by a warp, for walking its entries in order
+// without shared memory: lane l keeps the start of row r0 + l (INT_MAX past the
+// last row), end is where row r0 + 32 starts.  The row of an entry inside the
+// window is the last lane whose start is at most the entry (rows that start at
+// the same entry are empty but for the last), five shuffles per 32 entries.
+// xadj monotone.
+struct RowWindow {
+    int32_t r0, start, end;
+    __device__ __forceinline__ void load(const int32_t *__restrict__ xadj, int32_t n, int32_t first)
+    {
+        const int lane = threadIdx.x & 31;
+        r0 = first;
+        start = r0 + lane < n ? xadj[r0 + lane] : INT_MAX;
+        end = r0 + 32 < n ? xadj[r0 + 32] : INT_MAX;
+    }
+    // lane of the row of entry j (start of lane 0 <= j < end); all 32 lanes call
+    __device__ __forceinline__ int find(int32_t j) const
+    {
+        int l = 0;
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1) {
+            const int32_t st = __shfl_sync(HP_FULL_MASK, start, l + s);
+            if (st <= j) l += s;
+        }
+        return l;
+    }
+};
+
+// Entries per warp of an edge-parallel walk over m entries: whole batches of 128,
+// enough warps to fill the device (64 per SM), at most 2048 entries (one
+// warp_find_row and the window loads are spread over them).
+inline int64_t warp_entries(int64_t m, int sm_count)
+{
+    const int64_t e = (m / ((int64_t)sm_count * 64) + 127) / 128 * 128;
+    return e < 128 ? 128 : e > 2048 ? 2048 : e;
+}
+
 // Owner rows of a tile of CSR entries: owner[i] = the row of entry tb + i for
 // i < te - tb <= NT * ITEMS (xadj monotone, xadj[0] = 0, xadj[n] = m > tb).
 // The row holding entry tb comes from warp_find_row; every later row that

@@ -38,3 +38,65 @@ def test_edgecut_device(ctx):
     assert ctx.edgecut_device(t[0], t[1], t[2], t[3]) == oracle.edgecut(g, where)
     unit = graphs.Graph(g.xadj, g.adjncy, g.vwgt, np.ones_like(g.adjwgt))
     assert ctx.edgecut_device(t[0], t[1], None, t[3]) == oracle.edgecut(unit, where)
+
+
+def walk_graph(degrees, seed):
+    """A symmetric graph on the given target degrees (a multigraph's edges, repeats dropped)."""
+    rng = np.random.default_rng(seed)
+    stubs = np.repeat(np.arange(len(degrees)), degrees)
+    rng.shuffle(stubs)
+    stubs = stubs[: stubs.size // 2 * 2].reshape(-1, 2)
+    stubs = stubs[stubs[:, 0] != stubs[:, 1]]
+    e = np.unique(np.sort(stubs, 1), axis=0)
+    w = rng.integers(1, 1000, e.shape[0]).astype(np.int32)
+    s, d = np.concatenate([e[:, 0], e[:, 1]]), np.concatenate([e[:, 1], e[:, 0]])
+    order = np.lexsort((d, s))
+    xadj = np.zeros(len(degrees) + 1, np.int32)
+    xadj[1:] = np.cumsum(np.bincount(s, minlength=len(degrees)))
+    return xadj, d[order].astype(np.int32), np.concatenate([w, w])[order]
+
+
+# the edge-parallel walks: empty rows in runs longer than a window of 32, hub rows over
+# several warps' shares, one entry pair to several rounds of the grid
+WALKS = {
+    "pair": [1, 1],
+    "empty_runs": [0] * 70 + [3, 5, 2] + [0] * 33 + [4] * 40 + [0] * 200,
+    "hubs": [3000, 2500] + [2] * 5000 + [0] * 40 + [700] * 3 + [1] * 999,
+    "odd": [5] * 1001,
+    "large": [16] * 120001,
+}
+
+
+@pytest.mark.parametrize("name", list(WALKS))
+@pytest.mark.parametrize("unit", [False, True])
+def test_edgecut_walk(ctx, name, unit):
+    import torch
+    xadj, adj, w = walk_graph(WALKS[name], 3)
+    n = xadj.size - 1
+    where = np.random.default_rng(4).integers(0, 7, n).astype(np.int32)
+    rows = np.repeat(np.arange(n), np.diff(xadj))
+    cut = int((np.ones_like(w) if unit else w)[where[rows] != where[adj]].astype(np.int64).sum()) // 2
+    t = [torch.from_numpy(a).cuda() for a in (xadj, adj, w, where)]
+    torch.cuda.synchronize()
+    assert ctx.edgecut_device(t[0], t[1], None if unit else t[2], t[3]) == cut
+
+
+@pytest.mark.parametrize("at", [0, 31, 32, 127, 128, 129, 500])
+def test_validation_of_unsorted_rows(ctx, at):
+    """A row that is not ascending at one place is accepted, one that lists a neighbour twice
+    (there, or far apart) is refused, wherever the place falls in a warp's batches."""
+    import hunyuansc25_b200 as hp
+    n = 700
+    xadj = np.arange(0, n * (n - 1) + 1, n - 1).astype(np.int32)
+    adj = np.stack([np.delete(np.arange(n), v) for v in range(n)]).astype(np.int32)
+    v = 3 + at
+    ok = adj.copy()
+    ok[v, [at, at + 1]] = ok[v, [at + 1, at]]
+    part, cut = ctx.partition(xadj, ok.ravel(), 2)
+    ref, rcut = ctx.partition(xadj, adj.ravel(), 2)
+    assert cut == rcut
+    for other in (at + 1, (at + 300) % (n - 1)):
+        bad = adj.copy()
+        bad[v, other] = bad[v, at]
+        with pytest.raises(hp.HpError):
+            ctx.partition(xadj, bad.ravel(), 2)
