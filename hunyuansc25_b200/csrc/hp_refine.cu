@@ -408,26 +408,66 @@ gain_dense_kernel(const int32_t *__restrict__ list, const int32_t *__restrict__ 
     }
 }
 
-__device__ __forceinline__ int32_t row_conn(const int32_t *gp, const int32_t *gc, int32_t len, int32_t q,
-                                            int32_t k)
+// Calls f(part, connectivity) for the entries of a gain row up to its padding, in
+// order, ROW_BATCH loads of both arrays in flight at a time: a walk that tests every
+// entry before it loads the next one pays a memory latency per entry.
+constexpr int ROW_BATCH = 4;
+template <class F>
+__device__ __forceinline__ void row_walk(const int32_t *gpart, const int32_t *gconn, int32_t o, int32_t len, F &&f)
+{
+    for (int32_t j0 = 0; j0 < len; j0 += ROW_BATCH) {
+        int32_t q[ROW_BATCH], c[ROW_BATCH];
+#pragma unroll
+        for (int t = 0; t < ROW_BATCH; t++) {
+            const bool in = j0 + t < len;
+            q[t] = in ? gpart[o + j0 + t] : -1;
+            c[t] = in ? gconn[o + j0 + t] : 0;
+        }
+#pragma unroll
+        for (int t = 0; t < ROW_BATCH; t++) {
+            if (q[t] < 0) return;
+            f(q[t], c[t]);
+        }
+    }
+}
+
+// The connectivity to part q in a gain row of len entries (capacity).
+__device__ __forceinline__ int32_t row_conn(const int32_t *gp, const int32_t *gc, int32_t len, int32_t q, int32_t k)
 {
     if (len == k) return gc[q];   // dense row
     // rows are ascending by part and padded with -1: bisect to a short window
     // (entries before lo are parts below q; entries from hi on are padding or
-    // parts >= q), then walk to the first entry that is padding or >= q
+    // parts >= q), then read the window [lo, hi] at once
     int32_t lo = 0, hi = len;
-    while (hi - lo > 8) {
+    while (hi - lo > 7) {
         const int32_t mid = (lo + hi) >> 1;
         const int32_t p = gp[mid];
         if (p >= 0 && p < q) lo = mid + 1;
         else hi = mid;
     }
-    for (int32_t j = lo; j < len; j++) {
-        const int32_t p = gp[j];
-        if (p == q) return gc[j];
-        if (p < 0 || p > q) break;
+    int32_t at = -1;
+#pragma unroll
+    for (int t = 0; t < 8; t++)
+        if (lo + t < len && gp[lo + t] == q) at = lo + t;
+    return at >= 0 ? gc[at] : 0;
+}
+
+// conn(a) - conn(b) in a gain row: the two lookups' loads overlap in dense and in
+// short rows.
+__device__ __forceinline__ long long row_diff(const int32_t *gp, const int32_t *gc, int32_t len, int32_t a, int32_t b,
+                                              int32_t k)
+{
+    if (len == k) return (long long)gc[a] - gc[b];
+    if (len > 12) return (long long)row_conn(gp, gc, len, a, k) - row_conn(gp, gc, len, b, k);
+    int32_t ia = -1, ib = -1;
+#pragma unroll
+    for (int t = 0; t < 12; t++) {
+        const int32_t p = t < len ? gp[t] : -1;
+        if (p == a) ia = t;   // (a, b >= 0: never the padding)
+        if (p == b) ib = t;
     }
-    return 0;
+    const int32_t ca = ia >= 0 ? gc[ia] : 0, cb = ib >= 0 ? gc[ib] : 0;
+    return (long long)ca - cb;
 }
 
 __global__ void __launch_bounds__(256)
@@ -472,11 +512,9 @@ rowcut_kernel(int32_t n, const int32_t *__restrict__ goff, const int32_t *__rest
     // rows longer than 32 entries are summed by the whole warp, one at a time
     const bool coop = len > 32;
     if (!coop)
-        for (int32_t j = o; j < o + len; j++) {
-            const int32_t q = gpart[j];
-            if (q < 0) break;
-            if (q != p) acc += gconn[j];
-        }
+        row_walk(gpart, gconn, o, len, [&](int32_t q, int32_t cq) {
+            if (q != p) acc += cq;
+        });
     unsigned cm = __ballot_sync(HP_FULL_MASK, coop);
     while (cm) {
         const int src = __ffs(cm) - 1;
@@ -532,15 +570,12 @@ __device__ __forceinline__ RowBest row_best(const int32_t *__restrict__ gpart, c
     RowBest r{0, 0, 0, -1, 0};
     const bool coop = len > 32;
     if (!coop)
-        for (int32_t j = o; j < o + len; j++) {
-            const int32_t q = gpart[j];
-            if (q < 0) break;
-            const int32_t cq = gconn[j];
+        row_walk(gpart, gconn, o, len, [&](int32_t q, int32_t cq) {
             r.wd += cq;
             r.np += cq > 0;
-            if (q == p) { r.pc = cq; continue; }
+            if (q == p) { r.pc = cq; return; }
             if (cq > r.bc) { r.bc = cq; r.b = q; }   // ascending parts: first max = lowest part
-        }
+        });
     unsigned cm = __ballot_sync(HP_FULL_MASK, coop);
     while (cm) {
         const int src = __ffs(cm) - 1;
@@ -635,15 +670,12 @@ __device__ __forceinline__ RowBest row_best_cta(CoopRows<NT> &S, const int32_t *
     RowBest r{0, 0, 0, -1, 0};
     const bool coop = len > 32;
     if (!coop)
-        for (int32_t j = o; j < o + len; j++) {
-            const int32_t q = gpart[j];
-            if (q < 0) break;
-            const int32_t cq = gconn[j];
+        row_walk(gpart, gconn, o, len, [&](int32_t q, int32_t cq) {
             r.wd += cq;
             r.np += cq > 0;
-            if (q == p) { r.pc = cq; continue; }
+            if (q == p) { r.pc = cq; return; }
             if (cq > r.bc) { r.bc = cq; r.b = q; }   // ascending parts: first max = lowest part
-        }
+        });
     const int my = coop_queue<NT>(S, coop, o, len, p);
     const int nc = S.n;
     for (int i = wid; i < nc; i += NT / 32) {
@@ -851,7 +883,11 @@ __global__ void log_label_kernel(int64_t r0, int64_t r1, const int32_t *__restri
 // the cut-change sum c1 (conn(to) - conn(from) of every move, read from the mover's
 // own gain row before any move applies).  The kernels that decide the moves append
 // them through move_append and add the c1 terms per block, so no separate pass
-// over the moves precedes their application.
+// over the moves precedes their application.  The terms come from the gains the
+// selection left in pregain: an LP candidate's is its term; a weak rebalance
+// candidate's too (an undersized destination taken for want of a connected one has
+// connectivity 0: it would have been connected otherwise); a strong one's is
+// -conn(from), to which the destination's connectivity is added (goff .. k).
 struct MoveSink {
     int32_t *moves, *oldp;
     unsigned long long *d_nmoves, *d_c1;
@@ -859,18 +895,12 @@ struct MoveSink {
     int32_t k;
 };
 
-__device__ __forceinline__ int32_t row_conn(const int32_t *gp, const int32_t *gc, int32_t len, int32_t q,
-                                            int32_t k);
-
-// Appends the move of v from p to d; returns its c1 term.
-__device__ __forceinline__ long long move_append(const MoveSink &ms, int32_t v, int32_t p, int32_t d)
+// Appends the move of v out of part p.
+__device__ __forceinline__ void move_append(const MoveSink &ms, int32_t v, int32_t p)
 {
     const unsigned long long i = atomicAdd(ms.d_nmoves, 1ull);
     ms.moves[i] = v;
     ms.oldp[i] = p;
-    const int32_t o = ms.goff[v], len = ms.goff[v + 1] - o;
-    return (long long)row_conn(ms.gpart + o, ms.gconn + o, len, d, ms.k) -
-           row_conn(ms.gpart + o, ms.gconn + o, len, p, ms.k);
 }
 
 __device__ __forceinline__ long long ab_change(int32_t v, int32_t g, int32_t p, int32_t b,
@@ -988,7 +1018,10 @@ afterburner_small_kernel(int32_t n, const int32_t *__restrict__ xadj, const int3
                 J.accp[v] = selp;
                 listed = sel || selp;
             }
-            if (sel) c1 = move_append(ms, v, p, b);
+            if (sel) {
+                move_append(ms, v, p);
+                c1 = g;
+            }
         }
     }
     if (judge) {
@@ -1040,7 +1073,10 @@ afterburner_big_kernel(const int32_t *__restrict__ big, const int32_t *__restric
                 J.accp[v] = selp;
                 if (sel || selp) J.list[atomicAdd(J.d_n, 1)] = v;
             }
-            if (sel) c1 += move_append(ms, v, p, b);
+            if (sel) {
+                move_append(ms, v, p);
+                c1 += g;
+            }
         }
     }
     hp::block_add_to<256>(c1, ms.d_c1);
@@ -1195,7 +1231,10 @@ __global__ void afterburner_huge_final_kernel(const int32_t *__restrict__ huge, 
             if (sel || selp) J.list[atomicAdd(J.d_n, 1)] = v;
         }
         lock[v] = sel;
-        if (sel) c1 += move_append(ms, v, where[v], dest[v]);
+        if (sel) {
+            move_append(ms, v, where[v]);
+            c1 += g;
+        }
     }
     hp::block_add_to<256>(c1, ms.d_c1);
 }
@@ -1429,7 +1468,6 @@ __device__ __forceinline__ void undersized_block(int32_t k, const unsigned long 
 //         (und[v % nu]); gain = conn(dest) - conn(own)
 //   strong (jetrs, :2774-3135): v in an overweight part with vwgt < 2 (pw - opt);
 //         loss = -conn(own)
-// The part bounds pstart/pend are reset to -1 here for the rank kernel.
 constexpr int RB_TILE = 256;
 constexpr int RB_COOP = 32;   // weak rebalance: longer gain rows are walked by a warp
 
@@ -1441,9 +1479,8 @@ rb_candidates_kernel(int32_t n, const int32_t *__restrict__ where, const int32_t
                      const int32_t *__restrict__ gpart, const int32_t *__restrict__ gconn,
                      const int32_t *__restrict__ und, const int32_t *__restrict__ d_nu, int32_t k,
                      int32_t *__restrict__ K, int32_t *__restrict__ V, int32_t *__restrict__ dest,
-                     int32_t *__restrict__ d_cnt, int32_t *__restrict__ pstart, int32_t *__restrict__ pend,
-                     unsigned long long *tile_status, hp::LbCtl *lb, unsigned *status,
-                     const int8_t *__restrict__ ufl, BestCopy bcp)
+                     int32_t *__restrict__ d_cnt, unsigned long long *tile_status, hp::LbCtl *lb, unsigned *status,
+                     const int8_t *__restrict__ ufl, int32_t *__restrict__ pregain, BestCopy bcp)
 {
     hp::pdl_wait();
     __shared__ int32_t s_scan[RB_TILE / 32 + 2];
@@ -1452,10 +1489,6 @@ rb_candidates_kernel(int32_t n, const int32_t *__restrict__ where, const int32_t
     int64_t tile;
     unsigned epoch;
     hp::lb_begin(lb, &tile, &epoch);
-    for (int64_t q = tile * RB_TILE + threadIdx.x; q < k; q += (int64_t)gridDim.x * RB_TILE) {
-        pstart[q] = -1;
-        pend[q] = -1;
-    }
     const int64_t v64 = tile * RB_TILE + threadIdx.x;
     const int lane = threadIdx.x & 31;
     int32_t kk = -1;
@@ -1473,7 +1506,7 @@ rb_candidates_kernel(int32_t n, const int32_t *__restrict__ where, const int32_t
                       : (pwp > maxp[p] && 2 * (int64_t)vwgt[v] < 3 * (pwp - opt[p]));
     }
     const int32_t o = cand ? goff[v] : 0, len = cand ? goff[v + 1] - o : 0;
-    int32_t d = p;
+    int32_t d = p, gain = 0;
     if (!STRONG) {
         // best underweight part by connectivity (first, i.e. lowest part, among
         // equals) and the connectivity to the own part; rows of more than
@@ -1482,13 +1515,10 @@ rb_candidates_kernel(int32_t n, const int32_t *__restrict__ where, const int32_t
         int32_t b = -1;
         const bool coop = cand && len > RB_COOP;
         if (cand && !coop) {
-            for (int32_t j = o; j < o + len; j++) {
-                const int32_t q = gpart[j];
-                if (q < 0) break;
-                const int32_t cq = gconn[j];
+            row_walk(gpart, gconn, o, len, [&](int32_t q, int32_t cq) {
                 if (q == p) pc = cq;
-                if (ufl[q] && cq > bc) { bc = cq; b = q; }
-            }
+                if (cq > bc && ufl[q]) { bc = cq; b = q; }
+            });
         }
         // the CTA's long rows, shared by all its warps
         const int my = coop_queue<RB_TILE>(S, coop, o, len, p);
@@ -1524,13 +1554,14 @@ rb_candidates_kernel(int32_t n, const int32_t *__restrict__ where, const int32_t
                 if (nu == 0) ok = false;
                 else { b = und[v % nu]; g = -pc; }
             }
-            if (ok) { d = b; kk = p * 64 + hp::gain_bucket((int32_t)g, vwgt[v]); }
+            if (ok) { d = b; gain = (int32_t)g; kk = p * 64 + hp::gain_bucket(gain, vwgt[v]); }
         }
     } else if (cand) {
-        const int32_t pc = row_conn(gpart + o, gconn + o, len, p, k);
-        kk = p * 64 + hp::gain_bucket(-pc, vwgt[v]);
+        gain = -row_conn(gpart + o, gconn + o, len, p, k);
+        kk = p * 64 + hp::gain_bucket(gain, vwgt[v]);
     }
     if (in) dest[v] = d;
+    if (kk >= 0) pregain[v] = gain;   // the move's c1 term (MoveSink)
     int tot;
     const int local = hp::block_excl_scan<RB_TILE>(kk >= 0 ? 1 : 0, &tot, s_scan);
     if (threadIdx.x < 32) {
@@ -1548,8 +1579,8 @@ rb_candidates_kernel(int32_t n, const int32_t *__restrict__ where, const int32_t
 }
 
 // Over the sorted candidates: pre[i] = weight of the candidates before i in
-// the sorted order (pre[cnt] = total), and the part bounds pstart/pend (first
-// index, one past the last) from the sorted keys.  Tiles of RK_TILE items in
+// the sorted order (pre[cnt] = total), and pstart, the index of every part's first
+// candidate, from the sorted keys.  Tiles of RK_TILE items in
 // launch order with an epoch look-back, taken by a fixed grid of persistent
 // CTAs until the tile holding index cnt, so the work follows the count on
 // the device, not n.
@@ -1558,7 +1589,7 @@ constexpr int RK_THREADS = 256, RK_ITEMS = 4, RK_TILE = RK_THREADS * RK_ITEMS;
 __global__ void __launch_bounds__(RK_THREADS)
 rb_rank_kernel(const int32_t *__restrict__ K, const int32_t *__restrict__ V, const int32_t *__restrict__ d_cnt,
                const int32_t *__restrict__ vwgt, int32_t *__restrict__ pre, int32_t *__restrict__ pstart,
-               int32_t *__restrict__ pend, unsigned long long *tile_status, hp::LbCtl *lb, unsigned *status)
+               unsigned long long *tile_status, hp::LbCtl *lb, unsigned *status)
 {
     hp::pdl_wait();
     __shared__ int32_t s_scan[RK_THREADS / 32 + 2];
@@ -1593,7 +1624,6 @@ rb_rank_kernel(const int32_t *__restrict__ K, const int32_t *__restrict__ V, con
             if (i < cnt) {
                 const int32_t p = K[i] >> 6;
                 if (i == 0 || (K[i - 1] >> 6) != p) pstart[p] = (int32_t)i;
-                if (i == cnt - 1 || (K[i + 1] >> 6) != p) pend[p] = (int32_t)i + 1;
             }
         }
     }
@@ -1651,7 +1681,7 @@ __global__ void rw_select_kernel(const int32_t *__restrict__ K, const int32_t *_
                                  const int32_t *__restrict__ d_cnt, const int32_t *__restrict__ pre,
                                  const int32_t *__restrict__ pstart,
                                  const unsigned long long *__restrict__ pw,
-                                 const int64_t *__restrict__ maxp, const int32_t *__restrict__ dest, MoveSink ms)
+                                 const int64_t *__restrict__ maxp, const int32_t *__restrict__ pregain, MoveSink ms)
 {
     hp::pdl_wait();
     const int32_t cnt = *d_cnt;
@@ -1662,41 +1692,24 @@ __global__ void rw_select_kernel(const int32_t *__restrict__ K, const int32_t *_
         int64_t before = (int64_t)pre[i] - pre[pstart[p]];
         if (before < (int64_t)pw[p] - maxp[p]) {
             const int32_t v = V[i];
-            c1 += move_append(ms, v, p, dest[v]);
+            move_append(ms, v, p);
+            c1 += pregain[v];
         }
     }
     hp::block_add_to<256>(c1, ms.d_c1);
 }
 
-// Evicted prefix of every overweight part: smallest e in (s, end] with
-// pre[e] - pre[s] >= excess, else end.
-__global__ void evict_end_kernel(int32_t k, const int32_t *__restrict__ pstart,
-                                 const int32_t *__restrict__ pend, const int32_t *__restrict__ pre,
-                                 const unsigned long long *__restrict__ pw,
-                                 const int64_t *__restrict__ maxp, int32_t *__restrict__ ev_end)
-{
-    hp::pdl_wait();
-    int32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= k) return;
-    int32_t s = pstart[p], e = pend[p];
-    if (s < 0) { ev_end[p] = -1; return; }
-    const int64_t need = (int64_t)pw[p] - maxp[p];
-    int32_t lo = s, hi = e;
-    while (lo + 1 < hi) {
-        int32_t mid = (lo + hi) / 2;
-        if ((int64_t)pre[mid] - pre[s] >= need) hi = mid; else lo = mid;
-    }
-    ev_end[p] = hi;
-}
-
-// Strong rebalance: the evicted prefix of every overweight part (sorted index
-// i < ev_end[part]) compacted in sorted order -- P[j] = i and sp[j] = weight of
+// Strong rebalance: the evicted prefix of every overweight part (up to the first
+// candidate where the weight before it reaches the part's excess: the candidates
+// whose weight before them is less) compacted in sorted order -- P[j] = i and sp[j] = weight of
 // the evicted candidates before j (sp[np] = total), *d_np = np -- in one pass
 // with two epoch look-back chains (count: tile words [0, half); weight: words
 // [half, 2 half)); persistent CTAs as in rb_rank_kernel.
 __global__ void __launch_bounds__(RK_THREADS)
 rs_evict_kernel(const int32_t *__restrict__ K, const int32_t *__restrict__ V, const int32_t *__restrict__ d_cnt,
-                const int32_t *__restrict__ ev_end, const int32_t *__restrict__ vwgt, int32_t *__restrict__ P,
+                const int32_t *__restrict__ pre, const int32_t *__restrict__ pstart,
+                const unsigned long long *__restrict__ pw, const int64_t *__restrict__ maxp,
+                const int32_t *__restrict__ vwgt, int32_t *__restrict__ P,
                 int32_t *__restrict__ sp, int32_t *__restrict__ d_np, unsigned long long *tile_status,
                 int64_t half, hp::LbCtl *lb, unsigned *status)
 {
@@ -1716,7 +1729,11 @@ rs_evict_kernel(const int32_t *__restrict__ K, const int32_t *__restrict__ V, co
 #pragma unroll
         for (int q = 0; q < RK_ITEMS; q++) {
             const int64_t i = i0 + q;
-            f[q] = i < cnt && i < ev_end[K[i] >> 6];
+            f[q] = false;
+            if (i < cnt) {
+                const int32_t p = K[i] >> 6;
+                f[q] = (int64_t)pre[i] - pre[pstart[p]] < (int64_t)pw[p] - maxp[p];
+            }
             w[q] = f[q] ? vwgt[V[i]] : 0;
             nf += f[q];
             sw += w[q];
@@ -1853,7 +1870,7 @@ __device__ void cookie_cut_warp(int32_t k, const unsigned long long *__restrict_
 __global__ void rs_assign_kernel(int32_t k, const int32_t *__restrict__ P, const int32_t *__restrict__ d_np,
                                  const int32_t *__restrict__ V, const int32_t *__restrict__ es,
                                  const int32_t *__restrict__ ee, const int32_t *__restrict__ where,
-                                 int32_t *__restrict__ dest, MoveSink ms)
+                                 int32_t *__restrict__ dest, const int32_t *__restrict__ pregain, MoveSink ms)
 {
     hp::pdl_wait();
     const int32_t np = *d_np;
@@ -1871,7 +1888,9 @@ __global__ void rs_assign_kernel(int32_t k, const int32_t *__restrict__ P, const
         const int32_t from = where[v];
         if (j < ee[p] && p != from) {
             dest[v] = p;
-            c1 += move_append(ms, v, from, p);
+            move_append(ms, v, from);
+            const int32_t o = ms.goff[v], len = ms.goff[v + 1] - o;
+            c1 += (long long)row_conn(ms.gpart + o, ms.gconn + o, len, p, ms.k) + pregain[v];
         }
     }
     hp::block_add_to<256>(c1, ms.d_c1);
@@ -1892,7 +1911,7 @@ struct RefineBufs {
     int32_t *jlist, *joff;                 // its listed vertices and their row prefix
     unsigned long long *ab_acc2;           // learned-candidate sums of the hub rows
     int32_t *K, *V, *K2, *V2, *pre, *P, *sp;
-    int32_t *pstart, *pend, *und, *ev_end, *es, *ee;
+    int32_t *pstart, *und, *es, *ee;
     int8_t *ufl;   // per part: pw < maxp (a weak pass's destination rule), set by ctl_begin
     unsigned long long *pw;
     const int64_t *opt, *maxp;
@@ -2001,13 +2020,13 @@ int rank_candidates(hp_context *c, HpLevel &g, RefineBufs &B, int32_t k, int32_t
     const int64_t rt = ((int64_t)n + RK_TILE) / RK_TILE;   // a tile holds index cnt <= n
     if (ct > c->lb_cap || 2 * rt > c->lb_cap) return HP_ERR_INTERNAL;
     HP_LAUNCH(c, rb_candidates_kernel<STRONG>, (unsigned)ct, RB_TILE, 0, n, g.where, g.vwgt, B.pw, B.maxp, B.opt,
-              B.goff, B.gpart, B.gconn, B.und, (const int32_t *)&sc[S_NU], k, B.K, B.V, B.dest, d_cnt, B.pstart,
-              B.pend, c->lb_status, c->lb_ctl, c->d_status, B.ufl, bcp);
+              B.goff, B.gpart, B.gconn, B.und, (const int32_t *)&sc[S_NU], k, B.K, B.V, B.dest, d_cnt,
+              c->lb_status, c->lb_ctl, c->d_status, B.ufl, B.pregain, bcp);
     bool in_tmp = false;
     HP_TRY(hp_sort_pairs(c, B.K, B.V, B.K2, B.V2, n, d_cnt, key_bits_for(k), &in_tmp));
     *Ks = in_tmp ? B.K2 : B.K;
     *Vs = in_tmp ? B.V2 : B.V;
-    HP_LAUNCH(c, rb_rank_kernel, rank_grid(c, rt), RK_THREADS, 0, *Ks, *Vs, d_cnt, g.vwgt, B.pre, B.pstart, B.pend,
+    HP_LAUNCH(c, rb_rank_kernel, rank_grid(c, rt), RK_THREADS, 0, *Ks, *Vs, d_cnt, g.vwgt, B.pre, B.pstart,
               c->lb_status, c->lb_ctl, c->d_status);
     return HP_OK;
 }
@@ -2025,7 +2044,7 @@ int weak_rebalance(hp_context *c, HpLevel &g, RefineBufs &B, int32_t k, const Be
     int32_t *Ks, *Vs;
     HP_TRY(rank_candidates<false>(c, g, B, k, &Ks, &Vs, bcp));
     HP_LAUNCH(c, rw_select_kernel, (unsigned)(c->sm_count * 8), 256, 0, Ks, Vs,
-              (const int32_t *)&sc[S_LISTCNT], B.pre, B.pstart, B.pw, B.maxp, B.dest, move_sink(c, B, k));
+              (const int32_t *)&sc[S_LISTCNT], B.pre, B.pstart, B.pw, B.maxp, B.pregain, move_sink(c, B, k));
     return HP_OK;
 }
 
@@ -2038,13 +2057,13 @@ int strong_rebalance(hp_context *c, HpLevel &g, RefineBufs &B, int32_t k, const 
     const unsigned pg = (unsigned)(c->sm_count * 8);
     const int32_t *d_cnt = (const int32_t *)&sc[S_LISTCNT];
     int32_t *d_np = (int32_t *)&sc[S_NP];
-    HP_LAUNCH(c, evict_end_kernel, nblk(k), 256, 0, k, B.pstart, B.pend, B.pre, B.pw, B.maxp, B.ev_end);
     const int64_t rt = ((int64_t)n + RK_TILE) / RK_TILE;
-    HP_LAUNCH(c, rs_evict_kernel, rank_grid(c, rt), RK_THREADS, 0, Ks, Vs, d_cnt, B.ev_end, g.vwgt, B.P, B.sp, d_np,
+    HP_LAUNCH(c, rs_evict_kernel, rank_grid(c, rt), RK_THREADS, 0, Ks, Vs, d_cnt, B.pre, B.pstart, B.pw,
+              B.maxp, g.vwgt, B.P, B.sp, d_np,
               c->lb_status, c->lb_cap / 2, c->lb_ctl, c->d_status);
     HP_LAUNCH(c, cookie_cutter_kernel, 1, 1024, sizeof(int32_t) * COOKIE_SMEM_INTS, k, B.pw, B.maxp, B.sp, d_np,
               B.es, B.ee);
-    HP_LAUNCH(c, rs_assign_kernel, pg, 256, 0, k, B.P, d_np, Vs, B.es, B.ee, g.where, B.dest,
+    HP_LAUNCH(c, rs_assign_kernel, pg, 256, 0, k, B.P, d_np, Vs, B.es, B.ee, g.where, B.dest, B.pregain,
               move_sink(c, B, k));
     return HP_OK;
 }
@@ -2147,8 +2166,7 @@ pass_end_kernel(const int32_t *__restrict__ moves, const unsigned long long *d_n
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nm; i += (int64_t)gridDim.x * blockDim.x) {
         const int32_t v = moves[i];
         const int32_t o = goff[v], len = goff[v + 1] - o;
-        acc += (long long)row_conn(gpart + o, gconn + o, len, where[v], k) -
-               row_conn(gpart + o, gconn + o, len, oldp[i], k);
+        acc += row_diff(gpart + o, gconn + o, len, where[v], oldp[i], k);
     }
     hp::block_add_to<256>(acc, &sc[S_C2]);   // ends with a barrier
     if (threadIdx.x == 0) {
@@ -2777,11 +2795,9 @@ refine_cluster_kernel(SmallLevel a)
         if (!a.coarser) {   // the coarsest level: the cut from the gain rows
             for (int32_t v = vb + lane; v < ve; v += 32) {
                 const int32_t p = a.where[v], o = a.goff[v], len = a.goff[v + 1] - o;
-                for (int32_t j = o; j < o + len; j++) {
-                    const int32_t q = a.gpart[j];
-                    if (q < 0) break;
-                    if (q != p) cut[0] += a.gconn[j];
-                }
+                row_walk(a.gpart, a.gconn, o, len, [&](int32_t q, int32_t cq) {
+                    if (q != p) cut[0] += cq;
+                });
             }
         }
         cl_sum<1>(cut, X, buf, rank, nct);
@@ -2979,13 +2995,10 @@ refine_cluster_kernel(SmallLevel a)
                     int32_t b = -1;
                     const bool coop = cand && len > RB_COOP;
                     if (cand && !coop)
-                        for (int32_t j = o; j < o + len; j++) {
-                            const int32_t q = a.gpart[j];
-                            if (q < 0) break;
-                            const int32_t cq = a.gconn[j];
+                        row_walk(a.gpart, a.gconn, o, len, [&](int32_t q, int32_t cq) {
                             if (q == p) pc = cq;
-                            if (s_ufl[q] && cq > bc) { bc = cq; b = q; }
-                        }
+                            if (cq > bc && s_ufl[q]) { bc = cq; b = q; }
+                        });
                     unsigned cm = __ballot_sync(HP_FULL_MASK, coop);
                     while (cm) {
                         const int src = __ffs(cm) - 1;
@@ -3211,8 +3224,7 @@ refine_cluster_kernel(SmallLevel a)
             for (int32_t i = gtid; i < nmoves; i += gt) {
                 const int32_t v = a.moves[i];
                 const int32_t o = a.goff[v], len = a.goff[v + 1] - o;
-                c[1] += (long long)row_conn(a.gpart + o, a.gconn + o, len, a.where[v], k) -
-                        row_conn(a.gpart + o, a.gconn + o, len, a.oldp[i], k);
+                c[1] += row_diff(a.gpart + o, a.gconn + o, len, a.where[v], a.oldp[i], k);
             }
         }
         long long m = LLONG_MIN;
@@ -3397,7 +3409,7 @@ int refine_level(hp_context *c, HpLevel &g, int32_t k, bool finest, const int64_
                             &B.small_l, &B.big_l, &B.best_where, &B.K, &B.V, &B.K2, &B.V2, &B.pre,
                             &B.P, &B.sp, &B.huge_mv, &B.huge, &B.recof};
     for (auto pp : n_arrays) *pp = ralloc_t<int32_t>(c, (int64_t)n + 1);
-    int32_t **k_arrays[] = {&B.pstart, &B.pend, &B.und, &B.ev_end, &B.es, &B.ee};
+    int32_t **k_arrays[] = {&B.pstart, &B.und, &B.es, &B.ee};
     for (auto pp : k_arrays) *pp = ralloc_t<int32_t>(c, k);
     B.lock = ralloc_t<int8_t>(c, n);
     B.prune = ralloc_t<int8_t>(c, n);
