@@ -1131,6 +1131,13 @@ HP_API int hp_test_arena_restarts(hp_context *ctx)
     return ctx->arena_restarts;
 }
 
+HP_API int hp_test_wide_rows(hp_context *ctx, int32_t on)
+{
+    if (!ctx) return HP_ERR_INVALID_ARG;
+    ctx->wide_rows = on != 0;
+    return HP_OK;
+}
+
 // ---- legacy drop-in ------------------------------------------------------------------
 static std::mutex g_legacy_mu;
 static hp_context *g_legacy = nullptr;

@@ -15,8 +15,10 @@
 //                         thread's bitonic network in registers, written in
 //                         place by one ordered pass with a decoupled look-back
 //                         that also produces the coarse xadj
-//        33..256          one warp, LSD radix sort in shared memory
-//        257..4096        one CTA of 256, LSD radix sort in shared memory
+//        33..1024         one warp, bitonic network in registers (an LSD radix
+//                         sort in shared memory where the coarse ids leave no
+//                         room for the entry's index in 32 bits)
+//        1025..4096       one CTA of 128 or 256, LSD radix sort in shared memory
 //        4097..12288      one CTA of 1024, LSD radix sort in shared memory
 //        larger           one CTA, dense accumulator + presence bitmap
 //        (a level whose coarse ids fit contract_smem_cn merges every long row
@@ -686,12 +688,257 @@ struct ContractSrc {
     }
 };
 
+template <int G>
+__device__ __forceinline__ void group_sync()
+{
+    if (G == 32) __syncwarp();
+    else __syncthreads();
+}
+
+// Two exclusive scans across a group in one pass (a: int, b: wrapping uint32).
+template <int G>
+__device__ __forceinline__ void group_excl_scan2(int a, uint32_t b, int *ea, uint32_t *eb, int *ta, uint32_t *tb,
+                                                 int32_t *s_scan /* 2 * (G/32) + 2 */)
+{
+    const int lane = threadIdx.x & 31;
+    int ia = a;
+    uint32_t ib = b;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int xa = __shfl_up_sync(HP_FULL_MASK, ia, o);
+        const uint32_t xb = __shfl_up_sync(HP_FULL_MASK, ib, o);
+        if (lane >= o) { ia += xa; ib += xb; }
+    }
+    if (G == 32) {
+        *ta = __shfl_sync(HP_FULL_MASK, ia, 31);
+        *tb = __shfl_sync(HP_FULL_MASK, ib, 31);
+        *ea = ia - a;
+        *eb = ib - b;
+        return;
+    }
+    constexpr int W = G / 32;
+    const int wid = (threadIdx.x % G) >> 5;
+    if (lane == 31) { s_scan[wid] = ia; s_scan[W + wid] = (int32_t)ib; }
+    __syncthreads();
+    if (wid == 0) {
+        int t = lane < W ? s_scan[lane] : 0;
+        uint32_t u = lane < W ? (uint32_t)s_scan[W + lane] : 0u;
+        int ti = t;
+        uint32_t ui = u;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int xa = __shfl_up_sync(HP_FULL_MASK, ti, o);
+            const uint32_t xb = __shfl_up_sync(HP_FULL_MASK, ui, o);
+            if (lane >= o) { ti += xa; ui += xb; }
+        }
+        if (lane < W) { s_scan[lane] = ti - t; s_scan[W + lane] = (int32_t)(ui - u); }
+        if (lane == W - 1) { s_scan[2 * W] = ti; s_scan[2 * W + 1] = (int32_t)ui; }
+    }
+    __syncthreads();
+    *ea = s_scan[wid] + ia - a;
+    *eb = (uint32_t)s_scan[W + wid] + ib - b;
+    *ta = s_scan[2 * W];
+    *tb = (uint32_t)s_scan[2 * W + 1];
+    __syncthreads();
+}
+
 // ---- short rows: one thread per coarse row, aggregation in registers ------------
-// The row's entries come from the tile's staging buffer (packed key << 32 |
+// The row's entries come from the tile's staging buffer as words (key << ASM_IDX |
+// index in the row, the self key already WORD_NONE) with the weights beside them.  A
+// bitonic network of NET sorts the words; the weights of equal keys are summed into
+// the slot of the run's first entry, and the unique keys are counted.  A comparator is
+// two instructions instead of six on 64-bit entries, which the kernel was bound by:
+// RGG of 2^24 vertices, level 0 8.1 -> 5.9 ms, 128^3 grid 0.26 -> 0.23 ms.
+constexpr int ASM_IDX = 5;                                   // a short row has at most 32 entries
+constexpr int32_t ASM_KEY_MAX = (1 << (32 - ASM_IDX)) - 1;   // coarse ids below it fit a word
+
+template <int NET, int XN>
+__device__ __forceinline__ int sort_staged_row(const unsigned *key, int32_t *wgt, int32_t len, unsigned (&x)[XN])
+{
+#pragma unroll
+    for (int i = 0; i < NET; i++) x[i] = i < len ? key[i] : hp::WORD_NONE;
+    hp::sort_words<NET, XN>(x);
+    int u = 0;
+    int32_t acc = 0;          // weight of the entries after i that have its key
+    bool same_next = false;   // entry i + 1 has the key of entry i
+#pragma unroll
+    for (int b = NET - 8; b >= 0; b -= 8) {   // eight weights in flight
+        int32_t w[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) w[q] = wgt[x[b + q] == hp::WORD_NONE ? 0 : x[b + q] & ((1u << ASM_IDX) - 1u)];
+#pragma unroll
+        for (int q = 7; q >= 0; q--) {
+            const int i = b + q;
+            const bool same = i > 0 && (x[i] ^ x[i > 0 ? i - 1 : 0]) < (1u << ASM_IDX);   // the key of entry i - 1
+            const bool valid = x[i] != hp::WORD_NONE;
+            acc += w[q];
+            if (!same && valid && same_next) wgt[x[i] & ((1u << ASM_IDX) - 1u)] = acc;
+            u += valid && !same;
+            if (!same) acc = 0;
+            same_next = same && valid;
+        }
+    }
+    return u;
+}
+
+// The first word of every run of the sorted row into out[0..u), each tagged with the
+// tile row t; the run's weight is at the word's index of the row's staged weights.
+template <int NET, int XN>
+__device__ __forceinline__ void emit_staged_row(const unsigned (&x)[XN], unsigned *out, uint8_t *orow, uint8_t t)
+{
+    int r = 0;
+#pragma unroll
+    for (int i = 0; i < NET; i++) {
+        const bool same = i > 0 && (x[i] ^ x[i > 0 ? i - 1 : 0]) < (1u << ASM_IDX);
+        if (x[i] == hp::WORD_NONE || same) continue;
+        out[r] = x[i];
+        orow[r] = t;
+        r++;
+    }
+}
+
+// Coarse CSR assembly in one ordered pass: tiles of ASM_TILE coarse rows are
+// taken in order (dynamic tile counter).  The tile's short rows are staged in
+// shared memory: consecutive threads load consecutive entries of the rows (the
+// row reads coalesce, the cmap gathers of one row hit neighbouring ids), each
+// thread then sorts its row in registers (network of 8, 16 or 32 by the
+// longest short row in the warp) or takes the unique count of a long row
+// aggregated before; a block scan plus a decoupled look-back across tiles gives
+// every row its final offset; the merged short rows go back through shared
+// memory and are written with consecutive threads on consecutive entries.
+// cxadj is written directly, with no second scan and no compaction copy; long
+// rows are placed afterwards by copy_long_rows_kernel.
+constexpr int ASM_TILE = 256;
+
+// Dynamic shared memory: ASM_TILE * XN staged words, weights and tile rows.
+template <int XN>
+constexpr size_t asm_smem_bytes()
+{
+    return (sizeof(unsigned) + sizeof(int32_t) + sizeof(uint8_t)) * (size_t)ASM_TILE * XN;
+}
+
+// XN: the longest network the level needs (8, 16 or 32; the host reads the
+// longest short row) -- every short row has at most XN entries.
+template <int XN>
+__global__ void __launch_bounds__(ASM_TILE)
+contract_assemble_kernel(int32_t cn, ContractSrc src, const int32_t *__restrict__ ucnt,
+                         int32_t *__restrict__ cxadj, int32_t *__restrict__ cadjncy,
+                         int32_t *__restrict__ cadjwgt, unsigned long long *tile_status, hp::LbCtl *lb,
+                         unsigned *status, int32_t thread_row, int wcheck)
+{
+    hp::pdl_wait();
+    extern __shared__ unsigned asm_words[];                                  // ASM_TILE * XN, in and out
+    int32_t *s_wgt = reinterpret_cast<int32_t *>(asm_words + ASM_TILE * XN);   // staged weights, then run sums
+    uint8_t *s_row = reinterpret_cast<uint8_t *>(s_wgt + ASM_TILE * XN);       // tile row of each word
+    __shared__ int4 s_ri[ASM_TILE];
+    __shared__ int32_t s_off[ASM_TILE];     // staged offset of the row's input
+    __shared__ int32_t s_goff[ASM_TILE];    // the row's final offset minus the staged offset of its output
+    __shared__ int32_t s_scan[2 * (ASM_TILE / 32) + 2];
+    __shared__ int32_t s_excl;
+    int64_t tile;
+    unsigned epoch;
+    hp::lb_begin(lb, &tile, &epoch);
+    const int t = threadIdx.x;
+    const int32_t c0 = (int32_t)(tile * ASM_TILE);
+    const int32_t c = c0 + t;
+    RowInfo r{0, 0, 0, 0};
+    int32_t len = 0;
+    if (c < cn) src.row(c, r, len);
+    const bool small = c < cn && len <= thread_row;
+    int tin;
+    const int ioff = hp::block_excl_scan<ASM_TILE>(small ? len : 0, &tin, s_scan);
+    s_ri[t] = make_int4(r.s0, r.l0, r.s1, r.l1);
+    s_off[t] = ioff;
+    if (small)
+        for (int i = 0; i < len; i++) s_row[ioff + i] = (uint8_t)t;
+    __syncthreads();
+    // stage: four entries per thread in flight (row reads, then the cmap gathers)
+    for (int f0 = t; f0 < tin; f0 += 4 * ASM_TILE) {
+        int32_t a[4], w[4], rt[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int f = f0 + q * ASM_TILE;
+            rt[q] = -1;
+            a[q] = 0;
+            w[q] = 0;
+            if (f < tin) {
+                rt[q] = s_row[f];
+                const int4 ri = s_ri[rt[q]];
+                const int i = f - s_off[rt[q]];
+                const int32_t j = i < ri.y ? ri.x + i : ri.z + (i - ri.y);
+                a[q] = src.adjncy[j];
+                w[q] = src.adjwgt[j];
+            }
+        }
+        int32_t kq[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) kq[q] = rt[q] >= 0 ? src.cmap[a[q]] : 0;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            if (rt[q] < 0) continue;
+            const int32_t k = kq[q];
+            const int f = f0 + q * ASM_TILE;
+            asm_words[f] = k == c0 + rt[q] ? hp::WORD_NONE : ((unsigned)k << ASM_IDX) | (unsigned)(f - s_off[rt[q]]);
+            s_wgt[f] = w[q];
+        }
+    }
+    __syncthreads();
+    if (wcheck && small) {
+        // the coarse row's weighted degree (weight range, row_weight_range_kernel)
+        long long ws = 0;
+        for (int i = 0; i < len; i++) {
+            if (asm_words[ioff + i] != hp::WORD_NONE) ws += s_wgt[ioff + i];
+        }
+        if (ws >= (long long)INT32_MAX) atomicOr(status, HP_STATUS_WEIGHT_RANGE);
+    }
+    const unsigned wmax = __reduce_max_sync(HP_FULL_MASK, small ? (unsigned)len : 0u);
+    unsigned x[XN];
+    int u = 0;
+    if (c < cn && !small) u = ucnt[c];
+    if (XN == 8 || wmax <= 8) {
+        if (small) u = sort_staged_row<8, XN>(asm_words + ioff, s_wgt + ioff, len, x);
+    } else if (XN == 16 || wmax <= 16) {
+        if (small) u = sort_staged_row<(XN < 16 ? XN : 16), XN>(asm_words + ioff, s_wgt + ioff, len, x);
+    } else {
+        if (small) u = sort_staged_row<XN, XN>(asm_words + ioff, s_wgt + ioff, len, x);
+    }
+    int ooff, tout;
+    uint32_t local, agg;
+    group_excl_scan2<ASM_TILE>(small ? u : 0, (uint32_t)u, &ooff, &local, &tout, &agg, s_scan);   // (the staged words are read)
+    if (t < 32) {
+        const int32_t excl = hp::lookback_epoch(tile_status, tile, (int32_t)agg, epoch, status);
+        if (t == 0) s_excl = excl;
+    }
+    if (small) {
+        if (XN == 8 || wmax <= 8) emit_staged_row<8, XN>(x, asm_words + ooff, s_row + ooff, (uint8_t)t);
+        else if (XN == 16 || wmax <= 16)
+            emit_staged_row<(XN < 16 ? XN : 16), XN>(x, asm_words + ooff, s_row + ooff, (uint8_t)t);
+        else emit_staged_row<XN, XN>(x, asm_words + ooff, s_row + ooff, (uint8_t)t);
+    }
+    __syncthreads();
+    const int32_t off = s_excl + (int32_t)local;
+    s_goff[t] = off - ooff;
+    if (c < cn) {
+        cxadj[c] = off;
+        if (c == cn - 1) cxadj[cn] = off + u;
+    }
+    __syncthreads();
+    for (int f = t; f < tout; f += ASM_TILE) {
+        const int rt = s_row[f];
+        const int32_t pos = s_goff[rt] + f;
+        const unsigned e = asm_words[f];
+        cadjncy[pos] = (int32_t)(e >> ASM_IDX);
+        cadjwgt[pos] = s_wgt[s_off[rt] + (int)(e & ((1u << ASM_IDX) - 1u))];
+    }
+    hp::lb_end(lb);
+}
+
+// The same with 64-bit entries, for levels of ASM_KEY_MAX coarse vertices or more:
+// the row's entries come from the tile's staging buffer (packed key << 32 |
 // weight, the self key already PACK_NONE); a bitonic network of NET sorts them
 // and the unique keys are counted.
 template <int NET, int XN>
-__device__ __forceinline__ int sort_staged_row(const unsigned long long *stage, int32_t len,
+__device__ __forceinline__ int sort_wide_row(const unsigned long long *stage, int32_t len,
                                                unsigned long long (&x)[XN])
 {
 #pragma unroll
@@ -710,7 +957,7 @@ __device__ __forceinline__ int sort_staged_row(const unsigned long long *stage, 
 // The sorted row merged (weights of equal keys summed) into out[0..u), each
 // entry tagged with the tile row t.
 template <int NET, int XN>
-__device__ __forceinline__ void emit_staged_row(const unsigned long long (&x)[XN], unsigned long long *out,
+__device__ __forceinline__ void emit_wide_row(const unsigned long long (&x)[XN], unsigned long long *out,
                                                 uint8_t *orow, uint8_t t)
 {
     int r = -1;
@@ -734,31 +981,9 @@ __device__ __forceinline__ void emit_staged_row(const unsigned long long (&x)[XN
     if (r >= 0) out[r] = ((unsigned long long)prev << 32) | (uint32_t)acc;
 }
 
-// Coarse CSR assembly in one ordered pass: tiles of ASM_TILE coarse rows are
-// taken in order (dynamic tile counter).  The tile's short rows are staged in
-// shared memory: consecutive threads load consecutive entries of the rows (the
-// row reads coalesce, the cmap gathers of one row hit neighbouring ids), each
-// thread then sorts its row in registers (network of 8, 16 or 32 by the
-// longest short row in the warp) or takes the unique count of a long row
-// aggregated before; a block scan plus a decoupled look-back across tiles gives
-// every row its final offset; the merged short rows go back through shared
-// memory and are written with consecutive threads on consecutive entries.
-// cxadj is written directly, with no second scan and no compaction copy; long
-// rows are placed afterwards by copy_long_rows_kernel.
-constexpr int ASM_TILE = 256;
-
-// Dynamic shared memory: ASM_TILE * XN staged entries and their tile rows.
-template <int XN>
-constexpr size_t asm_smem_bytes()
-{
-    return (sizeof(unsigned long long) + sizeof(uint8_t)) * (size_t)ASM_TILE * XN;
-}
-
-// XN: the longest network the level needs (8, 16 or 32; the host reads the
-// longest short row) -- every short row has at most XN entries.
 template <int XN>
 __global__ void __launch_bounds__(ASM_TILE)
-contract_assemble_kernel(int32_t cn, ContractSrc src, const int32_t *__restrict__ ucnt,
+contract_assemble_wide_kernel(int32_t cn, ContractSrc src, const int32_t *__restrict__ ucnt,
                          int32_t *__restrict__ cxadj, int32_t *__restrict__ cadjncy,
                          int32_t *__restrict__ cadjwgt, unsigned long long *tile_status, hp::LbCtl *lb,
                          unsigned *status, int32_t thread_row, int wcheck)
@@ -832,11 +1057,11 @@ contract_assemble_kernel(int32_t cn, ContractSrc src, const int32_t *__restrict_
     int u = 0;
     if (c < cn && !small) u = ucnt[c];
     if (XN == 8 || wmax <= 8) {
-        if (small) u = sort_staged_row<8, XN>(asm_stage + ioff, len, x);
+        if (small) u = sort_wide_row<8, XN>(asm_stage + ioff, len, x);
     } else if (XN == 16 || wmax <= 16) {
-        if (small) u = sort_staged_row<(XN < 16 ? XN : 16), XN>(asm_stage + ioff, len, x);
+        if (small) u = sort_wide_row<(XN < 16 ? XN : 16), XN>(asm_stage + ioff, len, x);
     } else {
-        if (small) u = sort_staged_row<XN, XN>(asm_stage + ioff, len, x);
+        if (small) u = sort_wide_row<XN, XN>(asm_stage + ioff, len, x);
     }
     int agg, tout;
     const int local = hp::block_excl_scan<ASM_TILE>(u, &agg, s_scan);   // (the staged input is read)
@@ -846,10 +1071,10 @@ contract_assemble_kernel(int32_t cn, ContractSrc src, const int32_t *__restrict_
         if (t == 0) s_excl = excl;
     }
     if (small) {
-        if (XN == 8 || wmax <= 8) emit_staged_row<8, XN>(x, asm_stage + ooff, s_row + ooff, (uint8_t)t);
+        if (XN == 8 || wmax <= 8) emit_wide_row<8, XN>(x, asm_stage + ooff, s_row + ooff, (uint8_t)t);
         else if (XN == 16 || wmax <= 16)
-            emit_staged_row<(XN < 16 ? XN : 16), XN>(x, asm_stage + ooff, s_row + ooff, (uint8_t)t);
-        else emit_staged_row<XN, XN>(x, asm_stage + ooff, s_row + ooff, (uint8_t)t);
+            emit_wide_row<(XN < 16 ? XN : 16), XN>(x, asm_stage + ooff, s_row + ooff, (uint8_t)t);
+        else emit_wide_row<XN, XN>(x, asm_stage + ooff, s_row + ooff, (uint8_t)t);
     }
     s_off[t] = ooff;
     __syncthreads();
@@ -927,13 +1152,6 @@ copy_long_rows_kernel(const int32_t *__restrict__ lists, const int32_t *__restri
 // digit-major order (digit d of warp w before digit d of warp w+1), and a stable
 // scatter in which each warp walks its contiguous chunk 32 items at a time and
 // ranks equal digits with __match_any_sync.
-template <int G>
-__device__ __forceinline__ void group_sync()
-{
-    if (G == 32) __syncwarp();
-    else __syncthreads();
-}
-
 // Exclusive scan across the G threads of a group (one value per thread).
 template <int G>
 __device__ __forceinline__ int group_excl_scan(int v, int *total, int32_t *s_scan /* G/32 + 1 */)
@@ -958,51 +1176,6 @@ __device__ __forceinline__ int group_excl_scan(int v, int *total, int32_t *s_sca
     *total = s_scan[G / 32];
     __syncthreads();
     return r;
-}
-
-// Two exclusive scans across a group in one pass (a: int, b: wrapping uint32).
-template <int G>
-__device__ __forceinline__ void group_excl_scan2(int a, uint32_t b, int *ea, uint32_t *eb, int *ta,
-                                                 int32_t *s_scan /* 2 * (G/32) + 2 */)
-{
-    const int lane = threadIdx.x & 31;
-    int ia = a;
-    uint32_t ib = b;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int xa = __shfl_up_sync(HP_FULL_MASK, ia, o);
-        const uint32_t xb = __shfl_up_sync(HP_FULL_MASK, ib, o);
-        if (lane >= o) { ia += xa; ib += xb; }
-    }
-    if (G == 32) {
-        *ta = __shfl_sync(HP_FULL_MASK, ia, 31);
-        *ea = ia - a;
-        *eb = ib - b;
-        return;
-    }
-    constexpr int W = G / 32;
-    const int wid = (threadIdx.x % G) >> 5;
-    if (lane == 31) { s_scan[wid] = ia; s_scan[W + wid] = (int32_t)ib; }
-    __syncthreads();
-    if (wid == 0) {
-        int t = lane < W ? s_scan[lane] : 0;
-        uint32_t u = lane < W ? (uint32_t)s_scan[W + lane] : 0u;
-        int ti = t;
-        uint32_t ui = u;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int xa = __shfl_up_sync(HP_FULL_MASK, ti, o);
-            const uint32_t xb = __shfl_up_sync(HP_FULL_MASK, ui, o);
-            if (lane >= o) { ti += xa; ui += xb; }
-        }
-        if (lane < W) { s_scan[lane] = ti - t; s_scan[W + lane] = (int32_t)(ui - u); }
-        if (lane == W - 1) s_scan[2 * W] = ti;
-    }
-    __syncthreads();
-    *ea = s_scan[wid] + ia - a;
-    *eb = (uint32_t)s_scan[W + wid] + ib - b;
-    *ta = s_scan[2 * W];
-    __syncthreads();
 }
 
 // Sorts A[0..N) (result in A; B is scratch of the same size); hist holds
@@ -1074,8 +1247,8 @@ __device__ int group_merge_emit(const unsigned long long *A, int N, int32_t *out
         wsum += (uint32_t)A[i];
     }
     int o0, U;
-    uint32_t p0;
-    group_excl_scan2<G>(heads, wsum, &o0, &p0, &U, s_scan);
+    uint32_t p0, wtot;
+    group_excl_scan2<G>(heads, wsum, &o0, &p0, &U, &wtot, s_scan);
     int o = o0 - 1;   // ordinal of the current run
     uint32_t p = p0;  // weights before entry i
     for (int i = lo; i < hi; i++) {
@@ -1163,6 +1336,133 @@ __device__ void group_weight_range(long long wpart, long long *s64, unsigned *st
         if (tot >= (long long)INT32_MAX) atomicOr(status, HP_STATUS_WEIGHT_RANGE);
     }
     group_sync<G>();
+}
+
+// ---- rows of up to 1024 entries: one warp, a register network ---------------------
+// What bounds these rows is the sort.  The LSD radix sort of a row (a pass per 8 key
+// bits: histogram, scan of 256 counters, ranked scatter) is a chain of shared-memory
+// round trips whatever the row's length.  A bitonic network over 32-bit words (key and
+// index, hp::warp_sort_words) has no counters and no shared memory, NR independent
+// operations a lane in every step, and its size follows the row: NR = 2, 4, ... 32
+// words a lane for rows of up to 64, 128, ... 1024 entries.  The weights wait in shared
+// memory and are fetched by the sorted words' indexes; a run's weight is the difference
+// of two prefixes (wrapping 32-bit; every run sum is itself an int32 edge weight).
+// Key and index must fit 32 bits, else the row takes the radix sort.  Contraction of
+// R-MAT scale 22 (with the 32-bit network of the short rows): level 0 9.9 -> 7.5 ms,
+// level 1 7.9 -> 5.9; a row of 300-1000 entries is also cheaper here than in the
+// shared-memory and hybrid accumulators below (scale 20, 92K coarse ids: 3.0 -> 1.5 ms
+// a level), which hold a whole SM per row.
+constexpr int WS_SHORT_WARPS = 8, WS_SHORT_NR = 8;    // rows of up to 256 entries
+constexpr int WS_LONG_WARPS = 4, WS_LONG_NR = 32;     // rows of up to 1024 entries
+
+constexpr int ws_idx_bits(int nr) { return nr <= 1 ? 5 : 1 + ws_idx_bits(nr / 2); }
+constexpr int ws_buf(int nr) { return 33 * nr + 1; }   // 32 nr + 1 words, one pad every 32
+
+// Row c (len <= 32 * NR entries), gathered, sorted, merged and written to
+// out_k / out_w in ascending order; returns the unique count (all lanes).  buf:
+// 2 * ws_buf(NR) words.
+template <int NR>
+__device__ int warp_sort_row(const ContractSrc &src, int32_t c, const RowInfo &r, int32_t len, uint32_t *buf,
+                             int32_t *__restrict__ out_k, int32_t *__restrict__ out_w, int wcheck, unsigned *status)
+{
+    constexpr int IDX = ws_idx_bits(NR);
+    constexpr int D = NR < 8 ? NR : 8;   // loads of a lane in flight: the entries, then their coarse ids
+    const int lane = threadIdx.x & 31;
+    uint32_t *pre = buf, *sk = buf + ws_buf(NR);   // pre holds the weights until the sorted words fetched them
+    unsigned x[NR];
+    long long ws = 0;
+#pragma unroll
+    for (int b = 0; b < NR; b += D) {
+        if (b * 32 >= len) {   // (uniform over the warp)
+#pragma unroll
+            for (int q = 0; q < D; q++) x[b + q] = hp::WORD_NONE;
+            continue;
+        }
+        int32_t a[D], w[D];
+#pragma unroll
+        for (int q = 0; q < D; q++) {
+            const int i = (b + q) * 32 + lane;
+            const int32_t j = i < r.l0 ? r.s0 + i : r.s1 + (i - r.l0);
+            a[q] = i < len ? src.adjncy[j] : -1;
+            w[q] = i < len ? src.adjwgt[j] : 0;
+        }
+#pragma unroll
+        for (int q = 0; q < D; q++) {
+            const int i = (b + q) * 32 + lane;
+            const int32_t k = a[q] >= 0 ? src.cmap[a[q]] : c;
+            x[b + q] = k == c ? hp::WORD_NONE : ((unsigned)k << IDX) | (unsigned)i;
+            if (k != c) ws += w[q];
+            pre[i] = (uint32_t)w[q];
+        }
+    }
+    if (wcheck) group_weight_range<32>(ws, nullptr, status);
+    __syncwarp();
+    hp::warp_sort_words<NR>(x);
+    uint32_t w[NR];
+    const unsigned last = __shfl_up_sync(HP_FULL_MASK, x[NR - 1], 1);
+    unsigned heads = 0u;   // bit q: word q starts a run
+    uint32_t wsum = 0;
+#pragma unroll
+    for (int q = 0; q < NR; q++) {
+        const unsigned prev = q > 0 ? x[q > 0 ? q - 1 : 0] : (lane > 0 ? last : hp::WORD_NONE);
+        const bool valid = x[q] != hp::WORD_NONE;
+        w[q] = valid ? pre[x[q] & ((1u << IDX) - 1u)] : 0u;
+        if (valid && (x[q] >> IDX) != (prev >> IDX)) heads |= 1u << q;
+        wsum += w[q];
+    }
+    int o, U;
+    uint32_t p, wtot;
+    group_excl_scan2<32>(__popc(heads), wsum, &o, &p, &U, &wtot, nullptr);
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < NR; q++) {
+        if ((heads >> q) & 1u) {
+            sk[o + (o >> 5)] = x[q] >> IDX;
+            pre[o + (o >> 5)] = p;
+            o++;
+        }
+        p += w[q];
+    }
+    if (lane == 31) pre[U + (U >> 5)] = wtot;
+    __syncwarp();
+    for (int i = lane; i < U; i += 32) {
+        const int e = i + (i >> 5), e1 = i + 1 + ((i + 1) >> 5);
+        out_k[i] = (int32_t)sk[e];
+        out_w[i] = (int32_t)(pre[e1] - pre[e]);
+    }
+    __syncwarp();
+    return U;
+}
+
+// MAXNR: the longest rows of the list have 32 * MAXNR entries.
+template <int WARPS, int MAXNR>
+__global__ void __launch_bounds__(32 * WARPS)
+contract_warp_sort_kernel(const int32_t *__restrict__ list, const int32_t *__restrict__ d_count, ContractSrc src,
+                          const int32_t *__restrict__ toff, int32_t *__restrict__ tk, int32_t *__restrict__ tw,
+                          int32_t *__restrict__ ucnt, int wcheck, unsigned *status)
+{
+    hp::pdl_wait();
+    __shared__ uint32_t s_buf[WARPS][2 * ws_buf(MAXNR)];
+    const int wid = threadIdx.x >> 5;
+    uint32_t *buf = s_buf[wid];
+    const int32_t cnt = *d_count;
+    for (int64_t li = (int64_t)blockIdx.x * WARPS + wid; li < cnt; li += (int64_t)gridDim.x * WARPS) {
+        const int32_t c = list[li];
+        RowInfo r;
+        int32_t len;
+        src.row(c, r, len);
+        const int32_t off = toff[c];
+        int U;
+        if (MAXNR <= 8) {
+            if (len <= 64) U = warp_sort_row<2>(src, c, r, len, buf, tk + off, tw + off, wcheck, status);
+            else if (len <= 128) U = warp_sort_row<4>(src, c, r, len, buf, tk + off, tw + off, wcheck, status);
+            else U = warp_sort_row<8>(src, c, r, len, buf, tk + off, tw + off, wcheck, status);
+        } else {
+            if (len <= 512) U = warp_sort_row<16>(src, c, r, len, buf, tk + off, tw + off, wcheck, status);
+            else U = warp_sort_row<MAXNR>(src, c, r, len, buf, tk + off, tw + off, wcheck, status);
+        }
+        if ((threadIdx.x & 31) == 0) ucnt[c] = U;
+    }
 }
 
 constexpr int WROW_MAX = HP_TUNE_WARP_ROW_MAX;   // warp class: up to 256 entries
@@ -1907,43 +2207,59 @@ int contract_level(hp_context *c, HpLevel &g, int32_t cn, HpLevel &cg)
         // kbits bits of KEY_NONE and the dropped self key sorts last
         int kbits = 0;
         while ((1ll << kbits) <= (int64_t)cn) kbits++;
-        if (h.cnt[0] > 0)
+        // register networks where key and index fit a word, else the radix sorts
+        const bool words_short = !c->wide_rows && kbits + ws_idx_bits(WS_SHORT_NR) <= 32;
+        const bool words_long = !c->wide_rows && kbits + ws_idx_bits(WS_LONG_NR) <= 32;
+        if (h.cnt[0] > 0 && words_short)
+            HP_LAUNCH(c, (contract_warp_sort_kernel<WS_SHORT_WARPS, WS_SHORT_NR>),
+                      (unsigned)std::min<int64_t>((h.cnt[0] + WS_SHORT_WARPS - 1) / WS_SHORT_WARPS, c->sm_count * 8),
+                      32 * WS_SHORT_WARPS, 0, lists, &counts[0], src, toff, tk, tw, ucnt, wchk, c->d_status);
+        if (h.sub[0] > 0 && words_long)
+            HP_LAUNCH(c, (contract_warp_sort_kernel<WS_LONG_WARPS, WS_LONG_NR>),
+                      (unsigned)std::min<int64_t>((h.sub[0] + WS_LONG_WARPS - 1) / WS_LONG_WARPS, c->sm_count * 6),
+                      32 * WS_LONG_WARPS, 0, lists + 3 * (int64_t)cn, &sub_counts[0], src, toff, tk, tw, ucnt, wchk,
+                      c->d_status);
+        if (h.cnt[0] > 0 && !words_short)
             HP_LAUNCH(c, contract_warp_radix_kernel,
                       (unsigned)std::min<int64_t>((h.cnt[0] + WROW_WARPS - 1) / WROW_WARPS, c->sm_count * 6),
                       32 * WROW_WARPS, 0, lists, &counts[0], src, toff, tk, tw, ucnt, kbits, wchk, c->d_status);
         // a level whose coarse ids fit a shared-memory dense accumulator merges
         // every long row there (one atomic per entry, ordered extraction)
         const bool smem_dense = cn <= c->tune.contract_smem_cn;
+        // the lists those kernels take: the rows that a register network does not
+        const struct { int32_t list, n; int32_t *count; } accl[3] = {
+            {words_long ? 4 : 1, words_long ? h.sub[1] : h.cnt[1], words_long ? &sub_counts[1] : &counts[1]},
+            {5, words_long ? h.sub[2] : 0, &sub_counts[2]},
+            {2, h.cnt[2], &counts[2]}};
+        const int64_t acc_rows = (int64_t)accl[0].n + accl[1].n + accl[2].n;
         if (smem_dense) {
             const size_t acc = sizeof(int32_t) * ((size_t)cn + (cn + 31) / 32 + (cn + 1023) / 1024);
-            for (int cls = 1; cls <= 2; cls++)
-                if (h.cnt[cls] > 0)
-                    HP_LAUNCH(c, (contract_dense_kernel<1024, true>),
-                              (unsigned)std::min<int64_t>(h.cnt[cls], c->sm_count), 1024, acc,
-                              lists + cls * (int64_t)cn, &counts[cls], src, toff, tk, tw, ucnt, cn,
+            for (const auto &a : accl)
+                if (a.n > 0)
+                    HP_LAUNCH(c, (contract_dense_kernel<1024, true>), (unsigned)std::min<int64_t>(a.n, c->sm_count),
+                              1024, acc, lists + a.list * (int64_t)cn, a.count, src, toff, tk, tw, ucnt, cn,
                               (int32_t *)nullptr, (unsigned *)nullptr, (unsigned *)nullptr,
                               c->tune.dense_sparse_ratio, 0, wchk, c->d_status);
         }
-        // hybrid: the rows of lists 1 and 2 accumulate their low ids densely and
-        // radix-sort the rest; rows whose rest does not fit go to the spill list,
+        // hybrid: the same rows accumulate their low ids densely and radix-sort the rest; rows whose rest does not fit go to the spill list,
         // which the CTA radix (up to XROW_MAX) and dense slab kernels then take
-        const bool hybrid = !smem_dense && cn <= HY_MAX_CN && c->tune.contract_hybrid && h.cnt[1] + h.cnt[2] > 0;
+        const bool hybrid = !smem_dense && cn <= HY_MAX_CN && c->tune.contract_hybrid && acc_rows > 0;
         int32_t *spill = nullptr;
         int32_t *d_nspill = (int32_t *)&sc[4];
         if (hybrid) {
-            spill = ralloc_t<int32_t>(c, (int64_t)h.cnt[1] + h.cnt[2]);
+            spill = ralloc_t<int32_t>(c, acc_rows);
             HP_CHECK_OOM(c);
-            for (int cls = 1; cls <= 2; cls++)
-                if (h.cnt[cls] > 0)
-                    HP_LAUNCH(c, contract_hybrid_kernel, (unsigned)std::min<int64_t>(h.cnt[cls], c->sm_count),
-                              HY_THREADS, hybrid_smem(), lists + cls * (int64_t)cn, &counts[cls], src, toff, tk, tw,
-                              ucnt, kbits, 0, spill, d_nspill, wchk, c->d_status);
+            for (const auto &a : accl)
+                if (a.n > 0)
+                    HP_LAUNCH(c, contract_hybrid_kernel, (unsigned)std::min<int64_t>(a.n, c->sm_count), HY_THREADS,
+                              hybrid_smem(), lists + a.list * (int64_t)cn, a.count, src, toff, tk, tw, ucnt, kbits, 0,
+                              spill, d_nspill, wchk, c->d_status);
             HP_LAUNCH(c, (contract_cta_radix_kernel<XROW_THREADS, XROW_MAX>),
-                      (unsigned)std::min<int64_t>((int64_t)h.cnt[1] + h.cnt[2], c->sm_count), XROW_THREADS,
+                      (unsigned)std::min<int64_t>(acc_rows, c->sm_count), XROW_THREADS,
                       (cta_radix_smem<XROW_THREADS, XROW_MAX>()), spill, d_nspill, src, toff, tk, tw, ucnt, kbits, 0,
                       wchk, c->d_status);
         }
-        if (!smem_dense && !hybrid && h.sub[0] > 0)
+        if (!smem_dense && !hybrid && !words_long && h.sub[0] > 0)
             HP_LAUNCH(c, (contract_cta_radix_kernel<MROW_THREADS, MROW_MAX>),
                       (unsigned)std::min<int64_t>(h.sub[0], c->sm_count * 12), MROW_THREADS,
                       (cta_radix_smem<MROW_THREADS, MROW_MAX>()), lists + 3 * (int64_t)cn, &sub_counts[0], src, toff,
@@ -1982,15 +2298,16 @@ int contract_level(hp_context *c, HpLevel &g, int32_t cn, HpLevel &cg)
         }
     }
     // short rows + coarse xadj in one ordered pass, then the long rows' copies
-    if (h.small_max <= 8)
-        HP_LAUNCH(c, contract_assemble_kernel<8>, (unsigned)ntiles, ASM_TILE, asm_smem_bytes<8>(), cn, src, ucnt, cg.xadj,
-                  cg.adjncy, cg.adjwgt, c->lb_status, c->lb_ctl, c->d_status, c->tune.contract_thread_row, wchk);
-    else if (h.small_max <= 16)
-        HP_LAUNCH(c, contract_assemble_kernel<16>, (unsigned)ntiles, ASM_TILE, asm_smem_bytes<16>(), cn, src, ucnt, cg.xadj,
-                  cg.adjncy, cg.adjwgt, c->lb_status, c->lb_ctl, c->d_status, c->tune.contract_thread_row, wchk);
-    else
-        HP_LAUNCH(c, contract_assemble_kernel<32>, (unsigned)ntiles, ASM_TILE, asm_smem_bytes<32>(), cn, src, ucnt, cg.xadj,
-                  cg.adjncy, cg.adjwgt, c->lb_status, c->lb_ctl, c->d_status, c->tune.contract_thread_row, wchk);
+    const bool words_asm = !c->wide_rows && cn <= ASM_KEY_MAX;
+    auto assemble = [&](auto kernel, size_t smem) -> int {
+        HP_LAUNCH(c, kernel, (unsigned)ntiles, ASM_TILE, smem, cn, src, ucnt, cg.xadj, cg.adjncy, cg.adjwgt,
+                  c->lb_status, c->lb_ctl, c->d_status, c->tune.contract_thread_row, wchk);
+        return HP_OK;
+    };
+    if (!words_asm) HP_TRY(assemble(contract_assemble_wide_kernel<32>, asm_smem_bytes<32>()));
+    else if (h.small_max <= 8) HP_TRY(assemble(contract_assemble_kernel<8>, asm_smem_bytes<8>()));
+    else if (h.small_max <= 16) HP_TRY(assemble(contract_assemble_kernel<16>, asm_smem_bytes<16>()));
+    else HP_TRY(assemble(contract_assemble_kernel<32>, asm_smem_bytes<32>()));
     if (h.cnt[0] > 0)
         HP_LAUNCH(c, copy_long_rows_kernel<false>, std::min<unsigned>(blocks_for((int64_t)h.cnt[0] * 32),
                                                                      c->sm_count * 16),
@@ -2017,6 +2334,8 @@ int contract_level(hp_context *c, HpLevel &g, int32_t cn, HpLevel &cg)
 int hp_coarsen_init()
 {
     HP_CUDA(cudaFuncSetAttribute(contract_assemble_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)asm_smem_bytes<32>()));
+    HP_CUDA(cudaFuncSetAttribute(contract_assemble_wide_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)asm_smem_bytes<32>()));
     HP_CUDA(cudaFuncSetAttribute(match_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)ms_smem_bytes(HP_TUNE_SMALL_MATCH_MAX)));

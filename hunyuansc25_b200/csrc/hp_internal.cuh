@@ -94,6 +94,7 @@ struct hp_context {
     std::vector<hp_context *> workers;   // batch worker contexts (own streams and arenas)
     std::vector<HpLevel> levels;
     bool trace_valid = false;
+    bool wide_rows = false;              // hp_test_wide_rows: contraction rows take the 64-bit sorts
     bool weight_check = false;           // total edge weight >= 2^31: contractions check pair bounds
     bool learned_skewed = false;         // the input's degrees are skewed enough for the learned proposals
     hp_options opt = {};

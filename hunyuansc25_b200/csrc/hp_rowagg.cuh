@@ -83,6 +83,86 @@ __device__ __forceinline__ void sort_regs(unsigned long long (&x)[XN])
 
 constexpr unsigned long long PACK_NONE = (unsigned long long)(uint32_t)KEY_NONE << 32;
 
+// ---- one row per thread or per warp, in 32-bit words ---------------------------
+// An entry is packed as key << bits | (its index in the row), so a compare-exchange
+// is one min and one max of 32-bit registers, and the weight is fetched by the index
+// after the sort.  Padding and dropped keys are WORD_NONE, which sorts last: its key
+// part, all ones, must be no key (2^(32 - bits) > number of keys).
+constexpr unsigned WORD_NONE = 0xffffffffu;
+
+// Ascending bitonic network over the first NET of XN registers of one thread.  The
+// first step of every merge compares mirrored positions, so all comparators point
+// the same way.
+template <int NET, int XN>
+__device__ __forceinline__ void sort_words(unsigned (&x)[XN])
+{
+#pragma unroll
+    for (int size = 2; size <= NET; size <<= 1) {
+#pragma unroll
+        for (int i = 0; i < NET; i++) {
+            const int j = i ^ (size - 1);
+            if (j > i) {
+                const unsigned a = x[i], b = x[j];
+                x[i] = min(a, b);
+                x[j] = max(a, b);
+            }
+        }
+#pragma unroll
+        for (int stride = size >> 2; stride > 0; stride >>= 1)
+#pragma unroll
+            for (int i = 0; i < NET; i++) {
+                const int j = i ^ stride;
+                if (j > i) {
+                    const unsigned a = x[i], b = x[j];
+                    x[i] = min(a, b);
+                    x[j] = max(a, b);
+                }
+            }
+    }
+}
+
+// The same over 32 * NR words held by a warp, NR per lane: any order in, ascending
+// order out with lane l holding positions l * NR .. l * NR + NR - 1.
+template <int NR>
+__device__ __forceinline__ void warp_sort_words(unsigned (&x)[NR])
+{
+    const int lane = threadIdx.x & 31;
+    sort_words<NR, NR>(x);
+#pragma unroll 1
+    for (int g = 2; g <= 32; g <<= 1) {   // merges of g lanes' runs
+        {
+            const bool low = (lane & (g >> 1)) == 0;
+#pragma unroll
+            for (int r = 0; r < (NR + 1) / 2; r++) {
+                const unsigned a = __shfl_xor_sync(HP_FULL_MASK, x[NR - 1 - r], g - 1);
+                const unsigned b = __shfl_xor_sync(HP_FULL_MASK, x[r], g - 1);
+                x[r] = low ? min(x[r], a) : max(x[r], a);
+                if (NR > 1) x[NR - 1 - r] = low ? min(x[NR - 1 - r], b) : max(x[NR - 1 - r], b);
+            }
+        }
+#pragma unroll 1
+        for (int m = g >> 2; m > 0; m >>= 1) {
+            const bool low = (lane & m) == 0;
+#pragma unroll
+            for (int r = 0; r < NR; r++) {
+                const unsigned a = __shfl_xor_sync(HP_FULL_MASK, x[r], m);
+                x[r] = low ? min(x[r], a) : max(x[r], a);
+            }
+        }
+#pragma unroll
+        for (int stride = NR >> 1; stride > 0; stride >>= 1)
+#pragma unroll
+            for (int i = 0; i < NR; i++) {
+                const int j = i ^ stride;
+                if (j > i) {
+                    const unsigned a = x[i], b = x[j];
+                    x[i] = min(a, b);
+                    x[j] = max(a, b);
+                }
+            }
+    }
+}
+
 // Segmented version: the warp holds 32/S independent rows of up to S entries
 // (lanes [S*r, S*r+S) hold row r); each segment is sorted by its own bitonic
 // network (log2 S stages), equal keys are merged, and every segment writes its

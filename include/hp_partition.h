@@ -357,6 +357,11 @@ int hp_test_wait_expiry(hp_context *ctx);
 int hp_test_arena_first(hp_context *ctx, int64_t bytes);
 int hp_test_arena_restarts(hp_context *ctx);
 
+/* Test of the contraction's 64-bit row sorts, which levels of 2^22 (long rows) or
+ * 2^27 (short rows) coarse vertices take: on != 0 makes this context's calls take
+ * them on every level, 0 restores the rule.  Speed only; the rows are the same. */
+int hp_test_wide_rows(hp_context *ctx, int32_t on);
+
 /* ---- legacy drop-in ------------------------------------------------------------
  * Identical signature to the reference (hunyuangraph_partitiongraph.h:284).
  * Uses a process-wide context on device 0 and hp_options_default(); ubvec[0]

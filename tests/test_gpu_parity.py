@@ -509,3 +509,39 @@ def test_cluster_levels_learned(ctx):
         finally:
             ctx.set_tuning()
         assert a[1] == b[1] and np.array_equal(a[0], b[0])
+
+
+def row_length_graph(lengths, pool, seed):
+    """A ring of `pool` vertices and, for each length L, a hub that is matched with its own leaf (the
+    heaviest edge of both) and has L - 2 neighbours in the ring: its coarse row merges L entries."""
+    rng = np.random.default_rng(seed)
+    n = pool + 2 * len(lengths)
+    ring = np.arange(pool)
+    e = [np.stack([ring, (ring + 1) % pool])]
+    for i, length in enumerate(lengths):
+        hub = pool + 2 * i
+        e.append(np.array([[hub], [hub + 1]]))
+        e.append(np.stack([np.full(length - 2, hub), rng.choice(pool, length - 2, replace=False)]))
+    u, v = np.concatenate(e, axis=1)
+    w = np.where((u >= pool) & (v == u + 1), 1000, rng.integers(1, 100, u.size))
+    s, d, w = np.concatenate([u, v]), np.concatenate([v, u]), np.concatenate([w, w])
+    order = np.lexsort((d, s))
+    xadj = np.concatenate([[0], np.cumsum(np.bincount(s, minlength=n))]).astype(np.int32)
+    return graphs.Graph(xadj, d[order].astype(np.int32), np.ones(n, np.int32), w[order].astype(np.int32))
+
+
+# contraction rows around the sizes of the register networks (a thread up to 32 entries, a
+# warp's 2 to 32 words a lane up to 1024) and past them; wide: the 64-bit sorts of huge levels
+@pytest.mark.parametrize("wide", [0, 1])
+@pytest.mark.parametrize("smem_cn", [0, 49152])
+def test_contraction_row_lengths(ctx, wide, smem_cn):
+    lengths = [3, 7, 8, 9, 16, 17, 31, 32, 33, 34, 63, 64, 65, 127, 128, 129, 255, 256, 257, 511, 512, 513, 1023,
+               1024, 1025, 2047, 2048, 2049, 4095, 4096, 4097]
+    lib, h = ctx.lib, ctx.h
+    ctx.set_tuning(contract_smem_cn=smem_cn, contract_hybrid=0, small_match_n=64)
+    assert lib.hp_test_wide_rows(h, wide) == 0
+    try:
+        compare_runs(ctx, row_length_graph(lengths, 9000, 5), 4, 1.1)
+    finally:
+        lib.hp_test_wide_rows(h, 0)
+        ctx.set_tuning(None)
