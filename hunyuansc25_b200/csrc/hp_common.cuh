@@ -258,6 +258,26 @@ __device__ __forceinline__ void block_add_to(long long v, unsigned long long *ou
     __syncthreads();
 }
 
+// Two block-wide sums into *oa and *ob.
+template <int BLOCK>
+__device__ __forceinline__ void block_add2_to(long long a, unsigned long long *oa, long long b, unsigned long long *ob)
+{
+    __shared__ long long s_part[2][BLOCK / 32];
+    a = warp_sum64(a);
+    b = warp_sum64(b);
+    if ((threadIdx.x & 31) == 0) {
+        s_part[0][threadIdx.x >> 5] = a;
+        s_part[1][threadIdx.x >> 5] = b;
+    }
+    __syncthreads();
+    if (threadIdx.x < 64) {   // a warp per sum
+        const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
+        const long long t = warp_sum64(lane < BLOCK / 32 ? s_part[q][lane] : 0);
+        if (lane == 0 && t != 0) atomicAdd(q ? ob : oa, (unsigned long long)t);
+    }
+    __syncthreads();   // as in block_add_to
+}
+
 // Decoupled look-back (single-pass scan across CTAs).  tile_status[t] holds
 // flag << 32 | value: flag 1 = the tile's own aggregate, flag 2 = its inclusive
 // prefix.  Called by all 32 lanes of one warp of tile `tile` with the tile's

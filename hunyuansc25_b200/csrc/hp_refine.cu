@@ -192,10 +192,27 @@ gain_thread_kernel(const int32_t *__restrict__ list, const int32_t *__restrict__
 // by part, padded with part -1 up to min(deg, k).  A vertex with deg >= k has a
 // dense row instead: entry q is (q, conn to part q), zeros included; dense rows
 // are updated in place by atomics when a neighbour moves and never rebuilt.
+// Rows of a pass's rebuild.  A pass whose moves touch more than `over` entries of the
+// level's adjacency rebuilds every row (apply_moves_kernel then touches none), else
+// the rows that the moves queued.
+struct RebuildRule {
+    const unsigned long long *touch;   // entries of the moved vertices' rows; nullptr: the listed rows
+    unsigned long long over;
+    __device__ __forceinline__ bool all() const { return touch && *touch > over; }
+    // the count of the rows to build, both loads in flight together
+    __device__ __forceinline__ int32_t rows(const int32_t *d_count, const int32_t *d_all, bool &a) const
+    {
+        const int32_t c = *d_count, n = *d_all;
+        a = all();
+        return a ? n : c;
+    }
+};
+
 // Rebuild of the listed (dirty) rows of at most S entries (S >= the level's
 // longest short row): 32/S rows per warp, one segment of S lanes per row,
 // sorted and merged by seg_aggregate; dirty flags are cleared.  Rows with
 // deg >= k (k <= S here) are written dense.
+// list == nullptr: every vertex with a row of at most bigd (<= S) entries.
 // (warp, nwarps: this warp's index among the nwarps warps sharing the list)
 template <int S>
 __device__ __forceinline__ void gain_seg_rows(int64_t warp, int64_t nwarps, const int32_t *__restrict__ list,
@@ -203,7 +220,7 @@ __device__ __forceinline__ void gain_seg_rows(int64_t warp, int64_t nwarps, cons
                                               const int32_t *__restrict__ adjncy, const int32_t *__restrict__ adjwgt,
                                               const int32_t *__restrict__ where, const int32_t *__restrict__ goff,
                                               int32_t *__restrict__ gpart, int32_t *__restrict__ gconn, int32_t k,
-                                              int32_t *__restrict__ dirty)
+                                              int32_t *__restrict__ dirty, int32_t bigd = 0)
 {
     constexpr int R = 32 / S;
     const int lane = threadIdx.x & 31, sl = lane & (S - 1);
@@ -211,10 +228,14 @@ __device__ __forceinline__ void gain_seg_rows(int64_t warp, int64_t nwarps, cons
         const int64_t i = i0 + lane / S;
         int32_t v = -1, b = 0, d = 0;
         if (i < cnt) {
-            v = list[i];
+            v = list ? list[i] : (int32_t)i;
             b = xadj[v];
             d = xadj[v + 1] - b;
-            if (sl == 0) dirty[v] = 0;
+            if (list) {
+                if (sl == 0) dirty[v] = 0;
+            } else if (d > bigd) {
+                v = -1;
+            }
         }
         int32_t key = hp::KEY_NONE, w = 0;
         if (v >= 0 && sl < d) {
@@ -239,11 +260,14 @@ gain_seg_kernel(const int32_t *__restrict__ list, const int32_t *__restrict__ d_
                 const int32_t *__restrict__ xadj, const int32_t *__restrict__ adjncy,
                 const int32_t *__restrict__ adjwgt, const int32_t *__restrict__ where,
                 const int32_t *__restrict__ goff, int32_t *__restrict__ gpart, int32_t *__restrict__ gconn,
-                int32_t k, int32_t *__restrict__ dirty)
+                int32_t k, int32_t *__restrict__ dirty, RebuildRule rule, int32_t n, int32_t bigd)
 {
     hp::pdl_wait();
+    const int32_t cnt = *d_count;
+    const bool all = rule.all();
     gain_seg_rows<S>((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5, ((int64_t)gridDim.x * blockDim.x) >> 5,
-                     list, *d_count, xadj, adjncy, adjwgt, where, goff, gpart, gconn, k, dirty);
+                     all ? nullptr : list, all ? n : cnt, xadj, adjncy, adjwgt, where, goff, gpart, gconn, k,
+                     dirty, bigd);
 }
 
 // Gain rows of bigd+1 .. huged entries when k <= warp_dense_k: one warp per
@@ -261,7 +285,8 @@ __device__ __forceinline__ void gain_bigwarp_rows(int64_t warp, int64_t nwarps, 
                                                   const int32_t *__restrict__ adjwgt,
                                                   const int32_t *__restrict__ where, const int32_t *__restrict__ goff,
                                                   int32_t *__restrict__ gpart, int32_t *__restrict__ gconn, int32_t k,
-                                                  int32_t *__restrict__ dirty, int32_t bigd, int32_t huged)
+                                                  int32_t *__restrict__ dirty, int32_t bigd, int32_t huged,
+                                                  bool in_place = false)
 {
     const int lane = threadIdx.x & 31;
     const int nwords = (k + 31) >> 5;
@@ -292,9 +317,9 @@ __device__ __forceinline__ void gain_bigwarp_rows(int64_t warp, int64_t nwarps, 
         }
         __syncwarp();
         const int32_t o = goff[v], cap = goff[v + 1] - o;
-        if (dense) {   // (no presence bits were set)
+        if (dense) {   // (no presence bits were set; in_place: the parts are there from the level's build)
             for (int32_t q = lane; q < k; q += 32) {
-                gpart[o + q] = q;
+                if (!in_place) gpart[o + q] = q;
                 gconn[o + q] = dw[q];
                 dw[q] = 0;
             }
@@ -331,9 +356,13 @@ gain_bigwarp_kernel(const int32_t *__restrict__ list, const int32_t *__restrict_
                     const int32_t *__restrict__ adjwgt, const int32_t *__restrict__ where,
                     const int32_t *__restrict__ goff, int32_t *__restrict__ gpart,
                     int32_t *__restrict__ gconn, int32_t k, int32_t *__restrict__ dirty, int32_t bigd,
-                    int32_t huged)
+                    int32_t huged, RebuildRule rule, const int32_t *__restrict__ all_list,
+                    const int32_t *__restrict__ d_all)
 {
     hp::pdl_wait();
+    bool all;
+    const int32_t cnt = rule.rows(d_count, d_all, all);
+    if (all) list = all_list;
     extern __shared__ int32_t gsm[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int nwords = (k + 31) >> 5;
@@ -342,8 +371,8 @@ gain_bigwarp_kernel(const int32_t *__restrict__ list, const int32_t *__restrict_
     for (int i = lane; i < k; i += 32) dw[i] = 0;
     for (int i = lane; i < nwords; i += 32) bm[i] = 0u;
     __syncwarp();
-    gain_bigwarp_rows((int64_t)blockIdx.x * GW_WARPS + wid, (int64_t)gridDim.x * GW_WARPS, dw, bm, list, *d_count,
-                      xadj, adjncy, adjwgt, where, goff, gpart, gconn, k, dirty, bigd, huged);
+    gain_bigwarp_rows((int64_t)blockIdx.x * GW_WARPS + wid, (int64_t)gridDim.x * GW_WARPS, dw, bm, list, cnt,
+                      xadj, adjncy, adjwgt, where, goff, gpart, gconn, k, dirty, bigd, huged, dirty != nullptr);
 }
 
 template <int NT>
@@ -353,9 +382,14 @@ gain_dense_kernel(const int32_t *__restrict__ list, const int32_t *__restrict__ 
                   const int32_t *__restrict__ adjwgt, const int32_t *__restrict__ where,
                   const int32_t *__restrict__ goff, int32_t *__restrict__ gpart,
                   int32_t *__restrict__ gconn, int32_t k, int32_t *__restrict__ dirty, int32_t bigd,
-                  int32_t huged, int32_t warp_dense_k)
+                  int32_t huged, int32_t warp_dense_k, RebuildRule rule, const int32_t *__restrict__ all_list,
+                  const int32_t *__restrict__ d_all)
 {
     hp::pdl_wait();
+    bool all;
+    const int32_t cnt = rule.rows(d_count, d_all, all);
+    if (all) list = all_list;
+    if (!list || (int32_t)blockIdx.x >= cnt) return;
     extern __shared__ int32_t dsm[];
     __shared__ int32_t s_scan[NT / 32 + 2];
     int32_t *dw = dsm;
@@ -364,7 +398,6 @@ gain_dense_kernel(const int32_t *__restrict__ list, const int32_t *__restrict__ 
     for (int i = threadIdx.x; i < k; i += NT) dw[i] = 0;
     for (int i = threadIdx.x; i < nwords; i += NT) bm[i] = 0;
     __syncthreads();
-    const int32_t cnt = *d_count;
     for (int32_t li = blockIdx.x; li < cnt; li += gridDim.x) {
         const int32_t v = list[li];
         const int32_t b = xadj[v], e = xadj[v + 1];
@@ -395,7 +428,7 @@ gain_dense_kernel(const int32_t *__restrict__ list, const int32_t *__restrict__ 
         const int32_t o = goff[v], cap = goff[v + 1] - o;
         if (dense) {
             for (int32_t q = threadIdx.x; q < k; q += NT) {
-                gpart[o + q] = q;
+                if (!dirty) gpart[o + q] = q;
                 gconn[o + q] = dw[q];
                 dw[q] = 0;
             }
@@ -891,7 +924,8 @@ __global__ void log_label_kernel(int64_t r0, int64_t r1, const int32_t *__restri
 struct MoveSink {
     int32_t *moves, *oldp;
     unsigned long long *d_nmoves, *d_c1;
-    const int32_t *goff, *gpart, *gconn;
+    unsigned long long *d_touch;   // adjacency entries of the moved vertices (nullptr: not needed)
+    const int32_t *goff, *gpart, *gconn, *xadj;
     int32_t k;
 };
 
@@ -901,6 +935,13 @@ __device__ __forceinline__ void move_append(const MoveSink &ms, int32_t v, int32
     const unsigned long long i = atomicAdd(ms.d_nmoves, 1ull);
     ms.moves[i] = v;
     ms.oldp[i] = p;
+}
+
+// The block's sums over its moves (256 threads).
+__device__ __forceinline__ void sink_sums(const MoveSink &ms, long long c1, long long touch)
+{
+    if (ms.d_touch) hp::block_add2_to<256>(c1, ms.d_c1, touch, ms.d_touch);
+    else hp::block_add_to<256>(c1, ms.d_c1);
 }
 
 __device__ __forceinline__ long long ab_change(int32_t v, int32_t g, int32_t p, int32_t b,
@@ -996,7 +1037,7 @@ afterburner_small_kernel(int32_t n, const int32_t *__restrict__ xadj, const int3
     const bool judge = *J.flag != 0;
     if (*d_ncand == 0ull && !(judge && *J.d_ncandp != 0ull)) return;
     const int32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-    long long c1 = 0;
+    long long c1 = 0, touch = 0;
     bool listed = false;
     if (v < n) {
         const int32_t b0 = xadj[v], e0 = xadj[v + 1];
@@ -1021,6 +1062,7 @@ afterburner_small_kernel(int32_t n, const int32_t *__restrict__ xadj, const int3
             if (sel) {
                 move_append(ms, v, p);
                 c1 = g;
+                touch = e0 - b0;
             }
         }
     }
@@ -1028,7 +1070,7 @@ afterburner_small_kernel(int32_t n, const int32_t *__restrict__ xadj, const int3
         const int32_t pos = hp::warp_append(J.d_n, listed);
         if (listed) J.list[pos] = v;
     }
-    hp::block_add_to<256>(c1, ms.d_c1);
+    sink_sums(ms, c1, touch);
 }
 
 __global__ void __launch_bounds__(256)
@@ -1044,7 +1086,7 @@ afterburner_big_kernel(const int32_t *__restrict__ big, const int32_t *__restric
     if (*d_ncand == 0ull && !(judge && *J.d_ncandp != 0ull)) return;
     const int lane = threadIdx.x & 31;
     const int32_t cnt = *d_bigcnt;
-    long long c1 = 0;
+    long long c1 = 0, touch = 0;
     for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < cnt;
          i += ((int64_t)gridDim.x * blockDim.x) >> 5) {
         const int32_t v = big[i];
@@ -1076,10 +1118,11 @@ afterburner_big_kernel(const int32_t *__restrict__ big, const int32_t *__restric
             if (sel) {
                 move_append(ms, v, p);
                 c1 += g;
+                touch += xadj[v + 1] - xadj[v];
             }
         }
     }
-    hp::block_add_to<256>(c1, ms.d_c1);
+    sink_sums(ms, c1, touch);
 }
 
 // ---- long rows (longer than chunk_deg): chunk plans ------------------------------
@@ -1215,7 +1258,7 @@ __global__ void afterburner_huge_final_kernel(const int32_t *__restrict__ huge, 
     const bool judge = *J.flag != 0;
     if (*d_ncand == 0ull && !(judge && *J.d_ncandp != 0ull)) return;
     const int32_t nh = *d_nhuge;
-    long long c1 = 0;
+    long long c1 = 0, touch = 0;
     for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nh; i += gridDim.x * blockDim.x) {
         const int32_t v = huge[i];
         const int32_t g = pregain[v];
@@ -1234,9 +1277,10 @@ __global__ void afterburner_huge_final_kernel(const int32_t *__restrict__ huge, 
         if (sel) {
             move_append(ms, v, where[v]);
             c1 += g;
+            if (ms.d_touch) touch += ms.xadj[v + 1] - ms.xadj[v];
         }
     }
-    hp::block_add_to<256>(c1, ms.d_c1);
+    sink_sums(ms, c1, touch);
 }
 
 // ---- the judge's exact cut changes ---------------------------------------------------
@@ -1399,11 +1443,23 @@ apply_moves_kernel(const int32_t *__restrict__ moves, const unsigned long long *
                    const int32_t *__restrict__ adjwgt, const int32_t *__restrict__ goff,
                    int32_t *__restrict__ gconn, int32_t *__restrict__ dirty, int32_t *__restrict__ small_l,
                    int32_t *__restrict__ big_l, int32_t *counts, int32_t k, int32_t *__restrict__ huge_mv,
-                   int32_t *__restrict__ d_nhuge, int32_t bigd, int32_t chunkd)
+                   int32_t *__restrict__ d_nhuge, int32_t bigd, int32_t chunkd, RebuildRule rule)
 {
     hp::pdl_wait();
+    const int64_t nm = (int64_t)*d_nmoves;
+    if (rule.all()) {   // the rebuild takes every row: only the moves themselves
+        for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nm; i += (int64_t)gridDim.x * blockDim.x) {
+            const int32_t v = moves[i];
+            const int32_t p = where[v], d = dest[v];
+            const unsigned long long w = (unsigned long long)vwgt[v];
+            atomicAdd(&pw[d], w);
+            atomicAdd(&pw[p], (unsigned long long)(-(long long)w));
+            where[v] = d;
+        }
+        return;
+    }
     apply_moves_rows((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5, ((int64_t)gridDim.x * blockDim.x) >> 5,
-                     moves, (int64_t)*d_nmoves, where, dest, vwgt, pw, xadj, adjncy, adjwgt, goff, gconn, dirty,
+                     moves, nm, where, dest, vwgt, pw, xadj, adjncy, adjwgt, goff, gconn, dirty,
                      small_l, big_l, counts, k, huge_mv, d_nhuge, bigd, chunkd);
 }
 
@@ -1685,7 +1741,7 @@ __global__ void rw_select_kernel(const int32_t *__restrict__ K, const int32_t *_
 {
     hp::pdl_wait();
     const int32_t cnt = *d_cnt;
-    long long c1 = 0;
+    long long c1 = 0, touch = 0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < cnt;
          i += (int64_t)gridDim.x * blockDim.x) {
         int32_t p = K[i] >> 6;
@@ -1694,9 +1750,10 @@ __global__ void rw_select_kernel(const int32_t *__restrict__ K, const int32_t *_
             const int32_t v = V[i];
             move_append(ms, v, p);
             c1 += pregain[v];
+            if (ms.d_touch) touch += ms.xadj[v + 1] - ms.xadj[v];
         }
     }
-    hp::block_add_to<256>(c1, ms.d_c1);
+    sink_sums(ms, c1, touch);
 }
 
 // Strong rebalance: the evicted prefix of every overweight part (up to the first
@@ -1874,7 +1931,7 @@ __global__ void rs_assign_kernel(int32_t k, const int32_t *__restrict__ P, const
 {
     hp::pdl_wait();
     const int32_t np = *d_np;
-    long long c1 = 0;
+    long long c1 = 0, touch = 0;
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < np;
          j += (int64_t)gridDim.x * blockDim.x) {
         // last part with es[p] <= j
@@ -1889,11 +1946,12 @@ __global__ void rs_assign_kernel(int32_t k, const int32_t *__restrict__ P, const
         if (j < ee[p] && p != from) {
             dest[v] = p;
             move_append(ms, v, from);
+            if (ms.d_touch) touch += ms.xadj[v + 1] - ms.xadj[v];
             const int32_t o = ms.goff[v], len = ms.goff[v + 1] - o;
             c1 += (long long)row_conn(ms.gpart + o, ms.gconn + o, len, p, ms.k) + pregain[v];
         }
     }
-    hp::block_add_to<256>(c1, ms.d_c1);
+    sink_sums(ms, c1, touch);
 }
 
 
@@ -1917,6 +1975,7 @@ struct RefineBufs {
     const int64_t *opt, *maxp;
     int32_t small_max;  // longest row of at most bigd entries (picks the gain kernel's network)
     bool huge_rows;     // the level has rows longer than huged
+    bool dense_rows;    // the level has rows of at least k entries
 };
 
 // scalar slots used by refinement
@@ -1927,16 +1986,15 @@ struct RefineBufs {
 // S_BIGCNT (slots 16-18) holds the big-row count, the longest short row, the
 // longest row above huged, the long-row count and the hub-row count.
 enum { S_NMOVES = 0, S_C1 = 1, S_C2 = 2, S_EXCESS = 3, S_NCAND = 4, S_CUT2 = 5, S_DIRTY = 6,
-       S_HUGEMV = 7, S_LISTCNT = 8, S_NU = 9, S_NP = 10, S_NCANDP = 11, S_JN = 12, S_JP = 13, S_JL = 14,
+       S_HUGEMV = 7, S_LISTCNT = 8, S_NU = 9, S_NP = 10, S_NCANDP = 11, S_JN = 12, S_JP = 13, S_JL = 14, S_TOUCH = 15,
        S_PASS_END = 16, S_BIGCNT = 16, S_DONE = 20 };
 
-// hub_list (nullable): the rows longer than gain_hub_deg among big_list, which
-// the dense build walks instead of big_list when k <= warp_dense_k (its other
-// rows are gain_bigwarp_kernel's)
+// hub_list: the level's rows longer than gain_hub_deg, which a full dense build walks
+// instead of all long rows when k <= warp_dense_k (the others are gain_bigwarp_kernel's)
 int build_rows(hp_context *c, HpLevel &g, RefineBufs &B, int32_t k, const int32_t *small_list,
                const int32_t *d_small_cnt, const int32_t *big_list, const int32_t *d_big_cnt,
-               bool any_big, int32_t *dirty, const int32_t *hub_list = nullptr,
-               const int32_t *d_hub_cnt = nullptr)
+               bool any_big, int32_t *dirty, const int32_t *hub_list, const int32_t *d_hub_cnt,
+               const RebuildRule &rule = RebuildRule{nullptr, 0})
 {
     const hp_tuning &tn = c->tune;
     if (small_list) {
@@ -1945,13 +2003,13 @@ int build_rows(hp_context *c, HpLevel &g, RefineBufs &B, int32_t k, const int32_
         const unsigned grid = (unsigned)(c->sm_count * tn.grid_ctas_per_sm);
         if (B.small_max <= 8)
             HP_LAUNCH(c, gain_seg_kernel<8>, grid, 256, 0, small_list, d_small_cnt, g.xadj, g.adjncy, g.adjwgt,
-                      g.where, B.goff, B.gpart, B.gconn, k, dirty);
+                      g.where, B.goff, B.gpart, B.gconn, k, dirty, rule, g.n, tn.gain_thread_deg);
         else if (B.small_max <= 16)
             HP_LAUNCH(c, gain_seg_kernel<16>, grid, 256, 0, small_list, d_small_cnt, g.xadj, g.adjncy, g.adjwgt,
-                      g.where, B.goff, B.gpart, B.gconn, k, dirty);
+                      g.where, B.goff, B.gpart, B.gconn, k, dirty, rule, g.n, tn.gain_thread_deg);
         else
             HP_LAUNCH(c, gain_seg_kernel<32>, grid, 256, 0, small_list, d_small_cnt, g.xadj, g.adjncy, g.adjwgt,
-                      g.where, B.goff, B.gpart, B.gconn, k, dirty);
+                      g.where, B.goff, B.gpart, B.gconn, k, dirty, rule, g.n, tn.gain_thread_deg);
     } else {
         // full build of the level: one thread per row, register network
         const unsigned grid = nblk(g.n);
@@ -1966,19 +2024,24 @@ int build_rows(hp_context *c, HpLevel &g, RefineBufs &B, int32_t k, const int32_
                       g.where, B.goff, B.gpart, B.gconn, k, dirty, tn.gain_thread_deg);
     }
     if (any_big) {
+        // eight CTAs per SM in flight (where their accumulators fit): the rows are bound by
+        // gather latency (R-MAT scale 22, all levels: four and two CTAs 9.7 ms, eight 7.9)
         const size_t smem = sizeof(int32_t) * (size_t)k + sizeof(unsigned) * (size_t)((k + 31) / 32);
+        const int32_t *d_all = (const int32_t *)&c->d_scal[S_BIGCNT];
         if (k <= tn.warp_dense_k)
-            HP_LAUNCH(c, gain_bigwarp_kernel, (unsigned)(c->sm_count * 4), 32 * GW_WARPS, GW_WARPS * smem, big_list,
+            HP_LAUNCH(c, gain_bigwarp_kernel, (unsigned)(c->sm_count * 8), 32 * GW_WARPS, GW_WARPS * smem, big_list,
                       d_big_cnt, g.xadj, g.adjncy, g.adjwgt, g.where, B.goff, B.gpart, B.gconn, k, dirty,
-                      tn.gain_thread_deg, tn.gain_hub_deg);
-        // hub rows: every such row in a full build; in a rebuild only sparse
-        // ones (deg < k), which exist only when k > gain_hub_deg
-        const bool dense_rows = dirty ? (B.huge_rows && k > tn.gain_hub_deg) : B.huge_rows;
-        const bool hubs = hub_list && k <= tn.warp_dense_k;
-        if (k > tn.warp_dense_k || dense_rows)
-            HP_LAUNCH(c, gain_dense_kernel<256>, (unsigned)(c->sm_count * 2), 256, smem, hubs ? hub_list : big_list,
-                      hubs ? d_hub_cnt : d_big_cnt, g.xadj, g.adjncy, g.adjwgt, g.where, B.goff, B.gpart, B.gconn, k,
-                      dirty, tn.gain_thread_deg, tn.gain_hub_deg, tn.warp_dense_k);
+                      tn.gain_thread_deg, tn.gain_hub_deg, rule, B.big, d_all);
+        // hub rows: every such row in a full build (of a level or after a pass); among the
+        // queued rows only sparse ones (deg < k) exist, and only when k > gain_hub_deg
+        const bool hubs = k <= tn.warp_dense_k;
+        const int32_t *list = big_list, *d_cnt = d_big_cnt;
+        if (hubs && !dirty) { list = hub_list; d_cnt = d_hub_cnt; }
+        else if (hubs && k <= tn.gain_hub_deg) list = nullptr;
+        if (!hubs || B.huge_rows)
+            HP_LAUNCH(c, gain_dense_kernel<256>, (unsigned)(c->sm_count * 8), 256, smem, list, d_cnt, g.xadj, g.adjncy,
+                      g.adjwgt, g.where, B.goff, B.gpart, B.gconn, k, dirty, tn.gain_thread_deg, tn.gain_hub_deg,
+                      tn.warp_dense_k, rule, hubs ? hub_list : B.big, hubs ? d_hub_cnt : d_all);
     }
     return HP_OK;
 }
@@ -2031,10 +2094,10 @@ int rank_candidates(hp_context *c, HpLevel &g, RefineBufs &B, int32_t k, int32_t
     return HP_OK;
 }
 
-MoveSink move_sink(hp_context *c, const RefineBufs &B, int32_t k)
+MoveSink move_sink(hp_context *c, const HpLevel &g, const RefineBufs &B, int32_t k)
 {
     unsigned long long *sc = c->d_scal;
-    return MoveSink{B.moves, B.oldp, &sc[S_NMOVES], &sc[S_C1], B.goff, B.gpart, B.gconn, k};
+    return MoveSink{B.moves, B.oldp, &sc[S_NMOVES], &sc[S_C1], B.dense_rows ? &sc[S_TOUCH] : nullptr, B.goff, B.gpart, B.gconn, g.xadj, k};
 }
 
 // The undersized-part list of a weak pass is built by ctl_begin_kernel.
@@ -2044,7 +2107,7 @@ int weak_rebalance(hp_context *c, HpLevel &g, RefineBufs &B, int32_t k, const Be
     int32_t *Ks, *Vs;
     HP_TRY(rank_candidates<false>(c, g, B, k, &Ks, &Vs, bcp));
     HP_LAUNCH(c, rw_select_kernel, (unsigned)(c->sm_count * 8), 256, 0, Ks, Vs,
-              (const int32_t *)&sc[S_LISTCNT], B.pre, B.pstart, B.pw, B.maxp, B.pregain, move_sink(c, B, k));
+              (const int32_t *)&sc[S_LISTCNT], B.pre, B.pstart, B.pw, B.maxp, B.pregain, move_sink(c, g, B, k));
     return HP_OK;
 }
 
@@ -2064,7 +2127,7 @@ int strong_rebalance(hp_context *c, HpLevel &g, RefineBufs &B, int32_t k, const 
     HP_LAUNCH(c, cookie_cutter_kernel, 1, 1024, sizeof(int32_t) * COOKIE_SMEM_INTS, k, B.pw, B.maxp, B.sp, d_np,
               B.es, B.ee);
     HP_LAUNCH(c, rs_assign_kernel, pg, 256, 0, k, B.P, d_np, Vs, B.es, B.ee, g.where, B.dest, B.pregain,
-              move_sink(c, B, k));
+              move_sink(c, g, B, k));
     return HP_OK;
 }
 
@@ -2318,11 +2381,14 @@ lp_bytes_kernel(int32_t n, const int32_t *__restrict__ goff, const int32_t *__re
 __global__ void __launch_bounds__(256)
 rebuild_bytes_kernel(const int32_t *__restrict__ small_l, const int32_t *__restrict__ d_nsmall,
                      const int32_t *__restrict__ big_l, const int32_t *__restrict__ d_nbig,
-                     const int32_t *__restrict__ xadj, const int32_t *__restrict__ goff, unsigned long long *acc)
+                     const int32_t *__restrict__ xadj, const int32_t *__restrict__ goff, RebuildRule rule, int32_t n,
+                     unsigned long long *acc)
 {
     hp::pdl_wait();
     const int32_t ns = *d_nsmall, nb = *d_nbig;
     long long b = 0;
+    // every row: xadj, goff and the parts, the adjacency, the gain rows
+    if (rule.all() && blockIdx.x == 0 && threadIdx.x == 0) b = 12ll * n + 8ll * xadj[n] + 8ll * goff[n];
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (int64_t)ns + nb;
          i += (int64_t)gridDim.x * blockDim.x) {
         const int32_t v = i < ns ? small_l[i] : big_l[i - ns];
@@ -2416,10 +2482,10 @@ int pass_propose(hp_context *c, HpLevel &g, RefineBufs &B, const PassCfg &P, int
                       P.finest ? 1 : 0, B.pw, B.maxp, B.opt, B.dest, B.pregain, B.recof, c->log_x, c->log_v,
                       c->log_d, c->log_acc, c->log_count, c->log_cap);
         HP_LAUNCH(c, afterburner_small_kernel, nblk(n), 256, 0, n, g.xadj, g.adjncy, g.adjwgt, g.where, B.dest,
-                  B.pregain, B.lock, &sc[S_NCAND], move_sink(c, B, k), c->tune.gain_thread_deg, J);
+                  B.pregain, B.lock, &sc[S_NCAND], move_sink(c, g, B, k), c->tune.gain_thread_deg, J);
         if (P.any_big)
             HP_LAUNCH(c, afterburner_big_kernel, pg, 256, 0, B.big, d_bigcnt, g.xadj, g.adjncy, g.adjwgt, g.where,
-                      B.dest, B.pregain, B.lock, &sc[S_NCAND], move_sink(c, B, k), c->tune.chunk_deg, J);
+                      B.dest, B.pregain, B.lock, &sc[S_NCAND], move_sink(c, g, B, k), c->tune.chunk_deg, J);
         if (P.huge_rows) {
             const int32_t *d_nhuge = d_bigcnt + 3;
             HP_LAUNCH(c, hub_plan_kernel<false>, plan_grid(c, B.nhub_cap), PLAN_THREADS, 0, B.huge, d_nhuge, B.moves,
@@ -2429,7 +2495,7 @@ int pass_propose(hp_context *c, HpLevel &g, RefineBufs &B, const PassCfg &P, int
                       B.plan_off, B.plan_cnt, g.xadj, g.adjncy, g.adjwgt, g.where, B.dest, B.pregain, &sc[S_NCAND],
                       B.ab_acc, B.ab_acc2, J);
             HP_LAUNCH(c, afterburner_huge_final_kernel, (unsigned)c->sm_count, 256, 0, B.huge, d_nhuge, B.pregain,
-                      &sc[S_NCAND], B.ab_acc, B.ab_acc2, B.lock, g.where, B.dest, move_sink(c, B, k), J);
+                      &sc[S_NCAND], B.ab_acc, B.ab_acc2, B.lock, g.where, B.dest, move_sink(c, g, B, k), J);
         }
         if (judging) {   // the plain refiner's exact cut change on the same state (learned passes only)
             const int64_t rt = ((int64_t)n + RK_TILE) / RK_TILE;   // a tile holds index cnt <= n
@@ -2460,6 +2526,19 @@ int pass_propose(hp_context *c, HpLevel &g, RefineBufs &B, const PassCfg &P, int
     return HP_OK;
 }
 
+// When a pass rebuilds every gain row: on a level with dense rows, its moves touch more
+// than an eighth of the adjacency.  Touching an entry costs a gather of the neighbour's
+// row offset and, where the neighbour's row is dense, two scattered atomics; the full
+// build reads every entry once, in order, and adds in shared memory.  R-MAT scale 22,
+// k = 256, learned: moves and rebuilds 22.8 ms a call without the rule, 14.3 at an
+// eighth, 14.5 at a quarter, 15.4 at a sixteenth.  Levels without dense rows touch by
+// flags alone, and their passes are too short for the extra sum.
+constexpr int64_t REBUILD_SHARE = 8;
+RebuildRule rebuild_rule(hp_context *c, const HpLevel &g, const RefineBufs &B)
+{
+    return RebuildRule{B.dense_rows ? &c->d_scal[S_TOUCH] : nullptr, (unsigned long long)(g.m / REBUILD_SHARE)};
+}
+
 // Apply phase of one pass: simultaneous moves, exact cut change from the gain
 // rows before and after, gain-row maintenance, balance, then the control step.
 int pass_apply(hp_context *c, HpLevel &g, RefineBufs &B, const PassCfg &P, cudaGraphConditionalHandle hloop,
@@ -2469,11 +2548,12 @@ int pass_apply(hp_context *c, HpLevel &g, RefineBufs &B, const PassCfg &P, cudaG
     unsigned long long *sc = c->d_scal;
     const unsigned pg = (unsigned)(c->sm_count * c->tune.grid_ctas_per_sm);
     const unsigned mg = std::min(nblk(n), pg);   // grid-stride over the device move count
-    // (the proposal kernels appended the moves with their old parts and c1)
+    // (the proposal kernels appended the moves with their old parts, c1 and their entries)
+    const RebuildRule rule = rebuild_rule(c, g, B);
     int atok = hp_prof_begin(c);
     HP_LAUNCH(c, apply_moves_kernel, pg, 256, 0, B.moves, &sc[S_NMOVES], g.where, B.dest, g.vwgt, B.pw, g.xadj,
               g.adjncy, g.adjwgt, B.goff, B.gconn, B.dirty, B.small_l, B.big_l, (int32_t *)&sc[S_DIRTY], k,
-              B.huge_mv, (int32_t *)&sc[S_HUGEMV], c->tune.gain_thread_deg, c->tune.apply_chunk_deg);
+              B.huge_mv, (int32_t *)&sc[S_HUGEMV], c->tune.gain_thread_deg, c->tune.apply_chunk_deg, rule);
     if (P.huge_moves) {
         HP_LAUNCH(c, hub_plan_kernel<true>, plan_grid(c, B.nhub_cap), PLAN_THREADS, 0, B.huge_mv,
                   (const int32_t *)&sc[S_HUGEMV], B.moves, B.pregain, g.xadj, B.plan_v, B.plan_item, B.plan_off,
@@ -2485,11 +2565,12 @@ int pass_apply(hp_context *c, HpLevel &g, RefineBufs &B, const PassCfg &P, cudaG
     hp_prof_end(c, atok, HP_PROF_APPLY, 0);
     const int rtok = hp_prof_begin(c);
     HP_TRY(build_rows(c, g, B, k, B.small_l, (const int32_t *)&sc[S_DIRTY], B.big_l,
-                      ((const int32_t *)&sc[S_DIRTY]) + 1, P.any_big, B.dirty));
+                      ((const int32_t *)&sc[S_DIRTY]) + 1, P.any_big, B.dirty, B.hub,
+                      (const int32_t *)&sc[S_BIGCNT] + 4, rule));
     hp_prof_end(c, rtok, HP_PROF_REBUILD, 0);
     if (unsigned long long *cnt = hp_prof_counter(c, HP_PROF_REBUILD))
         HP_LAUNCH(c, rebuild_bytes_kernel, pg, 256, 0, B.small_l, (const int32_t *)&sc[S_DIRTY], B.big_l,
-                  ((const int32_t *)&sc[S_DIRTY]) + 1, g.xadj, B.goff, cnt);
+                  ((const int32_t *)&sc[S_DIRTY]) + 1, g.xadj, B.goff, rule, n, cnt);
     atok = hp_prof_begin(c);
     HP_LAUNCH(c, pass_end_kernel, mg, 256, 0, B.moves, &sc[S_NMOVES], B.goff, B.gpart, B.gconn, g.where, B.oldp, k,
               P.ctl, sc, hloop, graph, B.pw, B.maxp, c->d_status, (unsigned *)&sc[S_DONE]);
@@ -3526,6 +3607,7 @@ int refine_level(hp_context *c, HpLevel &g, int32_t k, bool finest, const int64_
     // count with G from the control block at the end of uncoarsening)
     B.small_max = ls.small_max;
     B.huge_rows = ls.maxdeg > huged;
+    B.dense_rows = ls.maxdeg >= k;
     B.gpart = ralloc_t<int32_t>(c, std::max<int64_t>(g.m, 1));
     B.gconn = ralloc_t<int32_t>(c, std::max<int64_t>(g.m, 1));
     HP_CHECK_OOM(c);

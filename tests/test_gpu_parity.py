@@ -545,3 +545,16 @@ def test_contraction_row_lengths(ctx, wide, smem_cn):
     finally:
         lib.hp_test_wide_rows(h, 0)
         ctx.set_tuning(None)
+
+
+# launched passes: gain rows of every short length (built by tiles of rows, dense where the
+# degree reaches k), hubs, and passes whose moves touch enough of the graph to rebuild all rows
+@pytest.mark.parametrize("k", [2, 9, 17, 33, 200])
+def test_launched_gain_rows(ctx, k):
+    lengths = list(range(2, 40)) + [64, 255, 256, 257, 1000, 5000]
+    ctx.set_tuning(small_level_n=0, gain_hub_deg=300, chunk_deg=512, apply_chunk_deg=512)
+    try:
+        compare_runs(ctx, row_length_graph(lengths, 6000, 8), k, 1.1)
+        compare_runs(ctx, graphs.rmat(12, 16, seed=5, wmin=1, wmax=100), k, 1.03)
+    finally:
+        ctx.set_tuning(None)
