@@ -743,43 +743,9 @@ __device__ __forceinline__ void group_excl_scan2(int a, uint32_t b, int *ea, uin
 }
 
 // ---- short rows: one thread per coarse row, aggregation in registers ------------
-// The row's entries come from the tile's staging buffer as words (key << ASM_IDX |
-// index in the row, the self key already WORD_NONE) with the weights beside them.  A
-// bitonic network of NET sorts the words; the weights of equal keys are summed into
-// the slot of the run's first entry, and the unique keys are counted.  A comparator is
-// two instructions instead of six on 64-bit entries, which the kernel was bound by:
-// RGG of 2^24 vertices, level 0 8.1 -> 5.9 ms, 128^3 grid 0.26 -> 0.23 ms.
-constexpr int ASM_IDX = 5;                                   // a short row has at most 32 entries
-constexpr int32_t ASM_KEY_MAX = (1 << (32 - ASM_IDX)) - 1;   // coarse ids below it fit a word
-
-template <int NET, int XN>
-__device__ __forceinline__ int sort_staged_row(const unsigned *key, int32_t *wgt, int32_t len, unsigned (&x)[XN])
-{
-#pragma unroll
-    for (int i = 0; i < NET; i++) x[i] = i < len ? key[i] : hp::WORD_NONE;
-    hp::sort_words<NET, XN>(x);
-    int u = 0;
-    int32_t acc = 0;          // weight of the entries after i that have its key
-    bool same_next = false;   // entry i + 1 has the key of entry i
-#pragma unroll
-    for (int b = NET - 8; b >= 0; b -= 8) {   // eight weights in flight
-        int32_t w[8];
-#pragma unroll
-        for (int q = 0; q < 8; q++) w[q] = wgt[x[b + q] == hp::WORD_NONE ? 0 : x[b + q] & ((1u << ASM_IDX) - 1u)];
-#pragma unroll
-        for (int q = 7; q >= 0; q--) {
-            const int i = b + q;
-            const bool same = i > 0 && (x[i] ^ x[i > 0 ? i - 1 : 0]) < (1u << ASM_IDX);   // the key of entry i - 1
-            const bool valid = x[i] != hp::WORD_NONE;
-            acc += w[q];
-            if (!same && valid && same_next) wgt[x[i] & ((1u << ASM_IDX) - 1u)] = acc;
-            u += valid && !same;
-            if (!same) acc = 0;
-            same_next = same && valid;
-        }
-    }
-    return u;
-}
+// (hp::sort_staged_row; the self key is dropped while staging.)  A comparator is two
+// instructions instead of six on 64-bit entries, which the kernel was bound by: RGG of
+// 2^24 vertices, level 0 8.1 -> 5.9 ms, 128^3 grid 0.26 -> 0.23 ms.
 
 // The first word of every run of the sorted row into out[0..u), each tagged with the
 // tile row t; the run's weight is at the word's index of the row's staged weights.
@@ -789,7 +755,7 @@ __device__ __forceinline__ void emit_staged_row(const unsigned (&x)[XN], unsigne
     int r = 0;
 #pragma unroll
     for (int i = 0; i < NET; i++) {
-        const bool same = i > 0 && (x[i] ^ x[i > 0 ? i - 1 : 0]) < (1u << ASM_IDX);
+        const bool same = i > 0 && hp::same_key(x[i], x[i > 0 ? i - 1 : 0]);
         if (x[i] == hp::WORD_NONE || same) continue;
         out[r] = x[i];
         orow[r] = t;
@@ -878,7 +844,7 @@ contract_assemble_kernel(int32_t cn, ContractSrc src, const int32_t *__restrict_
             if (rt[q] < 0) continue;
             const int32_t k = kq[q];
             const int f = f0 + q * ASM_TILE;
-            asm_words[f] = k == c0 + rt[q] ? hp::WORD_NONE : ((unsigned)k << ASM_IDX) | (unsigned)(f - s_off[rt[q]]);
+            asm_words[f] = k == c0 + rt[q] ? hp::WORD_NONE : ((unsigned)k << hp::ROW_IDX) | (unsigned)(f - s_off[rt[q]]);
             s_wgt[f] = w[q];
         }
     }
@@ -895,13 +861,9 @@ contract_assemble_kernel(int32_t cn, ContractSrc src, const int32_t *__restrict_
     unsigned x[XN];
     int u = 0;
     if (c < cn && !small) u = ucnt[c];
-    if (XN == 8 || wmax <= 8) {
-        if (small) u = sort_staged_row<8, XN>(asm_words + ioff, s_wgt + ioff, len, x);
-    } else if (XN == 16 || wmax <= 16) {
-        if (small) u = sort_staged_row<(XN < 16 ? XN : 16), XN>(asm_words + ioff, s_wgt + ioff, len, x);
-    } else {
-        if (small) u = sort_staged_row<XN, XN>(asm_words + ioff, s_wgt + ioff, len, x);
-    }
+    hp::by_net_size<XN>(wmax, [&](auto net) {
+        if (small) u = hp::sort_staged_row<decltype(net)::value, XN>(asm_words + ioff, s_wgt + ioff, len, x);
+    });
     int ooff, tout;
     uint32_t local, agg;
     group_excl_scan2<ASM_TILE>(small ? u : 0, (uint32_t)u, &ooff, &local, &tout, &agg, s_scan);   // (the staged words are read)
@@ -909,12 +871,9 @@ contract_assemble_kernel(int32_t cn, ContractSrc src, const int32_t *__restrict_
         const int32_t excl = hp::lookback_epoch(tile_status, tile, (int32_t)agg, epoch, status);
         if (t == 0) s_excl = excl;
     }
-    if (small) {
-        if (XN == 8 || wmax <= 8) emit_staged_row<8, XN>(x, asm_words + ooff, s_row + ooff, (uint8_t)t);
-        else if (XN == 16 || wmax <= 16)
-            emit_staged_row<(XN < 16 ? XN : 16), XN>(x, asm_words + ooff, s_row + ooff, (uint8_t)t);
-        else emit_staged_row<XN, XN>(x, asm_words + ooff, s_row + ooff, (uint8_t)t);
-    }
+    hp::by_net_size<XN>(wmax, [&](auto net) {
+        if (small) emit_staged_row<decltype(net)::value, XN>(x, asm_words + ooff, s_row + ooff, (uint8_t)t);
+    });
     __syncthreads();
     const int32_t off = s_excl + (int32_t)local;
     s_goff[t] = off - ooff;
@@ -927,13 +886,13 @@ contract_assemble_kernel(int32_t cn, ContractSrc src, const int32_t *__restrict_
         const int rt = s_row[f];
         const int32_t pos = s_goff[rt] + f;
         const unsigned e = asm_words[f];
-        cadjncy[pos] = (int32_t)(e >> ASM_IDX);
-        cadjwgt[pos] = s_wgt[s_off[rt] + (int)(e & ((1u << ASM_IDX) - 1u))];
+        cadjncy[pos] = (int32_t)(e >> hp::ROW_IDX);
+        cadjwgt[pos] = s_wgt[s_off[rt] + (int)(e & ((1u << hp::ROW_IDX) - 1u))];
     }
     hp::lb_end(lb);
 }
 
-// The same with 64-bit entries, for levels of ASM_KEY_MAX coarse vertices or more:
+// The same with 64-bit entries, for levels of hp::ROW_KEY_MAX coarse vertices or more:
 // the row's entries come from the tile's staging buffer (packed key << 32 |
 // weight, the self key already PACK_NONE); a bitonic network of NET sorts them
 // and the unique keys are counted.
@@ -2298,7 +2257,7 @@ int contract_level(hp_context *c, HpLevel &g, int32_t cn, HpLevel &cg)
         }
     }
     // short rows + coarse xadj in one ordered pass, then the long rows' copies
-    const bool words_asm = !c->wide_rows && cn <= ASM_KEY_MAX;
+    const bool words_asm = !c->wide_rows && cn <= hp::ROW_KEY_MAX;
     auto assemble = [&](auto kernel, size_t smem) -> int {
         HP_LAUNCH(c, kernel, (unsigned)ntiles, ASM_TILE, smem, cn, src, ucnt, cg.xadj, cg.adjncy, cg.adjwgt,
                   c->lb_status, c->lb_ctl, c->d_status, c->tune.contract_thread_row, wchk);

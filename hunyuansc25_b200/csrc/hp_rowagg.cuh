@@ -90,18 +90,22 @@ constexpr unsigned long long PACK_NONE = (unsigned long long)(uint32_t)KEY_NONE 
 // part, all ones, must be no key (2^(32 - bits) > number of keys).
 constexpr unsigned WORD_NONE = 0xffffffffu;
 
+constexpr int pow2_at_least(int n) { return n <= 1 ? 1 : 2 * pow2_at_least((n + 1) / 2); }
+
 // Ascending bitonic network over the first NET of XN registers of one thread.  The
 // first step of every merge compares mirrored positions, so all comparators point
-// the same way.
+// the same way; NET need not be a power of two: the missing high positions would hold
+// WORD_NONE, which such comparators leave in place, so they are left out.
 template <int NET, int XN>
 __device__ __forceinline__ void sort_words(unsigned (&x)[XN])
 {
+    constexpr int P = pow2_at_least(NET);
 #pragma unroll
-    for (int size = 2; size <= NET; size <<= 1) {
+    for (int size = 2; size <= P; size <<= 1) {
 #pragma unroll
         for (int i = 0; i < NET; i++) {
             const int j = i ^ (size - 1);
-            if (j > i) {
+            if (j > i && j < NET) {
                 const unsigned a = x[i], b = x[j];
                 x[i] = min(a, b);
                 x[j] = max(a, b);
@@ -112,13 +116,66 @@ __device__ __forceinline__ void sort_words(unsigned (&x)[XN])
 #pragma unroll
             for (int i = 0; i < NET; i++) {
                 const int j = i ^ stride;
-                if (j > i) {
+                if (j > i && j < NET) {
                     const unsigned a = x[i], b = x[j];
                     x[i] = min(a, b);
                     x[j] = max(a, b);
                 }
             }
     }
+}
+
+// f(integral constant) with the smallest network size that takes len entries (at most XN).
+template <int N> struct NetSize { static constexpr int value = N; };
+template <int XN, class F>
+__device__ __forceinline__ void by_net_size(unsigned len, F &&f)
+{
+    if (XN == 8 || len <= 8) f(NetSize<8>{});
+    else if (len <= 12) f(NetSize<(XN < 12 ? XN : 12)>{});
+    else if (XN == 16 || len <= 16) f(NetSize<(XN < 16 ? XN : 16)>{});
+    else if (len <= 20) f(NetSize<(XN < 20 ? XN : 20)>{});
+    else if (len <= 24) f(NetSize<(XN < 24 ? XN : 24)>{});
+    else f(NetSize<XN>{});
+}
+
+// ---- a thread's row staged in shared memory -------------------------------------
+// The row's entries are words (key << ROW_IDX | index in the row, a dropped key
+// WORD_NONE) with the weights beside them.  The words are sorted in registers, the
+// weights of equal keys are summed into the slot of the run's first entry, and the
+// unique keys are counted.
+constexpr int ROW_IDX = 5;                                    // at most 32 entries
+constexpr int32_t ROW_KEY_MAX = (1 << (32 - ROW_IDX)) - 1;    // keys below it fit a word
+
+__device__ __forceinline__ bool same_key(unsigned a, unsigned b) { return (a ^ b) < (1u << ROW_IDX); }
+
+template <int NET, int XN>
+__device__ __forceinline__ int sort_staged_row(const unsigned *key, int32_t *wgt, int32_t len, unsigned (&x)[XN])
+{
+#pragma unroll
+    for (int i = 0; i < NET; i++) x[i] = i < len ? key[i] : WORD_NONE;
+    sort_words<NET, XN>(x);
+    constexpr int Q = NET % 8 == 0 ? 8 : 4;   // weights in flight
+    int u = 0;
+    int32_t acc = 0;          // weight of the entries after i that have its key
+    bool same_next = false;   // entry i + 1 has the key of entry i
+#pragma unroll
+    for (int b = NET - Q; b >= 0; b -= Q) {
+        int32_t w[Q];
+#pragma unroll
+        for (int q = 0; q < Q; q++) w[q] = wgt[x[b + q] == WORD_NONE ? 0 : x[b + q] & ((1u << ROW_IDX) - 1u)];
+#pragma unroll
+        for (int q = Q - 1; q >= 0; q--) {
+            const int i = b + q;
+            const bool same = i > 0 && same_key(x[i], x[i > 0 ? i - 1 : 0]);   // the key of entry i - 1
+            const bool valid = x[i] != WORD_NONE;
+            acc += w[q];
+            if (!same && valid && same_next) wgt[x[i] & ((1u << ROW_IDX) - 1u)] = acc;
+            u += valid && !same;
+            if (!same) acc = 0;
+            same_next = same && valid;
+        }
+    }
+    return u;
 }
 
 // The same over 32 * NR words held by a warp, NR per lane: any order in, ascending
