@@ -15,10 +15,11 @@
 //                         thread's bitonic network in registers, written in
 //                         place by one ordered pass with a decoupled look-back
 //                         that also produces the coarse xadj
-//        33..1024         one warp, bitonic network in registers (an LSD radix
-//                         sort in shared memory where the coarse ids leave no
-//                         room for the entry's index in 32 bits)
-//        1025..4096       one CTA of 128 or 256, LSD radix sort in shared memory
+//        33..1024         one warp, bitonic network in registers
+//        1025..4096       one CTA of two or four warps, the same network merged
+//                         through shared memory (both: an LSD radix sort in
+//                         shared memory where the coarse ids leave no room for
+//                         the entry's index in 32 bits)
 //        4097..12288      one CTA of 1024, LSD radix sort in shared memory
 //        larger           one CTA, dense accumulator + presence bitmap
 //        (a level whose coarse ids fit contract_smem_cn merges every long row
@@ -1317,22 +1318,30 @@ constexpr int WS_LONG_WARPS = 4, WS_LONG_NR = 32;     // rows of up to 1024 entr
 constexpr int ws_idx_bits(int nr) { return nr <= 1 ? 5 : 1 + ws_idx_bits(nr / 2); }
 constexpr int ws_buf(int nr) { return 33 * nr + 1; }   // 32 nr + 1 words, one pad every 32
 
-// Row c (len <= 32 * NR entries), gathered, sorted, merged and written to
-// out_k / out_w in ascending order; returns the unique count (all lanes).  buf:
-// 2 * ws_buf(NR) words.
-template <int NR>
-__device__ int warp_sort_row(const ContractSrc &src, int32_t c, const RowInfo &r, int32_t len, uint32_t *buf,
-                             int32_t *__restrict__ out_k, int32_t *__restrict__ out_w, int wcheck, unsigned *status)
+// Row c (len <= 32 * NR * W entries) by W warps (one, or the whole CTA): gathered,
+// sorted, merged and written to out_k / out_w in ascending order; returns the unique
+// count (all threads).  buf: 2 * ws_buf(NR * W) words; sh: W > 1 only.
+template <int W> struct SortShared {
+    int32_t scan[2 * W + 2];
+    long long wsum[W];
+    unsigned last[W];
+};
+
+template <int NR, int W>
+__device__ int sort_row(const ContractSrc &src, int32_t c, const RowInfo &r, int32_t len, uint32_t *buf,
+                        int32_t *__restrict__ out_k, int32_t *__restrict__ out_w, int wcheck, unsigned *status,
+                        SortShared<W> *sh)
 {
-    constexpr int IDX = ws_idx_bits(NR);
+    constexpr int IDX = ws_idx_bits(NR * W);
+    constexpr int G = 32 * W;
     constexpr int D = NR < 8 ? NR : 8;   // loads of a lane in flight: the entries, then their coarse ids
-    const int lane = threadIdx.x & 31;
-    uint32_t *pre = buf, *sk = buf + ws_buf(NR);   // pre holds the weights until the sorted words fetched them
+    const int lane = threadIdx.x & 31, t = threadIdx.x % G;
+    uint32_t *pre = buf, *sk = buf + ws_buf(NR * W);   // pre holds the weights until the sorted words fetched them
     unsigned x[NR];
     long long ws = 0;
 #pragma unroll
     for (int b = 0; b < NR; b += D) {
-        if (b * 32 >= len) {   // (uniform over the warp)
+        if (b * G >= len) {   // (uniform over the group)
 #pragma unroll
             for (int q = 0; q < D; q++) x[b + q] = hp::WORD_NONE;
             continue;
@@ -1340,30 +1349,36 @@ __device__ int warp_sort_row(const ContractSrc &src, int32_t c, const RowInfo &r
         int32_t a[D], w[D];
 #pragma unroll
         for (int q = 0; q < D; q++) {
-            const int i = (b + q) * 32 + lane;
+            const int i = (b + q) * G + t;
             const int32_t j = i < r.l0 ? r.s0 + i : r.s1 + (i - r.l0);
             a[q] = i < len ? src.adjncy[j] : -1;
             w[q] = i < len ? src.adjwgt[j] : 0;
         }
 #pragma unroll
         for (int q = 0; q < D; q++) {
-            const int i = (b + q) * 32 + lane;
+            const int i = (b + q) * G + t;
             const int32_t k = a[q] >= 0 ? src.cmap[a[q]] : c;
             x[b + q] = k == c ? hp::WORD_NONE : ((unsigned)k << IDX) | (unsigned)i;
             if (k != c) ws += w[q];
             pre[i] = (uint32_t)w[q];
         }
     }
-    if (wcheck) group_weight_range<32>(ws, nullptr, status);
-    __syncwarp();
-    hp::warp_sort_words<NR>(x);
+    if (wcheck) group_weight_range<G>(ws, W > 1 ? sh->wsum : nullptr, status);
+    group_sync<G>();
+    if constexpr (W == 1) hp::warp_sort_words<NR>(x);
+    else hp::cta_sort_words<NR, W>(x, sk);
     uint32_t w[NR];
-    const unsigned last = __shfl_up_sync(HP_FULL_MASK, x[NR - 1], 1);
+    unsigned last = __shfl_up_sync(HP_FULL_MASK, x[NR - 1], 1);   // the word before this thread's
+    if constexpr (W > 1) {
+        if (lane == 31) sh->last[t >> 5] = x[NR - 1];
+        __syncthreads();
+        if (lane == 0 && t > 0) last = sh->last[(t >> 5) - 1];
+    }
     unsigned heads = 0u;   // bit q: word q starts a run
     uint32_t wsum = 0;
 #pragma unroll
     for (int q = 0; q < NR; q++) {
-        const unsigned prev = q > 0 ? x[q > 0 ? q - 1 : 0] : (lane > 0 ? last : hp::WORD_NONE);
+        const unsigned prev = q > 0 ? x[q > 0 ? q - 1 : 0] : (t > 0 ? last : hp::WORD_NONE);
         const bool valid = x[q] != hp::WORD_NONE;
         w[q] = valid ? pre[x[q] & ((1u << IDX) - 1u)] : 0u;
         if (valid && (x[q] >> IDX) != (prev >> IDX)) heads |= 1u << q;
@@ -1371,8 +1386,8 @@ __device__ int warp_sort_row(const ContractSrc &src, int32_t c, const RowInfo &r
     }
     int o, U;
     uint32_t p, wtot;
-    group_excl_scan2<32>(__popc(heads), wsum, &o, &p, &U, &wtot, nullptr);
-    __syncwarp();
+    group_excl_scan2<G>(__popc(heads), wsum, &o, &p, &U, &wtot, W > 1 ? sh->scan : nullptr);
+    group_sync<G>();
 #pragma unroll
     for (int q = 0; q < NR; q++) {
         if ((heads >> q) & 1u) {
@@ -1382,14 +1397,14 @@ __device__ int warp_sort_row(const ContractSrc &src, int32_t c, const RowInfo &r
         }
         p += w[q];
     }
-    if (lane == 31) pre[U + (U >> 5)] = wtot;
-    __syncwarp();
-    for (int i = lane; i < U; i += 32) {
+    if (t == G - 1) pre[U + (U >> 5)] = wtot;
+    group_sync<G>();
+    for (int i = t; i < U; i += G) {
         const int e = i + (i >> 5), e1 = i + 1 + ((i + 1) >> 5);
         out_k[i] = (int32_t)sk[e];
         out_w[i] = (int32_t)(pre[e1] - pre[e]);
     }
-    __syncwarp();
+    group_sync<G>();
     return U;
 }
 
@@ -1413,14 +1428,39 @@ contract_warp_sort_kernel(const int32_t *__restrict__ list, const int32_t *__res
         const int32_t off = toff[c];
         int U;
         if (MAXNR <= 8) {
-            if (len <= 64) U = warp_sort_row<2>(src, c, r, len, buf, tk + off, tw + off, wcheck, status);
-            else if (len <= 128) U = warp_sort_row<4>(src, c, r, len, buf, tk + off, tw + off, wcheck, status);
-            else U = warp_sort_row<8>(src, c, r, len, buf, tk + off, tw + off, wcheck, status);
+            if (len <= 64) U = sort_row<2, 1>(src, c, r, len, buf, tk + off, tw + off, wcheck, status, nullptr);
+            else if (len <= 128) U = sort_row<4, 1>(src, c, r, len, buf, tk + off, tw + off, wcheck, status, nullptr);
+            else U = sort_row<8, 1>(src, c, r, len, buf, tk + off, tw + off, wcheck, status, nullptr);
         } else {
-            if (len <= 512) U = warp_sort_row<16>(src, c, r, len, buf, tk + off, tw + off, wcheck, status);
-            else U = warp_sort_row<MAXNR>(src, c, r, len, buf, tk + off, tw + off, wcheck, status);
+            if (len <= 512) U = sort_row<16, 1>(src, c, r, len, buf, tk + off, tw + off, wcheck, status, nullptr);
+            else U = sort_row<MAXNR, 1>(src, c, r, len, buf, tk + off, tw + off, wcheck, status, nullptr);
         }
         if ((threadIdx.x & 31) == 0) ucnt[c] = U;
+    }
+}
+
+// Rows of up to 1024 * W entries, a CTA of W warps per row: a warp's network per 1024
+// entries, merged through shared memory.  Against the radix sorts and the accumulator
+// kernels below, rows of 1025-4096 entries: contraction of R-MAT scale 22 41.0 -> 35.7
+// ms, of scale 20 9.0 -> 7.6.
+template <int W>
+__global__ void __launch_bounds__(32 * W, 16 / W)
+contract_cta_sort_kernel(const int32_t *__restrict__ list, const int32_t *__restrict__ d_count, ContractSrc src,
+                         const int32_t *__restrict__ toff, int32_t *__restrict__ tk, int32_t *__restrict__ tw,
+                         int32_t *__restrict__ ucnt, int wcheck, unsigned *status)
+{
+    hp::pdl_wait();
+    __shared__ uint32_t s_buf[2 * ws_buf(WS_LONG_NR * W)];
+    __shared__ SortShared<W> sh;
+    const int32_t cnt = *d_count;
+    for (int32_t li = blockIdx.x; li < cnt; li += gridDim.x) {
+        const int32_t c = list[li];
+        RowInfo r;
+        int32_t len;
+        src.row(c, r, len);
+        const int32_t off = toff[c];
+        const int U = sort_row<WS_LONG_NR, W>(src, c, r, len, s_buf, tk + off, tw + off, wcheck, status, &sh);
+        if (threadIdx.x == 0) ucnt[c] = U;
     }
 }
 
@@ -2169,6 +2209,8 @@ int contract_level(hp_context *c, HpLevel &g, int32_t cn, HpLevel &cg)
         // register networks where key and index fit a word, else the radix sorts
         const bool words_short = !c->wide_rows && kbits + ws_idx_bits(WS_SHORT_NR) <= 32;
         const bool words_long = !c->wide_rows && kbits + ws_idx_bits(WS_LONG_NR) <= 32;
+        const bool words_cta2 = !c->wide_rows && kbits + ws_idx_bits(WS_LONG_NR * 2) <= 32;
+        const bool words_cta4 = !c->wide_rows && kbits + ws_idx_bits(WS_LONG_NR * 4) <= 32;
         if (h.cnt[0] > 0 && words_short)
             HP_LAUNCH(c, (contract_warp_sort_kernel<WS_SHORT_WARPS, WS_SHORT_NR>),
                       (unsigned)std::min<int64_t>((h.cnt[0] + WS_SHORT_WARPS - 1) / WS_SHORT_WARPS, c->sm_count * 8),
@@ -2178,6 +2220,12 @@ int contract_level(hp_context *c, HpLevel &g, int32_t cn, HpLevel &cg)
                       (unsigned)std::min<int64_t>((h.sub[0] + WS_LONG_WARPS - 1) / WS_LONG_WARPS, c->sm_count * 6),
                       32 * WS_LONG_WARPS, 0, lists + 3 * (int64_t)cn, &sub_counts[0], src, toff, tk, tw, ucnt, wchk,
                       c->d_status);
+        if (h.sub[1] > 0 && words_cta2)
+            HP_LAUNCH(c, contract_cta_sort_kernel<2>, (unsigned)std::min<int64_t>(h.sub[1], c->sm_count * 16), 64, 0,
+                      lists + 4 * (int64_t)cn, &sub_counts[1], src, toff, tk, tw, ucnt, wchk, c->d_status);
+        if (h.sub[2] > 0 && words_cta4)
+            HP_LAUNCH(c, contract_cta_sort_kernel<4>, (unsigned)std::min<int64_t>(h.sub[2], c->sm_count * 8), 128, 0,
+                      lists + 5 * (int64_t)cn, &sub_counts[2], src, toff, tk, tw, ucnt, wchk, c->d_status);
         if (h.cnt[0] > 0 && !words_short)
             HP_LAUNCH(c, contract_warp_radix_kernel,
                       (unsigned)std::min<int64_t>((h.cnt[0] + WROW_WARPS - 1) / WROW_WARPS, c->sm_count * 6),
@@ -2187,8 +2235,9 @@ int contract_level(hp_context *c, HpLevel &g, int32_t cn, HpLevel &cg)
         const bool smem_dense = cn <= c->tune.contract_smem_cn;
         // the lists those kernels take: the rows that a register network does not
         const struct { int32_t list, n; int32_t *count; } accl[3] = {
-            {words_long ? 4 : 1, words_long ? h.sub[1] : h.cnt[1], words_long ? &sub_counts[1] : &counts[1]},
-            {5, words_long ? h.sub[2] : 0, &sub_counts[2]},
+            {words_long ? 4 : 1, words_cta2 ? 0 : words_long ? h.sub[1] : h.cnt[1],
+             words_long ? &sub_counts[1] : &counts[1]},
+            {5, words_cta4 || !words_long ? 0 : h.sub[2], &sub_counts[2]},
             {2, h.cnt[2], &counts[2]}};
         const int64_t acc_rows = (int64_t)accl[0].n + accl[1].n + accl[2].n;
         if (smem_dense) {
@@ -2223,12 +2272,12 @@ int contract_level(hp_context *c, HpLevel &g, int32_t cn, HpLevel &cg)
                       (unsigned)std::min<int64_t>(h.sub[0], c->sm_count * 12), MROW_THREADS,
                       (cta_radix_smem<MROW_THREADS, MROW_MAX>()), lists + 3 * (int64_t)cn, &sub_counts[0], src, toff,
                       tk, tw, ucnt, kbits, 0, wchk, c->d_status);
-        if (!smem_dense && !hybrid && h.sub[1] > 0)
+        if (!smem_dense && !hybrid && !words_cta2 && h.sub[1] > 0)
             HP_LAUNCH(c, (contract_cta_radix_kernel<NROW_THREADS, NROW_MAX>),
                       (unsigned)std::min<int64_t>(h.sub[1], c->sm_count * 6), NROW_THREADS,
                       (cta_radix_smem<NROW_THREADS, NROW_MAX>()), lists + 4 * (int64_t)cn, &sub_counts[1], src, toff,
                       tk, tw, ucnt, kbits, MROW_MAX, wchk, c->d_status);
-        if (!smem_dense && !hybrid && h.sub[2] > 0)
+        if (!smem_dense && !hybrid && !words_cta4 && h.sub[2] > 0)
             HP_LAUNCH(c, (contract_cta_radix_kernel<CROW_THREADS, CROW_MAX>),
                       (unsigned)std::min<int64_t>(h.sub[2], c->sm_count * 3), CROW_THREADS,
                       (cta_radix_smem<CROW_THREADS, CROW_MAX>()), lists + 5 * (int64_t)cn, &sub_counts[2], src, toff,

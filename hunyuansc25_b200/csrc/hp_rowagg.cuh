@@ -178,7 +178,35 @@ __device__ __forceinline__ int sort_staged_row(const unsigned *key, int32_t *wgt
     return u;
 }
 
-// The same over 32 * NR words held by a warp, NR per lane: any order in, ascending
+// The strides below 32 * NR / 2 of a merge over the 32 * NR words of a warp (NR per
+// lane), from lane distance m down: m = 16 after a step at 16 * NR across lanes or more.
+template <int NR>
+__device__ __forceinline__ void warp_merge_words(unsigned (&x)[NR], int m)
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (; m > 0; m >>= 1) {
+        const bool low = (lane & m) == 0;
+#pragma unroll
+        for (int r = 0; r < NR; r++) {
+            const unsigned a = __shfl_xor_sync(HP_FULL_MASK, x[r], m);
+            x[r] = low ? min(x[r], a) : max(x[r], a);
+        }
+    }
+#pragma unroll
+    for (int stride = NR >> 1; stride > 0; stride >>= 1)
+#pragma unroll
+        for (int i = 0; i < NR; i++) {
+            const int j = i ^ stride;
+            if (j > i) {
+                const unsigned a = x[i], b = x[j];
+                x[i] = min(a, b);
+                x[j] = max(a, b);
+            }
+        }
+}
+
+// The network over 32 * NR words held by a warp, NR per lane: any order in, ascending
 // order out with lane l holding positions l * NR .. l * NR + NR - 1.
 template <int NR>
 __device__ __forceinline__ void warp_sort_words(unsigned (&x)[NR])
@@ -187,36 +215,48 @@ __device__ __forceinline__ void warp_sort_words(unsigned (&x)[NR])
     sort_words<NR, NR>(x);
 #pragma unroll 1
     for (int g = 2; g <= 32; g <<= 1) {   // merges of g lanes' runs
-        {
-            const bool low = (lane & (g >> 1)) == 0;
+        const bool low = (lane & (g >> 1)) == 0;
 #pragma unroll
-            for (int r = 0; r < (NR + 1) / 2; r++) {
-                const unsigned a = __shfl_xor_sync(HP_FULL_MASK, x[NR - 1 - r], g - 1);
-                const unsigned b = __shfl_xor_sync(HP_FULL_MASK, x[r], g - 1);
-                x[r] = low ? min(x[r], a) : max(x[r], a);
-                if (NR > 1) x[NR - 1 - r] = low ? min(x[NR - 1 - r], b) : max(x[NR - 1 - r], b);
-            }
+        for (int r = 0; r < (NR + 1) / 2; r++) {
+            const unsigned a = __shfl_xor_sync(HP_FULL_MASK, x[NR - 1 - r], g - 1);
+            const unsigned b = __shfl_xor_sync(HP_FULL_MASK, x[r], g - 1);
+            x[r] = low ? min(x[r], a) : max(x[r], a);
+            if (NR > 1) x[NR - 1 - r] = low ? min(x[NR - 1 - r], b) : max(x[NR - 1 - r], b);
         }
+        warp_merge_words<NR>(x, g >> 2);
+    }
+}
+
+// The network over 32 * NR * W words held by a CTA of W warps, thread t holding positions
+// t * NR .. t * NR + NR - 1 of the result.  Steps across warps go through buf (33 * NR * W
+// words, one pad every 32: a thread's NR consecutive words hit every bank once).
+template <int NR, int W>
+__device__ __forceinline__ void cta_sort_words(unsigned (&x)[NR], unsigned *buf)
+{
+    const int t = threadIdx.x, wid = t >> 5;
+    warp_sort_words<NR>(x);
 #pragma unroll 1
-        for (int m = g >> 2; m > 0; m >>= 1) {
-            const bool low = (lane & m) == 0;
+    for (int g = 2; g <= W; g <<= 1) {           // merges of g warps' runs
+#pragma unroll 1
+        for (int d = g; d >= 2; d >>= 1) {       // mirrored over g warps, then strides of g / 4 .. 1 warps
+            const bool mirror = d == g;
+            const int other = mirror ? 0 : (d >> 1);
 #pragma unroll
             for (int r = 0; r < NR; r++) {
-                const unsigned a = __shfl_xor_sync(HP_FULL_MASK, x[r], m);
+                const int e = t * NR + r;
+                buf[e + (e >> 5)] = x[r];
+            }
+            __syncthreads();
+            const bool low = (wid & (d >> 1)) == 0;
+#pragma unroll
+            for (int r = 0; r < NR; r++) {
+                const int e = mirror ? ((t * NR + r) ^ (g * 32 * NR - 1)) : ((t * NR + r) ^ (other * 32 * NR));
+                const unsigned a = buf[e + (e >> 5)];
                 x[r] = low ? min(x[r], a) : max(x[r], a);
             }
+            __syncthreads();
         }
-#pragma unroll
-        for (int stride = NR >> 1; stride > 0; stride >>= 1)
-#pragma unroll
-            for (int i = 0; i < NR; i++) {
-                const int j = i ^ stride;
-                if (j > i) {
-                    const unsigned a = x[i], b = x[j];
-                    x[i] = min(a, b);
-                    x[j] = max(a, b);
-                }
-            }
+        warp_merge_words<NR>(x, 16);
     }
 }
 
