@@ -2691,8 +2691,11 @@ __device__ __forceinline__ unsigned cl_size()
 // remote) are visible after it.
 __device__ __forceinline__ void cl_sync()
 {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n"
-                 "barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    // (not the .aligned forms: a warp may reach this diverged, and its parts would then
+    // arrive as if each were the whole warp)
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release;\n"
+                 "barrier.cluster.wait.acquire;" ::: "memory");
 }
 
 // The address of CTA `rank`'s copy of a shared-memory object.
@@ -2835,6 +2838,9 @@ refine_cluster_kernel(SmallLevel a)
     const int32_t vpw = (n + tw - 1) / tw;   // the warp's vertices [vb, ve)
     const int32_t vb = min(n, gw * vpw), ve = min(n, vb + vpw);
     int buf = 0;                             // exchange buffer (uniform over the cluster)
+    // no CTA writes another's shared memory before that CTA runs: being placed together
+    // does not mean having started
+    cl_sync();
     if (a.learned_mlp) hp::mlp_load_smem(s_mlp, a.mlp_params);
     // ---- the level's setup, as the launches of the multi-kernel levels:
     // gain-row capacities min(deg, k) and offsets, cleared locks and dirty
