@@ -604,6 +604,54 @@ struct RowBest {
     int32_t b, np;
 };
 
+// One gain row of more than 32 entries by a whole warp, the result in every lane:
+// conn(own), the best other part among those that ok() takes (the first, i.e. lowest,
+// of the most connected), the row's weight and its connected parts.  DEPTH loads per
+// lane are in flight (ROW_DEEP: a dense row of 256 parts is one batch; walked an entry
+// at a time, each load waited for the one before), and the warp reduces by redux.sync:
+// the weight and every connectivity are below 2^31.  The launched kernels take ROW_DEEP
+// on levels with dense rows of more than 64 parts, where most rows are long (R-MAT scale
+// 22, learned: selections 15.8 -> 12.2 ms), and two loads elsewhere: the registers of
+// eight cost the short rows' occupancy (RGG 2^24).
+constexpr int ROW_DEEP = 8, ROW_FLAT = 2;
+template <int DEPTH, class F>
+__device__ __forceinline__ RowBest warp_row_best(const int32_t *__restrict__ gpart, const int32_t *__restrict__ gconn,
+                                                 int32_t o, int32_t len, int32_t p, int32_t k, F &&ok)
+{
+    const int lane = threadIdx.x & 31;
+    unsigned lpc = 0, lbc = 0, lnp = 0, lwd = 0, lb = 0xffffffffu;
+    const bool dense = len == k;   // entry j is part j
+    for (int32_t j0 = lane; __any_sync(HP_FULL_MASK, j0 < len); j0 += 32 * DEPTH) {
+        int32_t q[DEPTH], c[DEPTH];
+#pragma unroll
+        for (int i = 0; i < DEPTH; i++) {
+            const int32_t j = j0 + 32 * i;
+            q[i] = j >= len ? -1 : (dense ? j : gpart[o + j]);
+            c[i] = j < len ? gconn[o + j] : 0;
+        }
+        bool end = false;   // padding runs to the end of the row
+#pragma unroll
+        for (int i = 0; i < DEPTH; i++) {
+            end |= q[i] < 0;
+            if (q[i] < 0) continue;
+            const unsigned cq = (unsigned)c[i];
+            lwd += cq;
+            lnp += cq > 0u;
+            if (q[i] == p) { lpc = cq; continue; }
+            if (cq > lbc && ok(q[i])) { lbc = cq; lb = (unsigned)q[i]; }
+        }
+        if (__any_sync(HP_FULL_MASK, end)) break;
+    }
+    RowBest r;
+    r.pc = __reduce_add_sync(HP_FULL_MASK, lpc);   // (one lane has it)
+    r.np = (int32_t)__reduce_add_sync(HP_FULL_MASK, lnp);
+    r.wd = __reduce_add_sync(HP_FULL_MASK, lwd);
+    const unsigned m = __reduce_max_sync(HP_FULL_MASK, lbc);
+    r.bc = m;
+    r.b = (int32_t)__reduce_min_sync(HP_FULL_MASK, lbc == m ? lb : 0xffffffffu);   // none: -1
+    return r;
+}
+
 // Called by every lane of the warp, each with its own row (len 0 for none).
 // Rows of at most 32 entries are walked by their lane; longer rows by the
 // whole warp, one row at a time, reduced in the serial walk's order.
@@ -626,28 +674,8 @@ __device__ __forceinline__ RowBest row_best(const int32_t *__restrict__ gpart, c
         cm &= cm - 1;
         const int32_t so = __shfl_sync(HP_FULL_MASK, o, src), sl = __shfl_sync(HP_FULL_MASK, len, src);
         const int32_t sp = __shfl_sync(HP_FULL_MASK, p, src);
-        int32_t lpc = 0, lbc = 0, lb = -1, lnp = 0;
-        long long lwd = 0;
-        const bool dense = sl == k;   // entry j is part j
-        for (int32_t j = lane; j < sl; j += 32) {
-            const int32_t q = dense ? j : gpart[so + j];
-            if (q < 0) break;   // padding runs to the end of the row
-            const int32_t cq = gconn[so + j];
-            lwd += cq;
-            lnp += cq > 0;
-            if (q == sp) { lpc = cq; continue; }
-            if (cq > lbc) { lbc = cq; lb = q; }
-        }
-        lpc = hp::warp_sum(lpc);
-        lnp = hp::warp_sum(lnp);
-        lwd = hp::warp_sum64(lwd);
-#pragma unroll
-        for (int sh = 16; sh > 0; sh >>= 1) {
-            const int32_t ob = __shfl_xor_sync(HP_FULL_MASK, lb, sh);
-            const int32_t oc = __shfl_xor_sync(HP_FULL_MASK, lbc, sh);
-            if (ob >= 0 && (lb < 0 || oc > lbc || (oc == lbc && ob < lb))) { lb = ob; lbc = oc; }
-        }
-        if (lane == src) { r.pc = lpc; r.bc = lbc; r.b = lb; r.wd = lwd; r.np = lnp; }
+        const RowBest w = warp_row_best<ROW_DEEP>(gpart, gconn, so, sl, sp, k, [](int32_t) { return true; });
+        if (lane == src) r = w;
     }
     return r;
 }
@@ -705,7 +733,7 @@ __device__ __forceinline__ int coop_queue(CoopRows<NT> &S, bool coop, int32_t o,
 
 // row_best with the CTA's long rows shared by all its warps (CoopRows).  All NT
 // threads call it.
-template <int NT>
+template <int NT, int DEPTH>
 __device__ __forceinline__ RowBest row_best_cta(CoopRows<NT> &S, const int32_t *__restrict__ gpart,
                                                 const int32_t *__restrict__ gconn, int32_t o, int32_t len,
                                                 int32_t p, int32_t k)
@@ -724,28 +752,8 @@ __device__ __forceinline__ RowBest row_best_cta(CoopRows<NT> &S, const int32_t *
     const int nc = S.n;
     for (int i = wid; i < nc; i += NT / 32) {
         const int32_t so = S.o[i], sl = S.len[i], sp = S.p[i];
-        int32_t lpc = 0, lbc = 0, lb = -1, lnp = 0;
-        long long lwd = 0;
-        const bool dense = sl == k;   // entry j is part j
-        for (int32_t j = lane; j < sl; j += 32) {
-            const int32_t q = dense ? j : gpart[so + j];
-            if (q < 0) break;   // padding runs to the end of the row
-            const int32_t cq = gconn[so + j];
-            lwd += cq;
-            lnp += cq > 0;
-            if (q == sp) { lpc = cq; continue; }
-            if (cq > lbc) { lbc = cq; lb = q; }
-        }
-        lpc = hp::warp_sum(lpc);
-        lnp = hp::warp_sum(lnp);
-        lwd = hp::warp_sum64(lwd);
-#pragma unroll
-        for (int sh = 16; sh > 0; sh >>= 1) {
-            const int32_t ob = __shfl_xor_sync(HP_FULL_MASK, lb, sh);
-            const int32_t oc = __shfl_xor_sync(HP_FULL_MASK, lbc, sh);
-            if (ob >= 0 && (lb < 0 || oc > lbc || (oc == lbc && ob < lb))) { lb = ob; lbc = oc; }
-        }
-        if (lane == 0) { S.pc[i] = lpc; S.bc[i] = lbc; S.b[i] = lb; S.wd[i] = lwd; S.np[i] = lnp; }
+        const RowBest w = warp_row_best<DEPTH>(gpart, gconn, so, sl, sp, k, [](int32_t) { return true; });
+        if (lane == 0) { S.pc[i] = w.pc; S.bc[i] = w.bc; S.b[i] = w.b; S.wd[i] = w.wd; S.np[i] = w.np; }
     }
     __syncthreads();
     if (my >= 0) { r.pc = S.pc[my]; r.bc = S.bc[my]; r.b = S.b[my]; r.wd = S.wd[my]; r.np = S.np[my]; }
@@ -753,7 +761,8 @@ __device__ __forceinline__ RowBest row_best_cta(CoopRows<NT> &S, const int32_t *
 }
 
 // ---- LP ------------------------------------------------------------------------
-__global__ void __launch_bounds__(256)
+template <int DEPTH>
+__global__ void __launch_bounds__(256, DEPTH == ROW_FLAT ? 8 : 5)
 lp_select_kernel(int32_t n, const int32_t *__restrict__ goff, const int32_t *__restrict__ gpart,
                  const int32_t *__restrict__ gconn, const int32_t *__restrict__ where,
                  const int8_t *__restrict__ lock, int finest, int32_t *__restrict__ dest,
@@ -774,7 +783,7 @@ lp_select_kernel(int32_t n, const int32_t *__restrict__ goff, const int32_t *__r
         len = goff[v + 1] - o;
         if (copy) bcp.best_where[v] = p;
     }
-    const RowBest rb = row_best_cta<256>(S, gpart, gconn, o, len, p, k);
+    const RowBest rb = row_best_cta<256, DEPTH>(S, gpart, gconn, o, len, p, k);
     const int64_t pc = rb.pc, bc = rb.bc;
     const int32_t b = rb.b;
     if (v < n) {
@@ -826,7 +835,7 @@ lp_select_learned_kernel(int32_t n, const int32_t *__restrict__ goff, const int3
         len = goff[v + 1] - o;
         if (copy) bcp.best_where[v] = p;
     }
-    const RowBest rb = row_best_cta<256>(S, gpart, gconn, o, len, p, k);
+    const RowBest rb = row_best_cta<256, ROW_DEEP>(S, gpart, gconn, o, len, p, k);
     if (v < n) {
         const int64_t pc = rb.pc, bc = rb.bc, wd = rb.wd;
         const int32_t b = rb.b, np = rb.np;
@@ -1538,7 +1547,7 @@ __device__ __forceinline__ void undersized_block(int32_t k, const unsigned long 
 constexpr int RB_TILE = 256;
 constexpr int RB_COOP = 32;   // weak rebalance: longer gain rows are walked by a warp
 
-template <bool STRONG>
+template <bool STRONG, int DEPTH>
 __global__ void __launch_bounds__(RB_TILE)
 rb_candidates_kernel(int32_t n, const int32_t *__restrict__ where, const int32_t *__restrict__ vwgt,
                      const unsigned long long *__restrict__ pw, const int64_t *__restrict__ maxp,
@@ -1592,23 +1601,8 @@ rb_candidates_kernel(int32_t n, const int32_t *__restrict__ where, const int32_t
         const int nc = S.n;
         for (int i = threadIdx.x >> 5; i < nc; i += RB_TILE / 32) {
             const int32_t so = S.o[i], sl = S.len[i], sp = S.p[i];
-            int32_t lpc = 0, lbc = 0, lb = -1;
-            const bool dense = sl == k;   // entry j is part j
-            for (int32_t j = lane; j < sl; j += 32) {
-                const int32_t q = dense ? j : gpart[so + j];
-                if (q < 0) break;   // padding runs to the end of the row
-                const int32_t cq = gconn[so + j];
-                if (q == sp) lpc = cq;
-                if (ufl[q] && cq > lbc) { lbc = cq; lb = q; }
-            }
-            lpc = hp::warp_sum(lpc);
-#pragma unroll
-            for (int sh = 16; sh > 0; sh >>= 1) {
-                const int32_t ob = __shfl_xor_sync(HP_FULL_MASK, lb, sh);
-                const int32_t oc = __shfl_xor_sync(HP_FULL_MASK, lbc, sh);
-                if (ob >= 0 && (lb < 0 || oc > lbc || (oc == lbc && ob < lb))) { lb = ob; lbc = oc; }
-            }
-            if (lane == 0) { S.pc[i] = lpc; S.bc[i] = lbc; S.b[i] = lb; }
+            const RowBest w = warp_row_best<DEPTH>(gpart, gconn, so, sl, sp, k, [&](int32_t q) { return ufl[q] != 0; });
+            if (lane == 0) { S.pc[i] = w.pc; S.bc[i] = w.bc; S.b[i] = w.b; }
         }
         __syncthreads();
         if (my >= 0) { pc = S.pc[my]; bc = S.bc[my]; b = S.b[my]; }
@@ -1987,6 +1981,7 @@ struct RefineBufs {
     int32_t small_max;  // longest row of at most bigd entries (picks the gain kernel's network)
     bool huge_rows;     // the level has rows longer than huged
     bool dense_rows;    // the level has rows of at least k entries
+    bool deep_rows;     // and k above 64: most gain rows are long (ROW_DEEP)
 };
 
 // scalar slots used by refinement
@@ -2092,9 +2087,14 @@ int rank_candidates(hp_context *c, HpLevel &g, RefineBufs &B, int32_t k, int32_t
     const int64_t ct = ((int64_t)n + RB_TILE - 1) / RB_TILE;
     const int64_t rt = ((int64_t)n + RK_TILE) / RK_TILE;   // a tile holds index cnt <= n
     if (ct > c->lb_cap || 2 * rt > c->lb_cap) return HP_ERR_INTERNAL;
-    HP_LAUNCH(c, rb_candidates_kernel<STRONG>, (unsigned)ct, RB_TILE, 0, n, g.where, g.vwgt, B.pw, B.maxp, B.opt,
-              B.goff, B.gpart, B.gconn, B.und, (const int32_t *)&sc[S_NU], k, B.K, B.V, B.dest, d_cnt,
-              c->lb_status, c->lb_ctl, c->d_status, B.ufl, B.pregain, bcp);
+    auto launch = [&](auto kernel) -> int {
+        HP_LAUNCH(c, kernel, (unsigned)ct, RB_TILE, 0, n, g.where, g.vwgt, B.pw, B.maxp, B.opt, B.goff, B.gpart,
+                  B.gconn, B.und, (const int32_t *)&sc[S_NU], k, B.K, B.V, B.dest, d_cnt, c->lb_status, c->lb_ctl,
+                  c->d_status, B.ufl, B.pregain, bcp);
+        return HP_OK;
+    };
+    HP_TRY(B.deep_rows ? launch(rb_candidates_kernel<STRONG, ROW_DEEP>)
+                       : launch(rb_candidates_kernel<STRONG, ROW_FLAT>));
     bool in_tmp = false;
     HP_TRY(hp_sort_pairs(c, B.K, B.V, B.K2, B.V2, n, d_cnt, key_bits_for(k), &in_tmp));
     *Ks = in_tmp ? B.K2 : B.K;
@@ -2484,9 +2484,14 @@ int pass_propose(hp_context *c, HpLevel &g, RefineBufs &B, const PassCfg &P, int
             HP_LAUNCH(c, lp_select_learned_kernel, nblk(n), 256, 0, n, B.goff, B.gpart, B.gconn, g.where, g.xadj,
                       B.lock, P.finest ? 1 : 0, B.pw, B.maxp, B.opt, c->mlp_params, c->mlp_threshold, B.dest,
                       B.pregain, &sc[S_NCAND], gate, k, B.prune, &sc[S_NCANDP], J.flag, best_copy(B, P));
-        if (both_lp || !learned_pass)
-            HP_LAUNCH(c, lp_select_kernel, nblk(n), 256, 0, n, B.goff, B.gpart, B.gconn, g.where, B.lock,
+        if (both_lp || !learned_pass) {
+            auto launch = [&](auto kernel) -> int {
+                HP_LAUNCH(c, kernel, nblk(n), 256, 0, n, B.goff, B.gpart, B.gconn, g.where, B.lock,
                       P.finest ? 1 : 0, B.dest, B.pregain, &sc[S_NCAND], gate, k, best_copy(B, P));
+                return HP_OK;
+            };
+            HP_TRY(B.deep_rows ? launch(lp_select_kernel<ROW_DEEP>) : launch(lp_select_kernel<ROW_FLAT>));
+        }
         if (P.recording)
             HP_LAUNCH(c, log_candidates_kernel, nblk(n), 256, 0, n, B.goff, B.gpart, B.gconn, g.where, g.xadj,
                       P.finest ? 1 : 0, B.pw, B.maxp, B.opt, B.dest, B.pregain, B.recof, c->log_x, c->log_v,
@@ -3102,22 +3107,8 @@ refine_cluster_kernel(SmallLevel a)
                         cm &= cm - 1;
                         const int32_t so = __shfl_sync(HP_FULL_MASK, o, src), sl = __shfl_sync(HP_FULL_MASK, len, src);
                         const int32_t sp_ = __shfl_sync(HP_FULL_MASK, p, src);
-                        int32_t lpc = 0, lbc = 0, lb = -1;
-                        for (int32_t j = lane; j < sl; j += 32) {
-                            const int32_t q = a.gpart[so + j];
-                            if (q < 0) break;
-                            const int32_t cq = a.gconn[so + j];
-                            if (q == sp_) lpc = cq;
-                            if (s_ufl[q] && cq > lbc) { lbc = cq; lb = q; }
-                        }
-                        lpc = hp::warp_sum(lpc);
-#pragma unroll
-                        for (int sh = 16; sh > 0; sh >>= 1) {
-                            const int32_t ob = __shfl_xor_sync(HP_FULL_MASK, lb, sh);
-                            const int32_t oc = __shfl_xor_sync(HP_FULL_MASK, lbc, sh);
-                            if (ob >= 0 && (lb < 0 || oc > lbc || (oc == lbc && ob < lb))) { lb = ob; lbc = oc; }
-                        }
-                        if (lane == src) { pc = lpc; bc = lbc; b = lb; }
+                        const RowBest w = warp_row_best<ROW_DEEP>(a.gpart, a.gconn, so, sl, sp_, k, [&](int32_t q) { return s_ufl[q] != 0; });
+                        if (lane == src) { pc = w.pc; bc = w.bc; b = w.b; }
                     }
                     if (cand) {
                         bool ok = true;
@@ -3624,6 +3615,7 @@ int refine_level(hp_context *c, HpLevel &g, int32_t k, bool finest, const int64_
     B.small_max = ls.small_max;
     B.huge_rows = ls.maxdeg > huged;
     B.dense_rows = ls.maxdeg >= k;
+    B.deep_rows = B.dense_rows && k > 64;
     B.gpart = ralloc_t<int32_t>(c, std::max<int64_t>(g.m, 1));
     B.gconn = ralloc_t<int32_t>(c, std::max<int64_t>(g.m, 1));
     HP_CHECK_OOM(c);
