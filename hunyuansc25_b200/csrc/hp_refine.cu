@@ -219,10 +219,14 @@ struct RebuildRule {
     }
 };
 
-// Rebuild of the listed (dirty) rows of at most S entries (S >= the level's
-// longest short row): 32/S rows per warp, one segment of S lanes per row,
-// sorted and merged by seg_aggregate; dirty flags are cleared.  Rows with
-// deg >= k (k <= S here) are written dense.
+// Rebuild of the listed (dirty) rows of at most S entries (S >= the level's longest
+// short row); dirty flags are cleared.  S/4 lanes per row with four entries each, so a
+// warp has 128/S rows in flight: the rebuild is bound by its chain of loads (row,
+// parts, weights) and exchanges.  The entries are sorted as words (part << ROW_IDX |
+// index) by the network of hp::warp_sort_words over the row's lanes, the weights fetched
+// by the words' indexes, equal parts summed by a segmented scan.  Rows with deg >= k
+// (k <= S here) are written dense.  One entry per lane before: a pass of 41,202 vertices
+// (128^3 grid, 16 CTAs) spent 88 us here.
 // list == nullptr: every vertex with a row of at most bigd (<= S) entries.
 // (warp, nwarps: this warp's index among the nwarps warps sharing the list)
 template <int S>
@@ -233,10 +237,10 @@ __device__ __forceinline__ void gain_seg_rows(int64_t warp, int64_t nwarps, cons
                                               int32_t *__restrict__ gpart, int32_t *__restrict__ gconn, int32_t k,
                                               int32_t *__restrict__ dirty, int32_t bigd = 0)
 {
-    constexpr int R = 32 / S;
-    const int lane = threadIdx.x & 31, sl = lane & (S - 1);
+    constexpr int L = S / 4, R = 32 / L;   // lanes per row, rows per warp
+    const int lane = threadIdx.x & 31, sl = lane & (L - 1);
     for (int64_t i0 = warp * R; i0 < cnt; i0 += nwarps * R) {
-        const int64_t i = i0 + lane / S;
+        const int64_t i = i0 + lane / L;
         int32_t v = -1, b = 0, d = 0;
         if (i < cnt) {
             v = list ? list[i] : (int32_t)i;
@@ -246,22 +250,79 @@ __device__ __forceinline__ void gain_seg_rows(int64_t warp, int64_t nwarps, cons
                 if (sl == 0) dirty[v] = 0;
             } else if (d > bigd) {
                 v = -1;
+                d = 0;
             }
         }
-        int32_t key = hp::KEY_NONE, w = 0;
-        if (v >= 0 && sl < d) {
-            key = where[adjncy[b + sl]];
-            w = adjwgt[b + sl];
+        const int32_t o = v >= 0 ? goff[v] : 0;
+        int32_t a[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) a[q] = sl + q * L < d ? adjncy[b + sl + q * L] : -1;
+        unsigned x[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            x[q] = a[q] >= 0 ? ((unsigned)where[a[q]] << hp::ROW_IDX) | (unsigned)(sl + q * L) : hp::WORD_NONE;
+        hp::lanes_sort_words<4, L>(x);   // lane sl: positions 4 sl .. 4 sl + 3
+        uint32_t w[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            w[q] = x[q] != hp::WORD_NONE ? (uint32_t)adjwgt[b + (x[q] & ((1u << hp::ROW_IDX) - 1u))] : 0u;
+        // w[q]: the weight from entry q to the end of its run -- in the lane, then over
+        // the row's lanes (a lane whose entries are all one run passes on what follows it)
+        const unsigned nx = __shfl_down_sync(HP_FULL_MASK, x[0], 1, L);
+#pragma unroll
+        for (int q = 2; q >= 0; q--)
+            if (hp::same_key(x[q], x[q + 1])) w[q] += w[q + 1];
+        bool open = sl + 1 < L && hp::same_key(x[3], nx);   // the run of entry 3 goes on
+        const bool single = hp::same_key(x[0], x[3]);       // (sorted: all four in one run)
+        uint32_t head = w[0];           // weight of the lane's first run, as far as scanned
+        bool through = single && open;  // it reaches past the lanes scanned so far
+        uint32_t carry = 0;             // what follows entry 3 in its run
+#pragma unroll
+        for (int st = 1; st < L; st <<= 1) {
+            const uint32_t h = __shfl_down_sync(HP_FULL_MASK, head, st, L);
+            const bool t = __shfl_down_sync(HP_FULL_MASK, (int)through, st, L) != 0;
+            if (through) { head += h; through = t; }
         }
-        const int32_t o = v >= 0 ? goff[v] : 0, cap = v >= 0 ? goff[v + 1] - o : 0;
-        const bool dense = v >= 0 && d >= k;
-        if (dense && sl < k) { gpart[o + sl] = sl; gconn[o + sl] = 0; }
+        const uint32_t next = __shfl_down_sync(HP_FULL_MASK, head, 1, L);
+        if (open) carry = next;
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if (carry && hp::same_key(x[q], x[3])) w[q] += carry;
+        const unsigned px = __shfl_up_sync(HP_FULL_MASK, x[3], 1, L);
+        bool hd[4];
+        int u = 0;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const unsigned prev = q > 0 ? x[q > 0 ? q - 1 : 0] : px;
+            hd[q] = x[q] != hp::WORD_NONE && ((q == 0 && sl == 0) || !hp::same_key(x[q], prev));
+            u += hd[q];
+        }
+        int incl = u;
+#pragma unroll
+        for (int st = 1; st < L; st <<= 1) {
+            const int t = __shfl_up_sync(HP_FULL_MASK, incl, st, L);
+            if (sl >= st) incl += t;
+        }
+        const int total = __shfl_sync(HP_FULL_MASK, incl, L - 1, L);
+        int r = incl - u;
+        if (v >= 0 && d >= k) {
+            const unsigned mask = (L == 32 ? 0xffffffffu : ((1u << L) - 1u) << (lane & ~(L - 1)));
+            for (int32_t q = sl; q < k; q += L) { gpart[o + q] = q; gconn[o + q] = 0; }
+            __syncwarp(mask);
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (hd[q]) gconn[o + (x[q] >> hp::ROW_IDX)] = (int32_t)w[q];
+        } else if (v >= 0) {
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (hd[q]) {
+                    gpart[o + r] = (int32_t)(x[q] >> hp::ROW_IDX);
+                    gconn[o + r] = (int32_t)w[q];
+                    r++;
+                }
+            for (int32_t t = total + sl; t < d; t += L) { gpart[o + t] = -1; gconn[o + t] = 0; }
+        }
         __syncwarp();
-        if (dense && key != hp::KEY_NONE) atomicAdd(&gconn[o + key], w);
-        const int c = hp::seg_aggregate<S>(key, w, (v >= 0 && !dense) ? gpart + o : nullptr,
-                                            (v >= 0 && !dense) ? gconn + o : nullptr);
-        if (v >= 0 && !dense)
-            for (int32_t t = c + sl; t < cap; t += S) { gpart[o + t] = -1; gconn[o + t] = 0; }
     }
 }
 

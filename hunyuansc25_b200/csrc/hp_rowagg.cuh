@@ -3,12 +3,12 @@
 // ascending order.  Used by contraction (key = coarse neighbour id, the self
 // key dropped) and by the gain table (key = neighbour's part).
 //
-// Size classes (chosen per row by its entry count):
-//   S   <= 32     one warp, register bitonic sort over the 32 lanes (shuffles)
-//   B   <= CAP    one CTA, shared-memory bitonic sort (CAP = 512 or 4096)
-//   D   larger    one CTA, dense accumulator + presence bitmap over the key
-//                 space, scanned in key order (global scratch per CTA for
-//                 contraction, shared memory for part keys)
+// Size classes (chosen per row by its entry count; the kernels' files give the bounds):
+//   registers   a sorting network over 32-bit words (key and index), by a thread, a few
+//               lanes, a warp or a CTA per row (64-bit entries where they do not fit)
+//   dense       one CTA, dense accumulator + presence bitmap over the key space,
+//               scanned in key order (global scratch per CTA for contraction, shared
+//               memory for part keys)
 // Every class produces the same canonical row, so the class boundaries are a
 // performance choice only.
 #pragma once
@@ -18,44 +18,6 @@
 namespace hp {
 
 constexpr int32_t KEY_NONE = 0x7fffffff;
-
-// Warp-wide aggregation of up to 32 entries already held one per lane.
-// Writes unique keys/sums to out_k/out_w (if non-null) and returns the count
-// (same value in all lanes).
-__device__ __forceinline__ int warp_aggregate32(int32_t key, int32_t w, int32_t *out_k,
-                                                int32_t *out_w)
-{
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int k = 2; k <= 32; k <<= 1) {
-#pragma unroll
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            int32_t pk = __shfl_xor_sync(HP_FULL_MASK, key, j);
-            int32_t pw = __shfl_xor_sync(HP_FULL_MASK, w, j);
-            bool up = (lane & k) == 0;
-            bool lower = (lane & j) == 0;
-            bool take = lower ? (up ? pk < key : pk > key) : (up ? pk > key : pk < key);
-            if (take) { key = pk; w = pw; }
-        }
-    }
-    // suffix sums inside runs of equal keys
-    int32_t s = w;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        int32_t t = __shfl_down_sync(HP_FULL_MASK, s, o);
-        int32_t kk = __shfl_down_sync(HP_FULL_MASK, key, o);
-        if (lane + o < 32 && kk == key) s += t;
-    }
-    int32_t prev = __shfl_up_sync(HP_FULL_MASK, key, 1);
-    bool head = key != KEY_NONE && (lane == 0 || prev != key);
-    unsigned hm = __ballot_sync(HP_FULL_MASK, head);
-    if (head && out_k) {
-        int r = __popc(hm & lanemask_lt());
-        out_k[r] = key;
-        out_w[r] = s;
-    }
-    return __popc(hm);
-}
 
 // ---- one row per thread, in registers ---------------------------------------
 // Entries are packed as key << 32 | weight (padding and dropped keys are
@@ -206,15 +168,16 @@ __device__ __forceinline__ void warp_merge_words(unsigned (&x)[NR], int m)
         }
 }
 
-// The network over 32 * NR words held by a warp, NR per lane: any order in, ascending
-// order out with lane l holding positions l * NR .. l * NR + NR - 1.
-template <int NR>
-__device__ __forceinline__ void warp_sort_words(unsigned (&x)[NR])
+// The network over NR * L words held by L consecutive lanes of a warp, NR per lane: any
+// order in, ascending order out with the group's lane l holding positions l * NR ..
+// l * NR + NR - 1.  All lanes of the warp call it; every group of L sorts its own.
+template <int NR, int L>
+__device__ __forceinline__ void lanes_sort_words(unsigned (&x)[NR])
 {
     const int lane = threadIdx.x & 31;
     sort_words<NR, NR>(x);
 #pragma unroll 1
-    for (int g = 2; g <= 32; g <<= 1) {   // merges of g lanes' runs
+    for (int g = 2; g <= L; g <<= 1) {   // merges of g lanes' runs
         const bool low = (lane & (g >> 1)) == 0;
 #pragma unroll
         for (int r = 0; r < (NR + 1) / 2; r++) {
@@ -225,6 +188,12 @@ __device__ __forceinline__ void warp_sort_words(unsigned (&x)[NR])
         }
         warp_merge_words<NR>(x, g >> 2);
     }
+}
+
+template <int NR>
+__device__ __forceinline__ void warp_sort_words(unsigned (&x)[NR])
+{
+    lanes_sort_words<NR, 32>(x);
 }
 
 // The network over 32 * NR * W words held by a CTA of W warps, thread t holding positions
@@ -258,116 +227,6 @@ __device__ __forceinline__ void cta_sort_words(unsigned (&x)[NR], unsigned *buf)
         }
         warp_merge_words<NR>(x, 16);
     }
-}
-
-// Segmented version: the warp holds 32/S independent rows of up to S entries
-// (lanes [S*r, S*r+S) hold row r); each segment is sorted by its own bitonic
-// network (log2 S stages), equal keys are merged, and every segment writes its
-// unique keys to its own out_k/out_w.  Returns the segment's unique count.
-template <int S>
-__device__ __forceinline__ int seg_aggregate(int32_t key, int32_t w, int32_t *out_k, int32_t *out_w)
-{
-    const int lane = threadIdx.x & 31;
-    const int sl = lane & (S - 1);
-#pragma unroll
-    for (int k = 2; k <= S; k <<= 1) {
-#pragma unroll
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            const int32_t pk = __shfl_xor_sync(HP_FULL_MASK, key, j);
-            const int32_t pw = __shfl_xor_sync(HP_FULL_MASK, w, j);
-            const bool up = (sl & k) == 0;
-            const bool lower = (sl & j) == 0;
-            const bool take = lower ? (up ? pk < key : pk > key) : (up ? pk > key : pk < key);
-            if (take) { key = pk; w = pw; }
-        }
-    }
-    int32_t s = w;
-#pragma unroll
-    for (int o = 1; o < S; o <<= 1) {
-        const int32_t t = __shfl_down_sync(HP_FULL_MASK, s, o, S);
-        const int32_t kk = __shfl_down_sync(HP_FULL_MASK, key, o, S);
-        if (sl + o < S && kk == key) s += t;
-    }
-    const int32_t prev = __shfl_up_sync(HP_FULL_MASK, key, 1, S);
-    const bool head = key != KEY_NONE && (sl == 0 || prev != key);
-    const unsigned seg = S == 32 ? 0xffffffffu : (((1u << S) - 1u) << (lane & ~(S - 1)));
-    const unsigned hm = __ballot_sync(HP_FULL_MASK, head) & seg;
-    if (head && out_k) {
-        const int r = __popc(hm & lanemask_lt());
-        out_k[r] = key;
-        out_w[r] = s;
-    }
-    return __popc(hm);
-}
-
-// Same aggregation written as a dense vector over keys [0, nkeys):
-// out_k[q] = q, out_w[q] = sum of the weights with key q (0 if none).
-__device__ __forceinline__ void warp_aggregate32_dense(int32_t key, int32_t w, int32_t nkeys,
-                                                       int32_t *out_k, int32_t *out_w)
-{
-    const int lane = threadIdx.x & 31;
-    for (int32_t q = lane; q < nkeys; q += 32) { out_k[q] = q; out_w[q] = 0; }
-    __syncwarp();
-    // duplicates of a key are summed with one atomic per entry (order-free)
-    if (key != KEY_NONE) atomicAdd(&out_w[key], w);
-    __syncwarp();
-}
-
-// CTA-wide shared-memory aggregation of len <= CAP entries staged in sk/sw
-// (entries beyond len must already be KEY_NONE up to the pow2 size P).
-template <int NT, int CAP>
-__device__ __forceinline__ int block_aggregate_smem(int32_t *sk, int32_t *sw, int P,
-                                                    int32_t *out_k, int32_t *out_w,
-                                                    int32_t *s_scan /* NT/32 + 2 */)
-{
-    const int tid = threadIdx.x;
-    // bitonic sort of P elements
-    for (int k = 2; k <= P; k <<= 1) {
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = tid; i < P; i += NT) {
-                int ixj = i ^ j;
-                if (ixj > i) {
-                    int32_t a = sk[i], b = sk[ixj];
-                    bool up = (i & k) == 0;
-                    if (up ? (a > b) : (a < b)) {
-                        sk[i] = b; sk[ixj] = a;
-                        int32_t t = sw[i]; sw[i] = sw[ixj]; sw[ixj] = t;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    }
-    // heads and their positions: thread t owns elements [t*per, (t+1)*per)
-    const int per = (P + NT - 1) / NT;
-    const int lo = tid * per, hiE = min(lo + per, P);
-    int cnt = 0;
-    for (int i = lo; i < hiE; i++)
-        cnt += (sk[i] != KEY_NONE && (i == 0 || sk[i - 1] != sk[i]));
-    const int lane = tid & 31, wid = tid >> 5;
-    int incl = warp_incl_scan(cnt);
-    if (lane == 31) s_scan[wid] = incl;
-    __syncthreads();
-    if (wid == 0) {
-        int t = lane < NT / 32 ? s_scan[lane] : 0;
-        int ti = warp_incl_scan(t);
-        if (lane < NT / 32) s_scan[lane] = ti - t;
-        if (lane == NT / 32 - 1) s_scan[NT / 32] = ti;
-    }
-    __syncthreads();
-    int pos = s_scan[wid] + incl - cnt;
-    const int total = s_scan[NT / 32];
-    for (int i = lo; i < hiE; i++) {
-        int32_t key = sk[i];
-        if (key == KEY_NONE || (i > 0 && sk[i - 1] == key)) continue;
-        int32_t sum = 0;
-        for (int j = i; j < P && sk[j] == key; j++) sum += sw[j];
-        out_k[pos] = key;
-        out_w[pos] = sum;
-        pos++;
-    }
-    __syncthreads();
-    return total;
 }
 
 // CTA-wide exclusive scan of one int per thread; returns exclusive value and
