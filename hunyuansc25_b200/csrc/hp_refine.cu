@@ -1928,65 +1928,85 @@ __device__ void cookie_cut_warp(int32_t k, const unsigned long long *__restrict_
                                 const int64_t *__restrict__ maxp, const int32_t *sp, int32_t np,
                                 int32_t *__restrict__ es, int32_t *__restrict__ ee)
 {
+    // The parts form one dependent chain (each starts where the one before ended), so the
+    // number of its steps and their latency are what counts: parts that take nothing are
+    // skipped 32 at a time, the 32 prefix weights after the window's start wb and the
+    // chain's own prefix stay in registers, in 32 bits (weights total below 2^31, a room
+    // is clamped to 2^31), and the ranges are stored 32 parts at a time.  RGG 2^24,
+    // k = 1024: a pass of the 8,517-vertex level 166 -> 61 us, of 1,942 vertices 102 -> 48.
     const int lane = threadIdx.x & 31;
-    int32_t st = 0;
+    const unsigned total = (unsigned)sp[np];
+    int32_t st = 0, wb = 0;
+    unsigned cur = (unsigned)sp[0];   // sp[st]
+    // positions past np count as reached: the answer is then np
+    auto window = [&](int32_t b) -> unsigned {
+        const int32_t pos = b + 1 + lane;
+        return pos <= np ? (unsigned)sp[pos] : 0xffffffffu;
+    };
+    unsigned w = window(0);
     for (int32_t p0 = 0; p0 < k; p0 += 32) {
         const int32_t pl = p0 + lane;
-        const int64_t my_room = pl < k && maxp[pl] > (int64_t)pw[pl] ? maxp[pl] - (int64_t)pw[pl] : 0;
+        const int64_t room64 = pl < k ? maxp[pl] - (int64_t)pw[pl] : 0;
+        const unsigned my_room = room64 <= 0 ? 0u : (unsigned)min(room64, (int64_t)1 << 31);
         const int cnt = min(32, k - p0);
-        for (int q = 0; q < cnt; q++) {
-            const int64_t room = __shfl_sync(HP_FULL_MASK, my_room, q);
-            const int32_t p = p0 + q;
-            const int32_t lo0 = st;
-            int32_t end = lo0;
-            if (room > 0) {
-                const int32_t hi0 = np;
-                const int64_t find = (int64_t)sp[lo0] + room;
-                // first idx in (lo0, hi0] with sp[idx] >= find, else hi0
-                int32_t lo = lo0, hi = hi0, e = hi0;
-                bool found = false;
-                {
-                    const int32_t pos = lo0 + 1 + lane;
-                    const bool ge = pos <= hi0 && (int64_t)sp[pos] >= find;
-                    const unsigned m = __ballot_sync(HP_FULL_MASK, ge);
-                    if (m) { e = lo0 + 1 + (__ffs(m) - 1); found = true; }
-                    else if (lo0 + 32 >= hi0) { e = hi0; found = true; }
-                    else lo = lo0 + 32;   // sp[lo0+32] < find: the answer lies in (lo0+32, hi0]
+        int32_t my_s = np, my_e = np;   // (parts after the list is used up: empty at np)
+        int q = 0;
+        while (q < cnt && st < np) {
+            // the next part that takes something: the first whose room is nearer to the
+            // first vertex's weight w1 than to nothing (the parts before it end where
+            // they start, at st)
+            if (st - wb >= 32) { wb = st; w = window(wb); }
+            const unsigned w1 = __shfl_sync(HP_FULL_MASK, w, st - wb) - cur;
+            const unsigned t = __ballot_sync(HP_FULL_MASK, lane >= q && lane < cnt && my_room > 0u &&
+                                                               (w1 < my_room || w1 - my_room < my_room));
+            const int nq = t ? __ffs(t) - 1 : cnt;
+            if (lane >= q && lane < nq) { my_s = st; my_e = st; }
+            q = nq;
+            if (q == cnt) break;
+            const unsigned room = __shfl_sync(HP_FULL_MASK, my_room, q);
+            int32_t end = st;
+            unsigned vend = cur;
+            {
+                // e: the first position after st with sp[e] >= find, else np
+                const unsigned find = cur + room;
+                unsigned m = __ballot_sync(HP_FULL_MASK, w >= find);
+                if (m == 0u) {
+                    wb = st;
+                    w = window(wb);
+                    m = __ballot_sync(HP_FULL_MASK, w >= find);
                 }
-                if (!found) {
+                if (m == 0u) {   // beyond the 32 positions after st (sp[st + 32] < find)
+                    int32_t lo = st + 32, hi = np;   // sp[lo] < find; the answer is in (lo, hi]
                     while (hi - lo > 32) {
-                        int64_t span = hi - lo;
-                        int32_t pos = lo + (int32_t)((span * (lane + 1)) / 32);
-                        bool ge = (int64_t)sp[pos] >= find;
-                        unsigned m = __ballot_sync(HP_FULL_MASK, ge);
-                        if (m == 0) { lo = __shfl_sync(HP_FULL_MASK, pos, 31); break; }
-                        int f = __ffs(m) - 1;
-                        int32_t nhi = __shfl_sync(HP_FULL_MASK, pos, f);
-                        int32_t nlo = f == 0 ? lo : __shfl_sync(HP_FULL_MASK, pos, f - 1);
-                        lo = nlo; hi = nhi;
+                        const int64_t span = hi - lo;
+                        const int32_t pos = lo + (int32_t)((span * (lane + 1)) / 32);
+                        const unsigned g = __ballot_sync(HP_FULL_MASK, (unsigned)sp[pos] >= find);
+                        if (g == 0u) { lo = np; break; }
+                        const int f = __ffs(g) - 1;
+                        hi = __shfl_sync(HP_FULL_MASK, pos, f);
+                        if (f > 0) lo = __shfl_sync(HP_FULL_MASK, pos, f - 1);
                     }
-                    e = hi;
-                    if (lo < hi) {
-                        int32_t pos = lo + 1 + lane;
-                        bool ge = pos <= hi && (int64_t)sp[pos] >= find;
-                        unsigned m = __ballot_sync(HP_FULL_MASK, ge);
-                        e = m ? lo + 1 + (__ffs(m) - 1) : hi;
-                    }
+                    wb = lo < np ? lo : np - 1;
+                    w = window(wb);
+                    m = __ballot_sync(HP_FULL_MASK, w >= find);
                 }
-                int32_t s0 = e > lo0 ? e - 1 : lo0;
-                int64_t dh = hp::iabs64((int64_t)sp[e] - find), dl = hp::iabs64((int64_t)sp[s0] - find);
-                end = dh < dl ? e : s0;
+                // (m == 0: np is the last position of the window)
+                const int f = m ? __ffs(m) - 1 : 31;
+                const int32_t e = min(wb + 1 + f, np);
+                const unsigned vw = __shfl_sync(HP_FULL_MASK, w, e - wb - 1);
+                const unsigned vb = __shfl_sync(HP_FULL_MASK, w, e - wb - 2 >= 0 ? e - wb - 2 : 0);
+                const unsigned ve = e == np ? total : vw;
+                const unsigned vs = e - 1 == st ? cur : (e - 1 == wb ? (unsigned)sp[wb] : vb);
+                const unsigned dh = ve >= find ? ve - find : find - ve, dl = find - vs;
+                end = dh < dl ? e : e - 1;
+                vend = dh < dl ? ve : vs;
             }
-            if (lane == 0) { es[p] = lo0; ee[p] = end; }
+            if (lane == q) { my_s = st; my_e = end; }
             st = end;
-            if (st == np) {
-                // the evicted list is used up: every later part starts at np and,
-                // room or not, ends there (nothing lies beyond np), so the rest is
-                // written in parallel
-                for (int32_t r = p + 1 + lane; r < k; r += 32) { es[r] = np; ee[r] = np; }
-                return;
-            }
+            cur = vend;
+            q++;
         }
+        if (pl < k) { es[pl] = my_s; ee[pl] = my_e; }
     }
 }
 
