@@ -552,9 +552,11 @@ int hp_lb_reserve(hp_context *c, int64_t tiles)
     c->lb_status = nullptr;
     c->lb_cap = 0;
     HP_CUDA(cudaMalloc((void **)&c->lb_status, sizeof(unsigned long long) * (size_t)cap));
-    HP_CUDA(cudaMemset(c->lb_status, 0, sizeof(unsigned long long) * (size_t)cap));
+    // on the call's stream: it does not wait for the legacy stream, where a plain memset
+    // could still run beside the first look-back kernels
+    HP_CUDA(cudaMemsetAsync(c->lb_status, 0, sizeof(unsigned long long) * (size_t)cap, c->stream));
     if (!c->lb_ctl) HP_CUDA(cudaMalloc((void **)&c->lb_ctl, sizeof(hp::LbCtl)));
-    HP_CUDA(cudaMemset(c->lb_ctl, 0, sizeof(hp::LbCtl)));
+    HP_CUDA(cudaMemsetAsync(c->lb_ctl, 0, sizeof(hp::LbCtl), c->stream));
     c->lb_cap = cap;
     return HP_OK;
 }

@@ -350,6 +350,7 @@ int hp_mlp_ensure(hp_context *c)
     c->mlp_m = c->mlp_grad + HP_MLP_NPARAM;
     c->mlp_v = c->mlp_m + HP_MLP_NPARAM;
     HP_CUDA(cudaMemset(p, 0, sizeof(float) * 4 * HP_MLP_NPARAM));
+    HP_CUDA(cudaStreamSynchronize(cudaStreamLegacy));   // (the library's streams do not wait for it)
     return HP_OK;
 }
 
@@ -376,6 +377,7 @@ HP_API int hp_mlp_set_params(hp_context *c, const float *params, int32_t count, 
     HP_TRY(hp_mlp_ensure(c));
     HP_CUDA(cudaMemcpy(c->mlp_params, params, sizeof(float) * HP_MLP_NPARAM, cudaMemcpyHostToDevice));
     HP_CUDA(cudaMemset(c->mlp_m, 0, sizeof(float) * 2 * HP_MLP_NPARAM));
+    HP_CUDA(cudaStreamSynchronize(cudaStreamLegacy));   // (the library's streams do not wait for it)
     c->mlp_threshold = threshold;
     c->mlp_ready = true;
     return HP_OK;
@@ -466,6 +468,7 @@ HP_API int hp_movelog_enable(hp_context *c, int64_t capacity)
     c->log_acc = c->log_d + capacity;
     c->log_count = (unsigned long long *)(c->log_acc + capacity);
     HP_CUDA(cudaMemset(c->log_count, 0, sizeof(unsigned long long)));
+    HP_CUDA(cudaStreamSynchronize(cudaStreamLegacy));   // (the library's streams do not wait for it)
     return HP_OK;
 }
 
@@ -494,5 +497,6 @@ HP_API int hp_movelog_reset(hp_context *c)
     if (!c || !c->log_x) return HP_ERR_INVALID_ARG;
     HP_CUDA(cudaSetDevice(c->device));
     HP_CUDA(cudaMemset(c->log_count, 0, sizeof(unsigned long long)));
+    HP_CUDA(cudaStreamSynchronize(cudaStreamLegacy));   // (the library's streams do not wait for it)
     return HP_OK;
 }

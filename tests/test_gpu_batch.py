@@ -53,3 +53,18 @@ def test_prepared_batch_matches_batch_call(ctx):
         assert [int(x) for x in c2] == [int(x) for x in cuts]
         for a, q in zip(parts, p2):
             assert np.array_equal(a, q)
+
+
+def test_batch_growing_graphs_fresh_contexts():
+    """Workers whose look-back regions are allocated and grow while the other workers'
+    kernels run: every context's first batch and one of larger graphs."""
+    import hunyuansc25_b200 as hp
+    small = [graphs.grid2d(40 + i, 30, seed=i, wmin=1, wmax=9) for i in range(16)]
+    large = [graphs.grid2d(1100, 1000 + i, seed=i, wmin=1, wmax=9) for i in range(4)]
+    want = None
+    for _ in range(4):
+        with hp.Context(0) as c:
+            got = [c.partition_batch(gs, [4] * len(gs), 1.03) for gs in (small, large)]
+        cuts = [list(r[1]) for r in got]
+        want = want or cuts
+        assert cuts == want
