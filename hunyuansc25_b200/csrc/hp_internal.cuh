@@ -25,7 +25,8 @@ struct HpLevel {
 struct hp_context {
     int device = 0;
     int sm_count = 148;
-    int max_cluster = 1;             // CTAs of the largest cluster refine_cluster_kernel can run in
+    int max_cluster = 1;             // CTAs of the largest cluster refine_loop_kernel can run in
+    int grid_ctas = 0;               // CTAs of its cooperative launches (0: not available)
     cudaStream_t stream = nullptr;   // stream of the current call
     cudaStream_t own_stream = nullptr;
 
@@ -106,7 +107,7 @@ constexpr int HP_TUNE_WARP_ROW_MAX = 256;        // contract_warp_radix_kernel's
 constexpr int HP_TUNE_CTA_ROW_MAX = 4096;        // contract_cta_radix_kernel<256, 4096>
 constexpr int HP_TUNE_WARP_DENSE_K_MAX = 1024;   // gain_bigwarp_kernel's shared accumulators
 constexpr int HP_TUNE_DEG_MAX = 1 << 24;
-constexpr int HP_TUNE_SMALL_LEVEL_MAX = 32768;   // vertices per CTA of refine_cluster_kernel's levels
+constexpr int HP_TUNE_SMALL_LEVEL_MAX = 32768;   // vertices per CTA of refine_loop_kernel's cluster levels
 constexpr int HP_TUNE_SMALL_MATCH_MAX = 8192;    // match_small_kernel's shared-memory state
 constexpr int HP_TUNE_SMEM_CN_MAX = 49152;       // shared-memory dense accumulator of the contraction
 constexpr int64_t HP_LEARNED_SKEW = 16;          // learned proposals: max degree / mean degree of the input
@@ -171,6 +172,25 @@ inline cudaError_t hp_launch_kernel(const hp_context *c, void (*kernel)(P...), u
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
+// A cooperative launch: every CTA is resident, so the CTAs may wait for one another.
+// (Not a programmatic dependent: it starts when the stream's previous kernel is done.)
+template <class... P, class... A>
+inline cudaError_t hp_launch_coop(const hp_context *c, void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
+                                  A &&...args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = c->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+
 // Count and check every kernel launch.  Once the arena has run out nothing more is
 // launched (a pointer allocated after that is null): the call unwinds with
 // HP_ERR_NOMEM and partition_common retries with a larger arena.
@@ -178,11 +198,19 @@ inline cudaError_t hp_launch_kernel(const hp_context *c, void (*kernel)(P...), u
     HP_LAUNCH_CLUSTER(ctx, kernel, 1, grid, block, smem, __VA_ARGS__)
 // The same with thread-block clusters of `cluster` CTAs.
 #define HP_LAUNCH_CLUSTER(ctx, kernel, cluster, grid, block, smem, ...)                     \
+    HP_LAUNCH_CHECKED(ctx, kernel, grid,                                                    \
+                      hp_launch_kernel((ctx), kernel, (unsigned)(grid), (unsigned)(block),  \
+                                       (size_t)(smem), (unsigned)(cluster), __VA_ARGS__))
+// A cooperative launch.
+#define HP_LAUNCH_COOP(ctx, kernel, grid, block, smem, ...)                                 \
+    HP_LAUNCH_CHECKED(ctx, kernel, grid,                                                    \
+                      hp_launch_coop((ctx), kernel, (unsigned)(grid), (unsigned)(block),    \
+                                     (size_t)(smem), __VA_ARGS__))
+#define HP_LAUNCH_CHECKED(ctx, kernel, grid, launch)                                        \
     do {                                                                                    \
         if ((ctx)->oom) return HP_ERR_NOMEM;                                                \
         if ((grid) > 0) {                                                                   \
-            cudaError_t e__ = hp_launch_kernel((ctx), kernel, (unsigned)(grid), (unsigned)(block), \
-                                               (size_t)(smem), (unsigned)(cluster), __VA_ARGS__); \
+            cudaError_t e__ = launch;                                                       \
             (ctx)->launches++;                                                              \
             if (e__ == cudaSuccess) e__ = cudaGetLastError();                               \
             if (e__ != cudaSuccess) {                                                       \

@@ -2725,6 +2725,10 @@ struct SmallLevel {
     const float *mlp_params;
     RefineCtl *ctl;
     unsigned *status;
+    // the grid variant's barrier counter (zero at launch) and exchange arrays
+    unsigned *bar;
+    long long *gx;          // 2 x CTAs x 3
+    int32_t *ghist;         // CTAs x 256
 };
 
 // Dynamic shared memory: the largest of the phases' needs (sort tables; the staged
@@ -2758,6 +2762,17 @@ int32_t cluster_level_n(const hp_context *c)
 {
     return (int32_t)std::min<int64_t>((int64_t)c->tune.small_level_n * c->max_cluster, CL_LEVEL_MAX);
 }
+
+// Levels above that run their passes in one cooperative launch over the whole GPU, a CTA
+// per SM: the same loop with a barrier through global memory (about 2.5 us against the
+// cluster's 1) and 148 SMs.  Launched passes take longer up to about two million vertices
+// (a pass of the 128^3 grid, k = 64: 110,557 vertices 68 -> 60 us, 614,464 89 -> 77,
+// 2,097,152 129 -> 112; RGG, k = 1024: 477,503 81 -> 66, 1,450,170 115 -> 92), and their
+// graphs cost the host half a millisecond a level; above it the launched kernels'
+// occupancy wins (2,598,047 vertices 194 us launched, about 210 here).  A longer row than
+// GRID_DEG_MAX would hold the one warp that walks it.
+constexpr int32_t GRID_LEVEL_MAX = 1 << 21;
+constexpr int32_t GRID_DEG_MAX = 1024;
 
 __device__ __forceinline__ unsigned cl_rank()
 {
@@ -2804,74 +2819,166 @@ __device__ __forceinline__ int32_t cl_ld32(unsigned addr)
     return v;
 }
 
-// Exchange of the CTAs' sums through a cluster barrier.  Two buffers in turn: a CTA
+// The barrier of the grid variant (a cooperative launch: every CTA is resident): an
+// arrival counter that only grows, *gen its value when the last barrier completed.
+// Writes before it are visible after it.  The wait is bounded: on expiry it sets
+// HP_STATUS_SPIN_TIMEOUT and returns false in every thread of the CTA, which then
+// leaves the kernel (as the CTAs that wait for it will).
+__device__ __forceinline__ bool grid_sync(unsigned *bar, unsigned *gen, unsigned *status)
+{
+    __shared__ bool s_ok;
+    *gen += gridDim.x;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(bar, 1u);
+        unsigned seen = 0, spins = 0;
+        for (;;) {
+            asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
+            if ((int)(seen - *gen) >= 0) break;
+            if (++spins > HP_SPIN_LIMIT) {
+                atomicOr(status, HP_STATUS_SPIN_TIMEOUT);
+                break;
+            }
+            if (spins > 64) __nanosleep(32);
+        }
+        __threadfence();
+        s_ok = (int)(seen - *gen) >= 0;
+    }
+    __syncthreads();
+    return s_ok;
+}
+
+// Exchange of the CTAs' sums through the barrier.  Two buffers in turn: a CTA
 // writes a buffer again only two barriers later, when every CTA has read it.
+// A cluster's CTAs write into each other's shared memory; a grid's go through
+// global memory, read by one warp of every CTA.
 struct ClXch {
     long long x[2][CL_MAX][3];
     long long w[CL_WARPS][3];
-    int buf;   // (thread 0 toggles it; read after a barrier)
+    long long tot[4];
 };
 
-// Sums of N (at most 3) values over all threads of the cluster; every thread gets
-// them.  Everything written before the call is visible after it.
-template <int N>
-__device__ __forceinline__ void cl_sum(long long (&v)[N], ClXch &X, int buf, unsigned rank, unsigned nct)
-{
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-    for (int i = 0; i < N; i++) {
-        const long long s = hp::warp_sum64(v[i]);
-        if (lane == 0) X.w[wid][i] = s;
+template <bool GRID>
+struct ClTeam {
+    unsigned rank, nct;
+    unsigned gen;       // grid: the barrier's count so far
+    const SmallLevel &a;
+    ClXch &X;
+    __device__ __forceinline__ ClTeam(const SmallLevel &a_, ClXch &X_) : gen(0), a(a_), X(X_)
+    {
+        rank = GRID ? blockIdx.x : cl_rank();
+        nct = GRID ? gridDim.x : cl_size();
     }
-    __syncthreads();
-    if (wid == 0) {
+    // All threads of the team; false: the wait expired and the kernel ends.
+    __device__ __forceinline__ bool sync()
+    {
+        if (GRID) return grid_sync(a.bar, &gen, a.status);
+        cl_sync();
+        return true;
+    }
+    __device__ __forceinline__ void put(int buf, int i, long long v)   // (the first warp, the same v in its lanes)
+    {
+        const int lane = threadIdx.x & 31;
+        if (GRID) {
+            if (lane == 0) a.gx[((size_t)buf * nct + rank) * 3 + i] = v;
+        } else if (lane < (int)nct) {
+            cl_st64(cl_map(&X.x[buf][rank][i], lane), v);
+        }
+    }
+    // Sums of N (at most 3) values over all threads of the team; every thread gets
+    // them.  Everything written before the call is visible after it.
+    template <int N>
+    __device__ __forceinline__ bool sum(long long (&v)[N], int buf)
+    {
+        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
         for (int i = 0; i < N; i++) {
-            const long long s = hp::warp_sum64(X.w[lane][i]);
-            if (lane < (int)nct) cl_st64(cl_map(&X.x[buf][rank][i], lane), s);
+            const long long s = hp::warp_sum64(v[i]);
+            if (lane == 0) X.w[wid][i] = s;
         }
-    }
-    cl_sync();
+        __syncthreads();
+        if (wid == 0) {
 #pragma unroll
-    for (int i = 0; i < N; i++) {
-        long long s = 0;
-        for (unsigned r = 0; r < nct; r++) s += X.x[buf][r][i];
-        v[i] = s;
-    }
-}
-
-// Exclusive prefix over the cluster's warps (rank, then warp order) of two values
-// per warp (the same in all its lanes), and their totals.
-__device__ __forceinline__ void cl_warp_scan2(int32_t a, int32_t b, int32_t *ea, int32_t *eb, int32_t *ta,
-                                              int32_t *tb, ClXch &X, int buf, unsigned rank, unsigned nct)
-{
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) { X.w[wid][0] = a; X.w[wid][1] = b; }
-    __syncthreads();
-    if (wid == 0) {
-        const int va = (int)X.w[lane][0], vb = (int)X.w[lane][1];
-        const int ia = hp::warp_incl_scan(va), ib = hp::warp_incl_scan(vb);
-        X.w[lane][0] = ia - va;
-        X.w[lane][1] = ib - vb;
-        const int sa = __shfl_sync(HP_FULL_MASK, ia, 31), sb = __shfl_sync(HP_FULL_MASK, ib, 31);
-        if (lane < (int)nct) {
-            cl_st64(cl_map(&X.x[buf][rank][0], lane), sa);
-            cl_st64(cl_map(&X.x[buf][rank][1], lane), sb);
+            for (int i = 0; i < N; i++) put(buf, i, hp::warp_sum64(X.w[lane][i]));
         }
+        if (!sync()) return false;
+        if (GRID) {
+            if (wid == 0) {
+#pragma unroll
+                for (int i = 0; i < N; i++) {
+                    long long s = 0;
+                    for (unsigned r = lane; r < nct; r += 32) s += __ldcg(&a.gx[((size_t)buf * nct + r) * 3 + i]);
+                    s = hp::warp_sum64(s);
+                    if (lane == 0) X.tot[i] = s;
+                }
+            }
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < N; i++) v[i] = X.tot[i];
+            return true;
+        }
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            long long s = 0;
+            for (unsigned r = 0; r < nct; r++) s += X.x[buf][r][i];
+            v[i] = s;
+        }
+        return true;
     }
-    cl_sync();
-    int32_t pa = (int32_t)X.w[wid][0], pb = (int32_t)X.w[wid][1], xa = 0, xb = 0;
-    for (unsigned r = 0; r < nct; r++) {
-        const int32_t qa = (int32_t)X.x[buf][r][0], qb = (int32_t)X.x[buf][r][1];
-        if (r < rank) { pa += qa; pb += qb; }
-        xa += qa;
-        xb += qb;
+    // Exclusive prefix over the team's warps (rank, then warp order) of two values
+    // per warp (the same in all its lanes), and their totals.
+    __device__ __forceinline__ bool warp_scan2(int32_t va, int32_t vb, int32_t *ea, int32_t *eb, int32_t *ta,
+                                               int32_t *tb, int buf)
+    {
+        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+        if (lane == 0) { X.w[wid][0] = va; X.w[wid][1] = vb; }
+        __syncthreads();
+        if (wid == 0) {
+            const int qa = (int)X.w[lane][0], qb = (int)X.w[lane][1];
+            const int ia = hp::warp_incl_scan(qa), ib = hp::warp_incl_scan(qb);
+            X.w[lane][0] = ia - qa;
+            X.w[lane][1] = ib - qb;
+            put(buf, 0, __shfl_sync(HP_FULL_MASK, ia, 31));
+            put(buf, 1, __shfl_sync(HP_FULL_MASK, ib, 31));
+        }
+        if (!sync()) return false;
+        int32_t pa = (int32_t)X.w[wid][0], pb = (int32_t)X.w[wid][1], xa = 0, xb = 0;
+        if (GRID) {
+            if (wid == 0) {
+                int32_t la = 0, lb = 0;   // the CTAs before this one
+                for (unsigned r = lane; r < nct; r += 32) {
+                    const int32_t qa = (int32_t)__ldcg(&a.gx[((size_t)buf * nct + r) * 3]);
+                    const int32_t qb = (int32_t)__ldcg(&a.gx[((size_t)buf * nct + r) * 3 + 1]);
+                    if (r < rank) { la += qa; lb += qb; }
+                    xa += qa;
+                    xb += qb;
+                }
+                la = hp::warp_sum(la); lb = hp::warp_sum(lb);
+                xa = hp::warp_sum(xa); xb = hp::warp_sum(xb);
+                if (lane == 0) { X.tot[0] = la; X.tot[1] = lb; X.tot[2] = xa; X.tot[3] = xb; }
+            }
+            __syncthreads();
+            pa += (int32_t)X.tot[0];
+            pb += (int32_t)X.tot[1];
+            xa = (int32_t)X.tot[2];
+            xb = (int32_t)X.tot[3];
+            __syncthreads();   // (the totals and the warps' prefixes are read)
+        } else {
+            for (unsigned r = 0; r < nct; r++) {
+                const int32_t qa = (int32_t)X.x[buf][r][0], qb = (int32_t)X.x[buf][r][1];
+                if (r < rank) { pa += qa; pb += qb; }
+                xa += qa;
+                xb += qb;
+            }
+        }
+        *ea = pa;
+        *eb = pb;
+        *ta = xa;
+        *tb = xb;
+        return true;
     }
-    *ea = pa;
-    *eb = pb;
-    *ta = xa;
-    *tb = xb;
-}
+};
 
 // The gain rows of the listed vertices (short rows by lane segments, long rows by a
 // warp's dense accumulator in shared memory).
@@ -2901,8 +3008,10 @@ __device__ __forceinline__ void cl_rebuild(const SmallLevel &a, int gw, int tw, 
     }
 }
 
+// GRID: the CTAs of a cooperative launch instead of a cluster (grid_level).
+template <bool GRID>
 __global__ void __launch_bounds__(CL_THREADS, 1)
-refine_cluster_kernel(SmallLevel a)
+refine_loop_kernel(const __grid_constant__ SmallLevel a)
 {
     hp::pdl_wait();
     extern __shared__ __align__(16) int32_t cl_dyn[];
@@ -2913,11 +3022,13 @@ refine_cluster_kernel(SmallLevel a)
     __shared__ int32_t s_part[CL_KMAX];      // weak: the undersized parts; strong: the parts' evicted ranges
     __shared__ int8_t s_ufl[CL_KMAX];        // weak: pw < maxp
     __shared__ int32_t s_hist[256], s_base[256];
+    __shared__ int32_t s_group[2][GRID ? CL_THREADS : 1];   // digit counts before this CTA and in all, by group
     __shared__ int32_t s_scan[CL_WARPS + 2];
     __shared__ int32_t s_nu;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const unsigned lt = hp::lanemask_lt();
-    const unsigned rank = cl_rank(), nct = cl_size();
+    ClTeam<GRID> team(a, X);
+    const unsigned rank = team.rank, nct = team.nct;
     const int tw = (int)nct * CL_WARPS, gw = (int)rank * CL_WARPS + wid;
     const int gt = (int)nct * CL_THREADS, gtid = (int)rank * CL_THREADS + tid;
     const int32_t n = a.n, k = a.k;
@@ -2926,7 +3037,7 @@ refine_cluster_kernel(SmallLevel a)
     int buf = 0;                             // exchange buffer (uniform over the cluster)
     // no CTA writes another's shared memory before that CTA runs: being placed together
     // does not mean having started
-    cl_sync();
+    if (!GRID && !team.sync()) return;
     if (a.learned_mlp) hp::mlp_load_smem(s_mlp, a.mlp_params);
     // ---- the level's setup, as the launches of the multi-kernel levels:
     // gain-row capacities min(deg, k) and offsets, cleared locks and dirty
@@ -2952,7 +3063,7 @@ refine_cluster_kernel(SmallLevel a)
         }
         caps = hp::warp_sum(caps);
         int32_t run, e1, total, t1;
-        cl_warp_scan2(caps, 0, &run, &e1, &total, &t1, X, buf, rank, nct);
+        if (!team.warp_scan2(caps, 0, &run, &e1, &total, &t1, buf)) return;
         buf ^= 1;
         for (int32_t v0 = vb; v0 < ve; v0 += 32) {
             const int32_t v = v0 + lane;
@@ -2969,10 +3080,10 @@ refine_cluster_kernel(SmallLevel a)
         if (gtid == 0) a.goff[n] = total;
         for (int32_t q = tid; q < k; q += CL_THREADS)
             if (spw[q]) atomicAdd(&a.pw[q], (unsigned long long)spw[q]);
-        cl_sync();
+        if (!team.sync()) return;
         const int32_t ns = __ldcg(&a.counts[1]), nb = __ldcg(&a.counts[2]);
         cl_rebuild(a, gw, tw, ns, nb, cl_dyn);
-        cl_sync();
+        if (!team.sync()) return;
         if (rank == 0 && tid < 4) a.counts[tid] = 0;   // (the first pass's; barriers follow before its use)
         long long cut[1] = {0};
         if (!a.coarser) {   // the coarsest level: the cut from the gain rows
@@ -2983,7 +3094,7 @@ refine_cluster_kernel(SmallLevel a)
                 });
             }
         }
-        cl_sum<1>(cut, X, buf, rank, nct);
+        if (!team.sum(cut, buf)) return;
         buf ^= 1;
         long long m = LLONG_MIN;
         for (int32_t q = tid; q < k; q += CL_THREADS) {
@@ -3058,7 +3169,7 @@ refine_cluster_kernel(SmallLevel a)
                 }
                 my[0] += cand;
             }
-            cl_sum<2>(my, X, buf, rank, nct);   // (barrier: every selection is visible)
+            if (!team.sum(my, buf)) return;   // (barrier: every selection is visible)
             buf ^= 1;
             ncand = my[0];
             judged = jdg;
@@ -3107,7 +3218,7 @@ refine_cluster_kernel(SmallLevel a)
                 if (jdg) {
                     // ---- the judge: exact cut decrease of the plain and the
                     // learned move sets on this state, as judge_delta_kernel
-                    cl_sync();   // every lock / accp is visible
+                    if (!team.sync()) return;   // every lock / accp is visible
                     long long sj[2] = {0, 0};
                     for (int32_t v0 = vb; v0 < ve; v0 += 32) {
                         const int32_t v = v0 + lane;
@@ -3134,7 +3245,7 @@ refine_cluster_kernel(SmallLevel a)
                                             a.lock, sj[0], sj[1]);
                         }
                     }
-                    cl_sum<2>(sj, X, buf, rank, nct);
+                    if (!team.sum(sj, buf)) return;
                     buf ^= 1;
                     jp2 = sj[0];
                     jl2 = sj[1];
@@ -3213,17 +3324,18 @@ refine_cluster_kernel(SmallLevel a)
                 cw += __popc(m);
             }
             __syncwarp();
-            // stable radix sort by key, 8-bit digits: per-warp digit counts, their
+            // stable radix sort by key, digits of at most 8 bits: per-warp digit counts, their
             // prefix over the CTA's warps, the CTAs' totals read through the cluster
             int32_t *ks = a.K, *vs = a.V, *kd = a.K2, *vd = a.V2;
             int32_t ib = vb, ie = vb + cw, cnt = 0;   // the warp's items
             int32_t *wc = cl_dyn + wid * 256;
-            for (int shift = 0; shift < a.key_bits; shift += 8) {
-                for (int q = lane; q < 256; q += 32) wc[q] = 0;
+            const int passes = (a.key_bits + 7) / 8, dbits = (a.key_bits + passes - 1) / passes, bins = 1 << dbits;
+            for (int shift = 0; shift < a.key_bits; shift += dbits) {
+                for (int q = lane; q < bins; q += 32) wc[q] = 0;
                 __syncwarp();
-                for (int32_t i = ib + lane; i < ie; i += 32) atomicAdd(&wc[((unsigned)ks[i] >> shift) & 255u], 1);
+                for (int32_t i = ib + lane; i < ie; i += 32) atomicAdd(&wc[((unsigned)ks[i] >> shift) & (bins - 1)], 1);
                 __syncthreads();
-                if (tid < 256) {
+                if (tid < bins) {
                     int32_t s = 0;
 #pragma unroll 8
                     for (int w = 0; w < CL_WARPS; w++) {
@@ -3231,24 +3343,44 @@ refine_cluster_kernel(SmallLevel a)
                         cl_dyn[w * 256 + tid] = s;
                         s += t;
                     }
-                    s_hist[tid] = s;
+                    if (GRID) a.ghist[(size_t)rank * 256 + tid] = s;
+                    else s_hist[tid] = s;
                 }
-                cl_sync();
+                if (!team.sync()) return;
                 int32_t before = 0, all = 0;
-                if (tid < 256)
+                if (GRID) {   // a group of threads per set of CTAs, a thread per digit
+                    const int groups = CL_THREADS >> dbits, per = ((int)nct + groups - 1) / groups;
+                    const int dg = tid & (bins - 1), r0 = (tid >> dbits) * per, r1 = min((int)nct, r0 + per);
+                    int32_t bg = 0, ag = 0;
+#pragma unroll 10
+                    for (int r = r0; r < r1; r++) {
+                        const int32_t t = __ldcg(&a.ghist[(size_t)r * 256 + dg]);
+                        if (r < (int)rank) bg += t;
+                        ag += t;
+                    }
+                    s_group[0][tid] = bg;
+                    s_group[1][tid] = ag;
+                    __syncthreads();
+                    if (tid < bins)
+                        for (int g = 0; g < groups; g++) {
+                            before += s_group[0][(g << dbits) + tid];
+                            all += s_group[1][(g << dbits) + tid];
+                        }
+                } else if (tid < bins) {
                     for (unsigned r = 0; r < nct; r++) {
                         const int32_t t = cl_ld32(cl_map(&s_hist[tid], r));
                         if (r < rank) before += t;
                         all += t;
                     }
+                }
                 const int ex = hp::block_excl_scan<CL_THREADS>(all, &cnt, s_scan);
-                if (tid < 256) s_base[tid] = ex + before;
+                if (tid < bins) s_base[tid] = ex + before;
                 __syncthreads();
                 for (int32_t i0 = ib; i0 < ie; i0 += 32) {
                     const int32_t i = i0 + lane;
                     const bool valid = i < ie;
                     const int32_t key = valid ? ks[i] : 0, val = valid ? vs[i] : 0;
-                    const unsigned dg = valid ? (((unsigned)key >> shift) & 255u) : 256u + lane;
+                    const unsigned dg = valid ? (((unsigned)key >> shift) & (bins - 1)) : 256u + lane;
                     const unsigned peers = __match_any_sync(HP_FULL_MASK, dg);
                     const int rk = __popc(peers & lt);
                     if (valid) {
@@ -3260,7 +3392,7 @@ refine_cluster_kernel(SmallLevel a)
                     if (valid && rk == 0) wc[dg] += __popc(peers);
                     __syncwarp();
                 }
-                cl_sync();
+                if (!team.sync()) return;
                 int32_t *t = ks; ks = kd; kd = t;
                 t = vs; vs = vd; vd = t;
                 const int32_t ipw = (cnt + tw - 1) / tw;
@@ -3272,7 +3404,7 @@ refine_cluster_kernel(SmallLevel a)
             for (int32_t i = ib + lane; i < ie; i += 32) wsum += a.vwgt[vs[i]];
             wsum = hp::warp_sum(wsum);
             int32_t run, e1, t0, t1;
-            cl_warp_scan2(wsum, 0, &run, &e1, &t0, &t1, X, buf, rank, nct);
+            if (!team.warp_scan2(wsum, 0, &run, &e1, &t0, &t1, buf)) return;
             buf ^= 1;
             for (int32_t i0 = ib; i0 < ie; i0 += 32) {
                 const int32_t i = i0 + lane;
@@ -3285,7 +3417,7 @@ refine_cluster_kernel(SmallLevel a)
                 }
                 run += __shfl_sync(HP_FULL_MASK, incl, 31);
             }
-            cl_sync();
+            if (!team.sync()) return;
             // a candidate leaves its part when the part's candidates before it weigh
             // less than the part's excess (weak: the moves; strong: the evicted prefix,
             // whose end is the first candidate where that weight reaches the excess)
@@ -3315,7 +3447,7 @@ refine_cluster_kernel(SmallLevel a)
                 nf = hp::warp_sum(nf);
                 fw = hp::warp_sum(fw);
                 int32_t pc, pr, np, wt;
-                cl_warp_scan2(nf, fw, &pc, &pr, &np, &wt, X, buf, rank, nct);
+                if (!team.warp_scan2(nf, fw, &pc, &pr, &np, &wt, buf)) return;
                 buf ^= 1;
                 // the evicted vertices in sorted order and their prefix weights (rs_evict_kernel)
                 for (int32_t i0 = ib; i0 < ie; i0 += 32) {
@@ -3338,7 +3470,7 @@ refine_cluster_kernel(SmallLevel a)
                     pr += __shfl_sync(HP_FULL_MASK, incl, 31);
                 }
                 if (gtid == 0) a.sp[np] = wt;
-                cl_sync();
+                if (!team.sync()) return;
                 if (rank == 0) {   // the cookie cutter, on staged prefix weights when they fit
                     const bool staged = np + 1 <= a.cookie_cap;
                     if (staged)
@@ -3348,7 +3480,7 @@ refine_cluster_kernel(SmallLevel a)
                         cookie_cut_warp(k, (const unsigned long long *)s_pw, a.maxp, staged ? cl_dyn : a.sp, np, a.es,
                                         a.ee);
                 }
-                cl_sync();
+                if (!team.sync()) return;
                 for (int32_t q = tid; q < k; q += CL_THREADS) s_part[q] = a.es[q];
                 __syncthreads();
                 for (int32_t j0 = gw * 32; j0 < np; j0 += tw * 32) {   // rs_assign_kernel
@@ -3376,20 +3508,20 @@ refine_cluster_kernel(SmallLevel a)
                 }
             }
         }
-        cl_sync();   // the moves are complete
+        if (!team.sync()) return;   // the moves are complete
         // ---- apply: moves, gain-row maintenance, cut change after
         const int32_t nmoves = __ldcg(&cn[0]);
         if (nmoves > 0) {
             apply_moves_rows(gw, tw, a.moves, nmoves, a.where, a.dest, a.vwgt, a.pw, a.xadj, a.adjncy, a.adjwgt,
                              a.goff, a.gconn, a.dirty, a.small_l, a.big_l, &cn[1], k, nullptr, nullptr, a.bigd,
                              INT_MAX);
-            cl_sync();
+            if (!team.sync()) return;
             cl_rebuild(a, gw, tw, __ldcg(&cn[1]), __ldcg(&cn[2]), cl_dyn);
         }
         if (rank == 0 && tid < 4) a.counts[4 * ((guard & 1) ^ 1) + tid] = 0;   // the next pass's set
         long long c[2] = {c1, 0};
         if (nmoves > 0) {
-            cl_sync();
+            if (!team.sync()) return;
             for (int32_t i = gtid; i < nmoves; i += gt) {
                 const int32_t v = a.moves[i];
                 const int32_t o = a.goff[v], len = a.goff[v + 1] - o;
@@ -3404,7 +3536,7 @@ refine_cluster_kernel(SmallLevel a)
             m = e > m ? e : m;
         }
         m = hp::warp_max64(m);
-        cl_sum<2>(c, X, buf, rank, nct);
+        if (!team.sum(c, buf)) return;
         buf ^= 1;
         if (lane == 0) X.w[wid][2] = m;
         __syncthreads();
@@ -3564,6 +3696,40 @@ struct LevelLaunches {
     int gain_tok = -1;   // profiler interval of the level's gain build (bytes completed at the end)
 };
 
+// Cooperative launches of one device, from any context and thread, follow one another:
+// each takes every SM, and two that were half resident would wait for each other.
+struct CoopOrder {
+    std::mutex mu;
+    cudaEvent_t last = nullptr;   // the end of the latest one
+};
+
+CoopOrder &coop_order(int device)
+{
+    static CoopOrder order[64];
+    return order[device & 63];
+}
+
+template <class F>
+int coop_launch(hp_context *c, F &&launch)
+{
+    CoopOrder &o = coop_order(c->device);
+    std::lock_guard<std::mutex> lk(o.mu);
+    if (o.last) HP_CUDA(cudaStreamWaitEvent(c->stream, o.last, 0));
+    else HP_CUDA(cudaEventCreateWithFlags(&o.last, cudaEventDisableTiming));
+    const int rc = launch();
+    HP_CUDA(cudaEventRecord(o.last, c->stream));
+    return rc;
+}
+
+// Levels above a cluster's that run their pass loop in one cooperative launch over the
+// whole GPU: see GRID_LEVEL_MAX.  Not under the eager loop (the batch workers' contexts
+// share the GPU, and a cooperative launch waits for all of it).
+bool grid_takes(const hp_context *c, const HpLevel &g, int32_t k, const LevelStat &ls)
+{
+    return c->grid_ctas > 0 && c->tune.small_level_n > 0 && !c->opt.eager && g.n <= GRID_LEVEL_MAX && k <= CL_KMAX &&
+           ls.maxdeg <= GRID_DEG_MAX && g.m <= CL_DEG * (int64_t)g.n;
+}
+
 int refine_level(hp_context *c, HpLevel &g, int32_t k, bool finest, const int64_t *d_opt,
                  const int64_t *d_maxp, const LevelStat &ls, RefineCtl *ctl, const RefineCtl *coarser,
                  LevelLaunches *ll, GraphKeep *keep)
@@ -3617,7 +3783,8 @@ int refine_level(hp_context *c, HpLevel &g, int32_t k, bool finest, const int64_
     // either loop mode unless the per-pass move log or pass log is on
     const int32_t cl_n = cluster_level_n(c);
     const bool small_level = !recording && !dbg && n <= cl_n && k <= CL_KMAX && g.m <= CL_DEG * cl_n;
-    if (small_level) {
+    const bool grid_level = !small_level && !recording && !dbg && !learned && grid_takes(c, g, k, ls);
+    if (small_level || grid_level) {
         // the level's setup (gain rows, part weights, cut, control block) runs
         // inside the kernel: no launch per setup step
         B.gpart = ralloc_t<int32_t>(c, std::max<int64_t>(g.m, 1));
@@ -3675,8 +3842,23 @@ int refine_level(hp_context *c, HpLevel &g, int32_t k, bool finest, const int64_
         a.ctl = ctl;
         const size_t smem = small_level_smem(n, k);
         a.cookie_cap = (int32_t)(smem / sizeof(int32_t));
+        if (grid_level) {
+            const int ctas = c->grid_ctas;
+            a.bar = ralloc_t<unsigned>(c, 1);
+            a.gx = ralloc_t<long long>(c, 2 * 3 * (int64_t)ctas);
+            a.ghist = ralloc_t<int32_t>(c, 256 * (int64_t)ctas);
+            HP_CHECK_OOM(c);
+            HP_CUDA(cudaMemsetAsync(a.bar, 0, sizeof(unsigned), c->stream));
+            HP_CUDA(cudaMemsetAsync(c->d_scal, 0, sizeof(unsigned long long) * S_PASS_END, c->stream));
+            HP_TRY(coop_launch(c, [&]() -> int {
+                HP_LAUNCH_COOP(c, refine_loop_kernel<true>, ctas, CL_THREADS, smem, a);
+                return HP_OK;
+            }));
+            c->hi = mark;
+            return HP_OK;
+        }
         const int ctas = cluster_ctas(c, n, g.m);
-        HP_LAUNCH_CLUSTER(c, refine_cluster_kernel, ctas, ctas, CL_THREADS, smem, a);
+        HP_LAUNCH_CLUSTER(c, refine_loop_kernel<false>, ctas, ctas, CL_THREADS, smem, a);
         c->hi = mark;
         return HP_OK;
     }
@@ -3769,8 +3951,14 @@ int hp_refine_init(hp_context *c)
     const int bytes = HP_MAX_PARTS * 4 + (HP_MAX_PARTS / 32) * 4;
     HP_CUDA(cudaFuncSetAttribute(gain_dense_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
     const size_t smem = small_level_smem(CL_LEVEL_MAX, CL_KMAX);
-    HP_CUDA(cudaFuncSetAttribute(refine_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    HP_CUDA(cudaFuncSetAttribute(refine_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    HP_CUDA(cudaFuncSetAttribute(refine_loop_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    HP_CUDA(cudaFuncSetAttribute(refine_loop_kernel<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    // the CTAs of a cooperative launch of the grid variant: one per SM
+    HP_CUDA(cudaFuncSetAttribute(refine_loop_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int per_sm = 0, coop = 0;
+    HP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, refine_loop_kernel<true>, CL_THREADS, smem));
+    HP_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device));
+    c->grid_ctas = coop && per_sm > 0 && c->device < 64 ? c->sm_count : 0;
     // the largest cluster the device can place
     c->max_cluster = 1;
     for (int q = CL_MAX; q > 1; q /= 2) {
@@ -3786,7 +3974,7 @@ int hp_refine_init(hp_context *c)
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int fit = 0;
-        if (cudaOccupancyMaxActiveClusters(&fit, refine_cluster_kernel, &cfg) == cudaSuccess && fit > 0) {
+        if (cudaOccupancyMaxActiveClusters(&fit, refine_loop_kernel<false>, &cfg) == cudaSuccess && fit > 0) {
             c->max_cluster = q;
             break;
         }

@@ -558,3 +558,45 @@ def test_launched_gain_rows(ctx, k):
         compare_runs(ctx, graphs.rmat(12, 16, seed=5, wmin=1, wmax=100), k, 1.03)
     finally:
         ctx.set_tuning(None)
+
+
+def _ring_lattice(n, reach, seed):
+    """Vertex v joined to v +- 1 .. reach (mod n), weights 1..9: rows of 2 * reach entries."""
+    u = np.repeat(np.arange(n), reach)
+    v = (u + np.tile(np.arange(1, reach + 1), n)) % n
+    w = np.random.default_rng(seed).integers(1, 10, u.size)
+    s, d, w = np.concatenate([u, v]), np.concatenate([v, u]), np.concatenate([w, w])
+    order = np.lexsort((d, s))
+    xadj = np.concatenate([[0], np.cumsum(np.bincount(s, minlength=n))]).astype(np.int32)
+    return graphs.Graph(xadj, d[order].astype(np.int32), np.ones(n, np.int32), w[order].astype(np.int32))
+
+
+# levels whose passes run in one cooperative launch (above 65,536 vertices): short and long
+# rows, dense rows (reach 8, k = 7), one to 1,024 parts, uneven targets
+@pytest.mark.parametrize("n,reach,k,ub,uneven", [(65537, 1, 3, 1.03, False), (66001, 8, 7, 1.03, True),
+                                                 (70001, 3, 1024, 1.05, False), (131072, 2, 100, 1.1, True)])
+def test_cooperative_levels(ctx, n, reach, k, ub, uneven):
+    tp = np.linspace(1.0, 3.0, k).astype(np.float32) if uneven else None
+    compare_runs(ctx, _ring_lattice(n, reach, n), k, ub, tpwgts=tp)
+
+
+def test_cooperative_levels_from_two_threads(ctx):
+    """Two contexts on two threads: their cooperative launches follow one another."""
+    import threading
+    gs = [graphs.grid2d(270, 280, seed=s, wmin=1, wmax=9) for s in (1, 2)]
+    want = [ctx.partition_graph(g, 16, 1.03) for g in gs]
+    got = [None, None]
+
+    def work(i):
+        with hp.Context(0) as c:
+            got[i] = [c.partition_graph(gs[i], 16, 1.03) for _ in range(4)]
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for i in range(2):
+        assert len(got[i]) == 4
+        for part, cut in got[i]:
+            assert cut == want[i][1] and np.array_equal(part, want[i][0])
