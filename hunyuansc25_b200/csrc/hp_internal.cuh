@@ -78,6 +78,12 @@ struct hp_context {
     unsigned long long *log_count = nullptr;
     int64_t log_cap = 0;
 
+    // Staging of large pageable uploads (stage_upload, hp_api.cu): pinned slots and the
+    // events of their last copies.  Batch workers upload directly.
+    char *stage = nullptr;
+    cudaEvent_t stage_ev[16] = {};
+    bool worker = false;
+
     // Graph reaper: executable graphs are released by a background thread once
     // the event recorded after their last launch has completed, so that their
     // destruction never delays the stream (hp_graph_retire, hp_api.cu).

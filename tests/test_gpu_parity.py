@@ -600,3 +600,16 @@ def test_cooperative_levels_from_two_threads(ctx):
         assert len(got[i]) == 4
         for part, cut in got[i]:
             assert cut == want[i][1] and np.array_equal(part, want[i][0])
+
+
+# host arrays above and around the staged upload's bound, weights given or not
+@pytest.mark.parametrize("n,weights", [(699000, True), (699100, False), (1048577, False)])
+def test_large_host_upload(ctx, n, weights):
+    g = _ring_lattice(n, 1, 3) if not weights else _ring_lattice(n // 2, 2, 3)
+    h = graphs.Graph(g.xadj, g.adjncy, g.vwgt if weights else None, g.adjwgt if weights else None)
+    part, cut = ctx.partition(h.xadj, h.adjncy, 4, h.vwgt, h.adjwgt, 1.1)
+    import torch
+    d = [None if a is None else torch.from_numpy(a).cuda() for a in (h.xadj, h.adjncy, h.vwgt, h.adjwgt)]
+    torch.cuda.synchronize()
+    dpart, dcut = ctx.partition_device(d[0], d[1], 4, d[2], d[3], 1.1)
+    assert cut == dcut and np.array_equal(part, dpart.cpu().numpy())
