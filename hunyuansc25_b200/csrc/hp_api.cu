@@ -109,12 +109,20 @@ validate_edges_kernel(int32_t n, int64_t m, int32_t share, const int32_t *__rest
                 const int32_t last = j0 + min(32 * q + 31, left - 1), j = in ? j0 + 32 * q + lane : last;
                 int l = win.find(j);
                 int32_t v = win.r0 + l, rs = __shfl_sync(HP_FULL_MASK, win.start, l);
-                while (last >= win.end) {   // entries of later rows: the next 32 rows
+                for (int step = 0; last >= win.end; step++) {   // entries of later rows
                     const int32_t end = win.end;
-                    win.load(xadj, n, win.r0 + 32);
-                    l = win.find(j);
-                    const int32_t s = __shfl_sync(HP_FULL_MASK, win.start, l);
-                    if (j >= end) { v = win.r0 + l; rs = s; }
+                    if (step < hp::ROW_WINDOWS) {   // the next 32 rows
+                        win.load(xadj, n, win.r0 + 32);
+                        l = win.find(j);
+                        const int32_t s = __shfl_sync(HP_FULL_MASK, win.start, l);
+                        if (j >= end) { v = win.r0 + l; rs = s; }
+                    } else {
+                        if (j >= end) {
+                            v = hp::row_from(xadj, n, win.r0 + 32, j);
+                            rs = xadj[v];
+                        }
+                        win.load(xadj, n, __shfl_sync(HP_FULL_MASK, v, 31));   // (lane 31: entry `last`)
+                    }
                 }
                 int32_t prev = __shfl_up_sync(HP_FULL_MASK, u[q], 1);
                 if (lane == 0) prev = carry;

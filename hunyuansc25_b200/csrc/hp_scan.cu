@@ -114,7 +114,7 @@ __global__ void scatter_flags_kernel(const int32_t *flags, const int32_t *pos, i
 // parts come from a register window (hp::RowWindow).  int64 block sums of 2 x cut.
 // The gathers bound it (one 32-byte L2 sector per entry).  Finding the rows by
 // markers and a max-scan in shared memory, as before, cost about ten shared-memory
-// operations per entry: 515 us against 292 us per call on an RGG of 2^22 vertices
+// operations per entry: 515 us against 280 us per call on an RGG of 2^22 vertices
 // (50 M entries, 436 MB), 2.1 ms against 1.0 ms on one of 2^24.
 constexpr int CUT_THREADS = 256;
 __global__ void __launch_bounds__(CUT_THREADS)
@@ -148,12 +148,22 @@ edgecut_kernel(int32_t n, int64_t m, int32_t share, const int32_t *__restrict__ 
                 const bool in = 32 * q + lane < left;
                 const int32_t last = j0 + min(32 * q + 31, left - 1), j = in ? j0 + 32 * q + lane : last;
                 int32_t own = __shfl_sync(HP_FULL_MASK, pr, win.find(j));
-                while (last >= win.end) {   // entries of later rows: the next 32 rows
+                for (int step = 0; last >= win.end; step++) {   // entries of later rows
                     const int32_t end = win.end;
-                    win.load(xadj, n, win.r0 + 32);
-                    pr = win.r0 + lane < n ? where[win.r0 + lane] : 0;
-                    const int32_t o = __shfl_sync(HP_FULL_MASK, pr, win.find(j));
-                    if (j >= end) own = o;
+                    if (step < hp::ROW_WINDOWS) {   // the next 32 rows
+                        win.load(xadj, n, win.r0 + 32);
+                        pr = win.r0 + lane < n ? where[win.r0 + lane] : 0;
+                        const int32_t o = __shfl_sync(HP_FULL_MASK, pr, win.find(j));
+                        if (j >= end) own = o;
+                    } else {
+                        int32_t r = 0;
+                        if (j >= end) {
+                            r = hp::row_from(xadj, n, win.r0 + 32, j);
+                            own = where[r];
+                        }
+                        win.load(xadj, n, __shfl_sync(HP_FULL_MASK, r, 31));   // (lane 31: entry `last`)
+                        pr = win.r0 + lane < n ? where[win.r0 + lane] : 0;
+                    }
                 }
                 if (in && pu[q] != own) acc += w[q];
             }

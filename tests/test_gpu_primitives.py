@@ -81,6 +81,71 @@ def test_edgecut_walk(ctx, name, unit):
     assert ctx.edgecut_device(t[0], t[1], None if unit else t[2], t[3]) == cut
 
 
+def _path_with_gaps(m, gap, every):
+    """A path over m vertices, `gap` vertices without edges before every `every`-th of them."""
+    at = np.arange(m) + gap * (np.arange(m) // every)
+    n = int(at[-1]) + 1 + gap
+    xadj = np.zeros(n + 1, np.int32)
+    xadj[at + 1] = 2
+    xadj[at[0] + 1] = xadj[at[-1] + 1] = 1
+    adj = np.stack([np.concatenate([[-1], at[:-1]]), np.concatenate([at[1:], [-1]])], 1).ravel()[1:-1]
+    return np.cumsum(xadj, dtype=np.int32), adj.astype(np.int32)
+
+
+# runs of empty rows that end at, before and after the walks' windows, between single rows
+# and between groups of them
+@pytest.mark.parametrize("gap", [31, 32, 63, 64, 65, 95, 96, 97, 129, 1000, 70001])
+@pytest.mark.parametrize("every", [1, 7, 40])
+def test_walks_over_runs_of_empty_rows(ctx, gap, every):
+    import torch
+
+    import hunyuansc25_b200 as hp
+    xadj, adj = _path_with_gaps(min(300, max(3 * every, 2_000_000 * every // gap)), gap, every)
+    n = xadj.size - 1
+    rows = np.repeat(np.arange(n), np.diff(xadj))
+    where = np.random.default_rng(gap).integers(0, 5, n).astype(np.int32)
+    t = [torch.from_numpy(a).cuda() for a in (xadj, adj, where)]
+    torch.cuda.synchronize()
+    assert ctx.edgecut_device(t[0], t[1], None, t[2]) == int((where[rows] != where[adj]).sum()) // 2
+    # the validation: accepted as it is, refused with one entry that has no reverse
+    if n < 20000:
+        ctx.partition(xadj, adj, 2)
+    bad = adj.copy()
+    bad[-1] = rows[0] if rows[0] != bad[-1] else rows[2]
+    with pytest.raises(hp.HpError):
+        ctx.partition(xadj, bad, 2)
+
+
+def test_long_run_of_empty_rows_is_passed_quickly(ctx):
+    """Eight million vertices without edges between two rows cost the edge cut and the
+    validation no walk over them (window by window they take over 80 ms)."""
+    import time
+
+    import torch
+
+    import hunyuansc25_b200 as hp
+    xadj, adj = _path_with_gaps(2000, 1 << 23, 1000)
+    n = xadj.size - 1
+    t = [torch.from_numpy(a).cuda() for a in (xadj, adj)]
+    where = torch.zeros(n, dtype=torch.int32, device="cuda")
+    adj[-1] = 5   # no reverse: refused right after the validation
+    bad = torch.from_numpy(adj).cuda()
+    part = torch.empty(n, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+
+    def refused():
+        with pytest.raises(hp.HpError):
+            ctx.partition_device(t[0], bad, 2, part=part)
+
+    for call in (lambda: ctx.edgecut_device(t[0], t[1], None, where), refused):
+        best = 1e9
+        for _ in range(4):
+            t0 = time.perf_counter()
+            call()
+            best = min(best, time.perf_counter() - t0)
+        assert best < 0.03, best
+
+
 @pytest.mark.parametrize("at", [0, 31, 32, 127, 128, 129, 500])
 def test_validation_of_unsorted_rows(ctx, at):
     """A row that is not ascending at one place is accepted, one that lists a neighbour twice
