@@ -75,26 +75,38 @@ __global__ void gain_cap_kernel(int32_t n, const int32_t *__restrict__ xadj, int
 // Degree statistics of a level, computed for every level at the start of
 // uncoarsening so that the host chooses each level's kernels without reading
 // anything back per level: rows longer than bigd, the longest row of 9..bigd
-// entries, the longest row overall.
+// entries, the longest row overall, the entries of the rows longer than LOOP_LONG_ROW, and
+// the most entries of `range` consecutive rows from a multiple of range on (0: not
+// asked for).
 struct LevelStat {
-    int32_t nbig, small_max, maxdeg, pad;
+    int32_t nbig, small_max, maxdeg, long_entries, range_entries;
 };
+constexpr int32_t LOOP_LONG_ROW = 1024;
 
 __global__ void __launch_bounds__(256)
-level_stats_kernel(int32_t n, const int32_t *__restrict__ xadj, LevelStat *st, int32_t bigd)
+level_stats_kernel(int32_t n, const int32_t *__restrict__ xadj, LevelStat *st, int32_t bigd, int32_t range)
 {
     hp::pdl_wait();
-    int32_t nbig = 0, smax = 0, dmax = 0;
+    int32_t nbig = 0, smax = 0, dmax = 0, lsum = 0, rmax = 0;
+    if (range > 0)
+        for (int64_t v = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * range; v < n;
+             v += (int64_t)gridDim.x * blockDim.x * range)
+            rmax = max(rmax, xadj[v + range < n ? v + range : n] - xadj[v]);
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
         const int32_t d = xadj[v + 1] - xadj[v];
         if (d > bigd) nbig++;
         else if (d > 8) smax = d > smax ? d : smax;
         dmax = d > dmax ? d : dmax;
+        lsum += d > LOOP_LONG_ROW ? d : 0;
     }
     nbig = hp::warp_sum(nbig);
+    lsum = hp::warp_sum(lsum);
     smax = __reduce_max_sync(HP_FULL_MASK, (unsigned)smax);
     dmax = __reduce_max_sync(HP_FULL_MASK, (unsigned)dmax);
+    rmax = __reduce_max_sync(HP_FULL_MASK, (unsigned)rmax);
     if ((threadIdx.x & 31) == 0) {
+        if (lsum) atomicAdd(&st->long_entries, lsum);
+        if (rmax) atomicMax(&st->range_entries, rmax);
         if (nbig) atomicAdd(&st->nbig, nbig);
         if (smax) atomicMax(&st->small_max, smax);
         if (dmax) atomicMax(&st->maxdeg, dmax);
@@ -2781,6 +2793,30 @@ int32_t cluster_level_n(const hp_context *c)
     return (int32_t)std::min<int64_t>((int64_t)c->tune.small_level_n * c->max_cluster, CL_LEVEL_MAX);
 }
 
+// Whether a level may be a cluster's by its size.
+bool cluster_size(const hp_context *c, const HpLevel &g, int32_t k)
+{
+    const int32_t n = cluster_level_n(c);
+    return g.n <= n && k <= CL_KMAX && g.m <= CL_DEG * n;
+}
+
+// ... and by its rows: a warp of the loop walks the rows of its own range of vertices and
+// a moved vertex's row, so a hub row, or many long rows side by side (the low ids of a
+// power-law graph), hold the cluster at its barriers, where the launched passes spread
+// rows over the grid.  Cluster / launched passes, us per pass, grids of 19,600 and 59,536
+// vertices with 1 to 64 hubs, by the most entries in a warp's range: 8,192 43-58 / 53-69,
+// 16,384 42-103 / 58-77, 32,768 44-140 / 57-86, 65,536 60-254 / 63-90; hubs spread over
+// the warps, by the entries of all: 32,768 41-67 / 60-85, 65,536 42-92 / 57-86, 131,072
+// 56-155 / 69-101, 262,144 73-145 / 75-100.  The smallest levels keep the cluster whatever
+// their rows (3,969 vertices, 30,400 entries in a warp's range, k = 256: 81 / 122).
+constexpr int32_t LOOP_WARP_ENTRIES = 16384, LOOP_LONG_ENTRIES = 98304;
+constexpr int32_t LOOP_ANY_ROWS_N = 4096;
+bool loop_rows(const HpLevel &g, const LevelStat &ls)
+{
+    return (g.n <= LOOP_ANY_ROWS_N && g.m <= CL_DEG * LOOP_ANY_ROWS_N) ||
+           (ls.range_entries <= LOOP_WARP_ENTRIES && ls.long_entries <= LOOP_LONG_ENTRIES);
+}
+
 // Levels above that run their passes in one cooperative launch over the whole GPU, a CTA
 // per SM: the same loop with a barrier through global memory (about 2.5 us against the
 // cluster's 1) and 148 SMs.  Launched passes take longer up to about two million vertices
@@ -3742,10 +3778,18 @@ int coop_launch(hp_context *c, F &&launch)
 // Levels above a cluster's that run their pass loop in one cooperative launch over the
 // whole GPU: see GRID_LEVEL_MAX.  Not under the eager loop (the batch workers' contexts
 // share the GPU, and a cooperative launch waits for all of it).
-bool grid_takes(const hp_context *c, const HpLevel &g, int32_t k, const LevelStat &ls)
+bool grid_size(const hp_context *c, const HpLevel &g, int32_t k)
 {
     return c->grid_ctas > 0 && c->tune.small_level_n > 0 && !c->opt.eager && g.n <= GRID_LEVEL_MAX && k <= CL_KMAX &&
-           ls.maxdeg <= GRID_DEG_MAX && g.m <= CL_DEG * (int64_t)g.n;
+           g.m <= CL_DEG * (int64_t)g.n;
+}
+
+// Vertices per warp of the loop kernel that may take the level (LevelStat::range_entries).
+int32_t loop_range(const hp_context *c, const HpLevel &g, int32_t k)
+{
+    const int64_t warps = CL_WARPS * (int64_t)(cluster_size(c, g, k) ? cluster_ctas(c, g.n, g.m) :
+                                               grid_size(c, g, k) ? c->grid_ctas : 0);
+    return warps > 0 ? (int32_t)((g.n + warps - 1) / warps) : 0;
 }
 
 int refine_level(hp_context *c, HpLevel &g, int32_t k, bool finest, const int64_t *d_opt,
@@ -3799,9 +3843,10 @@ int refine_level(hp_context *c, HpLevel &g, int32_t k, bool finest, const int64_
     const bool dbg = getenv("HP_DEBUG_PASSES") != nullptr;
     // small levels: the whole pass loop in one cluster (same rule, same result), in
     // either loop mode unless the per-pass move log or pass log is on
-    const int32_t cl_n = cluster_level_n(c);
-    const bool small_level = !recording && !dbg && n <= cl_n && k <= CL_KMAX && g.m <= CL_DEG * cl_n;
-    const bool grid_level = !small_level && !recording && !dbg && !learned && grid_takes(c, g, k, ls);
+    const bool loop = !recording && !dbg && loop_rows(g, ls);
+    const bool small_level = loop && cluster_size(c, g, k);
+    const bool grid_level = loop && !cluster_size(c, g, k) && !learned && ls.maxdeg <= GRID_DEG_MAX &&
+                            grid_size(c, g, k);
     if (small_level || grid_level) {
         // the level's setup (gain rows, part weights, cut, control block) runs
         // inside the kernel: no launch per setup step
@@ -4019,7 +4064,8 @@ int hp_uncoarsen(hp_context *c, int32_t nparts, const int64_t *h_opt, const int6
     for (int l = 0; l <= L; l++)
         if (c->levels[l].n > 0)
             HP_LAUNCH(c, level_stats_kernel, std::min<unsigned>(nblk(c->levels[l].n), (unsigned)(c->sm_count * 8)),
-                      256, 0, c->levels[l].n, c->levels[l].xadj, d_ls + l, c->tune.gain_thread_deg);
+                      256, 0, c->levels[l].n, c->levels[l].xadj, d_ls + l, c->tune.gain_thread_deg,
+                      loop_range(c, c->levels[l], nparts));
     std::vector<LevelStat> ls(L + 1);
     HP_CUDA(cudaMemcpyAsync(ls.data(), d_ls, sizeof(LevelStat) * (size_t)(L + 1), cudaMemcpyDeviceToHost,
                             c->stream));

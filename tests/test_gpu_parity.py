@@ -560,6 +560,48 @@ def test_launched_gain_rows(ctx, k):
         ctx.set_tuning(None)
 
 
+def hub_grid(side, hubs, deg, seed, scattered=False):
+    """A grid with `hubs` of its vertices joined to `deg` others each; the hubs are the first
+    vertices, or spread evenly."""
+    rng = np.random.default_rng(seed)
+    n = side * side
+    a = np.arange(n).reshape(side, side)
+    e = [np.stack([a[:, :-1].ravel(), a[:, 1:].ravel()]), np.stack([a[:-1].ravel(), a[1:].ravel()])]
+    for i in range(hubs):
+        h = i * (n // hubs) if scattered else i
+        e.append(np.stack([np.full(deg, h), rng.choice(n, deg, replace=False)]))
+    u, v = np.concatenate(e, axis=1)
+    lo, hi = np.minimum(u, v)[u != v], np.maximum(u, v)[u != v]
+    lo, hi = np.divmod(np.unique(lo.astype(np.int64) * n + hi), n)
+    s, d = np.concatenate([lo, hi]), np.concatenate([hi, lo])
+    order = np.lexsort((d, s))
+    xadj = np.concatenate([[0], np.cumsum(np.bincount(s, minlength=n))]).astype(np.int32)
+    return graphs.Graph(xadj, d[order].astype(np.int32), np.ones(n, np.int32), np.ones(d.size, np.int32))
+
+
+# one level (no coarsening): a warp of a cluster would walk the hubs of its 39 vertices (the
+# cooperative launch's: 15 or 43) by itself, so more than 16,384 entries there, or 98,304 in all
+# rows above 1,024, take launched passes (but for levels of 4,096 vertices and 65,536 entries)
+@pytest.mark.parametrize("side,hubs,deg,scattered,launched", [
+    (140, 0, 0, False, False), (140, 1, 16000, False, False), (140, 4, 4000, False, False),
+    (140, 1, 18000, False, True), (140, 5, 4000, False, True), (140, 5, 4000, True, False),
+    (63, 12, 1900, False, False), (140, 23, 4200, True, False), (140, 24, 4200, True, True), (264, 30, 4000, True, True),
+    (264, 17, 950, False, False), (450, 20, 1000, False, True)])
+def test_hub_rows_take_launched_passes(ctx, side, hubs, deg, scattered, launched):
+    g = hub_grid(side, hubs, deg, side + hubs, scattered)
+    opt = default_options(coarsen_to=g.nvtxs, init_starts=2, fm_passes=1)
+    part, cut = ctx.partition_graph(g, 3, 1.05, options=opt)
+    n = ctx.stats().kernel_launches
+    ctx.set_tuning(small_level_n=0)
+    try:
+        lpart, lcut = ctx.partition_graph(g, 3, 1.05, options=opt)
+        m = ctx.stats().kernel_launches
+    finally:
+        ctx.set_tuning(None)
+    assert cut == lcut and np.array_equal(part, lpart)
+    assert (n == m) if launched else (n < m), (n, m)
+
+
 def _ring_lattice(n, reach, seed):
     """Vertex v joined to v +- 1 .. reach (mod n), weights 1..9: rows of 2 * reach entries."""
     u = np.repeat(np.arange(n), reach)
