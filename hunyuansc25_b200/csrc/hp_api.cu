@@ -13,9 +13,9 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <exception>
 #include <mutex>
 #include <numeric>
-#include <system_error>
 #include <thread>
 
 #include "hp_internal.cuh"
@@ -808,13 +808,15 @@ static int check_args(int32_t nvtxs, const void *xadj, const void *adjncy, int32
     return HP_OK;
 }
 
-// Places the level-0 graph (copying host or device inputs into the arena).
 // Upload of pageable host arrays of a large graph.  The driver stages a pageable copy on
-// one thread (about 11 GB/s here); STAGE_THREADS threads copy into pinned slots, each slot
-// sent as it fills (a 73 MB graph: the call 19.1 -> 16.9 ms).  Below STAGE_MIN there is
-// less than a millisecond to save.
-constexpr size_t STAGE_MIN = 8u << 20, STAGE_SLOT = 512u << 10;
-constexpr int STAGE_THREADS = 8, STAGE_SLOTS = 16;
+// one thread (about 11 GB/s here); STAGE_THREADS threads copy into a pinned slot each, a
+// slot sent as it fills (a graph of 73 MB: the call 19.4 -> 17.0 ms; one of 13 MB gains
+// nothing, 20.0 ms both ways).  Pinning the slots takes 2-3 ms, what one such upload
+// saves, so a context's first large upload is copied directly: a program that partitions
+// once pays nothing for it, the second call half a millisecond (19.9 ms).
+constexpr size_t STAGE_MIN = 32u << 20, STAGE_SLOT = 512u << 10;
+constexpr int STAGE_THREADS = 4;   // two threads with two slots each: 17.7 ms
+static_assert(STAGE_THREADS <= sizeof(hp_context::stage_ev) / sizeof(cudaEvent_t), "an event per thread's slot");
 
 struct StageCopy {
     char *dst;
@@ -833,63 +835,71 @@ static bool pageable(const void *p)
 }
 
 // Whether the copies were staged (rc: how that went); false: the caller copies directly.
-static bool stage_upload(hp_context *c, const std::vector<StageCopy> &copies, int *rc)
+static bool stage_upload(hp_context *c, const StageCopy *copies, int ncopies, int *rc)
 {
     size_t total = 0;
-    for (const StageCopy &x : copies) {
-        if (x.bytes && !pageable(x.src)) return false;
-        total += x.bytes;
+    for (int i = 0; i < ncopies; i++) {
+        if (!pageable(copies[i].src)) return false;
+        total += copies[i].bytes;
     }
     if (c->worker || total < STAGE_MIN) return false;
     if (!c->stage) {
-        for (cudaEvent_t &e : c->stage_ev)
-            if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+        if (!c->stage_next) {
+            c->stage_next = true;
+            return false;
+        }
+        for (int i = 0; i < STAGE_THREADS; i++)
+            if (!c->stage_ev[i] && cudaEventCreateWithFlags(&c->stage_ev[i], cudaEventDisableTiming) != cudaSuccess) {
                 cudaGetLastError();
                 return false;
             }
-        if (cudaHostAlloc((void **)&c->stage, STAGE_SLOT * STAGE_SLOTS, cudaHostAllocDefault) != cudaSuccess) {
+        if (cudaHostAlloc((void **)&c->stage, STAGE_SLOT * STAGE_THREADS, cudaHostAllocDefault) != cudaSuccess) {
             cudaGetLastError();
             c->stage = nullptr;
             return false;
         }
     }
-    std::vector<StageCopy> chunks;
-    for (const StageCopy &x : copies)
-        for (size_t o = 0; o < x.bytes; o += STAGE_SLOT)
-            chunks.push_back({x.dst + o, x.src + o, std::min(STAGE_SLOT, x.bytes - o)});
-    std::atomic<size_t> next{0};
+    std::atomic<size_t> next{0};   // chunks of STAGE_SLOT bytes, in the order of the copies
     std::atomic<int> err{0};
-    // thread t owns slots t and t + STAGE_THREADS, in turn; a slot is filled again once
-    // its last copy is done (its event; a new event counts as done)
+    // a thread fills its slot again once the slot's last copy is done (its event; a new
+    // event counts as done)
     auto work = [&](int t) {
         if (cudaSetDevice(c->device) != cudaSuccess) { err = 1; return; }
-        for (int turn = 0;; turn ^= 1) {
-            const size_t i = next.fetch_add(1);
-            if (i >= chunks.size() || err) return;
-            const int s = t + turn * STAGE_THREADS;
-            char *slot = c->stage + (size_t)s * STAGE_SLOT;
-            cudaError_t e = cudaEventSynchronize(c->stage_ev[s]);
-            if (e == cudaSuccess) {
-                memcpy(slot, chunks[i].src, chunks[i].bytes);
-                e = cudaMemcpyAsync(chunks[i].dst, slot, chunks[i].bytes, cudaMemcpyHostToDevice, c->stream);
+        for (;;) {
+            size_t at = next.fetch_add(1);
+            int i = 0;
+            for (; i < ncopies; i++) {
+                const size_t chunks = (copies[i].bytes + STAGE_SLOT - 1) / STAGE_SLOT;
+                if (at < chunks) break;
+                at -= chunks;
             }
-            if (e == cudaSuccess) e = cudaEventRecord(c->stage_ev[s], c->stream);
+            if (i == ncopies || err) return;
+            const size_t off = at * STAGE_SLOT, bytes = std::min(STAGE_SLOT, copies[i].bytes - off);
+            char *slot = c->stage + (size_t)t * STAGE_SLOT;
+            cudaError_t e = cudaEventSynchronize(c->stage_ev[t]);
+            if (e == cudaSuccess) {
+                memcpy(slot, copies[i].src + off, bytes);
+                e = cudaMemcpyAsync(copies[i].dst + off, slot, bytes, cudaMemcpyHostToDevice, c->stream);
+            }
+            if (e == cudaSuccess) e = cudaEventRecord(c->stage_ev[t], c->stream);
             if (e != cudaSuccess) { err = 1; return; }
         }
     };
     std::thread th[STAGE_THREADS];
     try {
         for (int t = 1; t < STAGE_THREADS; t++) th[t] = std::thread(work, t);
-    } catch (const std::system_error &) {
-        // fewer threads: those that started and this one share the chunks
+    } catch (const std::exception &) {
+        // no thread or no memory for one: those that started and this one share the chunks
     }
     work(0);
     for (std::thread &t : th)
         if (t.joinable()) t.join();
     *rc = err ? HP_ERR_CUDA : HP_OK;
+    c->staged_uploads++;
     return true;
 }
 
+// Places the level-0 graph (copying host or device inputs into the arena).
 static int place_level0(hp_context *c, int32_t n, int64_t m, const int32_t *xadj, const int32_t *adjncy,
                         const int32_t *vwgt, const int32_t *adjwgt, cudaMemcpyKind kind)
 {
@@ -902,17 +912,19 @@ static int place_level0(hp_context *c, int32_t n, int64_t m, const int32_t *xadj
     g.adjwgt = lalloc_t<int32_t>(c, m);
     g.vwgt = lalloc_t<int32_t>(c, n);
     HP_CHECK_OOM(c);
-    std::vector<StageCopy> copies;
+    StageCopy copies[4];
+    int nc = 0;
     auto add = [&](int32_t *dst, const int32_t *src, int64_t count) {
-        if (src && count > 0) copies.push_back({(char *)dst, (const char *)src, sizeof(int32_t) * (size_t)count});
+        if (src && count > 0) copies[nc++] = {(char *)dst, (const char *)src, sizeof(int32_t) * (size_t)count};
     };
     add(g.xadj, xadj, (int64_t)n + 1);
     add(g.adjncy, adjncy, m);
     add(g.adjwgt, adjwgt, m);
     add(g.vwgt, vwgt, n);
     int rc = HP_OK;
-    if (kind != cudaMemcpyHostToDevice || !stage_upload(c, copies, &rc))
-        for (const StageCopy &x : copies) HP_CUDA(cudaMemcpyAsync(x.dst, x.src, x.bytes, kind, c->stream));
+    if (kind != cudaMemcpyHostToDevice || !stage_upload(c, copies, nc, &rc))
+        for (int i = 0; i < nc; i++)
+            HP_CUDA(cudaMemcpyAsync(copies[i].dst, copies[i].src, copies[i].bytes, kind, c->stream));
     HP_TRY(rc);
     if (!adjwgt && m > 0) HP_LAUNCH(c, fill_ones_kernel, gsz(c, m), 256, 0, m, g.adjwgt);
     if (!vwgt && n > 0) HP_LAUNCH(c, fill_ones_kernel, gsz(c, n), 256, 0, (int64_t)n, g.vwgt);
@@ -1227,6 +1239,11 @@ HP_API int hp_test_arena_restarts(hp_context *ctx)
 {
     if (!ctx) return HP_ERR_INVALID_ARG;
     return ctx->arena_restarts;
+}
+
+HP_API int hp_test_staged_uploads(const hp_context *ctx)
+{
+    return ctx ? ctx->staged_uploads : HP_ERR_INVALID_ARG;
 }
 
 HP_API int hp_test_wide_rows(hp_context *ctx, int32_t on)

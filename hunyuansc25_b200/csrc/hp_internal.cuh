@@ -79,10 +79,12 @@ struct hp_context {
     int64_t log_cap = 0;
 
     // Staging of large pageable uploads (stage_upload, hp_api.cu): pinned slots and the
-    // events of their last copies.  Batch workers upload directly.
+    // events of their last copies, from the context's second such upload on.  Batch
+    // workers upload directly.
     char *stage = nullptr;
-    cudaEvent_t stage_ev[16] = {};
-    bool worker = false;
+    cudaEvent_t stage_ev[4] = {};
+    bool stage_next = false, worker = false;
+    int staged_uploads = 0;
 
     // Graph reaper: executable graphs are released by a background thread once
     // the event recorded after their last launch has completed, so that their

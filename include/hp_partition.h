@@ -357,6 +357,10 @@ int hp_test_wait_expiry(hp_context *ctx);
 int hp_test_arena_first(hp_context *ctx, int64_t bytes);
 int hp_test_arena_restarts(hp_context *ctx);
 
+/* Uploads of this context that went through its pinned staging slots: pageable host
+ * arrays of 32 MiB or more, from the second such call on. */
+int hp_test_staged_uploads(const hp_context *ctx);
+
 /* Test of the contraction's 64-bit row sorts, which levels of 2^22 (long rows) or
  * 2^27 (short rows) coarse vertices take: on != 0 makes this context's calls take
  * them on every level, 0 restores the rule.  Speed only; the rows are the same. */

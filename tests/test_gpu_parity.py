@@ -644,14 +644,26 @@ def test_cooperative_levels_from_two_threads(ctx):
             assert cut == want[i][1] and np.array_equal(part, want[i][0])
 
 
-# host arrays above and around the staged upload's bound, weights given or not
-@pytest.mark.parametrize("n,weights", [(699000, True), (699100, False), (1048577, False)])
-def test_large_host_upload(ctx, n, weights):
-    g = _ring_lattice(n, 1, 3) if not weights else _ring_lattice(n // 2, 2, 3)
-    h = graphs.Graph(g.xadj, g.adjncy, g.vwgt if weights else None, g.adjwgt if weights else None)
-    part, cut = ctx.partition(h.xadj, h.adjncy, 4, h.vwgt, h.adjwgt, 1.1)
+# host arrays just below and above the staged upload's bound (32 MiB), and well above it, weights
+# given or not: direct below it and from pinned memory; above it direct the first time of a
+# context, then staged
+@pytest.mark.parametrize("n,weights,pinned,staged", [(699000, True, False, False), (2796202, False, False, False),
+                                                     (2796203, False, False, True), (1800001, True, False, True),
+                                                     (2900001, False, True, False)])
+def test_large_host_upload(n, weights, pinned, staged):
     import torch
-    d = [None if a is None else torch.from_numpy(a).cuda() for a in (h.xadj, h.adjncy, h.vwgt, h.adjwgt)]
+    g = _ring_lattice(n, 1, 3) if not weights else _ring_lattice(n // 2, 2, 3)
+    h = [g.xadj, g.adjncy, g.vwgt if weights else None, g.adjwgt if weights else None]
+    size = sum(a.nbytes for a in h if a is not None)
+    assert (size >= 32 << 20) == (staged or pinned)
+    keep = [None if a is None or not pinned else torch.from_numpy(a).pin_memory() for a in h]
+    h = [a if t is None else t.numpy() for a, t in zip(h, keep)]
+    d = [None if a is None else torch.from_numpy(a).cuda() for a in h]
     torch.cuda.synchronize()
-    dpart, dcut = ctx.partition_device(d[0], d[1], 4, d[2], d[3], 1.1)
-    assert cut == dcut and np.array_equal(part, dpart.cpu().numpy())
+    with hp.Context(0) as c:
+        dpart, dcut = c.partition_device(d[0], d[1], 4, d[2], d[3], 1.1)
+        dpart = dpart.cpu().numpy()
+        for call in range(3):
+            part, cut = c.partition(h[0], h[1], 4, h[2], h[3], 1.1)
+            assert cut == dcut and np.array_equal(part, dpart)
+            assert c.lib.hp_test_staged_uploads(c.h) == (call if staged else 0)
