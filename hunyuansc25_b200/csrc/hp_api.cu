@@ -779,6 +779,7 @@ HP_API void hp_context_destroy(hp_context *c)
     }
     cudaSetDevice(c->device);
     if (c->own_stream) cudaStreamSynchronize(c->own_stream);
+    hp_refine_close(c);
     if (c->arena) cudaFree(c->arena);
     if (c->d_status) cudaFree(c->d_status);
     if (c->lb_status) cudaFree(c->lb_status);

@@ -27,6 +27,8 @@ struct hp_context {
     int sm_count = 148;
     int max_cluster = 1;             // CTAs of the largest cluster refine_loop_kernel can run in
     int grid_ctas = 0;               // CTAs of its cooperative launches (0: not available)
+    cudaEvent_t coop_ev = nullptr;   // the end of this context's latest one
+    unsigned long long cuda_ctx = 0; // id of the CUDA context (another one after a device reset)
     cudaStream_t stream = nullptr;   // stream of the current call
     cudaStream_t own_stream = nullptr;
 
@@ -291,6 +293,7 @@ int hp_uncoarsen(hp_context *c, int32_t nparts, const int64_t *h_opt, const int6
 int hp_ensure_workers(hp_context *ctx, int nworkers);
 
 int hp_refine_init(hp_context *c);
+void hp_refine_close(hp_context *c);
 int hp_initpart_init();
 int hp_coarsen_init();
 int hp_mlp_ensure(hp_context *c);

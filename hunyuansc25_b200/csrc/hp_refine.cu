@@ -15,6 +15,8 @@
 // vertex id) via a stable radix sort, the cut is int64, balance is judged
 // against integer maximum part weights, and one status read per pass replaces
 // the reference's 4-6 blocking reads.
+#include <cuda.h>
+
 #include <chrono>
 #include <cstdlib>
 
@@ -3751,10 +3753,13 @@ struct LevelLaunches {
 };
 
 // Cooperative launches of one device, from any context and thread, follow one another:
-// each takes every SM, and two that were half resident would wait for each other.
+// each takes every SM, and two that were half resident would wait for each other.  The
+// event of the latest one belongs to the context that launched it, which takes itself out
+// when it is destroyed.  A context that the caller left behind at a device reset has
+// another CUDA context's id: its event is gone, and so is its launch.
 struct CoopOrder {
     std::mutex mu;
-    cudaEvent_t last = nullptr;   // the end of the latest one
+    const hp_context *last = nullptr;
 };
 
 CoopOrder &coop_order(int device)
@@ -3768,10 +3773,10 @@ int coop_launch(hp_context *c, F &&launch)
 {
     CoopOrder &o = coop_order(c->device);
     std::lock_guard<std::mutex> lk(o.mu);
-    if (o.last) HP_CUDA(cudaStreamWaitEvent(c->stream, o.last, 0));
-    else HP_CUDA(cudaEventCreateWithFlags(&o.last, cudaEventDisableTiming));
+    if (o.last && o.last->cuda_ctx == c->cuda_ctx) HP_CUDA(cudaStreamWaitEvent(c->stream, o.last->coop_ev, 0));
     const int rc = launch();
-    HP_CUDA(cudaEventRecord(o.last, c->stream));
+    HP_CUDA(cudaEventRecord(c->coop_ev, c->stream));
+    o.last = c;
     return rc;
 }
 
@@ -4021,7 +4026,13 @@ int hp_refine_init(hp_context *c)
     int per_sm = 0, coop = 0;
     HP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, refine_loop_kernel<true>, CL_THREADS, smem));
     HP_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device));
-    c->grid_ctas = coop && per_sm > 0 && c->device < 64 ? c->sm_count : 0;
+    using GetId = CUresult (*)(CUcontext, unsigned long long *);
+    void *get_id = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    HP_CUDA(cudaGetDriverEntryPoint("cuCtxGetId", &get_id, cudaEnableDefault, &found));
+    const bool id = found == cudaDriverEntryPointSuccess && ((GetId)get_id)(nullptr, &c->cuda_ctx) == CUDA_SUCCESS;
+    HP_CUDA(cudaEventCreateWithFlags(&c->coop_ev, cudaEventDisableTiming));
+    c->grid_ctas = id && coop && per_sm > 0 && c->device < 64 ? c->sm_count : 0;
     // the largest cluster the device can place
     c->max_cluster = 1;
     for (int q = CL_MAX; q > 1; q /= 2) {
@@ -4044,6 +4055,16 @@ int hp_refine_init(hp_context *c)
         cudaGetLastError();
     }
     return HP_OK;
+}
+
+void hp_refine_close(hp_context *c)
+{
+    {
+        CoopOrder &o = coop_order(c->device);
+        std::lock_guard<std::mutex> lk(o.mu);
+        if (o.last == c) o.last = nullptr;
+    }
+    if (c->coop_ev) cudaEventDestroy(c->coop_ev);
 }
 
 int hp_uncoarsen(hp_context *c, int32_t nparts, const int64_t *h_opt, const int64_t *h_maxp)

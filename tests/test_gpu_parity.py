@@ -644,6 +644,35 @@ def test_cooperative_levels_from_two_threads(ctx):
             assert cut == want[i][1] and np.array_equal(part, want[i][0])
 
 
+_RESET = """
+import ctypes, sys
+sys.path.insert(0, sys.argv[1])
+import numpy as np
+import hunyuansc25_b200 as hp
+from hunyuansc25_b200 import graphs
+g = graphs.grid2d(270, 280, seed=1, wmin=1, wmax=9)
+with hp.Context(0) as c:
+    want = c.partition_graph(g, 16, 1.03)
+cu, dev = ctypes.CDLL("libcuda.so.1"), ctypes.c_int()
+assert cu.cuDeviceGet(ctypes.byref(dev), 0) == 0 and cu.cuDevicePrimaryCtxReset_v2(dev) == 0
+for _ in range(2):
+    with hp.Context(0) as c:
+        part, cut = c.partition_graph(g, 16, 1.03)
+    assert cut == want[1] and np.array_equal(part, want[0])
+"""
+
+
+def test_contexts_after_a_device_reset():
+    """The caller closes its contexts, resets the device in its own process and makes new ones:
+    nothing of the old ones, such as the order of their cooperative launches, is still used."""
+    import subprocess
+    import sys
+
+    from conftest import ROOT
+    res = subprocess.run([sys.executable, "-c", _RESET, ROOT], capture_output=True, text=True, timeout=120)
+    assert res.returncode == 0, (res.returncode, res.stderr)
+
+
 # host arrays just below and above the staged upload's bound (32 MiB), and well above it, weights
 # given or not: direct below it and from pinned memory; above it direct the first time of a
 # context, then staged
