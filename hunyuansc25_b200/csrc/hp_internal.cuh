@@ -106,6 +106,7 @@ struct hp_context {
     std::vector<HpLevel> levels;
     bool trace_valid = false;
     bool wide_rows = false;              // hp_test_wide_rows: contraction rows take the 64-bit sorts
+    bool refuse_coop = false;            // hp_test_refuse_coop: cooperative launches are refused
     bool weight_check = false;           // total edge weight >= 2^31: contractions check pair bounds
     bool learned_skewed = false;         // the input's degrees are skewed enough for the learned proposals
     hp_options opt = {};
@@ -211,11 +212,6 @@ inline cudaError_t hp_launch_coop(const hp_context *c, void (*kernel)(P...), uns
     HP_LAUNCH_CHECKED(ctx, kernel, grid,                                                    \
                       hp_launch_kernel((ctx), kernel, (unsigned)(grid), (unsigned)(block),  \
                                        (size_t)(smem), (unsigned)(cluster), __VA_ARGS__))
-// A cooperative launch.
-#define HP_LAUNCH_COOP(ctx, kernel, grid, block, smem, ...)                                 \
-    HP_LAUNCH_CHECKED(ctx, kernel, grid,                                                    \
-                      hp_launch_coop((ctx), kernel, (unsigned)(grid), (unsigned)(block),    \
-                                     (size_t)(smem), __VA_ARGS__))
 #define HP_LAUNCH_CHECKED(ctx, kernel, grid, launch)                                        \
     do {                                                                                    \
         if ((ctx)->oom) return HP_ERR_NOMEM;                                                \

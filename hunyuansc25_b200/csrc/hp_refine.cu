@@ -3768,16 +3768,26 @@ CoopOrder &coop_order(int device)
     return order[device & 63];
 }
 
-template <class F>
-int coop_launch(hp_context *c, F &&launch)
+// Launches the level's loop on `ctas` CTAs.  *refused: the device does not place them all
+// at once (its SMs are shared out since the context was made); nothing was launched, and
+// the level takes launched passes.
+int coop_launch(hp_context *c, int ctas, size_t smem, const SmallLevel &a, bool *refused)
 {
     CoopOrder &o = coop_order(c->device);
     std::lock_guard<std::mutex> lk(o.mu);
     if (o.last && o.last->cuda_ctx == c->cuda_ctx) HP_CUDA(cudaStreamWaitEvent(c->stream, o.last->coop_ev, 0));
-    const int rc = launch();
+    const cudaError_t e = c->refuse_coop ? cudaErrorCooperativeLaunchTooLarge :
+                                           hp_launch_coop(c, refine_loop_kernel<true>, (unsigned)ctas, CL_THREADS, smem, a);
+    *refused = e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources;
+    if (*refused) {
+        cudaGetLastError();
+        return HP_OK;
+    }
+    HP_CUDA(e);
+    c->launches++;
     HP_CUDA(cudaEventRecord(c->coop_ev, c->stream));
     o.last = c;
-    return rc;
+    return HP_OK;
 }
 
 // Levels above a cluster's that run their pass loop in one cooperative launch over the
@@ -3852,6 +3862,7 @@ int refine_level(hp_context *c, HpLevel &g, int32_t k, bool finest, const int64_
     const bool small_level = loop && cluster_size(c, g, k);
     const bool grid_level = loop && !cluster_size(c, g, k) && !learned && ls.maxdeg <= GRID_DEG_MAX &&
                             grid_size(c, g, k);
+    const size_t loop_mark = c->hi;
     if (small_level || grid_level) {
         // the level's setup (gain rows, part weights, cut, control block) runs
         // inside the kernel: no launch per setup step
@@ -3918,17 +3929,19 @@ int refine_level(hp_context *c, HpLevel &g, int32_t k, bool finest, const int64_
             HP_CHECK_OOM(c);
             HP_CUDA(cudaMemsetAsync(a.bar, 0, sizeof(unsigned), c->stream));
             HP_CUDA(cudaMemsetAsync(c->d_scal, 0, sizeof(unsigned long long) * S_PASS_END, c->stream));
-            HP_TRY(coop_launch(c, [&]() -> int {
-                HP_LAUNCH_COOP(c, refine_loop_kernel<true>, ctas, CL_THREADS, smem, a);
+            bool refused = false;
+            HP_TRY(coop_launch(c, ctas, smem, a, &refused));
+            if (!refused) {
+                c->hi = mark;
                 return HP_OK;
-            }));
+            }
+            c->hi = loop_mark;   // (what the loop took)
+        } else {
+            const int ctas = cluster_ctas(c, n, g.m);
+            HP_LAUNCH_CLUSTER(c, refine_loop_kernel<false>, ctas, ctas, CL_THREADS, smem, a);
             c->hi = mark;
             return HP_OK;
         }
-        const int ctas = cluster_ctas(c, n, g.m);
-        HP_LAUNCH_CLUSTER(c, refine_loop_kernel<false>, ctas, ctas, CL_THREADS, smem, a);
-        c->hi = mark;
-        return HP_OK;
     }
     unsigned long long *sc = c->d_scal;
     HP_CUDA(cudaMemsetAsync(sc, 0, sizeof(unsigned long long) * (S_DONE + 1), c->stream));

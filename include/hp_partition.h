@@ -361,6 +361,11 @@ int hp_test_arena_restarts(hp_context *ctx);
  * arrays of 32 MiB or more, from the second such call on. */
 int hp_test_staged_uploads(const hp_context *ctx);
 
+/* Test of a device that refuses a cooperative launch (its SMs are shared out): on != 0
+ * makes every such launch of this context end with that error instead of being issued,
+ * 0 restores them.  The levels then take launched passes; the results are the same. */
+int hp_test_refuse_coop(hp_context *ctx, int32_t on);
+
 /* Test of the contraction's 64-bit row sorts, which levels of 2^22 (long rows) or
  * 2^27 (short rows) coarse vertices take: on != 0 makes this context's calls take
  * them on every level, 0 restores the rule.  Speed only; the rows are the same. */

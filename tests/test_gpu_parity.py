@@ -644,6 +644,22 @@ def test_cooperative_levels_from_two_threads(ctx):
             assert cut == want[i][1] and np.array_equal(part, want[i][0])
 
 
+def test_refused_cooperative_launch_takes_launched_passes(ctx):
+    """A device that does not place a cooperative launch: the same partition by launched passes,
+    and the cooperative launches again once it does."""
+    g = _ring_lattice(66001, 3, 8)
+    runs = []
+    for on in (0, 1, 0):
+        assert ctx.lib.hp_test_refuse_coop(ctx.h, on) == 0
+        try:
+            runs.append((*ctx.partition_graph(g, 7, 1.03), ctx.stats().kernel_launches))
+        finally:
+            ctx.lib.hp_test_refuse_coop(ctx.h, 0)
+    for part, cut, _ in runs[1:]:
+        assert cut == runs[0][1] and np.array_equal(part, runs[0][0])
+    assert runs[0][2] == runs[2][2] < runs[1][2]
+
+
 _RESET = """
 import ctypes, sys
 sys.path.insert(0, sys.argv[1])
