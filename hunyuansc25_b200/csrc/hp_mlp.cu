@@ -148,6 +148,8 @@ mlp_grad_kernel(const float *__restrict__ P, const float *__restrict__ X, const 
             y += wj.w * z[3];
             *reinterpret_cast<float4 *>(row2 + j) = make_float4(z[0], z[1], z[2], z[3]);
         }
+        if (!ok)   // no sample: no activations (they may overflow where no sample's do, and 0 x inf counts)
+            for (int j = 0; j < HP_MLP_H; j++) row1[j] = row2[j] = 0.f;
         // loss = softplus(y) - t*y ; dL/dy = sigmoid(y) - t
         const float sp = y > 0 ? y + log1pf(__expf(-y)) : log1pf(__expf(y));
         const float dy = ok ? (1.f / (1.f + __expf(-y)) - t) * scale : 0.f;

@@ -58,6 +58,31 @@ def test_gradient_sizes(ctx, n):
     assert np.linalg.norm(g - rg) <= 6e-6 * np.linalg.norm(rg)
 
 
+@pytest.mark.parametrize("n", [1, 31, 33])
+def test_gradient_of_the_last_tile_has_no_other_terms(ctx, n):
+    """Weights with which a sample of zeros would overflow, and none of the given ones does:
+    the lanes past the last sample add nothing to the gradient."""
+    import torch
+    x, y = _data(n, 3)
+    x[:, 0] = 1.0
+    p = learn.init_params(5)
+    p[0:8] = 0.0
+    p[0], p[256] = -2e38, 1e38          # unit 0 of layer 1: -1e38 for the samples, 1e38 for zeros
+    p[288:1312:32] = 10.0               # ... which layer 2 would turn into infinity
+    ctx.mlp_set_params(p)
+    xt, yt = torch.from_numpy(x).cuda(), torch.from_numpy(y).cuda()
+    loss, g = ctx.mlp_loss_grad(xt, yt)
+    q = torch.from_numpy(p).cuda().double().requires_grad_(True)
+    w1, b1, w2, b2, w3, b3 = torch.split(q, [256, 32, 1024, 32, 32, 1])
+    h = torch.relu(xt.double() @ w1.view(32, 8).T + b1)
+    h = torch.relu(h @ w2.view(32, 32).T + b2)
+    ref = torch.nn.functional.binary_cross_entropy_with_logits(h @ w3 + b3, yt.double())
+    ref.backward()
+    rg = q.grad.cpu().numpy()
+    assert abs(loss - ref.item()) <= 6e-6 * abs(ref.item())       # (the bound of test_gradient_sizes)
+    assert np.linalg.norm(g - rg) <= 6e-6 * np.linalg.norm(rg)
+
+
 def test_inference_tensor_cores_vs_fp32(ctx):
     import torch
     x, _ = _data(10007, 2)
