@@ -259,6 +259,7 @@ PROTOTYPES = {
     "hp_scan_exclusive_i32_noalloc": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p]),
     "hp_test_wait_expiry": (C.c_int, [C.c_void_p]),
     "hp_test_staged_uploads": (C.c_int, [C.c_void_p]),
+    "hp_test_grid_expiry": (C.c_int, [C.c_void_p, C.c_int32]),
     "hp_test_refuse_coop": (C.c_int, [C.c_void_p, C.c_int32]),
     "hp_test_wide_rows": (C.c_int, [C.c_void_p, C.c_int32]),
     "hp_test_arena_first": (C.c_int, [C.c_void_p, C.c_int64]),

@@ -1247,6 +1247,13 @@ HP_API int hp_test_staged_uploads(const hp_context *ctx)
     return ctx ? ctx->staged_uploads : HP_ERR_INVALID_ARG;
 }
 
+HP_API int hp_test_grid_expiry(hp_context *ctx, int32_t on)
+{
+    if (!ctx) return HP_ERR_INVALID_ARG;
+    ctx->grid_short = on != 0;
+    return HP_OK;
+}
+
 HP_API int hp_test_refuse_coop(hp_context *ctx, int32_t on)
 {
     if (!ctx) return HP_ERR_INVALID_ARG;

@@ -107,6 +107,7 @@ struct hp_context {
     bool trace_valid = false;
     bool wide_rows = false;              // hp_test_wide_rows: contraction rows take the 64-bit sorts
     bool refuse_coop = false;            // hp_test_refuse_coop: cooperative launches are refused
+    bool grid_short = false;             // hp_test_grid_expiry: their first barrier never completes
     bool weight_check = false;           // total edge weight >= 2^31: contractions check pair bounds
     bool learned_skewed = false;         // the input's degrees are skewed enough for the learned proposals
     hp_options opt = {};

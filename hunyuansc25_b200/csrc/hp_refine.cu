@@ -2759,6 +2759,7 @@ struct SmallLevel {
     unsigned *status;
     // the grid variant's barrier counter (zero at launch) and exchange arrays
     unsigned *bar;
+    unsigned spin_limit;
     long long *gx;          // 2 x CTAs x 3
     int32_t *ghist;         // CTAs x 256
 };
@@ -2877,10 +2878,10 @@ __device__ __forceinline__ int32_t cl_ld32(unsigned addr)
 
 // The barrier of the grid variant (a cooperative launch: every CTA is resident): an
 // arrival counter that only grows, *gen its value when the last barrier completed.
-// Writes before it are visible after it.  The wait is bounded: on expiry it sets
+// Writes before it are visible after it.  The wait is bounded by `limit`: on expiry it sets
 // HP_STATUS_SPIN_TIMEOUT and returns false in every thread of the CTA, which then
 // leaves the kernel (as the CTAs that wait for it will).
-__device__ __forceinline__ bool grid_sync(unsigned *bar, unsigned *gen, unsigned *status)
+__device__ __forceinline__ bool grid_sync(unsigned *bar, unsigned *gen, unsigned *status, unsigned limit)
 {
     __shared__ bool s_ok;
     *gen += gridDim.x;
@@ -2892,7 +2893,7 @@ __device__ __forceinline__ bool grid_sync(unsigned *bar, unsigned *gen, unsigned
         for (;;) {
             asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
             if ((int)(seen - *gen) >= 0) break;
-            if (++spins > HP_SPIN_LIMIT) {
+            if (++spins > limit) {
                 atomicOr(status, HP_STATUS_SPIN_TIMEOUT);
                 break;
             }
@@ -2929,7 +2930,7 @@ struct ClTeam {
     // All threads of the team; false: the wait expired and the kernel ends.
     __device__ __forceinline__ bool sync()
     {
-        if (GRID) return grid_sync(a.bar, &gen, a.status);
+        if (GRID) return grid_sync(a.bar, &gen, a.status, a.spin_limit);
         cl_sync();
         return true;
     }
@@ -3927,7 +3928,9 @@ int refine_level(hp_context *c, HpLevel &g, int32_t k, bool finest, const int64_
             a.gx = ralloc_t<long long>(c, 2 * 3 * (int64_t)ctas);
             a.ghist = ralloc_t<int32_t>(c, 256 * (int64_t)ctas);
             HP_CHECK_OOM(c);
-            HP_CUDA(cudaMemsetAsync(a.bar, 0, sizeof(unsigned), c->stream));
+            // (hp_test_grid_expiry: one arrival short, so the first barrier never completes)
+            a.spin_limit = c->grid_short ? 1u << 14 : HP_SPIN_LIMIT;
+            HP_CUDA(cudaMemsetAsync(a.bar, c->grid_short ? 0xff : 0, sizeof(unsigned), c->stream));
             HP_CUDA(cudaMemsetAsync(c->d_scal, 0, sizeof(unsigned long long) * S_PASS_END, c->stream));
             bool refused = false;
             HP_TRY(coop_launch(c, ctas, smem, a, &refused));

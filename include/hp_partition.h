@@ -361,6 +361,12 @@ int hp_test_arena_restarts(hp_context *ctx);
  * arrays of 32 MiB or more, from the second such call on. */
 int hp_test_staged_uploads(const hp_context *ctx);
 
+/* Test of the cooperative launches' barrier: on != 0 makes the barrier of this context's
+ * launches start one arrival short, with a limit of 2^14 polls, so that the first wait of
+ * every CTA runs out: all of them return and the call ends with HP_ERR_TIMEOUT.  0
+ * restores it; the context stays usable. */
+int hp_test_grid_expiry(hp_context *ctx, int32_t on);
+
 /* Test of a device that refuses a cooperative launch (its SMs are shared out): on != 0
  * makes every such launch of this context end with that error instead of being issued,
  * 0 restores them.  The levels then take launched passes; the results are the same. */

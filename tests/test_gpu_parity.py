@@ -243,6 +243,21 @@ def test_bounded_wait_expiry(ctx):
     compare_runs(ctx, graphs.grid2d(40, 30, seed=6, wmin=1, wmax=5), 8)
 
 
+def test_grid_barrier_expiry(ctx):
+    """The same for the barrier of the cooperative launches: one arrival that never comes, every
+    CTA gives up and returns, the call reports HP_ERR_TIMEOUT, and the context then partitions."""
+    g = graphs.grid2d(270, 280, seed=1, wmin=1, wmax=9)
+    assert ctx.lib.hp_test_grid_expiry(ctx.h, 1) == 0
+    try:
+        t0 = time.perf_counter()
+        with pytest.raises(hp.HpError) as e:
+            ctx.partition_graph(g, 16, 1.03)
+        assert e.value.code == HP_ERR_TIMEOUT and time.perf_counter() - t0 < 5
+    finally:
+        ctx.lib.hp_test_grid_expiry(ctx.h, 0)
+    compare_runs(ctx, g, 16)
+
+
 def test_arena_exhaustion_retry(ctx):
     """The arena's grow-and-retry path, driven from the host: the first attempt
     gets a small arena, runs out, launches nothing more and restarts with twice
