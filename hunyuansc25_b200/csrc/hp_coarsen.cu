@@ -897,13 +897,15 @@ contract_assemble_kernel(int32_t cn, ContractSrc src, const int32_t *__restrict_
 // the row's entries come from the tile's staging buffer (packed key << 32 |
 // weight, the self key already PACK_NONE); a bitonic network of NET sorts them
 // and the unique keys are counted.
-template <int NET, int XN>
+constexpr int ASM_WIDE = HP_TUNE_THREAD_ROW_MAX;
+
+template <int NET>
 __device__ __forceinline__ int sort_wide_row(const unsigned long long *stage, int32_t len,
-                                               unsigned long long (&x)[XN])
+                                             unsigned long long (&x)[ASM_WIDE])
 {
 #pragma unroll
     for (int i = 0; i < NET; i++) x[i] = i < len ? stage[i] : hp::PACK_NONE;
-    hp::sort_regs<NET, XN>(x);
+    hp::sort_regs<NET, ASM_WIDE>(x);
     int u = 0;
 #pragma unroll
     for (int i = 0; i < NET; i++) {
@@ -916,9 +918,9 @@ __device__ __forceinline__ int sort_wide_row(const unsigned long long *stage, in
 
 // The sorted row merged (weights of equal keys summed) into out[0..u), each
 // entry tagged with the tile row t.
-template <int NET, int XN>
-__device__ __forceinline__ void emit_wide_row(const unsigned long long (&x)[XN], unsigned long long *out,
-                                                uint8_t *orow, uint8_t t)
+template <int NET>
+__device__ __forceinline__ void emit_wide_row(const unsigned long long (&x)[ASM_WIDE], unsigned long long *out,
+                                              uint8_t *orow, uint8_t t)
 {
     int r = -1;
     uint32_t prev = 0xffffffffu;
@@ -941,16 +943,15 @@ __device__ __forceinline__ void emit_wide_row(const unsigned long long (&x)[XN],
     if (r >= 0) out[r] = ((unsigned long long)prev << 32) | (uint32_t)acc;
 }
 
-template <int XN>
 __global__ void __launch_bounds__(ASM_TILE)
 contract_assemble_wide_kernel(int32_t cn, ContractSrc src, const int32_t *__restrict__ ucnt,
-                         int32_t *__restrict__ cxadj, int32_t *__restrict__ cadjncy,
-                         int32_t *__restrict__ cadjwgt, unsigned long long *tile_status, hp::LbCtl *lb,
-                         unsigned *status, int32_t thread_row, int wcheck)
+                              int32_t *__restrict__ cxadj, int32_t *__restrict__ cadjncy,
+                              int32_t *__restrict__ cadjwgt, unsigned long long *tile_status, hp::LbCtl *lb,
+                              unsigned *status, int32_t thread_row, int wcheck)
 {
     hp::pdl_wait();
-    extern __shared__ unsigned long long asm_stage[];                      // ASM_TILE * XN
-    uint8_t *s_row = reinterpret_cast<uint8_t *>(asm_stage + ASM_TILE * XN);   // tile row of each entry
+    extern __shared__ unsigned long long asm_stage[];                      // ASM_TILE * ASM_WIDE
+    uint8_t *s_row = reinterpret_cast<uint8_t *>(asm_stage + ASM_TILE * ASM_WIDE);   // tile row of each entry
     __shared__ int4 s_ri[ASM_TILE];
     __shared__ int32_t s_off[ASM_TILE];     // staged offset of the row's input, then of its output
     __shared__ int32_t s_goff[ASM_TILE];    // the row's final offset
@@ -1013,15 +1014,15 @@ contract_assemble_wide_kernel(int32_t cn, ContractSrc src, const int32_t *__rest
         if (ws >= (long long)INT32_MAX) atomicOr(status, HP_STATUS_WEIGHT_RANGE);
     }
     const unsigned wmax = __reduce_max_sync(HP_FULL_MASK, small ? (unsigned)len : 0u);
-    unsigned long long x[XN];
+    unsigned long long x[ASM_WIDE];
     int u = 0;
     if (c < cn && !small) u = ucnt[c];
-    if (XN == 8 || wmax <= 8) {
-        if (small) u = sort_wide_row<8, XN>(asm_stage + ioff, len, x);
-    } else if (XN == 16 || wmax <= 16) {
-        if (small) u = sort_wide_row<(XN < 16 ? XN : 16), XN>(asm_stage + ioff, len, x);
+    if (wmax <= 8) {
+        if (small) u = sort_wide_row<8>(asm_stage + ioff, len, x);
+    } else if (wmax <= 16) {
+        if (small) u = sort_wide_row<16>(asm_stage + ioff, len, x);
     } else {
-        if (small) u = sort_wide_row<XN, XN>(asm_stage + ioff, len, x);
+        if (small) u = sort_wide_row<ASM_WIDE>(asm_stage + ioff, len, x);
     }
     int agg, tout;
     const int local = hp::block_excl_scan<ASM_TILE>(u, &agg, s_scan);   // (the staged input is read)
@@ -1031,10 +1032,9 @@ contract_assemble_wide_kernel(int32_t cn, ContractSrc src, const int32_t *__rest
         if (t == 0) s_excl = excl;
     }
     if (small) {
-        if (XN == 8 || wmax <= 8) emit_wide_row<8, XN>(x, asm_stage + ooff, s_row + ooff, (uint8_t)t);
-        else if (XN == 16 || wmax <= 16)
-            emit_wide_row<(XN < 16 ? XN : 16), XN>(x, asm_stage + ooff, s_row + ooff, (uint8_t)t);
-        else emit_wide_row<XN, XN>(x, asm_stage + ooff, s_row + ooff, (uint8_t)t);
+        if (wmax <= 8) emit_wide_row<8>(x, asm_stage + ooff, s_row + ooff, (uint8_t)t);
+        else if (wmax <= 16) emit_wide_row<16>(x, asm_stage + ooff, s_row + ooff, (uint8_t)t);
+        else emit_wide_row<ASM_WIDE>(x, asm_stage + ooff, s_row + ooff, (uint8_t)t);
     }
     s_off[t] = ooff;
     __syncthreads();
@@ -2233,13 +2233,14 @@ int contract_level(hp_context *c, HpLevel &g, int32_t cn, HpLevel &cg)
         // a level whose coarse ids fit a shared-memory dense accumulator merges
         // every long row there (one atomic per entry, ordered extraction)
         const bool smem_dense = cn <= c->tune.contract_smem_cn;
-        // the lists those kernels take: the rows that a register network does not
-        const struct { int32_t list, n; int32_t *count; } accl[3] = {
-            {words_long ? 4 : 1, words_cta2 ? 0 : words_long ? h.sub[1] : h.cnt[1],
-             words_long ? &sub_counts[1] : &counts[1]},
-            {5, words_cta4 || !words_long ? 0 : h.sub[2], &sub_counts[2]},
-            {2, h.cnt[2], &counts[2]}};
-        const int64_t acc_rows = (int64_t)accl[0].n + accl[1].n + accl[2].n;
+        // the lists those kernels take: the rows above CROW_MAX, and those below it where no
+        // register network runs (hp_test_wide_rows: at their sizes the ids leave room for
+        // every network's index)
+        static_assert(std::max(HY_MAX_CN, HP_TUNE_SMEM_CN_MAX) < 1 << (32 - ws_idx_bits(WS_LONG_NR * 4)),
+                      "networks of all row lengths run where the accumulators do");
+        const struct { int32_t list, n; int32_t *count; } accl[2] = {{1, words_long ? 0 : h.cnt[1], &counts[1]},
+                                                                     {2, h.cnt[2], &counts[2]}};
+        const int64_t acc_rows = (int64_t)accl[0].n + accl[1].n;
         if (smem_dense) {
             const size_t acc = sizeof(int32_t) * ((size_t)cn + (cn + 31) / 32 + (cn + 1023) / 1024);
             for (const auto &a : accl)
@@ -2249,8 +2250,9 @@ int contract_level(hp_context *c, HpLevel &g, int32_t cn, HpLevel &cg)
                               (int32_t *)nullptr, (unsigned *)nullptr, (unsigned *)nullptr,
                               c->tune.dense_sparse_ratio, 0, wchk, c->d_status);
         }
-        // hybrid: the same rows accumulate their low ids densely and radix-sort the rest; rows whose rest does not fit go to the spill list,
-        // which the CTA radix (up to XROW_MAX) and dense slab kernels then take
+        // hybrid: the same rows accumulate their low ids densely and radix-sort the rest;
+        // rows whose rest does not fit go to the spill list, which the CTA radix (up to
+        // XROW_MAX) and dense slab kernels then take
         const bool hybrid = !smem_dense && cn <= HY_MAX_CN && c->tune.contract_hybrid && acc_rows > 0;
         int32_t *spill = nullptr;
         int32_t *d_nspill = (int32_t *)&sc[4];
@@ -2312,7 +2314,7 @@ int contract_level(hp_context *c, HpLevel &g, int32_t cn, HpLevel &cg)
                   c->lb_status, c->lb_ctl, c->d_status, c->tune.contract_thread_row, wchk);
         return HP_OK;
     };
-    if (!words_asm) HP_TRY(assemble(contract_assemble_wide_kernel<32>, asm_smem_bytes<32>()));
+    if (!words_asm) HP_TRY(assemble(contract_assemble_wide_kernel, asm_smem_bytes<ASM_WIDE>()));
     else if (h.small_max <= 8) HP_TRY(assemble(contract_assemble_kernel<8>, asm_smem_bytes<8>()));
     else if (h.small_max <= 16) HP_TRY(assemble(contract_assemble_kernel<16>, asm_smem_bytes<16>()));
     else HP_TRY(assemble(contract_assemble_kernel<32>, asm_smem_bytes<32>()));
@@ -2343,7 +2345,7 @@ int hp_coarsen_init()
 {
     HP_CUDA(cudaFuncSetAttribute(contract_assemble_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)asm_smem_bytes<32>()));
-    HP_CUDA(cudaFuncSetAttribute(contract_assemble_wide_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    HP_CUDA(cudaFuncSetAttribute(contract_assemble_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)asm_smem_bytes<32>()));
     HP_CUDA(cudaFuncSetAttribute(match_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)ms_smem_bytes(HP_TUNE_SMALL_MATCH_MAX)));

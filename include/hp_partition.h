@@ -372,9 +372,11 @@ int hp_test_grid_expiry(hp_context *ctx, int32_t on);
  * 0 restores them.  The levels then take launched passes; the results are the same. */
 int hp_test_refuse_coop(hp_context *ctx, int32_t on);
 
-/* Test of the contraction's 64-bit row sorts, which levels of 2^22 (long rows) or
- * 2^27 (short rows) coarse vertices take: on != 0 makes this context's calls take
- * them on every level, 0 restores the rule.  Speed only; the rows are the same. */
+/* Test of the contraction's 64-bit row sorts, which levels of too many coarse vertices
+ * for an id and an index in 32 bits take: 2^27 for rows of up to 32 entries, 2^24 up to
+ * 256, 2^22 up to 1024, 2^21 up to 2048, 2^20 up to 4096.  on != 0 makes this context's
+ * calls take them on every level, 0 restores the rule.  Speed only; the rows are the
+ * same. */
 int hp_test_wide_rows(hp_context *ctx, int32_t on);
 
 /* ---- legacy drop-in ------------------------------------------------------------
