@@ -55,7 +55,9 @@ SPACE = {
     "warp_dense_k": [0, 256, 512, 1024],
     "grid_ctas_per_sm": [2, 4, 8, 12, 16],
     "dense_sparse_ratio": [1, 2, 4, 8, 32],
-    "small_level_n": [0, 2048, 4096, 8192, 16384, 32768],
+    # vertices per CTA of a cluster: 16 CTAs reach the bound of 65,536 at 4096; 0 also turns
+    # off the cooperative loop of the larger levels
+    "small_level_n": [0, 512, 1024, 2048, 4096],
     "chunk_deg": [512, 1024, 2048, 4096, 8192],
     "trial_cta_n": [128, 256, 512, 1024, 4096, 1 << 24],
     "contract_smem_cn": [0, 8192, 16384, 32768, 49152],

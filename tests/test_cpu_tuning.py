@@ -66,6 +66,12 @@ def test_every_search_value_is_in_range_alone():
             assert bad in (None, name), (name, v, bad)
 
 
+def test_small_level_values_differ():
+    """16 CTAs of small_level_n vertices, at most 65,536: every value searched is another bound."""
+    bounds = [min(16 * v, 65536) for v in tune.SPACE["small_level_n"]]
+    assert len(set(bounds)) == len(bounds)
+
+
 def test_tuning_file_round_trip(tmp_path):
     t = dict(TUNING_DEFAULTS, match_warp_deg=16, grid_ctas_per_sm=4)
     p = tmp_path / "x.json"
