@@ -640,7 +640,8 @@ def main():
                                     "launches": int(prof_launch[i]), "source": source[i]}
                     for i in timed},
     }
-    graph_vs_eager = {"timed_loop": "CUDA graph per level" if tuned["graph_passes"] else "launched passes",
+    graph_vs_eager = {"timed_loop": "one launch per level up to its bound, above it " +
+                                    ("a CUDA graph per level" if tuned["graph_passes"] else "launched passes"),
                       "graph_ms": round(graph_ms, 3), "eager_ms": round(eager_ms, 3),
                       "speedup": round(eager_ms / graph_ms, 4),
                       "identical_cut": int(ecut) == int(cut) == int(gcut),

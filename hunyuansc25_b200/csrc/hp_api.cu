@@ -81,7 +81,9 @@ validate_edges_kernel(int32_t n, int64_t m, int32_t share, const int32_t *__rest
                       int32_t *__restrict__ unsorted, unsigned long long *sums)
 {
     hp::pdl_wait();
-    if (*status & HP_STATUS_BAD_GRAPH) return;   // uniform over the grid
+    // (the same in all lanes of a warp; a warp that starts late may also see a flag of this
+    // launch: the graph is refused either way, and the sums are not read)
+    if (*status & HP_STATUS_BAD_GRAPH) return;
     const int lane = threadIdx.x & 31;
     bool bad = false;
     unsigned long long fp = 0;

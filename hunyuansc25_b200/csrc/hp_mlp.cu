@@ -48,7 +48,7 @@ __device__ __forceinline__ float mlp_fwd(const float *__restrict__ P, const floa
 // per sample for its 32 multiply-adds; four weights come with every broadcast
 // read of the forward and backward layers.  Writing every sample's 1,377
 // gradient terms to memory and summing them afterwards, as before, moved 11 KB
-// per sample: 2,107 us against 125 us (19.8 TFLOP/s) for 300,000 samples, with
+// per sample: 2,107 us against 125 us (17.5 TFLOP/s) for 300,000 samples, with
 // an error against 64-bit sums of 8.9e-8 against 2.7e-8.
 constexpr int MG_WARPS = 4;
 constexpr int MG_THREADS = 32 * MG_WARPS;

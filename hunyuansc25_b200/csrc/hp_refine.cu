@@ -42,6 +42,12 @@ __global__ void project_kernel(int32_t n, const int32_t *__restrict__ cmap,
     if (v < n) where[v] = cwhere[cmap[v]];
 }
 
+// Gain row of v: (part, connectivity) for every part adjacent to v, ascending
+// by part, padded with part -1 up to min(deg, k).  A vertex with deg >= k has a
+// dense row instead: entry q is (q, conn to part q), zeros included.  When a neighbour
+// moves, a dense row is updated in place by atomics and a sparse one rebuilt; a pass that
+// moves much of the level rebuilds both (RebuildRule).
+//
 // Row capacities min(deg, k); rows longer than bigd go on the big list, rows
 // longer than huged (the caller's chunk_deg) also on the long-row list (count
 // d_bigcnt[3]), rows longer than hubd (gain_hub_deg) on the hub list (count
@@ -213,10 +219,6 @@ gain_tile_kernel(int32_t n, const int32_t *__restrict__ xadj, const int32_t *__r
     }
 }
 
-// Gain row of v: (part, connectivity) for every part adjacent to v, ascending
-// by part, padded with part -1 up to min(deg, k).  A vertex with deg >= k has a
-// dense row instead: entry q is (q, conn to part q), zeros included; dense rows
-// are updated in place by atomics when a neighbour moves and never rebuilt.
 // Rows of a pass's rebuild.  A pass whose moves touch more than `over` entries of the
 // level's adjacency rebuilds every row (apply_moves_kernel then touches none), else
 // the rows that the moves queued.
@@ -2727,8 +2729,7 @@ int pass_apply(hp_context *c, HpLevel &g, RefineBufs &B, const PassCfg &P, cudaG
 // Per level and pass, one CTA or the launched kernels before, a cluster now: 128^3 grid
 // (k = 64) 2,817 vertices 100 -> 47 us, 8,854 93 -> 58, 25,181 85 -> 62; 256^2 grid
 // (k = 8) 10,870 vertices 62 -> 28 us, 65,536 63 -> 36.  Fewer than about 512 vertices
-// per CTA buy nothing: the passes are chains of L2 latencies and barriers; above
-// CL_LEVEL_MAX the grid-wide kernels' 148 SMs win.
+// per CTA buy nothing: the passes are chains of L2 latencies and barriers.
 constexpr int CL_THREADS = 1024;
 constexpr int CL_WARPS = CL_THREADS / 32;
 constexpr int CL_MAX = 16;                 // CTAs of a cluster (above 8: non-portable size)
@@ -2786,9 +2787,13 @@ int cluster_ctas(const hp_context *c, int32_t n, int64_t m)
     return q;
 }
 
-// The largest level a cluster takes: small_level_n vertices per CTA, at most
-// CL_LEVEL_MAX (above it the grid-wide kernels' memory parallelism wins), and at
-// most CL_DEG entries per vertex of that bound.
+// The largest level a cluster takes: small_level_n vertices per CTA, at most CL_LEVEL_MAX,
+// and at most CL_DEG entries per vertex of that bound.  Above CL_LEVEL_MAX the same loop
+// over the whole GPU has cheaper passes.  Cluster / cooperative launch, us per pass:
+// RGG (k = 100, 12 entries a vertex) 32,768 vertices 39 / 44, 49,152 46 / 45, 65,536
+// 47 / 46, 81,920 52 / 44, 131,072 68 / 47; 3-D grid (k = 64, 5.8 entries) 32,768 34 / 44,
+// 64,000 43 / 47, 81,356 48 / 48, 97,336 50 / 47, 130,050 57 / 49; 2-D grid (k = 8,
+// 4 entries) 65,536 35 / 39, 81,796 37 / 40, 98,596 42 / 40, 131,044 44 / 35.
 constexpr int32_t CL_LEVEL_MAX = 65536;
 constexpr int64_t CL_DEG = 16;
 int32_t cluster_level_n(const hp_context *c)
@@ -2822,12 +2827,14 @@ bool loop_rows(const HpLevel &g, const LevelStat &ls)
 
 // Levels above that run their passes in one cooperative launch over the whole GPU, a CTA
 // per SM: the same loop with a barrier through global memory (about 2.5 us against the
-// cluster's 1) and 148 SMs.  Launched passes take longer up to about two million vertices
-// (a pass of the 128^3 grid, k = 64: 110,557 vertices 68 -> 60 us, 614,464 89 -> 77,
-// 2,097,152 129 -> 112; RGG, k = 1024: 477,503 81 -> 66, 1,450,170 115 -> 92), and their
-// graphs cost the host half a millisecond a level; above it the launched kernels'
-// occupancy wins (2,598,047 vertices 194 us launched, about 210 here).  A longer row than
-// GRID_DEG_MAX would hold the one warp that walks it.
+// cluster's 1) and 148 SMs.  Against launched passes (a graph), us per pass: 3-D grid
+// (k = 64) 130,050 vertices 49 / 54, 1,000,000 74 / 94, 2,097,152 113 / 129, 8,000,000
+// 295 / 326; RGG (k = 100) 131,072 47 / 57, 1,000,000 95 / 116, 2,097,152 144 / 172,
+// 4,500,000 258 / 291.  It was not slower at any size, and saves the host half a
+// millisecond a level for the graph.  GRID_LEVEL_MAX is no crossing: it bounds how long a
+// launch that needs every SM keeps the other streams of the device out (about 3 ms for
+// the twenty passes of a level), which launched passes let in between their kernels.
+// A longer row than GRID_DEG_MAX would hold the one warp that walks it.
 constexpr int32_t GRID_LEVEL_MAX = 1 << 21;
 constexpr int32_t GRID_DEG_MAX = 1024;
 

@@ -70,11 +70,15 @@ typedef struct hp_options {
     int32_t  validate;         /* 0 none, 1 structural check on the device (default)          */
     int32_t  trace;            /* 1: keep every level for hp_trace_*() (tests)                */
     int32_t  profile;          /* 1: time kernel classes with CUDA events into hp_stats.prof_* */
-    int32_t  eager;            /* 0: each level's refinement passes run as one CUDA graph
-                                  (device-side WHILE/SWITCH control, default); 1: passes
-                                  launched one by one with a host read per pass.  Results
-                                  are identical.  With profile = 1 the graphed LP and
-                                  gain-rebuild launches are not timed (eager ones are).    */
+    int32_t  eager;            /* 0 (default): no host read between a level's refinement
+                                  passes.  They run in one launch of a thread-block cluster
+                                  (up to 65,536 vertices) or of the whole GPU (cooperative,
+                                  up to 2^21), else as one CUDA graph (device-side
+                                  WHILE/SWITCH control; hp_tuning.graph_passes).  1: only
+                                  the clusters; above them passes are launched one by one
+                                  with a host read per pass.  Results are identical.  With
+                                  profile = 1 only eager launches of the pass classes are
+                                  timed.                                                   */
     uint64_t seed;             /* matching tie-break seed (default 1)                         */
 } hp_options;
 
@@ -121,7 +125,12 @@ void        hp_options_default(hp_options *opt);
 const char *hp_strerror(int code);
 
 /* A context owns one device arena and the per-call state; one context per
- * thread (contexts share nothing). device = CUDA ordinal. */
+ * thread.  Contexts share no data, and their calls overlap on the device -- except
+ * that a cooperative launch (hp_options.eager = 0, levels of 65,537 to 2^21 vertices)
+ * needs every SM: it starts when the kernels then running on the device, of other
+ * contexts and streams too, leave them free, and such launches of a process follow one
+ * another.  A caller with kernels in flight that wait for this call to return sets
+ * eager = 1.  device = CUDA ordinal. */
 int  hp_context_create(int device, hp_context **out);
 void hp_context_destroy(hp_context *ctx);
 
@@ -163,8 +172,10 @@ typedef struct hp_tuning {
     int32_t match_cta_deg;       /* matching: rows longer than this take a CTA   [match_warp_deg, 2^24] 4096 */
     int32_t contract_thread_row; /* contraction: coarse rows up to this many
                                     entries merge in one thread's registers      [8, 32]       32 */
-    int32_t contract_warp_row;   /* ... up to this by a warp radix sort           [contract_thread_row, 256] 256 */
-    int32_t contract_cta_row;    /* ... up to this by a 256-thread CTA radix sort [contract_warp_row, 4096] 4096;
+    int32_t contract_warp_row;   /* ... up to this by a warp                      [contract_thread_row, 256] 256 */
+    int32_t contract_cta_row;    /* ... up to this by a warp or a CTA of two or four
+                                    (register networks; radix sorts where id and index do
+                                    not fit 32 bits)                   [contract_warp_row, 4096] 4096;
                                     longer rows: 1024-thread radix up to 12288, dense above */
     int32_t gain_thread_deg;     /* refinement: gain rows of up to this many entries by a
                                     thread or lane segment                        [8, 32]       32 */
@@ -178,7 +189,9 @@ typedef struct hp_tuning {
     int32_t small_level_n;       /* refinement: levels of at most this many vertices per CTA of
                                     a cluster (16 CTAs where the device has them; at most 65536
                                     vertices, 16x as many adjacency entries, nparts <= 1024)
-                                    run all their passes in one cluster; 0 = never [0, 32768]    4096 */
+                                    run all their passes in one cluster, unless hub rows
+                                    would hold single warps; 0 = never, and no cooperative
+                                    launches of larger levels either             [0, 32768]    4096 */
     int32_t chunk_deg;           /* refinement: the afterburner and move application
                                     split rows longer than this into chunks of 512
                                     entries over the whole grid                  [gain_thread_deg, 2^24] 4096 */
@@ -186,8 +199,9 @@ typedef struct hp_tuning {
                                     subgraph has at least this many vertices runs
                                     a CTA per trial instead of a warp             [1, 2^24]     512 */
     int32_t contract_smem_cn;    /* contraction: a level with at most this many coarse
-                                    vertices merges its long rows in a shared-memory
-                                    dense accumulator instead of radix sorts      [0, 49152]    49152 */
+                                    vertices merges its rows above contract_cta_row in a
+                                    shared-memory dense accumulator instead of radix sorts
+                                                                                  [0, 49152]    49152 */
     int32_t batch_workers;       /* hp_partition_batch: worker contexts (streams) that
                                     partition graphs concurrently                 [1, 64]       16 */
     int32_t small_match_n;       /* coarsening: levels of at most this many vertices (and
@@ -195,7 +209,7 @@ typedef struct hp_tuning {
                                     CTA; 0 = never                               [0, 8192]     8192 */
     int32_t contract_hybrid;     /* contraction: on levels with more coarse vertices than
                                     contract_smem_cn and at most 131072, rows longer than
-                                    contract_warp_row accumulate their ids below 32768 in
+                                    contract_cta_row accumulate their ids below 32768 in
                                     a shared-memory dense accumulator and radix-sort the
                                     rest (1), or radix-sort every entry (0)      [0, 1]        1 */
     int32_t apply_chunk_deg;     /* refinement: move application splits rows longer than
@@ -205,9 +219,10 @@ typedef struct hp_tuning {
                                     previous one drains and waits for it on the device
                                     (programmatic dependent launch) (1), or after it (0)
                                                                                   [0, 1]        1 */
-    int32_t graph_passes;        /* refinement: each level's pass loop as one CUDA graph with
-                                    device-side control (1), or its passes launched one by one
-                                    (0); hp_options.eager = 1 forces the latter.  Results are
+    int32_t graph_passes;        /* refinement: the pass loop of a level that does not run in one
+                                    launch (small_level_n) as one CUDA graph with device-side
+                                    control (1), or its passes launched one by one (0);
+                                    hp_options.eager = 1 forces the latter.  Results are
                                     identical                                     [0, 1]        1 */
     int32_t reserved[4];         /* zero */
 } hp_tuning;
