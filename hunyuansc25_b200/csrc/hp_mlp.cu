@@ -43,10 +43,11 @@ __device__ __forceinline__ float mlp_fwd(const float *__restrict__ P, const floa
 //                      partial gradients;
 //   mlp_finish_kernel  adds the CTAs' rows in a fixed order (in double: the rows
 //                      are few) and, in training, takes the Adam step.
-// The bound is FP32 arithmetic: about 3,600 multiply-adds per sample against 36
-// bytes.  The W2 block of 32 registers per lane takes three shared-memory reads
-// per sample for its 32 multiply-adds; four weights come with every broadcast
-// read of the forward and backward layers.  Writing every sample's 1,377
+// The work is about 3,600 multiply-adds per sample against 36 bytes; the bound is the
+// shared-memory pipe that feeds them (4 M samples: the pipe 93 % busy, issue 59 %).  The
+// W2 block of 32 registers per lane takes three shared-memory reads per sample for its 32
+// multiply-adds; four weights come with every broadcast read of the forward and backward
+// layers.  Writing every sample's 1,377
 // gradient terms to memory and summing them afterwards, as before, moved 11 KB
 // per sample: 2,107 us against 125 us (17.5 TFLOP/s) for 300,000 samples, with
 // an error against 64-bit sums of 8.9e-8 against 2.7e-8.

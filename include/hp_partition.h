@@ -129,8 +129,9 @@ const char *hp_strerror(int code);
  * that a cooperative launch (hp_options.eager = 0, levels of 65,537 to 2^21 vertices)
  * needs every SM: it starts when the kernels then running on the device, of other
  * contexts and streams too, leave them free, and such launches of a process follow one
- * another.  A caller with kernels in flight that wait for this call to return sets
- * eager = 1.  device = CUDA ordinal. */
+ * another; a cluster launch (levels of up to 65,536 vertices) needs up to 16 SMs side by
+ * side.  A caller with kernels in flight that never end, or that wait for this call to
+ * return, sets hp_tuning.small_level_n = 0: neither is used then.  device = CUDA ordinal. */
 int  hp_context_create(int device, hp_context **out);
 void hp_context_destroy(hp_context *ctx);
 
