@@ -18,6 +18,7 @@
 #include <cuda.h>
 
 #include <chrono>
+#include <cmath>
 #include <cstdlib>
 
 #include "hp_internal.cuh"
@@ -84,22 +85,36 @@ __global__ void gain_cap_kernel(int32_t n, const int32_t *__restrict__ xadj, int
 // uncoarsening so that the host chooses each level's kernels without reading
 // anything back per level: rows longer than bigd, the longest row of 9..bigd
 // entries, the longest row overall, the entries of the rows longer than LOOP_LONG_ROW, and
-// the most entries of `range` consecutive rows from a multiple of range on (0: not
-// asked for).
+// the most weighted entries of `range` consecutive rows from a multiple of range on (0: not
+// asked for): an entry counts LOOP_UNIT in a row longer than LOOP_LONG_ROW, `weight` in
+// others (loop_rows).
 struct LevelStat {
-    int32_t nbig, small_max, maxdeg, long_entries, range_entries;
+    int32_t nbig, small_max, maxdeg, long_entries;
+    unsigned long long range_entries;
 };
-constexpr int32_t LOOP_LONG_ROW = 1024;
+constexpr int32_t LOOP_LONG_ROW = 1024, LOOP_UNIT = 8;
 
 __global__ void __launch_bounds__(256)
-level_stats_kernel(int32_t n, const int32_t *__restrict__ xadj, LevelStat *st, int32_t bigd, int32_t range)
+level_stats_kernel(int32_t n, const int32_t *__restrict__ xadj, LevelStat *st, int32_t bigd, int32_t range,
+                   int32_t weight)
 {
     hp::pdl_wait();
-    int32_t nbig = 0, smax = 0, dmax = 0, lsum = 0, rmax = 0;
-    if (range > 0)
-        for (int64_t v = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * range; v < n;
-             v += (int64_t)gridDim.x * blockDim.x * range)
-            rmax = max(rmax, xadj[v + range < n ? v + range : n] - xadj[v]);
+    int32_t nbig = 0, smax = 0, dmax = 0, lsum = 0;
+    if (range > 0) {   // a warp per range
+        const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+        long long rmax = 0;
+        for (int64_t v0 = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * range; v0 < n; v0 += nwarps * range) {
+            const int64_t v1 = v0 + range < n ? v0 + range : n;
+            long long e = 0;
+            for (int64_t v = v0 + (threadIdx.x & 31); v < v1; v += 32) {
+                const int32_t d = xadj[v + 1] - xadj[v];
+                e += (long long)d * (d > LOOP_LONG_ROW ? LOOP_UNIT : weight);
+            }
+            e = hp::warp_sum64(e);
+            rmax = e > rmax ? e : rmax;
+        }
+        if ((threadIdx.x & 31) == 0 && rmax > 0) atomicMax(&st->range_entries, (unsigned long long)rmax);
+    }
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
         const int32_t d = xadj[v + 1] - xadj[v];
         if (d > bigd) nbig++;
@@ -111,10 +126,8 @@ level_stats_kernel(int32_t n, const int32_t *__restrict__ xadj, LevelStat *st, i
     lsum = hp::warp_sum(lsum);
     smax = __reduce_max_sync(HP_FULL_MASK, (unsigned)smax);
     dmax = __reduce_max_sync(HP_FULL_MASK, (unsigned)dmax);
-    rmax = __reduce_max_sync(HP_FULL_MASK, (unsigned)rmax);
     if ((threadIdx.x & 31) == 0) {
         if (lsum) atomicAdd(&st->long_entries, lsum);
-        if (rmax) atomicMax(&st->range_entries, rmax);
         if (nbig) atomicAdd(&st->nbig, nbig);
         if (smax) atomicMax(&st->small_max, smax);
         if (dmax) atomicMax(&st->maxdeg, dmax);
@@ -2811,18 +2824,30 @@ bool cluster_size(const hp_context *c, const HpLevel &g, int32_t k)
 // ... and by its rows: a warp of the loop walks the rows of its own range of vertices and
 // a moved vertex's row, so a hub row, or many long rows side by side (the low ids of a
 // power-law graph), hold the cluster at its barriers, where the launched passes spread
-// rows over the grid.  Cluster / launched passes, us per pass, grids of 19,600 and 59,536
-// vertices with 1 to 64 hubs, by the most entries in a warp's range: 8,192 43-58 / 53-69,
-// 16,384 42-103 / 58-77, 32,768 44-140 / 57-86, 65,536 60-254 / 63-90; hubs spread over
-// the warps, by the entries of all: 32,768 41-67 / 60-85, 65,536 42-92 / 57-86, 131,072
-// 56-155 / 69-101, 262,144 73-145 / 75-100.  The smallest levels keep the cluster whatever
-// their rows (3,969 vertices, 30,400 entries in a warp's range, k = 256: 81 / 122).
-constexpr int32_t LOOP_WARP_ENTRIES = 16384, LOOP_LONG_ENTRIES = 98304;
+// rows over the grid.  The entries in a range at which both take the same time:
+//   rows above LOOP_LONG_ROW (grids of 19,600 and 59,536 vertices with 1 to 64 hubs,
+//   k = 8 to 256; us per pass cluster / launched): 8,192 43-58 / 53-69, 16,384 42-103 /
+//   58-77, 32,768 44-140 / 57-86, 65,536 60-254 / 63-90;
+//   rows below it (R-MAT, 8,000 to 65,536 vertices), where every gain row of more than 32
+//   parts is a warp's turn: about 32,000 for k = 8 (31,111 76 / 82, 36,033 97 / 83),
+//   24,000 for 16 (18,187 81 / 78, 26,784 69 / 75), 16,000 for 32 (16,240 80 / 72, 15,410
+//   70 / 74), 12,000 for 64 (11,628 77 / 85, 14,306 93 / 87), 9,500 for 200 (8,758 91 / 83,
+//   15,410 127 / 95): so an entry counts sqrt(k) / 5.6 there, at most 1.75.
+// Hubs spread over the warps count by all their entries (us per pass): 32,768 41-67 / 60-85,
+// 65,536 42-92 / 57-86, 131,072 56-155 / 69-101, 262,144 73-145 / 75-100.  The smallest
+// levels keep the cluster whatever their rows (3,969 vertices, 30,400 entries in a warp's
+// range, k = 256: 81 / 122).
+constexpr int64_t LOOP_WARP_ENTRIES = 16384;
+constexpr int32_t LOOP_LONG_ENTRIES = 98304;
+int32_t loop_weight(int32_t k)
+{
+    return (int32_t)std::lround(LOOP_UNIT * std::min(1.75, std::sqrt((double)k) / 5.6));
+}
 constexpr int32_t LOOP_ANY_ROWS_N = 4096;
 bool loop_rows(const HpLevel &g, const LevelStat &ls)
 {
     return (g.n <= LOOP_ANY_ROWS_N && g.m <= CL_DEG * LOOP_ANY_ROWS_N) ||
-           (ls.range_entries <= LOOP_WARP_ENTRIES && ls.long_entries <= LOOP_LONG_ENTRIES);
+           ((int64_t)ls.range_entries <= LOOP_UNIT * LOOP_WARP_ENTRIES && ls.long_entries <= LOOP_LONG_ENTRIES);
 }
 
 // Levels above that run their passes in one cooperative launch over the whole GPU, a CTA
@@ -4109,7 +4134,7 @@ int hp_uncoarsen(hp_context *c, int32_t nparts, const int64_t *h_opt, const int6
         if (c->levels[l].n > 0)
             HP_LAUNCH(c, level_stats_kernel, std::min<unsigned>(nblk(c->levels[l].n), (unsigned)(c->sm_count * 8)),
                       256, 0, c->levels[l].n, c->levels[l].xadj, d_ls + l, c->tune.gain_thread_deg,
-                      loop_range(c, c->levels[l], nparts));
+                      loop_range(c, c->levels[l], nparts), loop_weight(nparts));
     std::vector<LevelStat> ls(L + 1);
     HP_CUDA(cudaMemcpyAsync(ls.data(), d_ls, sizeof(LevelStat) * (size_t)(L + 1), cudaMemcpyDeviceToHost,
                             c->stream));

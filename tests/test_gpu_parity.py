@@ -595,21 +595,24 @@ def hub_grid(side, hubs, deg, seed, scattered=False):
 
 
 # one level (no coarsening): a warp of a cluster would walk the hubs of its 39 vertices (the
-# cooperative launch's: 15 or 43) by itself, so more than 16,384 entries there, or 98,304 in all
-# rows above 1,024, take launched passes (but for levels of 4,096 vertices and 65,536 entries)
-@pytest.mark.parametrize("side,hubs,deg,scattered,launched", [
-    (140, 0, 0, False, False), (140, 1, 16000, False, False), (140, 4, 4000, False, False),
-    (140, 1, 18000, False, True), (140, 5, 4000, False, True), (140, 5, 4000, True, False),
-    (63, 12, 1900, False, False), (140, 23, 4200, True, False), (140, 24, 4200, True, True), (264, 30, 4000, True, True),
-    (264, 17, 950, False, False), (450, 20, 1000, False, True)])
-def test_hub_rows_take_launched_passes(ctx, side, hubs, deg, scattered, launched):
+# cooperative launch's: 15 or 43) by itself, so more than 16,384 entries there (rows up to
+# 1,024: four times as many for k = 3, 0.57 times for k = 200), or 98,304 in all rows above
+# 1,024, take launched passes (but for levels of 4,096 vertices and 65,536 entries)
+@pytest.mark.parametrize("side,hubs,deg,scattered,k,launched", [
+    (140, 0, 0, False, 3, False), (140, 1, 16000, False, 3, False), (140, 4, 4000, False, 3, False),
+    (140, 1, 18000, False, 3, True), (140, 5, 4000, False, 3, True), (140, 5, 4000, True, 3, False),
+    (140, 39, 1000, False, 3, False), (140, 20, 1000, False, 20, False), (140, 21, 1000, False, 40, True),
+    (140, 12, 1000, False, 200, True), (140, 9, 900, False, 200, False), (63, 12, 1900, False, 3, False),
+    (140, 23, 4200, True, 3, False), (140, 24, 4200, True, 3, True), (264, 30, 4000, True, 3, True),
+    (264, 17, 950, False, 3, False), (450, 20, 1000, False, 3, False), (450, 20, 1000, False, 50, True)])
+def test_hub_rows_take_launched_passes(ctx, side, hubs, deg, scattered, k, launched):
     g = hub_grid(side, hubs, deg, side + hubs, scattered)
     opt = default_options(coarsen_to=g.nvtxs, init_starts=2, fm_passes=1)
-    part, cut = ctx.partition_graph(g, 3, 1.05, options=opt)
+    part, cut = ctx.partition_graph(g, k, 1.05, options=opt)
     n = ctx.stats().kernel_launches
     ctx.set_tuning(small_level_n=0)
     try:
-        lpart, lcut = ctx.partition_graph(g, 3, 1.05, options=opt)
+        lpart, lcut = ctx.partition_graph(g, k, 1.05, options=opt)
         m = ctx.stats().kernel_launches
     finally:
         ctx.set_tuning(None)
